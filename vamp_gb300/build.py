@@ -52,25 +52,16 @@ def sources() -> list[Path]:
 
 def _defines() -> list[str]:
     # VG_MIN_BLOCKS: resident 128-thread blocks per SM the kernels are compiled for.
-    # VG_FORM_COMPACT=1: pass frames to the fine checks in registers instead of staging them in
-    # shared memory; VG_SELF_UNROLLED=1: one block of code per self-collision link pair instead
-    # of a loop over a table; VG_STAGED_ALL=1: the staged form for the robots whose default is the
-    # table-driven form (all schedule forms give identical results).
+    # VG_STAGED_ALL=1: the staged form for the robots whose default is the table-driven form
+    # (both forms give identical results).
     out = []
     mb = os.environ.get("VG_MIN_BLOCKS")
     if mb:
         out.append(f"-DVG_MIN_BLOCKS={int(mb)}")
-    if os.environ.get("VG_FORM_COMPACT") == "1":
-        out.append("-DVG_FORM_COMPACT")
-    if os.environ.get("VG_SELF_UNROLLED") == "1":
-        out.append("-DVG_SELF_UNROLLED")
     if os.environ.get("VG_STAGED_ALL") == "1":
         out.append("-DVG_STAGED_ALL")
     # VG_CAPT_SHARED_WEIGHT=w: the pointcloud query scans one lane's list with the whole warp
     # when 4 x the longest list exceeds w x the warp's shared steps
-    # VG_DEFAULT_LOOPED_ENV=1: the default edge kernel runs the environment section as loops
-    if os.environ.get("VG_DEFAULT_LOOPED_ENV") == "1":
-        out.append("-DVG_DEFAULT_LOOPED_ENV=1")
     w = os.environ.get("VG_CAPT_SHARED_WEIGHT")
     if w:
         out.append(f"-DVG_CAPT_SHARED_WEIGHT={int(w)}")

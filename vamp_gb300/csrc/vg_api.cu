@@ -166,6 +166,23 @@ namespace vg
 
     static_assert(sizeof(CaptView) % sizeof(float4) == 0, "CaptView must pack into float4s");
 
+    // A device copy of a pointcloud's points for the clearance field.  Without memory for it the
+    // field reads the tree's blocks instead (CloudPoints::n = 0).
+    static CloudPoints keep_points(const float *xyz, size_t n, cudaMemcpyKind kind, cudaStream_t s)
+    {
+        CloudPoints p;
+        const size_t bytes = 3 * n * sizeof(float);
+        if (n && cudaMalloc(&p.d, bytes) == cudaSuccess && cudaMemcpyAsync(p.d, xyz, bytes, kind, s) == cudaSuccess)
+        {
+            p.n = n;
+        }
+        else
+        {
+            cudaGetLastError();
+        }
+        return p;
+    }
+
     // Uploads each pointcloud's tree once: kCloudBuffers device buffers per cloud (tests, aabbs,
     // starts, the reference-layout blocks, the ring-ordered blocks the queries scan, and the
     // query tables).  A host-built cloud's reference-layout blocks are freed once ordered (the
@@ -215,6 +232,7 @@ namespace vg
             e->d_clouds.push_back(q.aff_q);
             e->d_clouds.push_back(q.tables);
             e->capt_q.push_back(q);
+            e->d_points.push_back(keep_points(c.points.data(), c.points.size() / 3, cudaMemcpyHostToDevice, 0));
         }
         return VG_OK;
     }
@@ -307,6 +325,8 @@ namespace vg
             VG_CUDA(cudaMalloc(&e->d_counter, 64), "cudaMalloc(counter)");
         }
         e->image_f4 = img.size();
+        e->field_ready.store(false);
+        e->field_states = 0.0;
         e->device = dev;
         e->dirty = false;
         ++e->version;
@@ -330,6 +350,7 @@ namespace vg
         d.att_off = e->att_off;
         d.n_hf = static_cast<int>(e->hf.size());
         d.hf_off = e->hf_off;
+        d.field = e->field_ready.load(std::memory_order_acquire) ? e->d_field : nullptr;
         return d;
     }
 
@@ -723,6 +744,13 @@ void vg_env_destroy(vg_env *env)
         cudaFree(env->d_stage);
     if (env->d_order)
         cudaFree(env->d_order);
+    if (env->d_field)
+        cudaFree(env->d_field);
+    for (const CloudPoints &p : env->d_points)
+    {
+        if (p.d)
+            cudaFree(p.d);
+    }
     if (env->h_pin)
         cudaFreeHost(env->h_pin);
     for (void *p : env->d_clouds)
@@ -832,6 +860,7 @@ int vg_env_add_pointcloud(vg_env *env, const float *xyz, size_t n, float r_min, 
     {
         CaptHost c;
         capt_build(xyz, n, r_min, r_max, r_point, c);
+        c.points.assign(xyz, xyz + 3 * n);
         env->clouds.push_back(std::move(c));
     }
     catch (...)
@@ -869,6 +898,7 @@ int vg_env_add_pointcloud_device(vg_env *env, const float *xyz, size_t n, float 
         d.release();
         return rc;
     }
+    env->d_points.push_back(keep_points(xyz, n, cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream)));
     CaptHost c;
     c.nlog2 = d.nlog2;
     std::memcpy(c.top, d.top, sizeof(c.top));
@@ -984,6 +1014,7 @@ int vg_validate_states_device(const char *robot, vg_env *env, const float *q, si
     int occ = 0;
     if (int rc = prepare_kernel(ext ? r->states_ext_fn : r->states_fn, smem, kBlock, &occ))
         return rc;
+    want_field(env, static_cast<double>(n), static_cast<cudaStream_t>(stream));
     const long long want = (static_cast<long long>(n) + kBlock - 1) / kBlock;
     const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));
     StatesParams p{q, static_cast<long long>(n), out, env_device(env)};
@@ -1114,6 +1145,7 @@ int vg_validate_motions_device(
         return VG_OK;
     if (int rc = commit(env))
         return rc;
+    want_field(env, kEdgeStates * static_cast<double>(n), static_cast<cudaStream_t>(stream));
     MotionLaunch m{r, env, a, b, n, resolution, nullptr, 0, out, blocks, env->d_counter};
     tuned_for(env, r, &m.schedule, &m.blocks_per_sm);
     return launch_motions(m, static_cast<cudaStream_t>(stream));
@@ -1144,6 +1176,7 @@ int vg_validate_vectors_device(
         return VG_OK;
     if (int rc = commit(env))
         return rc;
+    want_field(env, kEdgeStates * static_cast<double>(n), static_cast<cudaStream_t>(stream));
     MotionLaunch m{r, env, start, vector, n, resolution, nullptr, 0, out, blocks, env->d_counter};
     m.dist = distance;
     tuned_for(env, r, &m.schedule, &m.blocks_per_sm);
@@ -1187,6 +1220,7 @@ int vg_validate_motions_scored_device(
         VG_CUDA(cudaMalloc(&env->d_order, n * 16), "cudaMalloc(group orders)");
         env->order_cap = n * 16;
     }
+    want_field(env, kEdgeStates * static_cast<double>(n), static_cast<cudaStream_t>(stream));
     MotionLaunch m{r, env, a, b, n, resolution, scores, probes, out, blocks, env->d_counter};
     m.order = env->d_order;
     int schedule = 1;
@@ -1282,6 +1316,7 @@ int vg_fkcc_blocks_device(const char *robot, vg_env *env, const float *q, size_t
     int occ = 0;
     if (int rc = prepare_kernel(ext ? r->blocks_ext_fn[which] : r->blocks_fn[which], smem, kBlock, &occ))
         return rc;
+    want_field(env, static_cast<double>(n_blocks) * env->lanes, static_cast<cudaStream_t>(stream));
     const long long per_block = (kBlock / 32) * (32 / env->lanes);  // configuration blocks per thread block
     const long long want = (static_cast<long long>(n_blocks) + per_block - 1) / per_block;
     const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));

@@ -59,7 +59,7 @@ namespace
     int record(vg_batch *bt, cudaStream_t s);
 
     // every allocation and upload a launch needs, done outside any capture
-    int prepare(vg_batch *bt)
+    int prepare(vg_batch *bt, cudaStream_t s)
     {
         int dev = 0;
         VG_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
@@ -71,6 +71,8 @@ namespace
             if (int rc = commit(p.env))
                 return rc;
         }
+        for (auto &p : bt->parts)
+            want_field(p.env, kEdgeStates * static_cast<double>(p.n), s);
         const size_t need = bt->parts.size() * 16;
         if (need > bt->counters_cap)
         {
@@ -199,7 +201,7 @@ int vg_batch_launch(vg_batch *b, void *stream)
         drop_graph(b);  // an environment changed since the capture: upload it and capture again
     if (b->stale)
     {
-        if (int rc = prepare(b))
+        if (int rc = prepare(b, s))
             return rc;
         // the capture records the launches without running them
         VG_CUDA(cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
@@ -238,6 +240,7 @@ int vg_autotune_motions(const char *robot, vg_env *env, const float *a, const fl
     if (int rc = commit(env))
         return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    want_field(env, kEdgeStates * static_cast<double>(n), s);
     uint8_t *out = nullptr;
     VG_CUDA(cudaMalloc(&out, n), "cudaMalloc(autotune)");
     cudaEvent_t e0, e1;

@@ -18,6 +18,7 @@ namespace vg
         std::vector<float> aabbs;           // 2^nlog2 leaves x 6: lower xyz, upper xyz
         std::vector<uint32_t> aff_starts;   // 2^nlog2 + 1, in 8-point blocks
         std::vector<float> aff;             // blocks x 24: x[8], y[8], z[8]
+        std::vector<float> points;          // the input points x y z (host-built trees)
         float top[6] = {0, 0, 0, 0, 0, 0};  // box of all finite points
         float r_min = 0, r_max = 0, r_point = 0;
         // built on the GPU: the arrays exist only in device memory (sizes below)

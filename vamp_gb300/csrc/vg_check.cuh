@@ -17,6 +17,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 namespace vg
 {
@@ -216,7 +217,62 @@ namespace vg
         int n_att;          // -1: none
         const HeightView *hf;
         int n_hf;
+        const uint8_t *field;  // clearance field (below); null: not built
     };
+
+    // ------------------------------------------------------------------- clearance field
+    //
+    // A grid over the robots' workspace, one byte per cell: a lower bound of the distance from any
+    // point of the cell to anything in the environment, in steps of 1 / kFieldSteps m (0: none
+    // known; 255: that far or farther), with a margin that covers the FP32 rounding of every
+    // exact test (vg_field.cu).  A sphere whose radius is below the bound of its centre's cell
+    // cannot give a negative test value, so its exact query is skipped: the answer is the same.
+    // What bounded the edge check before it was the exact coarse queries (57 % of a warp's time;
+    // 97 % of the coarse spheres are out of every object's reach).
+    //
+    // 128 cells of 2.5 cm per axis: 2 MB, which the L2 holds, and cells small enough that 0.6 of
+    // the Panda's 11 coarse spheres per warp iteration keep their exact query (5 cm cells: 1.0).
+    constexpr int kFieldBits = 7;
+    constexpr int kFieldCells = 1 << kFieldBits;
+    constexpr float kFieldInv = 40.0f;         // cells per metre
+    constexpr float kFieldX = 64.0f;           // cell index of x = 0 and y = 0
+    constexpr float kFieldZ = 40.0f;           // cell index of z = 0
+    constexpr float kFieldSteps = 400.0f;
+    constexpr float kFieldMagic = 8388608.0f;  // 2^23: floats from here on hold integers exactly
+    constexpr unsigned kFieldMagicBits = 0x4b000000u;
+
+    // The field's value at a point: that of the cell whose centre is nearest, 0 outside the grid
+    // (and for NaN).  fma(x, 40, 2^23 + 64) is the cell index rounded to an integer, in the low
+    // mantissa bits; any bit above the index means outside.
+    __device__ __forceinline__ unsigned field_value(const uint8_t *field, float x, float y, float z)
+    {
+        const unsigned ux = __float_as_uint(__fmaf_rn(x, kFieldInv, kFieldMagic + kFieldX)) ^ kFieldMagicBits;
+        const unsigned uy = __float_as_uint(__fmaf_rn(y, kFieldInv, kFieldMagic + kFieldX)) ^ kFieldMagicBits;
+        const unsigned uz = __float_as_uint(__fmaf_rn(z, kFieldInv, kFieldMagic + kFieldZ)) ^ kFieldMagicBits;
+        unsigned v = 0u;
+        if ((ux | uy | uz) < static_cast<unsigned>(kFieldCells))
+        {
+            v = __ldg(field + ((uz << (2 * kFieldBits)) + (uy << kFieldBits) + ux));
+        }
+        return v;
+    }
+
+    // The smallest field value that rules a sphere of radius r out (256: none does).
+    __host__ __device__ constexpr unsigned field_reach(float r)
+    {
+        const float a = (r < 0.0f ? -r : r) * kFieldSteps;
+        return a < 255.0f ? static_cast<unsigned>(a) + 1u : 256u;  // NaN: 256
+    }
+
+    __device__ __forceinline__ int lowest_bit(unsigned m)
+    {
+        return __ffs(static_cast<int>(m)) - 1;
+    }
+
+    __device__ __forceinline__ int lowest_bit(unsigned long long m)
+    {
+        return __ffsll(static_cast<long long>(m)) - 1;
+    }
 
     // sphere_heightfield (collision/sphere_heightfield.hh:9-30), sign bit set iff the sphere is
     // below the surface: the cell floor(clamp(xs * (x0 - x) + xd / 2, 0, xd)) (one fused
@@ -545,16 +601,15 @@ namespace vg
         return __ballot_sync(kFull, hit);
     }
 
-    // sphere_environment_in_collision (validity.hh:47-150) for NS spheres at once, each over the
-    // segments in `mask`.  hit[s] receives the lanes of the segments whose block collides for
+    // sphere_environment_in_collision (validity.hh:47-150) for NS spheres at once, sphere s over
+    // the segments in mask[s].  hit[s] receives the lanes of the segments whose block collides for
     // sphere s.  Warp-uniform; all 32 lanes must call.
     // kExt: also the heightfields (kernels built for environments with heightfields or an
     // attachment; the default kernels leave them out)
     template <int W, int NS, bool kExt = false>
-    __device__ __forceinline__ void env_multi(const EnvView &e, const float4 *sph, unsigned mask, unsigned *hit)
+    __device__ __forceinline__ void env_multi(const EnvView &e, const float4 *sph, const unsigned *mask, unsigned *hit)
     {
         const int lane = threadIdx.x & 31;
-        const bool on = (mask >> lane) & 1u;
         float x[NS], y[NS], z[NS], r[NS], rsq[NS], M[NS], Mw[NS];
         unsigned bits[NS];
         float Mall = -__int_as_float(0x7f800000);
@@ -562,6 +617,7 @@ namespace vg
         for (int s = 0; s < NS; ++s)
         {
             const float4 c = sph[s];
+            const bool on = (mask[s] >> lane) & 1u;
             x[s] = c.x;
             y[s] = c.y;
             z[s] = c.z;
@@ -596,7 +652,7 @@ namespace vg
 #pragma unroll
         for (int s = 0; s < NS; ++s)
         {
-            hit[s] = seg_any<W>(__ballot_sync(kFull, bits[s] >> 31)) & mask;
+            hit[s] = seg_any<W>(__ballot_sync(kFull, bits[s] >> 31)) & mask[s];
         }
         // pointclouds, for the blocks the primitives did not already put in collision
 #pragma unroll 1
@@ -605,10 +661,10 @@ namespace vg
 #pragma unroll
             for (int s = 0; s < NS; ++s)
             {
-                const bool ask = on && !((hit[s] >> lane) & 1u);
-                if (__any_sync(kFull, ask))
+                const bool ask = ((mask[s] & ~hit[s]) >> lane) & 1u;
+                if (mask[s] & ~hit[s])
                 {
-                    hit[s] |= seg_any<W>(capt_warp(e.clouds[c], x[s], y[s], z[s], r[s], ask)) & mask;
+                    hit[s] |= seg_any<W>(capt_warp(e.clouds[c], x[s], y[s], z[s], r[s], ask)) & mask[s];
                 }
             }
         }
@@ -643,34 +699,8 @@ namespace vg
     {
         const float4 s = make_float4(x, y, z, r);
         unsigned hit;
-        env_multi<W, 1, kExt>(e, &s, mask, &hit);
+        env_multi<W, 1, kExt>(e, &s, &mask, &hit);
         return hit;
-    }
-
-    // Single-sphere form.
-    template <int W, bool kExt = false>
-    __device__ __noinline__ unsigned env_query(const EnvView &e, float x, float y, float z, float r, unsigned mask)
-    {
-        const float4 s = make_float4(x, y, z, r);
-        unsigned hit;
-        env_multi<W, 1, kExt>(e, &s, mask, &hit);
-        return hit;
-    }
-
-    // Fine tests of one link's NS spheres (one function per distinct NS): the segments in `mask`
-    // whose block collides for any of the spheres.
-    template <int W, int NS, bool kExt = false>
-    __device__ __noinline__ unsigned env_any(const EnvView &e, const float4 *sph, unsigned mask)
-    {
-        unsigned hit[NS];
-        env_multi<W, NS, kExt>(e, sph, mask, hit);
-        unsigned any = 0;
-#pragma unroll
-        for (int s = 0; s < NS; ++s)
-        {
-            any |= hit[s];
-        }
-        return any;
     }
 
     // sphere_sphere_self_collision (validity.hh:23-44) for the segments in `mask`.
@@ -722,15 +752,54 @@ namespace vg
         }
 
         template <int NS>
-        __device__ __forceinline__ void env_many(const float4 *s, unsigned mask, unsigned *hit)
+        __device__ __forceinline__ void env_many(const float4 *s, const unsigned *mask, unsigned *hit)
         {
             env_multi<W, NS, kExt>(env, s, mask, hit);
         }
 
-        template <int NS>
-        __device__ __forceinline__ unsigned env_any_hit(const float4 *s, unsigned mask)
+        // the field's value at a point (0, which rules nothing out, without a field)
+        __device__ __forceinline__ unsigned clearance(float x, float y, float z)
         {
-            return env_any<W, NS, kExt>(env, s, mask);
+            return env.field ? field_value(env.field, x, y, z) : 0u;
+        }
+
+        // the segments of `mask` in which any lane's sphere may touch something
+        __device__ __forceinline__ unsigned vote_near(bool may, unsigned mask)
+        {
+            return seg_any<W>(__ballot_sync(kFull, may) & mask);
+        }
+
+        __device__ __forceinline__ unsigned near(const float4 s, unsigned mask)
+        {
+            return vote_near(clearance(s.x, s.y, s.z) < field_reach(s.w), mask);
+        }
+
+        // vote_near of N spheres over the segments alive, sphere k's into masks[k]; a bit per
+        // sphere with any such segment.  The N lookups are independent loads in flight together.
+        template <int N>
+        __device__ __forceinline__ auto near_all(const float4 (&s)[N], unsigned *masks)
+        {
+            static_assert(N <= 64, "one bit per sphere");
+            using Bits = std::conditional_t<(N > 32), unsigned long long, unsigned>;
+            unsigned v[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+            {
+                v[k] = clearance(s[k].x, s[k].y, s[k].z);
+            }
+            Bits any = 0;
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+            {
+                const unsigned m = vote_near(v[k] < field_reach(s[k].w), alive);
+                any |= m ? Bits(1) << k : Bits(0);
+                if ((threadIdx.x & 31) == 0)
+                {
+                    masks[k] = m;  // warp-uniform
+                }
+            }
+            __syncwarp();
+            return any;
         }
 
         __device__ __forceinline__ unsigned self_hit(
@@ -761,64 +830,4 @@ namespace vg
             return seg_any<W>(__ballot_sync(kFull, bits >> 31)) & mask;
         }
     };
-
-    // Fine environment tests of one link's spheres, in order, for the segments in `need`.
-    // Clears colliding segments from ctx.alive; returns true once none is left.
-    template <int N, typename Ctx>
-    __device__ __forceinline__ bool env_fine(Ctx &ctx, const float4 *s, unsigned need)
-    {
-#pragma unroll 1
-        for (int k = 0; k < N; ++k)
-        {
-            const float4 c = s[k];
-            const unsigned hit = ctx.env_hit(c.x, c.y, c.z, c.w, need);
-            if (hit)
-            {
-                need &= ~hit;
-                if (!ctx.kill(hit))
-                {
-                    return true;
-                }
-                need &= ctx.alive;
-                if (!need)
-                {
-                    return false;
-                }
-            }
-        }
-        return false;
-    }
-
-    // Fine self-collision tests of one link pair: every sphere of link A against every sphere
-    // of link B (the reference's generated pair list is this cross product), for the segments
-    // in `need`.  Clears colliding segments from ctx.alive; returns true once none is left.
-    template <int NA, int NB, typename Ctx>
-    __device__ __forceinline__ bool self_cross(Ctx &ctx, const float4 *sa, const float4 *sb, unsigned need)
-    {
-#pragma unroll 1
-        for (int i = 0; i < NA; ++i)
-        {
-            const float4 a = sa[i];
-#pragma unroll 1
-            for (int j = 0; j < NB; ++j)
-            {
-                const float4 b = sb[j];
-                const unsigned hit = ctx.self_hit(a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, need);
-                if (hit)
-                {
-                    need &= ~hit;
-                    if (!ctx.kill(hit))
-                    {
-                        return true;
-                    }
-                    need &= ctx.alive;
-                    if (!need)
-                    {
-                        return false;
-                    }
-                }
-            }
-        }
-        return false;
-    }
 }  // namespace vg

@@ -3,7 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -97,6 +99,14 @@ namespace vg
                             // 3: as 2 with free segments starting on the next edge
         int blocks_per_sm;  // resident blocks per SM (0: as many as fit)
     };
+
+    // The input points of a pointcloud on the device, for the clearance field (n = 0: the tree was
+    // given as a layout; its blocks hold the points).
+    struct CloudPoints
+    {
+        float *d = nullptr;
+        size_t n = 0;
+    };
 }  // namespace vg
 
 // The C-ABI environment handle.
@@ -135,6 +145,13 @@ struct vg_env
     std::vector<vg::CaptHost> clouds;
     std::vector<void *> d_clouds;        // kCloudBuffers buffers per uploaded cloud
     std::vector<vg::CaptQuery> capt_q;   // per uploaded cloud (pointers into d_clouds)
+    std::vector<vg::CloudPoints> d_points;  // per uploaded cloud
+    // clearance field (vg_field.cu): built by want_field once the states checked since the last
+    // upload make it worth while, dropped by the next upload
+    uint8_t *d_field = nullptr;
+    std::atomic<bool> field_ready{false};
+    double field_states = 0.0;
+    std::mutex field_mu;
     // learned-order group orders (vg_validate_motions_scored_device), 16 bytes per edge
     uint8_t *d_order = nullptr;
     size_t order_cap = 0;
@@ -176,6 +193,14 @@ namespace vg
 
     int commit(vg_env *e);
     EnvDevice env_device(const vg_env *e);
+    // States checked in an environment since its last change from which its clearance field is
+    // built (about 0.1 ms, allocations and the synchronisation included).
+    constexpr double kFieldStates = 131072.0;
+    // states an edge is taken to hold where its length is not known on the host
+    constexpr double kEdgeStates = 64.0;
+    // Counts `states` about to be checked on stream s in a committed environment and builds its
+    // clearance field when due.  Failure to build leaves the environment without one.
+    void want_field(vg_env *e, double states, cudaStream_t s);
     int sm_count();
     int prepare_kernel(const void *fn, int smem, int block, int *blocks_per_sm);
     void tuned_for(const vg_env *env, const RobotOps *r, int *schedule, int *blocks_per_sm);

@@ -23,12 +23,6 @@
 #ifndef VG_MIN_BLOCKS_WIDE
 #define VG_MIN_BLOCKS_WIDE 3
 #endif
-// Environment section form of the default same-edge kernel: 0 unrolled, 1 loops (the
-// register-rich variant and the states kernel always use loops).
-#ifndef VG_DEFAULT_LOOPED_ENV
-#define VG_DEFAULT_LOOPED_ENV 0
-#endif
-
 namespace vg
 {
     // Device image of an environment: the x86 RSQRTPS table followed by the primitive records
@@ -46,6 +40,7 @@ namespace vg
         int att_off;        // attachment block: 3 transform rows, then the spheres, in float4
         int n_hf;           // HeightView descriptors
         int hf_off;         // their offset, in float4
+        const uint8_t *field;  // clearance field (null: not built)
     };
 
     constexpr int kRsqrtF4 = 2048 / 4;
@@ -75,6 +70,7 @@ namespace vg
         v.n_att = d.n_att;
         v.hf = reinterpret_cast<const HeightView *>(smem + d.hf_off - kRsqrtF4);
         v.n_hf = d.n_hf;
+        v.field = d.field;
         for (int k = 0; k < 5; ++k)
         {
             v.rec[k] = smem + d.off[k] - kRsqrtF4;
@@ -157,18 +153,17 @@ namespace vg
         return ctx.alive;
     }
 
-    // kLoopedEnv: the robot's environment section as loops (smaller code) instead of unrolled;
     // kExt: the extended checks, for environments with heightfields or an attachment: every
     // environment query also tests the heightfields, and with an attachment the block runs
     // Robot::fkcc_attach
     // kOrdered: the segments are consecutive blocks of one edge (CheckCtx)
-    template <typename Robot, int W, bool kLoopedEnv = false, bool kExt = false, bool kOrdered = false>
+    template <typename Robot, int W, bool kExt = false, bool kOrdered = false>
     __device__ __forceinline__ unsigned run_fkcc(const EnvView &ev, const float *q, unsigned alive, float *stage)
     {
         static_assert(Robot::kEnvChecks <= kWarpScratch, "per-warp scratch holds one word per environment check");
         __shared__ unsigned warp_scratch[kStageStride / 32][kWarpScratch];
         CheckCtx<W, kExt, kOrdered> ctx{ev, alive, false, stage, warp_scratch[threadIdx.x >> 5]};
-        Robot::template fkcc<CheckCtx<W, kExt, kOrdered>, kLoopedEnv>(q, ctx);
+        Robot::fkcc(q, ctx);
         if constexpr (kExt)
         {
             if (ctx.alive && ev.n_att >= 0)
@@ -208,7 +203,7 @@ namespace vg
             {
                 q[d] = in ? p.q[idx * D + d] : 0.0f;
             }
-            const unsigned alive = run_fkcc<Robot, 1, true, kExt>(ev, q, __ballot_sync(kFull, in), stage);
+            const unsigned alive = run_fkcc<Robot, 1, kExt>(ev, q, __ballot_sync(kFull, in), stage);
             if (in)
             {
                 p.out[idx] = static_cast<uint8_t>((alive >> (threadIdx.x & 31)) & 1u);
@@ -243,7 +238,7 @@ namespace vg
             {
                 q[d] = in ? p.q[(blk * W + lane % W) * D + d] : 0.0f;
             }
-            const unsigned alive = run_fkcc<Robot, W, true, kExt>(ev, q, __ballot_sync(kFull, in), stage);
+            const unsigned alive = run_fkcc<Robot, W, kExt>(ev, q, __ballot_sync(kFull, in), stage);
             if (in && lane % W == 0)
             {
                 p.out[blk] = static_cast<uint8_t>((alive >> lane) & 1u);
@@ -486,7 +481,7 @@ namespace vg
             {
                 break;
             }
-            const unsigned alive = run_fkcc<Robot, W, false, kExt>(ev, q, active, stage);
+            const unsigned alive = run_fkcc<Robot, W, kExt>(ev, q, active, stage);
             bool finish = false;
             if (e >= 0)
             {
@@ -528,7 +523,7 @@ namespace vg
     // (block i = block 0 minus v / (W n), i times).  The edge is invalid if any checked block is,
     // and the reference would have stopped at the first invalid block, so the block count
     // reported is that block's index + 1.
-    template <typename Robot, int W, bool kLearned, int kMinBlocks = VG_MIN_BLOCKS, bool kLoopedEnv = VG_DEFAULT_LOOPED_ENV != 0>
+    template <typename Robot, int W, bool kLearned, int kMinBlocks = VG_MIN_BLOCKS>
     __global__ void __launch_bounds__(128, kMinBlocks) edges_grouped_kernel(EdgesParams p)
     {
         extern __shared__ float4 smem[];
@@ -620,7 +615,7 @@ namespace vg
                         }
                     }
                     const unsigned mask = __ballot_sync(kFull, active);
-                    const unsigned alive = run_fkcc<Robot, W, kLoopedEnv, false, true>(ev, q, mask, stage);
+                    const unsigned alive = run_fkcc<Robot, W, false, true>(ev, q, mask, stage);
                     const unsigned dead = mask & ~alive;
                     // one bit per active segment (its first lane)
                     const unsigned leaders = mask & kSegLeaders;
@@ -649,7 +644,7 @@ namespace vg
                 {
                     const bool active = i0 + seg < n;
                     const unsigned mask = __ballot_sync(kFull, active);
-                    const unsigned alive = run_fkcc<Robot, W, kLoopedEnv, false, true>(ev, q, mask, stage);
+                    const unsigned alive = run_fkcc<Robot, W, false, true>(ev, q, mask, stage);
                     const unsigned dead = mask & ~alive;
                     if (dead)
                     {
@@ -689,7 +684,7 @@ namespace vg
     // the last segment (same lane of the segment) and subtracts bs seg + 1 more times.  Every
     // block is therefore still block 0 minus bs repeated i times, as the reference computes it
     // (planning/validate.hh:50-56), and verdicts and block counts equal edges_grouped_kernel's.
-    template <typename Robot, int W, int kMinBlocks = VG_MIN_BLOCKS, bool kLoopedEnv = VG_DEFAULT_LOOPED_ENV != 0>
+    template <typename Robot, int W, int kMinBlocks = VG_MIN_BLOCKS>
     __global__ void __launch_bounds__(128, kMinBlocks) edges_packed_kernel(EdgesParams p)
     {
         static_assert(W == 8 || W == 4, "packed schedule: 4 or 8 segments per warp");
@@ -803,7 +798,7 @@ namespace vg
             {
                 break;  // nothing carried and the queue is empty
             }
-            const unsigned alive = run_fkcc<Robot, W, kLoopedEnv>(ev, q, mask, stage);
+            const unsigned alive = run_fkcc<Robot, W>(ev, q, mask, stage);
             const unsigned dead = mask & ~alive;
             const unsigned cmask = r >= S ? kFull : ((1u << (r * W)) - 1u);  // the carried edge's lanes
             if (ce >= 0)

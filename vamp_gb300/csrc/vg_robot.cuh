@@ -38,10 +38,10 @@ namespace vg
         return cudaGetLastError();
     }
 
-    template <typename R, int W, bool kLearned, int kMinBlocks = VG_MIN_BLOCKS, bool kLoopedEnv = VG_DEFAULT_LOOPED_ENV != 0>
+    template <typename R, int W, bool kLearned, int kMinBlocks = VG_MIN_BLOCKS>
     cudaError_t launch_edges_grouped(const EdgesParams &p, int grid, int block, int smem, cudaStream_t s)
     {
-        edges_grouped_kernel<R, W, kLearned, kMinBlocks, kLoopedEnv><<<grid, block, smem, s>>>(p);
+        edges_grouped_kernel<R, W, kLearned, kMinBlocks><<<grid, block, smem, s>>>(p);
         return cudaGetLastError();
     }
 
@@ -52,10 +52,10 @@ namespace vg
         return cudaGetLastError();
     }
 
-    template <typename R, int W, int kMinBlocks, bool kLoopedEnv>
+    template <typename R, int W, int kMinBlocks>
     cudaError_t launch_edges_packed(const EdgesParams &p, int grid, int block, int smem, cudaStream_t s)
     {
-        edges_packed_kernel<R, W, kMinBlocks, kLoopedEnv><<<grid, block, smem, s>>>(p);
+        edges_packed_kernel<R, W, kMinBlocks><<<grid, block, smem, s>>>(p);
         return cudaGetLastError();
     }
 
@@ -115,21 +115,21 @@ namespace vg
         o.edges_grouped[1] = &launch_edges_grouped<R, 4, false>;
         o.edges_grouped_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, false>);
         o.edges_grouped_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, false>);
-        o.edges_wide[0] = &launch_edges_grouped<R, 8, false, VG_MIN_BLOCKS_WIDE, true>;
-        o.edges_wide[1] = &launch_edges_grouped<R, 4, false, VG_MIN_BLOCKS_WIDE, true>;
-        o.edges_wide_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, false, VG_MIN_BLOCKS_WIDE, true>);
-        o.edges_wide_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, false, VG_MIN_BLOCKS_WIDE, true>);
-        o.edges_packed[0] = &launch_edges_packed<R, 8, VG_MIN_BLOCKS_WIDE, true>;
-        o.edges_packed[1] = &launch_edges_packed<R, 4, VG_MIN_BLOCKS_WIDE, true>;
-        o.edges_packed_fn[0] = reinterpret_cast<const void *>(&edges_packed_kernel<R, 8, VG_MIN_BLOCKS_WIDE, true>);
-        o.edges_packed_fn[1] = reinterpret_cast<const void *>(&edges_packed_kernel<R, 4, VG_MIN_BLOCKS_WIDE, true>);
+        o.edges_wide[0] = &launch_edges_grouped<R, 8, false, VG_MIN_BLOCKS_WIDE>;
+        o.edges_wide[1] = &launch_edges_grouped<R, 4, false, VG_MIN_BLOCKS_WIDE>;
+        o.edges_wide_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, false, VG_MIN_BLOCKS_WIDE>);
+        o.edges_wide_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, false, VG_MIN_BLOCKS_WIDE>);
+        o.edges_packed[0] = &launch_edges_packed<R, 8, VG_MIN_BLOCKS_WIDE>;
+        o.edges_packed[1] = &launch_edges_packed<R, 4, VG_MIN_BLOCKS_WIDE>;
+        o.edges_packed_fn[0] = reinterpret_cast<const void *>(&edges_packed_kernel<R, 8, VG_MIN_BLOCKS_WIDE>);
+        o.edges_packed_fn[1] = reinterpret_cast<const void *>(&edges_packed_kernel<R, 4, VG_MIN_BLOCKS_WIDE>);
         // the learned order in the form of the fastest plain schedule for the Panda, UR5 and Fetch
-        // (register-rich build, looped environment section); the group order comes precomputed
+        // (register-rich build); the group order comes precomputed
         // (edge_order_kernel), which keeps it within the registers of 4 resident blocks
-        o.edges_learned[0] = &launch_edges_grouped<R, 8, true, VG_MIN_BLOCKS_WIDE, true>;
-        o.edges_learned[1] = &launch_edges_grouped<R, 4, true, VG_MIN_BLOCKS_WIDE, true>;
-        o.edges_learned_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, true, VG_MIN_BLOCKS_WIDE, true>);
-        o.edges_learned_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, true, VG_MIN_BLOCKS_WIDE, true>);
+        o.edges_learned[0] = &launch_edges_grouped<R, 8, true, VG_MIN_BLOCKS_WIDE>;
+        o.edges_learned[1] = &launch_edges_grouped<R, 4, true, VG_MIN_BLOCKS_WIDE>;
+        o.edges_learned_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, true, VG_MIN_BLOCKS_WIDE>);
+        o.edges_learned_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, true, VG_MIN_BLOCKS_WIDE>);
         o.edge_order[0] = &launch_edge_order<R, 8>;
         o.edge_order[1] = &launch_edge_order<R, 4>;
         // extended checks (heightfields, fkcc_attach): the segment-per-edge and states kernels

@@ -404,10 +404,10 @@ TABLED = {"ur5", "fetch", "baxter"}
 # 1.570796325 leave ~1e-9 residues that only cost operations (their effect is below 1e-8 m)
 SNAP32 = 1e-7
 # Coarse spheres queried together (one pass over the objects, up to the largest bound among
-# them): four in the unrolled environment section (one inlined copy per batch), two in the looped
-# one (one copy in all), the fastest of 1-11 measured on the Panda's 65,536-edge workload.
-COARSE_BATCH = int(os.environ.get("VG_COARSE_BATCH", "4"))
-LOOPED_BATCH = int(os.environ.get("VG_LOOPED_BATCH", "2"))
+# them): two, the fastest of 1-11 measured on the Panda's 65,536-edge workload.
+COARSE_BATCH = 2
+# Coarse spheres of the table-driven form whose field lookups are in flight together
+TABLE_NEAR = 4
 
 
 def f32_down(v: float) -> float:
@@ -717,14 +717,14 @@ def gen_cuda(model: dict) -> str:
     w("    static __device__ __forceinline__ int2 self_pair(int i) { return k%sAllPair[i]; }" % S)
     lay = stage_layout(model, kin, load_cull(name))
     w("    // floats of shared-memory staging per thread (non-constant entries of the fine checks' frames)")
-    w("#if defined(VG_FORM_COMPACT)%s" % (" || !defined(VG_STAGED_ALL)" if tabled else ""))
-    w("    static constexpr int kStage = 0;")
-    w("#elif defined(VG_SELF_UNROLLED)")
-    w("    static constexpr int kStage = %d;" % lay["n_frame"])
-    w("#else")
-    w("    // the coarse centres the self-check loop reads and the joint values its danger boxes test")
+    if tabled:
+        w("#ifndef VG_STAGED_ALL")
+        w("    static constexpr int kStage = 0;")
+        w("#else")
+    w("    // and the coarse centres the self-check loop reads and the joint values its danger boxes test")
     w("    static constexpr int kStage = %d;" % lay["total"])
-    w("#endif")
+    if tabled:
+        w("#endif")
     w("    static constexpr int kResolution = %d;" % model["resolution"])
     w("    static constexpr float kMinRadius = %s;" % lit32(model["min_radius"]))
     w("    static constexpr float kMaxRadius = %s;" % lit32(model["max_radius"]))
@@ -800,25 +800,60 @@ def gen_cuda(model: dict) -> str:
     }}
 
     // Robot::fkcc for the lanes of ctx.alive.  Clears the lanes of every segment found in collision.
-    template <typename Ctx, bool kLoopedEnv = false>
+    template <typename Ctx>
     static __device__ __forceinline__ void fkcc(const float *q, Ctx &ctx)
     {{
         float F[kFrames * 12];
         frames(q, F);
 {chr(10).join("        " + l for l in limits_code(model, load_cull(name)))}
-        // coarse centres, computed once: the self loop reads them for every link pair
+        // coarse centres, computed once (the self loop reads them for every link pair), and the
+        // segments where each may touch anything, four lookups in flight at a time
         float4 CC[{len(model['env_checks'])}];
+        unsigned *const near = ctx.wsc;
+#pragma unroll 1
+        for (int c0 = 0; c0 < {len(model['env_checks'])}; c0 += {TABLE_NEAR})
+        {{
+            float4 k[{TABLE_NEAR}];
+            unsigned clear[{TABLE_NEAR}];
+#pragma unroll
+            for (int j = 0; j < {TABLE_NEAR}; ++j)
+            {{
+                const int c = {"c0 + j" if len(model['env_checks']) % TABLE_NEAR == 0 else f"min(c0 + j, {len(model['env_checks']) - 1})"};
+                k[j] = centre(F, {pre}EnvCoarse[c]);
+                CC[c] = k[j];
+                clear[j] = ctx.clearance(k[j].x, k[j].y, k[j].z);
+            }}
+#pragma unroll
+            for (int j = 0; j < {TABLE_NEAR}; ++j)
+            {{
+                const unsigned m = ctx.vote_near(clear[j] < vg::field_reach(k[j].w), ctx.alive);
+                if ((threadIdx.x & 31) == 0)
+                {{
+                    near[c0 + j] = m;
+                }}
+            }}
+        }}
+        __syncwarp();
 #pragma unroll 1
         for (int c = 0; c < {len(model['env_checks'])}; ++c)
         {{
-            const float4 k = centre(F, {pre}EnvCoarse[c]);
-            CC[c] = k;
-            unsigned need = ctx.env_hit(k.x, k.y, k.z, k.w, ctx.alive);
+            unsigned need = near[c] & ctx.alive;
+            if (!need)
+            {{
+                continue;
+            }}
+            const float4 k = CC[c];
+            need = ctx.env_hit(k.x, k.y, k.z, k.w, need);
 #pragma unroll 1
             for (int i = {pre}EnvStart[c]; need && i < {pre}EnvStart[c + 1]; ++i)
             {{
                 const float4 s = centre(F, {pre}EnvFine[i]);
-                const unsigned hit = ctx.env_hit(s.x, s.y, s.z, s.w, need);
+                const unsigned may = ctx.near(s, need);
+                if (!may)
+                {{
+                    continue;
+                }}
+                const unsigned hit = ctx.env_hit(s.x, s.y, s.z, s.w, may);
                 need &= ~hit;
                 if (hit && !ctx.kill(hit))
                 {{
@@ -873,12 +908,10 @@ def gen_cuda(model: dict) -> str:
         w("#else")
 
 
-    # ---- compact and staged schedules.  Both: frames in registers while the kinematics run,
-    # coarse link spheres queried together, per-check code unrolled, per-sphere and per-pair work
-    # in rolled loops over constant tables.  Compact passes the frames to those loops in
-    # registers; staged (the default) writes the frames the fine checks need to shared memory
-    # once, so that the call sites pass frame indices and the frames need no registers across
-    # the checks (smaller code for the instruction cache, fewer live registers).
+    # ---- staged schedule.  The frames the fine checks need, the coarse centres and the joint
+    # values the danger boxes test are written to shared memory once, and the environment and
+    # self-collision sections are loops over constant tables that read them from there (small code
+    # for the instruction cache, few live registers).
     pre = f"k{S}"
     cull = load_cull(name)
     em = Emitter("cuda", SNAP32)
@@ -888,12 +921,7 @@ def gen_cuda(model: dict) -> str:
     fvals = frame_values(kin, fr)
     sid = lay["frames"]
 
-    def frame_expr(fid):
-        return "vg::Frame{{" + ", ".join(em.ref(v) for v in fvals[fidx[fid]]) + "}}"
-
     n_env = len(model["env_checks"])
-    env_index = {e["link"]: k for k, e in enumerate(model["env_checks"])}
-
     def centre(i, tag):
         em.lines = []
         link, p, r = slots[i]
@@ -908,76 +936,11 @@ def gen_cuda(model: dict) -> str:
         coarse += ["    " + l for l in ls]
         coarse.append(f"    cs[{k}] = make_float4({x}, {y}, {z}, {r});  // {e['link']}")
         coarse.append("}")
-    coarse.append(f"unsigned ch[{n_env}];")
-    nb = -(-n_env // COARSE_BATCH)
-    base = 0
-    for bi in range(nb):
-        size = n_env // nb + (1 if bi < n_env % nb else 0)
-        coarse.append(f"ctx.template env_many<{size}>(cs + {base}, ctx.alive, ch + {base});")
-        base += size
-
     stage = []
     vals_ = [f"(-{v[1:]})" if v.startswith("-") else v for v in lay["values"]]
     for i in range(0, len(vals_), 6):
         stage.append(" ".join(f"st[{j} * vg::kStageStride] = {vals_[j]};" for j in range(i, min(i + 6, len(vals_)))))
 
-    def env_section(staged):
-        out = []
-        for k, e in enumerate(model["env_checks"]):
-            fid = kin.sphere_in_frame(slots[e["fine"][0]][0], slots[e["fine"][0]][1])[0]
-            for sidx in e["fine"]:
-                assert kin.sphere_in_frame(slots[sidx][0], slots[sidx][1])[0] == fid
-            fa = str(sid[fid]) if staged else frame_expr(fid)
-            out.append(f"// environment: {e['link']} ({len(e['fine'])} fine spheres)")
-            out.append("{")
-            out.append(f"    const unsigned need = ch[{k}] & ctx.alive;")
-            out.append(f"    if (need)")
-            out.append("    {")
-            if staged:
-                out.append(f"        const unsigned hit = env_fine<Ctx::kW, Ctx::kExt>(ctx.env, st, {fa}, {env_start[k]}, {env_start[k + 1]}, need);")
-            else:
-                out.append(f"        const unsigned hit = env_fine<Ctx::kW, Ctx::kExt>(ctx.env, {fa}, {env_start[k]}, {env_start[k + 1]}, need);")
-            out.append("        if (hit && !ctx.kill(hit)) return;")
-            out.append("    }")
-            out.append("}")
-        return out
-
-    full_start, full_pairs, lv_start, lv_pairs = [0], [], [0], []
-    for ci, e in enumerate(model["self_checks"]):
-        full_pairs += [tuple(p_) for p_ in e["fine"]]
-        full_start.append(len(full_pairs))
-        sel = range(len(e["fine"])) if cull is None or cull["live"][ci] is None else cull["live"][ci]
-        lv_pairs += [tuple(e["fine"][pi]) for pi in sel]
-        lv_start.append(len(lv_pairs))
-
-    def self_section(staged):
-        out = []
-        for ci, e in enumerate(model["self_checks"]):
-            a, b = e["links"]
-            A, B = _pairs_ab(e)
-            fa = kin.sphere_in_frame(slots[A[0]][0], slots[A[0]][1])[0]
-            fb = kin.sphere_in_frame(slots[B[0]][0], slots[B[0]][1])[0]
-            ka, kb = env_index[a], env_index[b]
-            nl = lv_start[ci + 1] - lv_start[ci]
-            out.append(f"// self: {a} vs. {b} ({nl} of {len(e['fine'])} fine pairs can collide inside the limits)")
-            out.append("{")
-            out.append(f"    const unsigned need = ctx.self_hit(cs[{ka}].x, cs[{ka}].y, cs[{ka}].z, cs[{ka}].w, cs[{kb}].x, cs[{kb}].y, cs[{kb}].z, cs[{kb}].w, ctx.alive);")
-            out.append("    if (need)")
-            out.append("    {")
-            if staged:
-                cbc = f"make_float4(cs[{kb}].x, cs[{kb}].y, cs[{kb}].z, {pre}ContainR[{kb}])"
-                out.append(f"        const unsigned acc = ctx.in_limits ? self_pairs(st, {sid[fa]}, {sid[fb]}, {pre}LivePair, {lv_start[ci]}, {lv_start[ci + 1]}, {cbc})")
-                out.append(f"                                           : self_pairs(st, {sid[fa]}, {sid[fb]}, {pre}FullPair, {full_start[ci]}, {full_start[ci + 1]}, {cbc});")
-            else:
-                out.append(f"        const unsigned acc = ctx.in_limits ? self_pairs({frame_expr(fa)}, {frame_expr(fb)}, {pre}LivePair, {lv_start[ci]}, {lv_start[ci + 1]})")
-                out.append(f"                                           : self_pairs({frame_expr(fa)}, {frame_expr(fb)}, {pre}FullPair, {full_start[ci]}, {full_start[ci + 1]});")
-            out.append("        const unsigned hit = ctx.vote(acc, need);")
-            out.append("        if (hit && !ctx.kill(hit)) return;")
-            out.append("    }")
-            out.append("}")
-        return out
-
-    compact_body = head + coarse + env_section(False) + self_section(False)
     c0 = lay["coarse0"]
     coarse_stage = [" ".join(f"st[{c0 + 3 * i + j} * vg::kStageStride] = cs[{k}].{'xyz'[j]};" for j in range(3))
                     for i, k in enumerate(lay["coarse"])]
@@ -1016,108 +979,61 @@ for (int c = 0; c < {len(model['self_checks'])}; ++c)
         if (hit && !ctx.kill(hit)) return;
     }}
 }}""".split("\n")
-    staged_body = head + ["float *const st = ctx.stage;"] + stage + coarse + env_section(True) + self_section(True)
-    cut = next(i for i, l in enumerate(coarse) if l.startswith("unsigned ch["))
-    lb = LOOPED_BATCH
-    nb = -(-n_env // lb)
-    env_loops = f"""// coarse spheres of every environment-checked link, {lb} at a time (one copy of the batched query)
+    lb = COARSE_BATCH
+    env_loops = f"""// the segments where each coarse sphere may touch anything; a bit per sphere that has any
 unsigned *const chs = ctx.wsc;
+auto todo = ctx.template near_all<{n_env}>(cs, chs);
+// those spheres' exact queries, {lb} at a time (one copy of the batched query)
+decltype(todo) hits = 0;
 #pragma unroll 1
-for (int b = 0; b < {nb}; ++b)
+while (todo)
 {{
     float4 sp[{lb}];
+    unsigned need[{lb}], h[{lb}];
+    int id[{lb}];
 #pragma unroll
     for (int s = 0; s < {lb}; ++s)
     {{
-        const int k = {lb} * b + s;
+        const int k = vg::lowest_bit(todo);
+        id[s] = k;
+        todo &= todo - 1;
         // padding sphere: far away with radius -inf, it is never tested and never hits
-        sp[s] = k < {n_env} ? make_float4(st[({c0} + 3 * k) * vg::kStageStride], st[({c0} + 3 * k + 1) * vg::kStageStride],
-                                          st[({c0} + 3 * k + 2) * vg::kStageStride], {pre}CoarseR[k])
-                            : make_float4(1.0e10f, 0.0f, 0.0f, -__int_as_float(0x7f800000));
+        sp[s] = k >= 0 ? make_float4(st[({c0} + 3 * k) * vg::kStageStride], st[({c0} + 3 * k + 1) * vg::kStageStride],
+                                     st[({c0} + 3 * k + 2) * vg::kStageStride], {pre}CoarseR[k])
+                       : make_float4(1.0e10f, 0.0f, 0.0f, -__int_as_float(0x7f800000));
+        need[s] = k >= 0 ? chs[k] : 0u;
     }}
-    unsigned h[{lb}];
-    ctx.template env_many<{lb}>(sp, ctx.alive, h);
+    ctx.template env_many<{lb}>(sp, need, h);
 #pragma unroll
     for (int s = 0; s < {lb}; ++s)
     {{
-        if ({lb} * b + s < {n_env} && (threadIdx.x & 31) == 0)
+        if (h[s])
         {{
-            chs[{lb} * b + s] = h[s];  // warp-uniform
+            hits |= decltype(hits)(1) << id[s];
+            if ((threadIdx.x & 31) == 0)
+            {{
+                chs[id[s]] = h[s];  // warp-uniform
+            }}
         }}
     }}
 }}
 __syncwarp();
 // fine spheres of the links whose coarse sphere hit
 #pragma unroll 1
-for (int k = 0; k < {n_env}; ++k)
+while (hits)
 {{
+    const int k = vg::lowest_bit(hits);
+    hits &= hits - 1;
     const unsigned need = chs[k] & ctx.alive;
     if (need)
     {{
-        const unsigned hit = env_fine_inline<Ctx::kW, Ctx::kExt>(ctx.env, st, {pre}EnvFrameS[k], {pre}EnvStart[k], {pre}EnvStart[k + 1], need);
+        const unsigned hit = env_fine<Ctx::kW, Ctx::kExt>(ctx, st, {pre}EnvFrameS[k], {pre}EnvStart[k], {pre}EnvStart[k + 1], need);
         if (hit && !ctx.kill(hit)) return;
     }}
 }}""".split("\n")
-    # the environment section either as loops (one copy of the batched query: small code) or
-    # unrolled (the coarse centres stay in registers: fewer instructions); chosen per kernel
-    looped_body = (head + ["float *const st = ctx.stage;"] + stage + q_stage + coarse[:cut]
-                   + ["if constexpr (kLoopedEnv)", "{"] + ["    " + l for l in coarse_stage + env_loops] + ["}", "else", "{"]
-                   + ["    " + l for l in coarse[cut:] + coarse_stage + env_section(True)] + ["}"]
+    staged_body = (head + ["float *const st = ctx.stage;"] + stage + q_stage + coarse + coarse_stage + env_loops
                    + ["// self-collision link pairs, in the reference's order"] + self_loop)
 
-    w("#ifdef VG_FORM_COMPACT")
-    w(f"""    // Fine environment tests of the spheres EnvFine[k0..k1) of one frame, for the segments in
-    // `need`: the segments whose block collides.
-    template <int W, bool kExt = false>
-    static __device__ __noinline__ unsigned env_fine(const vg::EnvView &ev, const vg::Frame f, int k0, int k1, unsigned need)
-    {{
-        unsigned dead = 0u;
-#pragma unroll 1
-        for (int k = k0; k < k1; ++k)
-        {{
-            const float4 o = {pre}SlotOff[{pre}EnvFine[k]];
-            const float4 c = vg::frame_point(f, o);
-            const unsigned hit = vg::env_query_inline<W, kExt>(ev, c.x, c.y, c.z, c.w, need);
-            dead |= hit;
-            need &= ~hit;
-            if (!need)
-            {{
-                break;
-            }}
-        }}
-        return dead;
-    }}
-
-    // OR of the sign bits of the fine self-collision tests of pairs[k0..k1) (slot ids), the first
-    // slot of each pair in frame a, the second in frame b.
-    static __device__ __noinline__ unsigned self_pairs(const vg::Frame a, const vg::Frame b, const int2 *pairs, int k0, int k1)
-    {{
-        unsigned acc = 0u;
-        int last = -1;
-        float4 ca = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 1
-        for (int k = k0; k < k1; ++k)
-        {{
-            const int2 pr = pairs[k];
-            if (pr.x != last)
-            {{
-                ca = vg::frame_point(a, {pre}SlotOff[pr.x]);
-                last = pr.x;
-            }}
-            const float4 cb = vg::frame_point(b, {pre}SlotOff[pr.y]);
-            acc |= vg::self_bits(ca.x, ca.y, ca.z, cb.x, cb.y, cb.z, __fadd_rn(ca.w, cb.w));
-        }}
-        return acc;
-    }}
-""")
-    w("    // Robot::fkcc for the lanes of ctx.alive.  Clears the lanes of every segment found in collision.")
-    w("    template <typename Ctx, bool kLoopedEnv = false>")
-    w("    static __device__ __forceinline__ void fkcc(const float *q, Ctx &ctx)")
-    w("    {")
-    for l in compact_body:
-        w("        " + l)
-    w("    }")
-    w("#else")
     w(f"""    // Staged frame f: its non-constant entries from this thread's stage, the rest constants.
     static __device__ __forceinline__ vg::Frame frame_at(const float *st, int f)
     {{
@@ -1133,16 +1049,8 @@ for (int k = 0; k < {n_env}; ++k)
 
     // Fine environment tests of the spheres EnvFine[k0..k1) of staged frame f, for the segments
     // in `need`: the segments whose block collides.
-    template <int W, bool kExt = false>
-    static __device__ __noinline__ unsigned env_fine(const vg::EnvView &ev, const float *st, int f, int k0, int k1, unsigned need)
-    {{
-        return env_fine_inline<W, kExt>(ev, st, f, k0, k1, need);
-    }}
-
-    // The same, inlined into its caller (the looped environment section calls it from one place).
-    template <int W, bool kExt = false>
-    static __device__ __forceinline__ unsigned env_fine_inline(const vg::EnvView &ev, const float *st, int f, int k0, int k1,
-                                                               unsigned need)
+    template <int W, bool kExt, typename Ctx>
+    static __device__ __forceinline__ unsigned env_fine(Ctx &ctx, const float *st, int f, int k0, int k1, unsigned need)
     {{
         const vg::Frame fr = frame_at(st, f);
         unsigned dead = 0u;
@@ -1151,7 +1059,12 @@ for (int k = 0; k < {n_env}; ++k)
         {{
             const float4 o = {pre}SlotOff[{pre}EnvFine[k]];
             const float4 c = vg::frame_point(fr, o);
-            const unsigned hit = vg::env_query_inline<W, kExt>(ev, c.x, c.y, c.z, c.w, need);
+            const unsigned may = ctx.near(c, need);
+            if (!may)
+            {{
+                continue;
+            }}
+            const unsigned hit = ctx.env_hit(c.x, c.y, c.z, c.w, may);
             dead |= hit;
             need &= ~hit;
             if (!need)
@@ -1243,18 +1156,12 @@ for (int k = 0; k < {n_env}; ++k)
     }}
 """)
     w("    // Robot::fkcc for the lanes of ctx.alive.  Clears the lanes of every segment found in collision.")
-    w("    template <typename Ctx, bool kLoopedEnv = false>")
+    w("    template <typename Ctx>")
     w("    static __device__ __forceinline__ void fkcc(const float *q, Ctx &ctx)")
     w("    {")
-    w("#ifdef VG_SELF_UNROLLED")
     for l in staged_body:
         w("        " + l)
-    w("#else")
-    for l in looped_body:
-        w("        " + l)
-    w("#endif")
     w("    }")
-    w("#endif")
     if tabled:
         w("#endif  // VG_STAGED_ALL")
     w("};")
