@@ -158,7 +158,7 @@ int vg_env_set_mode(vg_env *env, int lanes, int sqrt_mode);
  * 1 = a warp checks consecutive blocks of one edge, 0 = each lane-block checks its own edge, 2 = as
  * 1 with the kernel built for fewer resident blocks and more registers per thread, 3 = as 2 with
  * the segments an edge's last blocks leave free starting on the next edge, -1 (default) = each
- * robot's own (2 for the Panda, UR5 and Fetch, 1 for Baxter).  An autotuner pick
+ * robot's own (1 for all four).  An autotuner pick
  * (vg_autotune_motions) takes precedence until this is called again.
  * No reference counterpart: the reference validates one edge at a time on one core. */
 int vg_env_set_schedule(vg_env *env, int schedule);

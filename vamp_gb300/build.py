@@ -32,10 +32,10 @@ NVCC_FLAGS = [
     "-fPIC,-ffp-contract=off,-O2",
 ]
 
-# ptxas optimisation level for the translation units where it was measured to matter.  The
-# Panda's same-edge edge kernel is bound by instruction fetch; built with ptxas -O1 it checked the
-# 65,536-edge workload in 2.665 ms against 2.748 ms at the default -O3 (two builds each, same box).
-# The other robots' kernels were as fast or faster at -O3, so they keep it.
+# ptxas optimisation level for the translation units where it was measured to matter: the Panda's
+# same-edge kernel checks 16,384 edges among 60 primitives in 275 us built with ptxas -O1 and 282 us
+# at the default -O3 (-O1 schedules less aggressively: less instruction fetch).  The other robots'
+# kernels were as fast or faster at -O3, so they keep it.
 PTXAS_LEVEL = {"robot_panda.cu": 1}
 
 
@@ -52,14 +52,10 @@ def sources() -> list[Path]:
 
 def _defines() -> list[str]:
     # VG_MIN_BLOCKS: resident 128-thread blocks per SM the kernels are compiled for.
-    # VG_STAGED_ALL=1: the staged form for the robots whose default is the table-driven form
-    # (both forms give identical results).
     out = []
     mb = os.environ.get("VG_MIN_BLOCKS")
     if mb:
         out.append(f"-DVG_MIN_BLOCKS={int(mb)}")
-    if os.environ.get("VG_STAGED_ALL") == "1":
-        out.append("-DVG_STAGED_ALL")
     # VG_CAPT_SHARED_WEIGHT=w: the pointcloud query scans one lane's list with the whole warp
     # when 4 x the longest list exceeds w x the warp's shared steps
     w = os.environ.get("VG_CAPT_SHARED_WEIGHT")

@@ -17,7 +17,6 @@
 #pragma once
 
 #include <cstdint>
-#include <type_traits>
 
 namespace vg
 {
@@ -264,14 +263,10 @@ namespace vg
         return a < 255.0f ? static_cast<unsigned>(a) + 1u : 256u;  // NaN: 256
     }
 
-    __device__ __forceinline__ int lowest_bit(unsigned m)
+    // word << 1 with the top bit of v below: a per-lane bit word filled first bit highest
+    __device__ __forceinline__ unsigned shift_in(unsigned word, unsigned v)
     {
-        return __ffs(static_cast<int>(m)) - 1;
-    }
-
-    __device__ __forceinline__ int lowest_bit(unsigned long long m)
-    {
-        return __ffsll(static_cast<long long>(m)) - 1;
+        return __funnelshift_l(v, word, 1);
     }
 
     // sphere_heightfield (collision/sphere_heightfield.hh:9-30), sign bit set iff the sphere is
@@ -719,11 +714,16 @@ namespace vg
         return __float_as_uint(__fmaf_rn(-rs, rs, sql2(ax, ay, az, bx, by, bz)));
     }
 
+    // whether the spheres a and b (w the radius) overlap
+    __device__ __forceinline__ bool spheres_meet(const float4 a, const float4 b)
+    {
+        const float rr = __fadd_rn(a.w, b.w);
+        return sql2(a.x, a.y, a.z, b.x, b.y, b.z) < __fmul_rn(rr, rr);
+    }
+
     // Threads per block of every checking kernel, and the stride of the per-thread columns of
     // the robots' shared-memory stage.
     constexpr int kStageStride = 128;
-    // words of per-warp shared scratch available to a generated fkcc (environment checks per robot)
-    constexpr int kWarpScratch = 64;
 
     // The context a generated Robot::fkcc body runs against.  kExt: the environment queries also
     // test heightfields.  kOrdered: the warp's segments are consecutive blocks of one edge in the
@@ -741,20 +741,10 @@ namespace vg
         bool in_limits = false;
         // this thread's column of the robot's shared-memory stage: element i at stage[i * kStageStride]
         float *stage = nullptr;
-        // this warp's scratch (kWarpScratch words) for warp-uniform values such as per-link hit masks
-        unsigned *wsc = nullptr;
 
-        // inlined at each call site: the table-driven robot forms call it from two places (coarse
-        // and fine spheres), and an out-of-line query costs them more than the second copy
         __device__ __forceinline__ unsigned env_hit(float x, float y, float z, float r, unsigned mask)
         {
             return env_query_inline<W, kExt>(env, x, y, z, r, mask);
-        }
-
-        template <int NS>
-        __device__ __forceinline__ void env_many(const float4 *s, const unsigned *mask, unsigned *hit)
-        {
-            env_multi<W, NS, kExt>(env, s, mask, hit);
         }
 
         // the field's value at a point (0, which rules nothing out, without a field)
@@ -772,34 +762,6 @@ namespace vg
         __device__ __forceinline__ unsigned near(const float4 s, unsigned mask)
         {
             return vote_near(clearance(s.x, s.y, s.z) < field_reach(s.w), mask);
-        }
-
-        // vote_near of N spheres over the segments alive, sphere k's into masks[k]; a bit per
-        // sphere with any such segment.  The N lookups are independent loads in flight together.
-        template <int N>
-        __device__ __forceinline__ auto near_all(const float4 (&s)[N], unsigned *masks)
-        {
-            static_assert(N <= 64, "one bit per sphere");
-            using Bits = std::conditional_t<(N > 32), unsigned long long, unsigned>;
-            unsigned v[N];
-#pragma unroll
-            for (int k = 0; k < N; ++k)
-            {
-                v[k] = clearance(s[k].x, s[k].y, s[k].z);
-            }
-            Bits any = 0;
-#pragma unroll
-            for (int k = 0; k < N; ++k)
-            {
-                const unsigned m = vote_near(v[k] < field_reach(s[k].w), alive);
-                any |= m ? Bits(1) << k : Bits(0);
-                if ((threadIdx.x & 31) == 0)
-                {
-                    masks[k] = m;  // warp-uniform
-                }
-            }
-            __syncwarp();
-            return any;
         }
 
         __device__ __forceinline__ unsigned self_hit(

@@ -2,11 +2,13 @@
 // distance from any point of the cell to anything in the environment, so that the checking
 // kernels skip the exact queries of spheres that are out of everything's reach.
 //
-// Every bound is rigorous against the exact tests as they round (collision/sphere_*.hh,
-// capt.hh:425-506): the test of an object is negative only if its distance function f at the
-// sphere's centre is below the radius, up to a few FP32 roundings; f changes by at most L times
-// the distance moved, so f(cell centre) - L * (half the cell's diagonal) - margin bounds it over
-// the cell.  The margin is 1 mm + 1e-5 of the coordinates involved, hundreds of times the
+// A cell's bound C is rigorous against the exact tests as they round (collision/sphere_*.hh,
+// capt.hh:425-506): no sphere inside the ball of radius C about any point of the cell tests
+// negative, neither one about that point nor the members of a larger sphere about it.  The test of
+// a primitive or a cloud is negative only if its distance function f at the sphere's centre is
+// below the radius, up to a few FP32 roundings; f changes by at most L times the distance moved, so
+// f(cell centre) - L * (half the cell's diagonal) - margin bounds it over the cell (and L > 1
+// scales it).  The margin is 1 mm + 1e-5 of the coordinates involved, hundreds of times the
 // rounding.  min_distance plays no part: a skipped test would have been non-negative, whether or
 // not the sorted walk would have reached it.
 //
@@ -41,9 +43,10 @@ namespace vg
             return fmaf(1e-5f, size, 1e-3f);
         }
 
-        // Lower bound of (distance of a sphere's centre at which object o of a kind may test
-        // negative, minus the sphere's radius) over the ball of radius `reach` about (x, y, z).
-        // NaN for objects with non-finite fields.
+        // A C as above for object o of a kind, over the ball of radius `reach` about (x, y, z):
+        // spheres of radius r whose centre is d from there need f >= r, f falls by at most L d, and
+        // d + r <= C, so C = (f - L * reach - margin) / max(L, 1).  NaN for objects with non-finite
+        // fields.
         __device__ __forceinline__ float object_bound(int kind, const float4 *o, float x, float y, float z, float reach)
         {
             const float4 a = o[0];
@@ -89,7 +92,7 @@ namespace vg
                 e[i] = v > 0.0f || !(v == v) ? v : 0.0f;
             }
             const float size = (1.0f + L) * place + fabsf(h[0]) + fabsf(h[1]) + fabsf(h[2]);
-            return len3(e[0], e[1], e[2]) - L * reach - margin(size);
+            return (len3(e[0], e[1], e[2]) - L * reach - margin(size)) / fmaxf(L, 1.0f);
         }
 
         __device__ __forceinline__ float3 cell_centre(int ix, int iy, int iz)
@@ -255,13 +258,20 @@ namespace vg
         }
 
         // Heightfields (t_heightfield, vg_check.cuh): the test is z - r - z0 < zs * h for the
-        // sample of the centre's cell, so the bound over a cell is its lowest z - z0 minus the
-        // largest zs * h among the samples its columns can reach (one more on each side, for
-        // the rounding of the index).
-        __global__ void __launch_bounds__(kFieldCells) field_heights(const HeightView h, uint8_t *out)
+        // sample of the sphere's own column.  The field also stands for spheres about other
+        // centres (a link group's members), so its bound C at p has to keep every sphere inside the
+        // ball of radius C about p above the surface: z - z0 - C >= the largest zs * h within C of
+        // p, sideways.  Largest zs * h per column of cells first (one more sample on each side,
+        // for the rounding of the index), on a grid kMaxGap columns wider than the field; infinity
+        // where a field or sample is not finite.
+        constexpr int kWide = kFieldCells + 2 * kMaxGap;
+
+        __global__ void field_columns(const HeightView h, float *tops)
         {
-            const int ix = threadIdx.x, iy = blockIdx.x;
-            const float3 p = cell_centre(ix, iy, 0);
+            const int ix = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), iy = blockIdx.y;
+            if (ix >= kWide)
+                return;
+            const float3 p = cell_centre(ix - kMaxGap, iy - kMaxGap, 0);
             const float half = 0.5f * kCell + 1e-4f;
             auto range = [&](float scale, float at, float from, int n, int &lo, int &hi) {
                 const float c = fmaf(scale, from - at, static_cast<float>(n / 2)), w = fabsf(scale) * half + 1.0f;
@@ -285,17 +295,57 @@ namespace vg
                     top = fmaxf(top, v);
                 }
             }
-            const float spare = margin(8.0f + fabsf(h.z) + fabsf(top)) + half;
+            tops[iy * kWide + ix] = fine ? top : __int_as_float(0x7f800000);
+        }
+
+        // A window of R columns to each side holds everything within (R - 1) cells of the middle
+        // column's points: C is the best of min((R - 1) cells, z - z0 - the window's largest) over
+        // a few R.
+        __global__ void __launch_bounds__(kFieldCells) field_heights(const HeightView h, const float *tops, uint8_t *out)
+        {
+            constexpr int kRings = 5;
+            constexpr int kWindow[kRings] = {2, 4, 8, 16, kMaxGap};
+            const int ix = threadIdx.x, iy = blockIdx.x;
+            float top[kRings];
+            float best = -3.4e38f;
+            int done = -1;
+#pragma unroll
+            for (int r = 0; r < kRings; ++r)
+            {
+                for (int dy = -kWindow[r]; dy <= kWindow[r]; ++dy)
+                {
+                    const float *row = tops + (iy + kMaxGap + dy) * kWide + ix + kMaxGap;
+                    const bool inner = dy >= -done && dy <= done;
+                    for (int dx = -kWindow[r]; dx <= kWindow[r]; ++dx)
+                    {
+                        if (inner && dx == -done)
+                            dx = done + 1;  // columns of the window before
+                        best = fmaxf(best, row[dx]);
+                    }
+                }
+                done = kWindow[r];
+                top[r] = best;
+            }
             for (int iz = 0; iz < kFieldCells; ++iz)
             {
                 uint8_t *cell = out + (iz << (2 * kFieldBits)) + (iy << kFieldBits) + ix;
                 const float z = (static_cast<float>(iz) - kFieldZ) * kCell;
-                const unsigned v = fine ? step_of(z - h.z - top - spare) : 0u;
-                *cell = static_cast<uint8_t>(min(static_cast<unsigned>(*cell), v));
+                float clear = 0.0f;
+#pragma unroll
+                for (int r = 0; r < kRings; ++r)
+                {
+                    const float up = z - h.z - top[r] - 0.5f * kCell - margin(8.0f + fabsf(h.z) + fabsf(top[r]));
+                    clear = fmaxf(clear, fminf(static_cast<float>(kWindow[r] - 1) * kCell - margin(8.0f), up));
+                }
+                *cell = static_cast<uint8_t>(min(static_cast<unsigned>(*cell), step_of(clear)));
             }
         }
 
-        // launches that fill e->d_field on stream s (scratch: occupancy bits and gaps, for clouds)
+        // launches that fill e->d_field on stream s (scratch: occupancy bits and gaps of the clouds,
+        // then a heightfield's columns)
+        constexpr size_t kScratch = kCells / 8 + 3 * static_cast<size_t>(kCells);
+        static_assert(kScratch >= kWide * kWide * sizeof(float), "a heightfield's columns fit the scratch");
+
         cudaError_t launch_build(vg_env *e, char *scratch, cudaStream_t s)
         {
             field_primitives<<<kCells / 512, 256, 0, s>>>(env_device(e), e->d_field);
@@ -334,7 +384,9 @@ namespace vg
             {
                 HeightView h = e->hf[i];
                 h.data = static_cast<const float *>(e->d_hf[i]);
-                field_heights<<<kFieldCells, kFieldCells, 0, s>>>(h, e->d_field);
+                float *tops = reinterpret_cast<float *>(scratch);
+                field_columns<<<dim3((kWide + 127) / 128, kWide), 128, 0, s>>>(h, tops);
+                field_heights<<<kFieldCells, kFieldCells, 0, s>>>(h, tops, e->d_field);
                 err = cudaGetLastError();
             }
             return err;
@@ -365,8 +417,8 @@ namespace vg
         if (!e->d_field)
             err = cudaMalloc(&e->d_field, kCells);
         char *scratch = nullptr;
-        if (err == cudaSuccess && !e->clouds.empty())
-            err = cudaMalloc(&scratch, kCells / 8 + 3 * static_cast<size_t>(kCells));
+        if (err == cudaSuccess && !(e->clouds.empty() && e->hf.empty()))
+            err = cudaMalloc(&scratch, kScratch);
         if (err == cudaSuccess)
             err = launch_build(e, scratch, s);
         // complete before any other stream or thread can see it

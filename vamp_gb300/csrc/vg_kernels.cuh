@@ -89,7 +89,7 @@ namespace vg
     template <typename Robot, int W, bool kExt>
     __device__ __noinline__ unsigned attach_check(const EnvView &ev, const float *q, unsigned alive)
     {
-        CheckCtx<W, kExt> ctx{ev, alive, false, nullptr, nullptr};
+        CheckCtx<W, kExt> ctx{ev, alive, false, nullptr};
         float T[12], NR[9], Nt[3];
         Robot::ee_pose(q, T);
         const float4 *A = ev.att;
@@ -116,7 +116,10 @@ namespace vg
         for (int k = 0; k < ev.n_att && need; ++k)
         {
             const float4 c = posed(k);
-            const unsigned hit = ctx.env_hit(c.x, c.y, c.z, c.w, need);
+            const unsigned may = ctx.near(c, need);
+            if (!may)
+                continue;
+            const unsigned hit = ctx.env_hit(c.x, c.y, c.z, c.w, may);
             ctx.alive &= ~hit;
             need &= ~hit;
         }
@@ -160,9 +163,7 @@ namespace vg
     template <typename Robot, int W, bool kExt = false, bool kOrdered = false>
     __device__ __forceinline__ unsigned run_fkcc(const EnvView &ev, const float *q, unsigned alive, float *stage)
     {
-        static_assert(Robot::kEnvChecks <= kWarpScratch, "per-warp scratch holds one word per environment check");
-        __shared__ unsigned warp_scratch[kStageStride / 32][kWarpScratch];
-        CheckCtx<W, kExt, kOrdered> ctx{ev, alive, false, stage, warp_scratch[threadIdx.x >> 5]};
+        CheckCtx<W, kExt, kOrdered> ctx{ev, alive, false, stage};
         Robot::fkcc(q, ctx);
         if constexpr (kExt)
         {
@@ -523,7 +524,7 @@ namespace vg
     // (block i = block 0 minus v / (W n), i times).  The edge is invalid if any checked block is,
     // and the reference would have stopped at the first invalid block, so the block count
     // reported is that block's index + 1.
-    template <typename Robot, int W, bool kLearned, int kMinBlocks = VG_MIN_BLOCKS>
+    template <typename Robot, int W, bool kLearned, int kMinBlocks = Robot::kEdgeBlocks>
     __global__ void __launch_bounds__(128, kMinBlocks) edges_grouped_kernel(EdgesParams p)
     {
         extern __shared__ float4 smem[];

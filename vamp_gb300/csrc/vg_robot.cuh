@@ -38,7 +38,7 @@ namespace vg
         return cudaGetLastError();
     }
 
-    template <typename R, int W, bool kLearned, int kMinBlocks = VG_MIN_BLOCKS>
+    template <typename R, int W, bool kLearned, int kMinBlocks = R::kEdgeBlocks>
     cudaError_t launch_edges_grouped(const EdgesParams &p, int grid, int block, int smem, cudaStream_t s)
     {
         edges_grouped_kernel<R, W, kLearned, kMinBlocks><<<grid, block, smem, s>>>(p);
@@ -123,13 +123,12 @@ namespace vg
         o.edges_packed[1] = &launch_edges_packed<R, 4, VG_MIN_BLOCKS_WIDE>;
         o.edges_packed_fn[0] = reinterpret_cast<const void *>(&edges_packed_kernel<R, 8, VG_MIN_BLOCKS_WIDE>);
         o.edges_packed_fn[1] = reinterpret_cast<const void *>(&edges_packed_kernel<R, 4, VG_MIN_BLOCKS_WIDE>);
-        // the learned order in the form of the fastest plain schedule for the Panda, UR5 and Fetch
-        // (register-rich build); the group order comes precomputed
-        // (edge_order_kernel), which keeps it within the registers of 4 resident blocks
-        o.edges_learned[0] = &launch_edges_grouped<R, 8, true, VG_MIN_BLOCKS_WIDE>;
-        o.edges_learned[1] = &launch_edges_grouped<R, 4, true, VG_MIN_BLOCKS_WIDE>;
-        o.edges_learned_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, true, VG_MIN_BLOCKS_WIDE>);
-        o.edges_learned_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, true, VG_MIN_BLOCKS_WIDE>);
+        // the learned order as the same-edge schedule; the group order comes precomputed
+        // (edge_order_kernel), which keeps its registers out of the check
+        o.edges_learned[0] = &launch_edges_grouped<R, 8, true>;
+        o.edges_learned[1] = &launch_edges_grouped<R, 4, true>;
+        o.edges_learned_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, true>);
+        o.edges_learned_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, true>);
         o.edge_order[0] = &launch_edge_order<R, 8>;
         o.edge_order[1] = &launch_edge_order<R, 4>;
         // extended checks (heightfields, fkcc_attach): the segment-per-edge and states kernels

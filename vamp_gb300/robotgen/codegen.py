@@ -313,7 +313,12 @@ def emit_centre(em: Emitter, frames, kin: Kin, link: str, p, prefix: str):
     are (constants are not folded into the chain), so a centre computed from frame values held in
     registers, in local memory or on the CPU rounds identically."""
     fid, v = kin.sphere_in_frame(link, p)
-    R, t = frames[fid]
+    return emit_point(em, frames[fid], v, prefix)
+
+
+def emit_point(em: Emitter, frame, v, prefix: str):
+    """A point at offset v of a frame (R, t), in emit_centre's order of operations."""
+    R, t = frame
     out = []
     for r in range(3):
         acc = t[r]
@@ -396,19 +401,9 @@ def slot_table(model: dict):
 # CUDA output
 
 
-# Robots whose check schedule is emitted as table-driven loops (frames in local memory) rather
-# than straight-line code: their schedules are large enough (hundreds of link pairs) that
-# straight-line code spends minutes in ptxas and spills heavily.  Results are identical either way.
-TABLED = {"ur5", "fetch", "baxter"}
 # FP32 constants this close to 0 or +-1 are folded to exact values: URDF angles such as
 # 1.570796325 leave ~1e-9 residues that only cost operations (their effect is below 1e-8 m)
 SNAP32 = 1e-7
-# Coarse spheres queried together (one pass over the objects, up to the largest bound among
-# them): two, the fastest of 1-11 measured on the Panda's 65,536-edge workload.
-COARSE_BATCH = 2
-# Coarse spheres of the table-driven form whose field lookups are in flight together
-TABLE_NEAR = 4
-
 
 def f32_down(v: float) -> float:
     """Largest float32 <= v (a conservative lower bound in FP32)."""
@@ -450,6 +445,11 @@ def danger_boxes(model: dict, cull) -> tuple:
     return checks, pairs
 
 
+# Resident 128-thread blocks per SM that the same-edge kernels are built for: five for the robots
+# whose checks then stay in registers (102 a thread; 16,384 motions among 60 primitives, built for
+# 4 -> 5 -> 6 blocks: Panda 302 -> 278 -> 299 us, UR5 396 -> 388 -> 401, Fetch 571 -> 492 -> 541);
+# Baxter's stage leaves room for three (built for 4, with spills: 1,270 us; for 3: 1,224).
+EDGE_BLOCKS = {"panda": 5, "ur5": 5, "fetch": 5, "baxter": 3}
 CONTAIN_MARGIN = 1e-4  # metres between a link's fine spheres and its containing sphere
 
 
@@ -500,15 +500,13 @@ def _aliases(lines) -> dict:
 
 
 def stage_layout(model: dict, kin, cull) -> dict:
-    """The staged form's shared-memory stage, per thread: each distinct non-constant value among
-    the entries of the frames the fine checks use (an entry that is a copy of another takes that
-    value's slot), then the centres of every coarse sphere, then the joint values the danger
-    boxes test."""
+    """The shared-memory stage, per thread: each distinct non-constant value among the entries of
+    the frames the checks use (an entry that is a copy of another takes that value's slot), then
+    the joint values the danger boxes test."""
     slots, _ = slot_table(model)
     em = Emitter("cuda", SNAP32)
     fr = emit_frames(kin, em, "q", sc_fn=lambda x, s_, c: "")
-    # VG_STAGE_NO_DEDUP=1 (generator switch): one slot per frame entry, copies included
-    alias = {} if os.environ.get("VG_STAGE_NO_DEDUP") == "1" else _aliases(em.lines)
+    alias = _aliases(em.lines)
 
     def resolve(name):
         sign = 1
@@ -517,15 +515,9 @@ def stage_layout(model: dict, kin, cull) -> dict:
             sign *= sg
         return name, sign
 
-    order = []
-    for e in model["env_checks"]:
-        order.append(kin.sphere_in_frame(slots[e["fine"][0]][0], slots[e["fine"][0]][1])[0])
-    for e in model["self_checks"]:
-        A, B = _pairs_ab(e)
-        order.append(kin.sphere_in_frame(slots[A[0]][0], slots[A[0]][1])[0])
-        order.append(kin.sphere_in_frame(slots[B[0]][0], slots[B[0]][1])[0])
     frames, fslots, fconsts, values = {}, [], [], {}
-    for fid in order:
+    for e in model["env_checks"]:
+        fid = kin.sphere_in_frame(slots[e["fine"][0]][0], slots[e["fine"][0]][1])[0]
         if fid in frames:
             continue
         frames[fid] = len(fslots)
@@ -548,14 +540,55 @@ def stage_layout(model: dict, kin, cull) -> dict:
             row_c.append(0.0)
         fslots.append(row_s)
         fconsts.append(row_c)
-    n = len(values)
-    n_env = len(model["env_checks"])
     checks, _ = danger_boxes(model, cull)
-    joints = sorted({j for (j0, j1, b0), _ in checks if b0 >= 0 for j in (j0, j1)}) or [0]
-    return {"frames": frames, "slots": fslots, "consts": fconsts, "n_frame": n, "values": list(values),
-            "coarse": list(range(n_env)), "coarse_pos": {k: k for k in range(n_env)},
+    joints = sorted({j for (j0, j1, b0), _ in checks if b0 >= 0 for j in (j0, j1)})
+    return {"frames": frames, "slots": fslots, "consts": fconsts, "values": list(values),
             "joints": joints, "joint_pos": {j: i for i, j in enumerate(joints)},
-            "coarse0": n, "q0": n + 3 * n_env, "total": n + 3 * n_env + len(joints)}
+            "q0": len(values), "total": len(values) + len(joints)}
+
+
+def enclosing_sphere(spheres) -> tuple:
+    """A sphere that contains the given ones ((x, y, z), r), near the smallest: Badoiu and
+    Clarkson's iteration (move towards the farthest by 1 / (i + 1)), the radius then rounded up
+    with CONTAIN_MARGIN to spare."""
+    c = [sum(p[k] for p, _ in spheres) / len(spheres) for k in range(3)]
+
+    def far(q):
+        return max((math.sqrt(sum((p[k] - q[k]) ** 2 for k in range(3))) + r, p) for p, r in spheres)
+
+    for i in range(1, 400):
+        d, p = far(c)
+        n = math.sqrt(sum((p[k] - c[k]) ** 2 for k in range(3)))
+        if n == 0.0:
+            break
+        # towards the farthest point of the farthest sphere
+        c = [c[k] + (p[k] - c[k]) / n * d / (i + 1) * 0.5 for k in range(3)]
+    best = c
+    return best, f32_up(far(best)[0] + CONTAIN_MARGIN)
+
+
+def link_groups(model: dict, kin) -> dict:
+    """The environment-checked links grouped by the frame their coarse spheres are fixed in: a
+    rigid group's coarse spheres lie in one sphere of that frame, which stands for all of them
+    until something comes near it (Baxter: 349 self checks of 33 links are 64 pairs of 15 groups)."""
+    slots, coarse_slot = slot_table(model)
+    groups = {}
+    for k, e in enumerate(model["env_checks"]):
+        link, p, r = slots[coarse_slot[e["link"]]]
+        fid, off = kin.sphere_in_frame(link, p)
+        for f in e["fine"]:
+            assert kin.sphere_in_frame(slots[f][0], slots[f][1])[0] == fid
+        assert e["fine"] == list(range(e["fine"][0], e["fine"][0] + len(e["fine"]))), "a link's fine slots are consecutive"
+        groups.setdefault(fid, []).append((k, [float(v) for v in off], float(r)))
+    order = list(groups)
+    of = {k: g for g, fid in enumerate(order) for k, _, _ in groups[fid]}
+    pairs = {}
+    env_ix = {e["link"]: k for k, e in enumerate(model["env_checks"])}
+    for c, e in enumerate(model["self_checks"]):
+        a, b = of[env_ix[e["links"][0]]], of[env_ix[e["links"][1]]]
+        assert a != b, "links of one rigid group are not checked against each other"
+        pairs.setdefault((a, b), []).append(c)
+    return {"frames": order, "members": [groups[f] for f in order], "pairs": pairs, "env_ix": env_ix}
 
 
 def _pairs_ab(e):
@@ -573,20 +606,28 @@ def _pairs_ab(e):
 def gen_cuda(model: dict) -> str:
     name = model["name"]
     S = struct_name(name)
+    pre = f"k{S}"
     kin = Kin(model)
     slots, coarse_slot = slot_table(model)
     dim = model["dimension"]
-    tabled = name in TABLED
-    fidx = frame_index(kin)
+    cull = load_cull(name)
+    lay = stage_layout(model, kin, cull)
+    groups = link_groups(model, kin)
+    members, pairs = groups["members"], groups["pairs"]
+    n_groups = len(members)
+    assert n_groups <= 32, "one bit of a word per link group"
+    boxes_of, live_boxes = danger_boxes(model, cull)
+    all_pairs = [tuple(p_) for e in model["self_checks"] for p_ in e["fine"]]
     lines = []
     w = lines.append
     w("// Generated by vamp_gb300/robotgen/codegen.py from vamp_gb300/robots/%s.json. Do not edit." % name)
     w("//")
-    w("// FP32 forward kinematics and the fkcc check schedule of the %s robot, one configuration" % name)
-    w("// per thread.  Schedule order follows the reference's generated Robot::fkcc")
-    w("// (src/impl/vamp/robots/%s.hh): environment checks link by link, each a coarse link sphere" % name)
-    w("// gating that link's fine spheres, then self-collision link pairs, a coarse pair gating the")
-    w("// cross product of the two links' fine spheres.  Schedule form: %s." % ("table-driven loops" if tabled else "straight-line"))
+    w("// FP32 forward kinematics and the fkcc checks of the %s robot, one configuration per thread." % name)
+    w("// The checks are the reference's generated Robot::fkcc (src/impl/vamp/robots/%s.hh): environment" % name)
+    w("// checks link by link, each a coarse link sphere gating that link's fine spheres, then")
+    w("// self-collision link pairs, a coarse pair gating the cross product of the two links' fine")
+    w("// spheres.  A state collides if any check does, so their order is free: here a straight-line")
+    w("// pass over rigid groups of links finds the checks that can matter, and loops run those.")
     w("#pragma once")
     w("")
     w('#include "../vg_check.cuh"')
@@ -597,113 +638,92 @@ def gen_cuda(model: dict) -> str:
     def frames_block(em):
         return emit_frames(kin, em, "q", sc_fn=lambda x, s_, c: f"float {s_}, {c}; vg_sincos_ref({x}, &{s_}, &{c});")
 
-    # ---- tables (constant memory) for the table-driven form, and slot data for both
-    env_start, env_fine = [0], []
-    for e in model["env_checks"]:
-        env_fine += e["fine"]
-        env_start.append(len(env_fine))
-    self_rows, self_list = [], []
+    def table(kind, ctype, ident, rows, fmt):
+        body = ", ".join(fmt(r) for r in rows) if rows else fmt(None)
+        w(f"    {kind} {ctype} {pre}{ident}[{max(1, len(rows))}] = {{{body}}};")
+
+    def i4(r):
+        return "{%d, %d, %d, %d}" % tuple(r if r is not None else (0, 0, 0, 0))
+
+    def f4(r):
+        return "{%s}" % ", ".join(lit32(v) for v in (r if r is not None else (0.0, 0.0, 0.0, 0.0)))
+
+    # ---- tables
+    em0 = Emitter("cuda", SNAP32)
+    offs = []
+    for l, p, r in slots:
+        v = kin.sphere_in_frame(l, p)[1]
+        offs.append((em0.const(float(v[0])), em0.const(float(v[1])), em0.const(float(v[2])), r))
+    w("    // slot -> its centre's offset in its frame, and its radius")
+    table("__constant__", "float4", "SlotOff", offs, f4)
+    w("    // per staged frame and entry: its stage slot, or -1 and the constant value")
+    nfr = len(lay["slots"])
+    w(f"    __constant__ int {pre}FrameSlot[{nfr}][12] = {{{', '.join('{' + ', '.join(map(str, r)) + '}' for r in lay['slots'])}}};")
+    w(f"    __constant__ float {pre}FrameConst[{nfr}][12] = {{{', '.join('{' + ', '.join(lit32(v) for v in r) + '}' for r in lay['consts'])}}};")
+    env_rows, group_rows = [], []
+    for g, fid in enumerate(groups["frames"]):
+        first = len(env_rows)
+        for k, _, _ in members[g]:
+            e = model["env_checks"][k]
+            env_rows.append((coarse_slot[e["link"]], e["fine"][0], e["fine"][0] + len(e["fine"]), 0))
+        group_rows.append((lay["frames"][fid], first, len(env_rows), 0))
+    w("    // rigid link groups: staged frame, their environment checks; per check its coarse slot and")
+    w("    // fine slots")
+    table("__constant__", "int4", "Group", group_rows, i4)
+    table("__constant__", "int4", "Env", env_rows, i4)
+    pair_rows, check_a, check_b, check_box, contain, row_rows, row_b, row_box = [], [], [], [], [], [], [], []
+    full0 = [0]
     for e in model["self_checks"]:
-        A, B = _pairs_ab(e)
-        a0 = len(self_list)
-        self_list += A
-        b0 = len(self_list)
-        self_list += B
-        self_rows.append((coarse_slot[e["links"][0]], coarse_slot[e["links"][1]], a0, b0, len(A), len(B)))
-    if True:
-        pre = f"k{S}"
-        w(f"    // slot -> frame, and the slot's centre offset in that frame and radius")
-        w(f"    __constant__ int {pre}SlotFrame[{len(slots)}] = {{{', '.join(str(fidx[kin.sphere_in_frame(l, p)[0]]) for l, p, r in slots)}}};")
-        offs = []
-        em0 = Emitter("cuda", SNAP32)
-        for l, p, r in slots:
-            v = kin.sphere_in_frame(l, p)[1]
-            offs.append(f"{{{lit32(em0.const(float(v[0])))}, {lit32(em0.const(float(v[1])))}, {lit32(em0.const(float(v[2])))}, {lit32(r)}}}")
-        w(f"    __constant__ float4 {pre}SlotOff[{len(slots)}] = {{{', '.join(offs)}}};")
-        # tables of the table-driven form: only for the robots that compile that form (and
-        # only while VG_STAGED_ALL does not switch them to the staged form)
-        w(f"    __constant__ int {pre}EnvStart[{len(env_start)}] = {{{', '.join(map(str, env_start))}}};")
-        if tabled:
-            w("#ifndef VG_STAGED_ALL")
-            w(f"    __constant__ int {pre}EnvCoarse[{len(model['env_checks'])}] = {{{', '.join(str(coarse_slot[e['link']]) for e in model['env_checks'])}}};")
-            w("#endif")
-        w(f"    __constant__ int {pre}EnvFine[{len(env_fine)}] = {{{', '.join(map(str, env_fine))}}};")
-        if tabled:
-            w("#ifndef VG_STAGED_ALL")
-            w(f"    // per link pair: coarse slot A, coarse slot B, start of A's and B's fine lists, their sizes")
-            w(f"    __constant__ int4 {pre}SelfRow[{len(self_rows)}] = {{{', '.join('{%d, %d, %d, %d}' % r[:4] for r in self_rows)}}};")
-            w(f"    __constant__ int2 {pre}SelfLen[{len(self_rows)}] = {{{', '.join('{%d, %d}' % r[4:] for r in self_rows)}}};")
-            w(f"    __constant__ int {pre}SelfList[{len(self_list)}] = {{{', '.join(map(str, self_list))}}};")
-            env_of = {e["link"]: k for k, e in enumerate(model["env_checks"])}
-            w(f"    // per link pair: environment-check index of link A's and link B's coarse sphere")
-            w(f"    __constant__ int2 {pre}SelfEnvIdx[{len(self_rows)}] = {{{', '.join('{%d, %d}' % (env_of[e['links'][0]], env_of[e['links'][1]]) for e in model['self_checks'])}}};")
-            w("#endif")
-        cull = load_cull(name)
-        live_start, live_pairs = [0], []
-        for ci, e in enumerate(model["self_checks"]):
-            sel = range(len(e["fine"])) if cull is None or cull["live"][ci] is None else cull["live"][ci]
-            live_pairs += [tuple(e["fine"][pi]) for pi in sel]
-            live_start.append(len(live_pairs))
-        w(f"    // fine pairs that can collide inside the widened joint limits, per self check")
-        w(f"    __constant__ int {pre}LiveStart[{len(live_start)}] = {{{', '.join(map(str, live_start))}}};")
-        w(f"    __constant__ int2 {pre}LivePair[{max(1, len(live_pairs))}] = {{{', '.join('{%d, %d}' % p for p in live_pairs) or '{0, 0}'}}};")
-        all_pairs = [tuple(p_) for e in model["self_checks"] for p_ in e["fine"]]
-        w(f"    // every fine self pair, in the reference's order (debug reports; global memory)")
-        w(f"    __device__ const int2 {pre}AllPair[{max(1, len(all_pairs))}] = {{{', '.join('{%d, %d}' % p for p in all_pairs) or '{0, 0}'}}};")
-        arows, afine = attach_tables(model, coarse_slot)
-        w(f"    // links checked against an attachment (fkcc_attach): coarse slot, fine range; fine slots")
-        w(f"    __device__ const int4 {pre}AttachLink[{max(1, len(arows))}] = {{{', '.join('{%d, %d, %d, 0}' % r for r in arows) or '{0, 0, 0, 0}'}}};")
-        w(f"    __device__ const int {pre}AttachFine[{max(1, len(afine))}] = {{{', '.join(map(str, afine)) or '0'}}};")
-        # tables of the staged form: every robot's default except the table-driven ones
-        if tabled:
-            w("#ifdef VG_STAGED_ALL")
-        w(f"    __constant__ int2 {pre}FullPair[{max(1, len(all_pairs))}] = {{{', '.join('{%d, %d}' % p for p in all_pairs) or '{0, 0}'}}};")
-        if True:
-            lay = stage_layout(model, kin, load_cull(name))
-            nfr = len(lay["slots"])
-            env_frames = [lay["frames"][kin.sphere_in_frame(slots[e["fine"][0]][0], slots[e["fine"][0]][1])[0]]
-                          for e in model["env_checks"]]
-            w(f"    // staged frame of each environment check's fine spheres")
-            w(f"    __constant__ int {pre}EnvFrameS[{len(env_frames)}] = {{{', '.join(map(str, env_frames))}}};")
-            w(f"    // per staged frame and entry: its stage slot, or -1 and the constant value")
-            w(f"    __constant__ int {pre}FrameSlot[{nfr}][12] = {{{', '.join('{' + ', '.join(map(str, r)) + '}' for r in lay['slots'])}}};")
-            w(f"    __constant__ float {pre}FrameConst[{nfr}][12] = {{{', '.join('{' + ', '.join(lit32(v) for v in r) + '}' for r in lay['consts'])}}};")
-            env_ix = {e["link"]: k for k, e in enumerate(model["env_checks"])}
-            rows_a, rows_b = [], []
-            lvs, fls = 0, 0
-            cull1 = load_cull(name)
-            for ci, e in enumerate(model["self_checks"]):
-                A, B = _pairs_ab(e)
-                fa = kin.sphere_in_frame(slots[A[0]][0], slots[A[0]][1])[0]
-                fb = kin.sphere_in_frame(slots[B[0]][0], slots[B[0]][1])[0]
-                sel = range(len(e["fine"])) if cull1 is None or cull1["live"][ci] is None else cull1["live"][ci]
-                nl, nf = len(list(sel)), len(e["fine"])
-                rows_a.append((lay["coarse_pos"][env_ix[e["links"][0]]], lay["coarse_pos"][env_ix[e["links"][1]]],
-                               lay["frames"][fa], lay["frames"][fb]))
-                rows_b.append((lvs, lvs + nl, fls, fls + nf))
-                lvs += nl
-                fls += nf
-            w(f"    // self-check loop: staged coarse centre of link A and B, their staged frames;")
-            w(f"    // live pair range, full pair range")
-            w(f"    __constant__ int4 {pre}SelfA[{len(rows_a)}] = {{{', '.join('{%d, %d, %d, %d}' % r for r in rows_a)}}};")
-            w(f"    __constant__ int4 {pre}SelfB[{len(rows_b)}] = {{{', '.join('{%d, %d, %d, %d}' % r for r in rows_b)}}};")
-            w(f"    __constant__ float {pre}CoarseR[{len(lay['coarse'])}] = {{{', '.join(lit32(model['coarse_spheres'][model['env_checks'][k]['link']]['r']) for k in lay['coarse'])}}};")
-            w(f"    // per environment-check link: radius about its coarse centre that contains every fine sphere")
-            w(f"    // of the link with {CONTAIN_MARGIN} m to spare (exact geometry, rounded up to FP32)")
-            w(f"    __constant__ float {pre}ContainR[{len(model['env_checks'])}] = {{{', '.join(lit32(f32_up(containing_radius(model, kin, e) + CONTAIN_MARGIN)) for e in model['env_checks'])}}};")
-            cb_checks, cb_pairs = danger_boxes(model, cull1)
-            box = lambda b: "{%s}" % ", ".join(lit32(v) for v in b)  # noqa: E731
-            w(f"    // danger boxes (joint space, inside the widened limits): a live pair can come within the")
-            w(f"    // culling margin only for joint values inside its box; per self check the two joints and")
-            w(f"    // the union of its pairs' boxes (and where its live pairs' boxes start, -1: none), per")
-            w(f"    // live pair of an analysed check its box (lo0, hi0, lo1, hi1)")
+        full0.append(full0[-1] + len(e["fine"]))
+    for (ga, gb), cs in pairs.items():
+        first = len(check_a)
+        for c in cs:
+            e = model["self_checks"][c]
+            sel = range(len(e["fine"])) if cull is None or cull["live"][c] is None else cull["live"][c]
+            (j0, j1, box0), union = boxes_of[c]
+            r0 = len(row_rows)
+            last = None
+            for n_, i in enumerate(sel):
+                x, y = e["fine"][i]
+                if x != last:
+                    row_rows.append([x, len(row_b), len(row_b), 0])
+                    last = x
+                row_b.append(y)
+                row_rows[-1][2] = len(row_b)
+                row_box.append(box0 + n_ if box0 >= 0 else -1)
+            check_a.append((coarse_slot[e["links"][0]], coarse_slot[e["links"][1]], r0, len(row_rows)))
             jp = lay["joint_pos"]
-            w(f"    __constant__ int4 {pre}SelfJoint[{len(cb_checks)}] = {{{', '.join('{%d, %d, %d, 0}' % ((jp[c[0][0]], jp[c[0][1]], c[0][2]) if c[0][2] >= 0 else (0, 0, -1)) for c in cb_checks)}}};")
-            w(f"    __constant__ float4 {pre}SelfBox[{len(cb_checks)}] = {{{', '.join(box(c[1]) for c in cb_checks)}}};")
-            w(f"    __constant__ float4 {pre}LiveBox[{max(1, len(cb_pairs))}] = {{{', '.join(box(p_) for p_ in cb_pairs) or box((0, 0, 0, 0))}}};")
-        if tabled:
-            w("#endif")
-        w("")
+            check_b.append((full0[c], full0[c + 1], jp[j0] if box0 >= 0 else -1, jp[j1] if box0 >= 0 else -1))
+            check_box.append(union)
+            contain.append(f32_up(containing_radius(model, kin, model["env_checks"][groups["env_ix"][e["links"][1]]]) + CONTAIN_MARGIN))
+        fa, fb = groups["frames"][ga], groups["frames"][gb]
+        pair_rows.append((lay["frames"][fa], lay["frames"][fb], first, len(check_a)))
+    w("    // pairs of link groups: staged frames A and B, their self checks")
+    table("__constant__", "int4", "Pair", pair_rows, i4)
+    w("    // per self check: coarse slots A and B, its rows of live fine pairs (those that can collide")
+    w("    // inside the widened joint limits); all its fine pairs and, where its danger boxes were")
+    w("    // found, the staged joints they test (-1: none)")
+    table("__constant__", "int4", "CheckA", check_a, i4)
+    table("__constant__", "int4", "CheckB", check_b, i4)
+    w("    // per self check the union of its live pairs' danger boxes (lo0, hi0, lo1, hi1), joint-space")
+    w("    // boxes outside which a live pair keeps the culling margin, and the radius about B's coarse")
+    w(f"    // centre that contains B's fine spheres with {CONTAIN_MARGIN} m to spare")
+    table("__constant__", "float4", "CheckBox", check_box, f4)
+    w(f"    __constant__ float {pre}ContainR[{len(contain)}] = {{{', '.join(lit32(v) for v in contain)}}};")
+    w("    // rows: a fine slot of A, its live pairs' range; per live pair the fine slot of B, and the box")
+    table("__constant__", "int4", "Row", row_rows, i4)
+    w(f"    __constant__ int {pre}RowB[{max(1, len(row_b))}] = {{{', '.join(map(str, row_b)) or '0'}}};")
+    if live_boxes:
+        boxed = [live_boxes[i] if i >= 0 else (-BIG, BIG, -BIG, BIG) for i in row_box]
+        table("__constant__", "float4", "RowBox", boxed, f4)
+    w("    // every fine self pair, in the reference's order (debug reports, and configurations outside")
+    w("    // the widened joint limits; global memory)")
+    w(f"    __device__ const int2 {pre}AllPair[{max(1, len(all_pairs))}] = {{{', '.join('{%d, %d}' % p for p in all_pairs) or '{0, 0}'}}};")
+    arows, afine = attach_tables(model, coarse_slot)
+    w("    // links checked against an attachment (fkcc_attach): coarse slot, fine range; fine slots")
+    w(f"    __device__ const int4 {pre}AttachLink[{max(1, len(arows))}] = {{{', '.join('{%d, %d, %d, 0}' % r for r in arows) or '{0, 0, 0, 0}'}}};")
+    w(f"    __device__ const int {pre}AttachFine[{max(1, len(afine))}] = {{{', '.join(map(str, afine)) or '0'}}};")
+    w("")
 
     w("struct %s" % S)
     w("{")
@@ -711,20 +731,13 @@ def gen_cuda(model: dict) -> str:
     w("    static constexpr int kDim = %d;" % dim)
     w("    static constexpr int kFine = %d;" % len(model["fine_spheres"]))
     w("    static constexpr int kSlots = %d;" % len(slots))
-    w("    static constexpr int kFrames = %d;" % (len(kin.frames) + 1))
-    w("    static constexpr int kEnvChecks = %d;" % len(model["env_checks"]))
-    w("    static constexpr int kSelfPairs = %d;" % sum(len(e["fine"]) for e in model["self_checks"]))
-    w("    static __device__ __forceinline__ int2 self_pair(int i) { return k%sAllPair[i]; }" % S)
-    lay = stage_layout(model, kin, load_cull(name))
-    w("    // floats of shared-memory staging per thread (non-constant entries of the fine checks' frames)")
-    if tabled:
-        w("#ifndef VG_STAGED_ALL")
-        w("    static constexpr int kStage = 0;")
-        w("#else")
-    w("    // and the coarse centres the self-check loop reads and the joint values its danger boxes test")
+    w("    static constexpr int kSelfPairs = %d;" % len(all_pairs))
+    w(f"    static __device__ __forceinline__ int2 self_pair(int i) {{ return {pre}AllPair[i]; }}")
+    w("    // floats of shared-memory staging per thread: the non-constant entries of the checks' frames")
+    w("    // and the joint values the danger boxes test")
     w("    static constexpr int kStage = %d;" % lay["total"])
-    if tabled:
-        w("#endif")
+    w("    // resident blocks per SM of the same-edge kernels")
+    w("    static constexpr int kEdgeBlocks = %d;" % EDGE_BLOCKS[name])
     w("    static constexpr int kResolution = %d;" % model["resolution"])
     w("    static constexpr float kMinRadius = %s;" % lit32(model["min_radius"]))
     w("    static constexpr float kMaxRadius = %s;" % lit32(model["max_radius"]))
@@ -760,280 +773,155 @@ def gen_cuda(model: dict) -> str:
     for l in body:
         w("        " + l)
     w("    }")
-    rows, afine = attach_tables(model, coarse_slot)
     w("    // links checked against an attachment, in the reference's order: coarse slot, fine range")
-    w(f"    static constexpr int kAttachLinks = {len(rows)};")
+    w(f"    static constexpr int kAttachLinks = {len(arows)};")
     w(f"    static __device__ __forceinline__ int4 attach_link(int i) {{ return k{S}AttachLink[i]; }}")
     w(f"    static __device__ __forceinline__ int attach_fine(int i) {{ return k{S}AttachFine[i]; }}")
     w("")
 
-    if tabled:
-        w("#ifndef VG_STAGED_ALL")
-        em = Emitter("cuda", SNAP32)
-        fr = frames_block(em)
-        body = list(em.lines)
-        for i, vals in enumerate(frame_values(kin, fr)):
-            body.append(" ".join(f"F[{12 * i + j}] = {em.ref(v)};" for j, v in enumerate(vals)))
-        w("    // Frames (root first): R row-major then t, 12 floats each.")
-        w("    static __device__ __forceinline__ void frames(const float *q, float *F)")
-        w("    {")
-        for l in body:
-            w("        " + l)
-        w("    }")
-        w("")
-        pre = f"k{S}"
-        w(f"""    static __device__ __forceinline__ float4 centre(const float *F, int slot)
-    {{
-        const float *f = F + 12 * {pre}SlotFrame[slot];
-        const float4 o = {pre}SlotOff[slot];
-        float c[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-        {{
-            float acc = f[9 + r];
-            acc = __fmaf_rn(f[3 * r + 0], o.x, acc);
-            acc = __fmaf_rn(f[3 * r + 1], o.y, acc);
-            acc = __fmaf_rn(f[3 * r + 2], o.z, acc);
-            c[r] = acc;
-        }}
-        return make_float4(c[0], c[1], c[2], o.w);
-    }}
-
-    // Robot::fkcc for the lanes of ctx.alive.  Clears the lanes of every segment found in collision.
-    template <typename Ctx>
-    static __device__ __forceinline__ void fkcc(const float *q, Ctx &ctx)
-    {{
-        float F[kFrames * 12];
-        frames(q, F);
-{chr(10).join("        " + l for l in limits_code(model, load_cull(name)))}
-        // coarse centres, computed once (the self loop reads them for every link pair), and the
-        // segments where each may touch anything, four lookups in flight at a time
-        float4 CC[{len(model['env_checks'])}];
-        unsigned *const near = ctx.wsc;
-#pragma unroll 1
-        for (int c0 = 0; c0 < {len(model['env_checks'])}; c0 += {TABLE_NEAR})
-        {{
-            float4 k[{TABLE_NEAR}];
-            unsigned clear[{TABLE_NEAR}];
-#pragma unroll
-            for (int j = 0; j < {TABLE_NEAR}; ++j)
-            {{
-                const int c = {"c0 + j" if len(model['env_checks']) % TABLE_NEAR == 0 else f"min(c0 + j, {len(model['env_checks']) - 1})"};
-                k[j] = centre(F, {pre}EnvCoarse[c]);
-                CC[c] = k[j];
-                clear[j] = ctx.clearance(k[j].x, k[j].y, k[j].z);
-            }}
-#pragma unroll
-            for (int j = 0; j < {TABLE_NEAR}; ++j)
-            {{
-                const unsigned m = ctx.vote_near(clear[j] < vg::field_reach(k[j].w), ctx.alive);
-                if ((threadIdx.x & 31) == 0)
-                {{
-                    near[c0 + j] = m;
-                }}
-            }}
-        }}
-        __syncwarp();
-#pragma unroll 1
-        for (int c = 0; c < {len(model['env_checks'])}; ++c)
-        {{
-            unsigned need = near[c] & ctx.alive;
-            if (!need)
-            {{
-                continue;
-            }}
-            const float4 k = CC[c];
-            need = ctx.env_hit(k.x, k.y, k.z, k.w, need);
-#pragma unroll 1
-            for (int i = {pre}EnvStart[c]; need && i < {pre}EnvStart[c + 1]; ++i)
-            {{
-                const float4 s = centre(F, {pre}EnvFine[i]);
-                const unsigned may = ctx.near(s, need);
-                if (!may)
-                {{
-                    continue;
-                }}
-                const unsigned hit = ctx.env_hit(s.x, s.y, s.z, s.w, may);
-                need &= ~hit;
-                if (hit && !ctx.kill(hit))
-                {{
-                    return;
-                }}
-            }}
-        }}
-#pragma unroll 1
-        for (int c = 0; c < {len(self_rows)}; ++c)
-        {{
-            const int4 row = {pre}SelfRow[c];
-            const int2 ce = {pre}SelfEnvIdx[c];
-            const float4 a = CC[ce.x], b = CC[ce.y];
-            unsigned need = ctx.self_hit(a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, ctx.alive);
-            if (!need)
-            {{
-                continue;
-            }}
-            unsigned acc = 0u;
-            if (ctx.in_limits)
-            {{
-#pragma unroll 1
-                for (int k = {pre}LiveStart[c]; k < {pre}LiveStart[c + 1]; ++k)
-                {{
-                    const int2 pr = {pre}LivePair[k];
-                    const float4 sa = centre(F, pr.x), sb = centre(F, pr.y);
-                    acc |= vg::self_bits(sa.x, sa.y, sa.z, sb.x, sb.y, sb.z, __fadd_rn(sa.w, sb.w));
-                }}
-            }}
-            else
-            {{
-                const int2 len = {pre}SelfLen[c];
-#pragma unroll 1
-                for (int i = 0; i < len.x; ++i)
-                {{
-                    const float4 sa = centre(F, {pre}SelfList[row.z + i]);
-#pragma unroll 1
-                    for (int j = 0; j < len.y; ++j)
-                    {{
-                        const float4 sb = centre(F, {pre}SelfList[row.w + j]);
-                        acc |= vg::self_bits(sa.x, sa.y, sa.z, sb.x, sb.y, sb.z, __fadd_rn(sa.w, sb.w));
-                    }}
-                }}
-            }}
-            const unsigned hit = ctx.vote(acc, need);
-            if (hit && !ctx.kill(hit))
-            {{
-                return;
-            }}
-        }}
-    }}""")
-        w("#else")
-
-
-    # ---- staged schedule.  The frames the fine checks need, the coarse centres and the joint
-    # values the danger boxes test are written to shared memory once, and the environment and
-    # self-collision sections are loops over constant tables that read them from there (small code
-    # for the instruction cache, few live registers).
-    pre = f"k{S}"
-    cull = load_cull(name)
+    # ---- fkcc.  Straight-line: the kinematics, the frames to the shared-memory stage, one sphere
+    # per link group, the groups' field lookups and the group pairs' tests into per-lane bit words
+    # (independent operations, no votes).  Then loops over the set bits of the words' warp-wide OR.
+    # What bounds it is latency: the loop over every link pair that this replaces was a chain of
+    # table loads, shared-memory loads and a vote per pair, 60 % of the edge check once the field
+    # had taken most environment queries out.  65,536 Panda motions 1.70 -> 0.69 ms, 9,973 UR5
+    # vectors 0.23 -> 0.13, four robots' graph 5.36 -> 3.37 (the smaller stage, 33 instead of 53 KB
+    # a block for the Panda, and five resident blocks instead of four included).
     em = Emitter("cuda", SNAP32)
     fr = frames_block(em)
-    head = list(em.lines)
-    head += limits_code(model, cull)
-    fvals = frame_values(kin, fr)
-    sid = lay["frames"]
-
-    n_env = len(model["env_checks"])
-    def centre(i, tag):
-        em.lines = []
-        link, p, r = slots[i]
-        x, y, z = emit_centre(em, fr, kin, link, p, f"{tag}{i}_")
-        return list(em.lines), (x, y, z, lit32(r))
-
-    # coarse spheres of every environment-checked link: queried together, reused by self checks
-    coarse = [f"float4 cs[{n_env}];"]
-    for k, e in enumerate(model["env_checks"]):
-        ls, (x, y, z, r) = centre(coarse_slot[e["link"]], "c")
-        coarse.append("{")
-        coarse += ["    " + l for l in ls]
-        coarse.append(f"    cs[{k}] = make_float4({x}, {y}, {z}, {r});  // {e['link']}")
-        coarse.append("}")
-    stage = []
+    body = list(em.lines)
+    body += limits_code(model, cull)
+    body.append("float *const st = ctx.stage;")
     vals_ = [f"(-{v[1:]})" if v.startswith("-") else v for v in lay["values"]]
     for i in range(0, len(vals_), 6):
-        stage.append(" ".join(f"st[{j} * vg::kStageStride] = {vals_[j]};" for j in range(i, min(i + 6, len(vals_)))))
-
-    c0 = lay["coarse0"]
-    coarse_stage = [" ".join(f"st[{c0 + 3 * i + j} * vg::kStageStride] = cs[{k}].{'xyz'[j]};" for j in range(3))
-                    for i, k in enumerate(lay["coarse"])]
-    qb = lay["q0"]
-    q_stage = [" ".join(f"st[{qb + i} * vg::kStageStride] = q[{d}];" for i, d in enumerate(lay["joints"]))]
-    self_loop = f"""#pragma unroll 1
-for (int c = 0; c < {len(model['self_checks'])}; ++c)
-{{
-    const int4 t = {pre}SelfA[c];
-    const float *ca = st + ({c0} + 3 * t.x) * vg::kStageStride;
-    const float *cb = st + ({c0} + 3 * t.y) * vg::kStageStride;
-    const unsigned need = ctx.self_hit(ca[0], ca[vg::kStageStride], ca[2 * vg::kStageStride], {pre}CoarseR[t.x],
-                                       cb[0], cb[vg::kStageStride], cb[2 * vg::kStageStride], {pre}CoarseR[t.y], ctx.alive);
-    if (need)
-    {{
-        const int4 u = {pre}SelfB[c];
-        const float4 cbc = make_float4(cb[0], cb[vg::kStageStride], cb[2 * vg::kStageStride], {pre}ContainR[t.y]);
-        unsigned acc = 0u;
-        if (ctx.in_limits)
-        {{
-            // live pairs only, and only while some lane's joints lie in the check's danger box
-            const int4 jj = {pre}SelfJoint[c];
-            const float4 bx = {pre}SelfBox[c];
-            const float qa = st[({qb} + jj.x) * vg::kStageStride], qb = st[({qb} + jj.y) * vg::kStageStride];
-            const bool in = (qa >= bx.x) & (qa <= bx.y) & (qb >= bx.z) & (qb <= bx.w);
-            if (__any_sync(vg::kFull, in))
-            {{
-                acc = self_pairs_boxed(st, t.z, t.w, u.x, u.y, jj.z, qa, qb, cbc);
-            }}
-        }}
-        else
-        {{
-            acc = self_pairs(st, t.z, t.w, {pre}FullPair, u.z, u.w, cbc);
-        }}
-        const unsigned hit = ctx.vote(acc, need);
-        if (hit && !ctx.kill(hit)) return;
-    }}
-}}""".split("\n")
-    lb = COARSE_BATCH
-    env_loops = f"""// the segments where each coarse sphere may touch anything; a bit per sphere that has any
-unsigned *const chs = ctx.wsc;
-auto todo = ctx.template near_all<{n_env}>(cs, chs);
-// those spheres' exact queries, {lb} at a time (one copy of the batched query)
-decltype(todo) hits = 0;
+        body.append(" ".join(f"st[{j} * vg::kStageStride] = {vals_[j]};" for j in range(i, min(i + 6, len(vals_)))))
+    for i, d in enumerate(lay["joints"]):
+        body.append(f"st[{lay['q0'] + i} * vg::kStageStride] = q[{d}];")
+    group_sphere = []
+    for g, fid in enumerate(groups["frames"]):
+        names = ", ".join(model["env_checks"][k]["link"] for k, _, _ in members[g])
+        body.append(f"// group {g}: {names}")
+        em.lines = []
+        if len(members[g]) == 1:
+            link, p, r = slots[coarse_slot[model["env_checks"][members[g][0][0]]["link"]]]
+            xyz = emit_centre(em, fr, kin, link, p, f"g{g}_")
+        else:
+            c, r = enclosing_sphere([(tuple(off), rad) for _, off, rad in members[g]])
+            xyz = emit_point(em, fr[fid], c, f"g{g}_")
+        body += em.lines
+        group_sphere.append((xyz, float(r)))
+        body.append(f"const unsigned v{g} = ctx.clearance({', '.join(xyz)});")
+    em.lines = []
+    body.append("// per lane: the pairs of groups that overlap, and those whose joints lie in a danger box")
+    plist = list(pairs)
+    n_words = -(-len(plist) // 32)
+    for wd in range(n_words):
+        part = plist[32 * wd:32 * wd + 32]
+        body.append(f"unsigned over{wd} = 0u;")
+        gate = []
+        for j, (ga, gb) in enumerate(part):
+            (A, ra), (B, rb) = group_sphere[ga], group_sphere[gb]
+            # the reference's own coarse test where both groups are single links, else one that
+            # contains it
+            body.append(f"over{wd} = vg::shift_in(over{wd}, vg::self_bits({', '.join(A)}, {', '.join(B)}, "
+                        f"__fadd_rn({lit32(ra)}, {lit32(rb)})));")
+            if all(boxes_of[c][0][2] >= 0 for c in pairs[(ga, gb)]):
+                gate.append((len(part) - 1 - j, [boxes_of[c] for c in pairs[(ga, gb)]]))
+        body.append(f"unsigned boxed{wd} = ~0u;")
+        if gate:
+            body.append("if (ctx.in_limits)")
+            body.append("{")
+            for bit, bs in gate:
+                cond = " | ".join("((q[%d] >= %s) & (q[%d] <= %s) & (q[%d] >= %s) & (q[%d] <= %s))" % (
+                    b[0][0], lit32(b[1][0]), b[0][0], lit32(b[1][1]), b[0][1], lit32(b[1][2]), b[0][1], lit32(b[1][3])) for b in bs)
+                body.append(f"    boxed{wd} &= {cond} ? ~0u : ~{1 << bit}u;")
+            body.append("}")
+    body.append("// per lane: the groups that may touch something")
+    body.append("unsigned near = 0u;")
+    for g in range(n_groups):
+        body.append(f"near = vg::shift_in(near, v{g} - vg::field_reach({lit32(group_sphere[g][1])}));")
+    body.append("const unsigned on = (ctx.alive >> (threadIdx.x & 31)) & 1u ? ~0u : 0u;")
+    body += f"""// environment checks of those groups
+unsigned todo = __reduce_or_sync(vg::kFull, near & on);
 #pragma unroll 1
 while (todo)
 {{
-    float4 sp[{lb}];
-    unsigned need[{lb}], h[{lb}];
-    int id[{lb}];
-#pragma unroll
-    for (int s = 0; s < {lb}; ++s)
+    const int bit = 31 - __clz(static_cast<int>(todo));
+    todo ^= 1u << bit;
+    const unsigned m = ctx.vote_near((near >> bit) & 1u, ctx.alive);
+    if (!m)
     {{
-        const int k = vg::lowest_bit(todo);
-        id[s] = k;
-        todo &= todo - 1;
-        // padding sphere: far away with radius -inf, it is never tested and never hits
-        sp[s] = k >= 0 ? make_float4(st[({c0} + 3 * k) * vg::kStageStride], st[({c0} + 3 * k + 1) * vg::kStageStride],
-                                     st[({c0} + 3 * k + 2) * vg::kStageStride], {pre}CoarseR[k])
-                       : make_float4(1.0e10f, 0.0f, 0.0f, -__int_as_float(0x7f800000));
-        need[s] = k >= 0 ? chs[k] : 0u;
+        continue;
     }}
-    ctx.template env_many<{lb}>(sp, need, h);
-#pragma unroll
-    for (int s = 0; s < {lb}; ++s)
+    const int4 g = {pre}Group[{n_groups - 1} - bit];
+    const vg::Frame f = frame_at(st, g.x);
+#pragma unroll 1
+    for (int k = g.y; k < g.z; ++k)
     {{
-        if (h[s])
+        // the coarse sphere, then (where it hit) the fine ones: one copy of the query
+        const int4 e = {pre}Env[k];
+        unsigned need = m & ctx.alive;
+        int next = e.y;
+        bool coarse = true;
+#pragma unroll 1
+        for (int slot = e.x;; slot = next++)
         {{
-            hits |= decltype(hits)(1) << id[s];
-            if ((threadIdx.x & 31) == 0)
+            const float4 c = vg::frame_point(f, {pre}SlotOff[slot]);
+            const unsigned may = ctx.near(c, need);
+            const unsigned hit = may ? ctx.env_hit(c.x, c.y, c.z, c.w, may) : 0u;
+            if (coarse)
             {{
-                chs[id[s]] = h[s];  // warp-uniform
+                need = hit;
+                coarse = false;
+            }}
+            else if (hit)
+            {{
+                if (!ctx.kill(hit))
+                {{
+                    return;
+                }}
+                need &= ctx.alive;
+            }}
+            if (!need || next >= e.z)
+            {{
+                break;
             }}
         }}
     }}
-}}
-__syncwarp();
-// fine spheres of the links whose coarse sphere hit
-#pragma unroll 1
-while (hits)
-{{
-    const int k = vg::lowest_bit(hits);
-    hits &= hits - 1;
-    const unsigned need = chs[k] & ctx.alive;
-    if (need)
-    {{
-        const unsigned hit = env_fine<Ctx::kW, Ctx::kExt>(ctx, st, {pre}EnvFrameS[k], {pre}EnvStart[k], {pre}EnvStart[k + 1], need);
-        if (hit && !ctx.kill(hit)) return;
-    }}
 }}""".split("\n")
-    staged_body = (head + ["float *const st = ctx.stage;"] + stage + q_stage + coarse + coarse_stage + env_loops
-                   + ["// self-collision link pairs, in the reference's order"] + self_loop)
-
+    for wd in range(n_words):
+        part = plist[32 * wd:32 * wd + 32]
+        body += f"""// self checks of the group pairs that overlap
+if (!self_checks(ctx, st, over{wd}, boxed{wd}, on, {32 * wd + len(part) - 1}))
+{{
+    return;
+}}""".split("\n")
+    box_gate = box_row = ""
+    if live_boxes:
+        box_gate = f"""
+                const int4 cb4 = {pre}CheckB[k];
+                float qa = 0.0f, qb = 0.0f;
+                if (cb4.z >= 0)
+                {{
+                    // only while some lane's joints lie in the check's danger box
+                    const float4 bx = {pre}CheckBox[k];
+                    qa = st[({lay['q0']} + cb4.z) * vg::kStageStride];
+                    qb = st[({lay['q0']} + cb4.w) * vg::kStageStride];
+                    const bool in = (qa >= bx.x) & (qa <= bx.y) & (qb >= bx.z) & (qb <= bx.w);
+                    if (!(__ballot_sync(vg::kFull, in) & need))
+                    {{
+                        continue;
+                    }}
+                }}"""
+        box_row = f"""
+                        if (cb4.z >= 0)
+                        {{
+                            const float4 bx = {pre}RowBox[i];
+                            if (!__any_sync(vg::kFull, (qa >= bx.x) & (qa <= bx.y) & (qb >= bx.z) & (qb <= bx.w)))
+                            {{
+                                continue;
+                            }}
+                        }}"""
     w(f"""    // Staged frame f: its non-constant entries from this thread's stage, the rest constants.
     static __device__ __forceinline__ vg::Frame frame_at(const float *st, int f)
     {{
@@ -1047,123 +935,92 @@ while (hits)
         return r;
     }}
 
-    // Fine environment tests of the spheres EnvFine[k0..k1) of staged frame f, for the segments
-    // in `need`: the segments whose block collides.
-    template <int W, bool kExt, typename Ctx>
-    static __device__ __forceinline__ unsigned env_fine(Ctx &ctx, const float *st, int f, int k0, int k1, unsigned need)
+    // Self checks of the group pairs last, last - 1, ... whose bit (0, 1, ...) is set in some
+    // lane's word `over` and in some lane's word `boxed`; `on`: all bits in the lanes checked.
+    // Each pair's checks run the reference's coarse test; where it overlaps, each fine sphere of A
+    // against B's containing sphere (every fine sphere of B lies inside it with CONTAIN_MARGIN to
+    // spare), and only rows that may touch it against B's spheres.  False once no segment is left.
+    template <typename Ctx>
+    static __device__ __forceinline__ bool self_checks(Ctx &ctx, const float *st, unsigned over, unsigned boxed, unsigned on, int last)
     {{
-        const vg::Frame fr = frame_at(st, f);
-        unsigned dead = 0u;
+        const int lane = threadIdx.x & 31;
+        unsigned todo = __reduce_or_sync(vg::kFull, over & on) & __reduce_or_sync(vg::kFull, boxed & on);
 #pragma unroll 1
-        for (int k = k0; k < k1; ++k)
+        while (todo)
         {{
-            const float4 o = {pre}SlotOff[{pre}EnvFine[k]];
-            const float4 c = vg::frame_point(fr, o);
-            const unsigned may = ctx.near(c, need);
-            if (!may)
+            const int bit = 31 - __clz(static_cast<int>(todo));
+            todo ^= 1u << bit;
+            const unsigned some = ctx.vote_near((over >> bit) & 1u, ctx.alive) & ctx.vote_near((boxed >> bit) & 1u, ctx.alive);
+            if (!some)
             {{
                 continue;
             }}
-            const unsigned hit = ctx.env_hit(c.x, c.y, c.z, c.w, may);
-            dead |= hit;
-            need &= ~hit;
-            if (!need)
-            {{
-                break;
-            }}
-        }}
-        return dead;
-    }}
-
-    // OR of the sign bits of the fine self-collision tests of pairs[k0..k1) (slot ids), the first
-    // slot of each pair in staged frame fa, the second in staged frame fb.
-    // A's fine sphere ca against B's containing sphere cbc (every fine sphere of B lies inside it
-    // with CONTAIN margin to spare): whether any lane's sphere may touch one of B's fine spheres.
-    // Where no lane's does, the pair tests of this sphere have clear sign bits and are skipped.
-    static __device__ __forceinline__ bool row_may_hit(const float4 ca, const float4 cbc)
-    {{
-        const float dx = __fsub_rn(ca.x, cbc.x), dy = __fsub_rn(ca.y, cbc.y), dz = __fsub_rn(ca.z, cbc.z);
-        const float rr = __fadd_rn(ca.w, cbc.w);
-        return __any_sync(vg::kFull, __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))) < __fmul_rn(rr, rr));
-    }}
-
-    static __device__ __noinline__ unsigned self_pairs(const float *st, int fa, int fb, const int2 *pairs, int k0, int k1,
-                                                       float4 cbc)
-    {{
-        const vg::Frame a = frame_at(st, fa), b = frame_at(st, fb);
-        unsigned acc = 0u;
-        int last = -1;
-        bool row = false;
-        float4 ca = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const int4 p = {pre}Pair[last - bit];
+            const vg::Frame a = frame_at(st, p.x), b = frame_at(st, p.y);
 #pragma unroll 1
-        for (int k = k0; k < k1; ++k)
-        {{
-            const int2 pr = pairs[k];
-            if (pr.x != last)
+            for (int k = p.z; k < p.w; ++k)
             {{
-                ca = vg::frame_point(a, {pre}SlotOff[pr.x]);
-                last = pr.x;
-                row = row_may_hit(ca, cbc);
-            }}
-            if (!row)
-            {{
-                continue;
-            }}
-            const float4 cb = vg::frame_point(b, {pre}SlotOff[pr.y]);
-            acc |= vg::self_bits(ca.x, ca.y, ca.z, cb.x, cb.y, cb.z, __fadd_rn(ca.w, cb.w));
-        }}
-        return acc;
-    }}
-
-    // The same over the live pairs LivePair[k0..k1), skipping a pair when no lane's joint values
-    // (qa, qb: the check's two joints) lie in its danger box LiveBox[box0 + k - k0] (box0 < 0:
-    // the check has no boxes): outside it the pair keeps the culling margin, so its test value
-    // cannot be negative.  Warp-uniform; all 32 lanes call.
-    static __device__ __noinline__ unsigned self_pairs_boxed(const float *st, int fa, int fb, int k0, int k1, int box0,
-                                                             float qa, float qb, float4 cbc)
-    {{
-        const vg::Frame a = frame_at(st, fa), b = frame_at(st, fb);
-        unsigned acc = 0u;
-        int last = -1;
-        bool row = false;
-        float4 ca = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 1
-        for (int k = k0; k < k1; ++k)
-        {{
-            if (box0 >= 0)
-            {{
-                const float4 bx = {pre}LiveBox[box0 + k - k0];
-                if (!__any_sync(vg::kFull, (qa >= bx.x) & (qa <= bx.y) & (qb >= bx.z) & (qb <= bx.w)))
+                const int4 ck = {pre}CheckA[k];
+                const float4 ca = vg::frame_point(a, {pre}SlotOff[ck.x]);
+                float4 cb = vg::frame_point(b, {pre}SlotOff[ck.y]);
+                const unsigned need = ctx.self_hit(ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w, some & ctx.alive);
+                if (!need)
                 {{
                     continue;
                 }}
+                unsigned acc = 0u;
+                if (!ctx.in_limits)
+                {{
+                    const int4 all = {pre}CheckB[k];
+#pragma unroll 1
+                    for (int i = all.x; i < all.y; ++i)
+                    {{
+                        const int2 pr = {pre}AllPair[i];
+                        const float4 sa = vg::frame_point(a, {pre}SlotOff[pr.x]), sb = vg::frame_point(b, {pre}SlotOff[pr.y]);
+                        acc |= vg::self_bits(sa.x, sa.y, sa.z, sb.x, sb.y, sb.z, __fadd_rn(sa.w, sb.w));
+                    }}
+                    const unsigned hit = ctx.vote(acc, need);
+                    if (hit && !ctx.kill(hit))
+                    {{
+                        return false;
+                    }}
+                    continue;
+                }}{box_gate}
+                cb.w = {pre}ContainR[k];
+                const bool mine = (need >> lane) & 1u;
+#pragma unroll 1
+                for (int r = ck.z; r < ck.w; ++r)
+                {{
+                    const int4 row = {pre}Row[r];
+                    const float4 sa = vg::frame_point(a, {pre}SlotOff[row.x]);
+                    if (!__any_sync(vg::kFull, mine && vg::spheres_meet(sa, cb)))
+                    {{
+                        continue;
+                    }}
+#pragma unroll 1
+                    for (int i = row.y; i < row.z; ++i)
+                    {{{box_row}
+                        const float4 sb = vg::frame_point(b, {pre}SlotOff[{pre}RowB[i]]);
+                        acc |= vg::self_bits(sa.x, sa.y, sa.z, sb.x, sb.y, sb.z, __fadd_rn(sa.w, sb.w));
+                    }}
+                }}
+                const unsigned hit = ctx.vote(acc, need);
+                if (hit && !ctx.kill(hit))
+                {{
+                    return false;
+                }}
             }}
-            const int2 pr = {pre}LivePair[k];
-            if (pr.x != last)
-            {{
-                ca = vg::frame_point(a, {pre}SlotOff[pr.x]);
-                last = pr.x;
-                row = row_may_hit(ca, cbc);
-            }}
-            if (!row)
-            {{
-                continue;
-            }}
-            const float4 cb = vg::frame_point(b, {pre}SlotOff[pr.y]);
-            acc |= vg::self_bits(ca.x, ca.y, ca.z, cb.x, cb.y, cb.z, __fadd_rn(ca.w, cb.w));
         }}
-        return acc;
+        return true;
     }}
 """)
     w("    // Robot::fkcc for the lanes of ctx.alive.  Clears the lanes of every segment found in collision.")
     w("    template <typename Ctx>")
     w("    static __device__ __forceinline__ void fkcc(const float *q, Ctx &ctx)")
     w("    {")
-    for l in staged_body:
+    for l in body:
         w("        " + l)
     w("    }")
-    if tabled:
-        w("#endif  // VG_STAGED_ALL")
     w("};")
     w("}  // namespace vg::robots")
     return "\n".join(lines) + "\n"
