@@ -190,7 +190,8 @@ extern "C" int vg_gemm_bf16_device(const void *a, const void *b, float *d, int M
 // =============================================================================================
 // The MLP: features (sin, cos of each joint, zero-padded to a multiple of 16) -> 256 -> 256 -> 1
 // with ReLU, BF16 weights and activations, FP32 accumulation and FP32 master weights (Adam).
-// The forward and backward GEMMs run on gemm_bf16_kernel; small reductions on CUDA cores.
+// Training runs mlp_rows_kernel and mlp_weights_kernel (vg_mlp_train.cuh), inference
+// mlp_infer_kernel; vg_mlp_predict_device runs the layers one by one on gemm_bf16_kernel.
 
 namespace vg
 {
@@ -211,28 +212,8 @@ namespace vg
         x[i] = __float2bfloat16_rn(v);
     }
 
-    // out[c][r] = in[r][c] for a [R][C] bf16 matrix
-    __global__ void transpose_kernel(const __nv_bfloat16 *in, __nv_bfloat16 *out, int R, int C)
-    {
-        __shared__ __nv_bfloat16 tile[32][33];
-        const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-        for (int k = threadIdx.y; k < 32; k += blockDim.y)
-        {
-            const int r = r0 + k, c = c0 + threadIdx.x;
-            if (r < R && c < C)
-                tile[k][threadIdx.x] = in[static_cast<size_t>(r) * C + c];
-        }
-        __syncthreads();
-        for (int k = threadIdx.y; k < 32; k += blockDim.y)
-        {
-            const int c = c0 + k, r = r0 + threadIdx.x;
-            if (r < R && c < C)
-                out[static_cast<size_t>(c) * R + r] = tile[threadIdx.x][k];
-        }
-    }
-
-    // z = H2 w3 + b3, p = sigmoid(z): one warp per row
-    __global__ void head_kernel(const __nv_bfloat16 *h2, const float *w3, const float *b3, int rows, float *z, float *p)
+    // p = sigmoid(H2 w3 + b3): one warp per row
+    __global__ void head_kernel(const __nv_bfloat16 *h2, const float *w3, const float *b3, int rows, float *p)
     {
         const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
         const int lane = threadIdx.x & 31;
@@ -246,106 +227,34 @@ namespace vg
         if (lane == 0)
         {
             const float zz = acc + b3[0];
-            if (z)
-                z[row] = zz;
             p[row] = 1.0f / (1.0f + expf(-zz));
         }
     }
 
-    // Binary cross-entropy on the logit: dz = (p - y) / n (rows >= n contribute nothing);
-    // dH2 = dz w3 masked by H2 > 0 (bf16); loss accumulated into *loss.
-    __global__ void head_backward_kernel(const __nv_bfloat16 *h2, const float *w3, const float *p, const float *z,
-                                         const uint8_t *valid, int n, int rows, float *dz, __nv_bfloat16 *dh2, float *loss)
-    {
-        const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-        const int lane = threadIdx.x & 31;
-        if (row >= rows)
-            return;
-        float g = 0.0f;
-        if (row < n)
-        {
-            const float y = valid[row] ? 0.0f : 1.0f;  // label: 1 = in collision
-            g = (p[row] - y) / static_cast<float>(n);
-            if (lane == 0)
-            {
-                const float zz = z[row];
-                // log(1 + exp(z)) - y z, evaluated stably
-                const float l = fmaxf(zz, 0.0f) - zz * y + log1pf(expf(-fabsf(zz)));
-                atomicAdd(loss, l / static_cast<float>(n));
-            }
-        }
-        if (lane == 0)
-            dz[row] = g;
-        for (int j = lane; j < kHidden; j += 32)
-        {
-            const float h = __bfloat162float(h2[static_cast<size_t>(row) * kHidden + j]);
-            dh2[static_cast<size_t>(row) * kHidden + j] = __float2bfloat16_rn(h > 0.0f ? g * w3[j] : 0.0f);
-        }
-    }
+}  // namespace vg
 
-    // out[j] = sum_r a[r][j] * (w ? w[r] : 1) over rows, for a [rows][cols] matrix (bf16 or f32).
-    // Block (32, 32): threadIdx.x picks the column of a 32-column group (coalesced loads),
-    // threadIdx.y the row phase; a fixed-order reduction keeps the sums deterministic.
-    template <typename T>
-    __global__ void colsum_kernel(const T *a, const float *w, int rows, int cols, float *out)
-    {
-        const int j = blockIdx.x * 32 + threadIdx.x;
-        float acc = 0.0f;
-        if (j < cols)
-        {
-            for (int r = threadIdx.y; r < rows; r += 32)
-            {
-                float v;
-                if constexpr (sizeof(T) == 2)
-                    v = __bfloat162float(a[static_cast<size_t>(r) * cols + j]);
-                else
-                    v = a[static_cast<size_t>(r) * cols + j];
-                acc = fmaf(v, w ? w[r] : 1.0f, acc);
-            }
-        }
-        __shared__ float red[32][33];
-        red[threadIdx.y][threadIdx.x] = acc;
-        __syncthreads();
-        if (threadIdx.y == 0 && j < cols)
-        {
-            float sum = 0.0f;
-            for (int k = 0; k < 32; ++k)
-                sum += red[k][threadIdx.x];
-            out[j] = sum;
-        }
-    }
+#include "vg_mlp_train.cuh"
 
-    // dH1 = (dH2 W2) masked by H1 > 0, as bf16
-    __global__ void relu_mask_kernel(const float *g, const __nv_bfloat16 *h, int count, __nv_bfloat16 *out)
+namespace vg
+{
+    // The BF16 weights from the FP32 masters: row-major and in core-matrix layout.
+    __global__ void pack_weights_kernel(const float *w1, const float *w2, int kin, __nv_bfloat16 *w1b, __nv_bfloat16 *w2b,
+                                        CoreWeights core)
     {
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i < count)
-            out[i] = __float2bfloat16_rn(__bfloat162float(h[i]) > 0.0f ? g[i] : 0.0f);
-    }
-
-    // Adam on FP32 master weights, writing the BF16 copy the GEMMs read (when given)
-    __global__ void adam_kernel(float *w, const float *g, float *m, float *v, int count, float lr, float b1, float b2,
-                                float eps, float c1, float c2, __nv_bfloat16 *wb)
-    {
-        const int i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i >= count)
-            return;
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        w[i] = wi;
-        if (wb)
-            wb[i] = __float2bfloat16_rn(wi);
-    }
-
-    __global__ void to_bf16_kernel(const float *in, __nv_bfloat16 *out, int count)
-    {
-        const int i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i < count)
-            out[i] = __float2bfloat16_rn(in[i]);
+        if (i < kHidden * kin)
+        {
+            const __nv_bfloat16 b = __float2bfloat16_rn(w1[i]);
+            w1b[i] = b;
+            *reinterpret_cast<__nv_bfloat16 *>(core.w1 + tc::tile_offset(i / kin, i % kin, kin)) = b;
+        }
+        if (i < kHidden * kHidden)
+        {
+            const __nv_bfloat16 b = __float2bfloat16_rn(w2[i]);
+            w2b[i] = b;
+            *reinterpret_cast<__nv_bfloat16 *>(core.w2 + tc::tile_offset(i / kHidden, i % kHidden, kHidden)) = b;
+            *reinterpret_cast<__nv_bfloat16 *>(core.w2t + tc::tile_offset(i % kHidden, i / kHidden, kHidden)) = b;
+        }
     }
 }  // namespace vg
 
@@ -357,12 +266,17 @@ struct vg_mlp
     // fp32 masters: W1 [256][kin], b1 [256], W2 [256][256], b2 [256], w3 [256], b3 [1]
     float *w = nullptr;
     float *grad = nullptr, *m1 = nullptr, *m2 = nullptr;
-    __nv_bfloat16 *w1b = nullptr, *w2b = nullptr, *w2tb = nullptr;
+    __nv_bfloat16 *w1b = nullptr, *w2b = nullptr;  // row-major
+    vg::CoreWeights core{};                        // one allocation, at core.w2
     int step = 0;
     // workspace for `cap` rows
     int cap = 0;
-    __nv_bfloat16 *x = nullptr, *h1 = nullptr, *h2 = nullptr, *dh2 = nullptr, *dh1 = nullptr, *t0 = nullptr, *t1 = nullptr;
-    float *f32 = nullptr, *z = nullptr, *p = nullptr, *dz = nullptr, *loss = nullptr;
+    __nv_bfloat16 *x = nullptr, *h1 = nullptr, *h2 = nullptr;
+    float *p = nullptr, *loss = nullptr;
+    // operands of a training step's weight gradients for train_cap rows, one allocation
+    int train_cap = 0;
+    unsigned char *step_mem = nullptr;
+    vg::StepBuffers step_buf{};
     int *err = nullptr;
     uint32_t wait_limit = vg::kWaitLimit;  // vg_mlp_set_wait_limit
     float *scores = nullptr;  // probe scores of the last learned edge check
@@ -385,10 +299,12 @@ namespace vg
     {
         if (rows <= m->cap)
             return VG_OK;
-        void *old[] = {m->x, m->h1, m->h2, m->dh2, m->dh1, m->t0, m->t1, m->f32, m->z, m->p, m->dz};
+        void *old[] = {m->x, m->h1, m->h2, m->p};
         for (void *o : old)
             if (o)
                 cudaFree(o);
+        m->x = m->h1 = m->h2 = nullptr;
+        m->p = nullptr;
         const size_t H = static_cast<size_t>(rows) * kHidden;
         cudaError_t e = cudaSuccess;
         auto get = [&](void **ptr, size_t bytes) {
@@ -398,14 +314,7 @@ namespace vg
         get(reinterpret_cast<void **>(&m->x), static_cast<size_t>(rows) * m->kin * 2);
         get(reinterpret_cast<void **>(&m->h1), H * 2);
         get(reinterpret_cast<void **>(&m->h2), H * 2);
-        get(reinterpret_cast<void **>(&m->dh2), H * 2);
-        get(reinterpret_cast<void **>(&m->dh1), H * 2);
-        get(reinterpret_cast<void **>(&m->t0), H * 2);
-        get(reinterpret_cast<void **>(&m->t1), H * 2);
-        get(reinterpret_cast<void **>(&m->f32), H * 4);
-        get(reinterpret_cast<void **>(&m->z), static_cast<size_t>(rows) * 4);
         get(reinterpret_cast<void **>(&m->p), static_cast<size_t>(rows) * 4);
-        get(reinterpret_cast<void **>(&m->dz), static_cast<size_t>(rows) * 4);
         if (e != cudaSuccess)
         {
             m->cap = 0;
@@ -415,10 +324,38 @@ namespace vg
         return VG_OK;
     }
 
-    static void sync_bf16(vg_mlp *m, cudaStream_t s)
+    // buffers of a training step of `rows` rows (a multiple of 128); x holds row-major features for
+    // callers that want them
+    static int mlp_reserve_step(vg_mlp *m, int rows)
     {
-        to_bf16_kernel<<<(m->n_w1() + 255) / 256, 256, 0, s>>>(m->W1(), m->w1b, static_cast<int>(m->n_w1()));
-        to_bf16_kernel<<<256, 256, 0, s>>>(m->W2(), m->w2b, 256 * 256);
+        VG_CUDA(cudaFuncSetAttribute(mlp_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(rows_smem_bytes())),
+                "MLP training kernels");
+        VG_CUDA(cudaFuncSetAttribute(mlp_weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(weights_smem_bytes())),
+                "MLP training kernels");
+        if (rows <= m->train_cap)
+            return VG_OK;
+        if (m->step_mem)
+            cudaFree(m->step_mem);
+        m->step_mem = nullptr;
+        m->train_cap = 0;
+        const size_t tiles = static_cast<size_t>(rows) / 128, xt = tiles * 256 * m->kin, h = tiles * kTileT;
+        if (cudaMalloc(&m->step_mem, xt + 4 * h + static_cast<size_t>(rows) * 4) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return set_error(VG_ERR_NOMEM, "MLP training workspace");
+        }
+        unsigned char *at = m->step_mem;
+        m->step_buf = {at, at + xt, at + xt + h, at + xt + 2 * h, at + xt + 3 * h, reinterpret_cast<float *>(at + xt + 4 * h)};
+        m->train_cap = rows;
+        return VG_OK;
+    }
+
+    static cudaError_t pack_weights(vg_mlp *m, cudaStream_t s)
+    {
+        pack_weights_kernel<<<kHidden * kHidden / 256, 256, 0, s>>>(m->W1(), m->W2(), m->kin, m->w1b, m->w2b, m->core);
+        return cudaGetLastError();
     }
 
     // forward for `rows` rows (a multiple of 128) of configurations q[n][dim]; p receives
@@ -435,7 +372,7 @@ namespace vg
             e = gemm_bf16(g2, kEpiBiasReluBf16, s);
         if (e == cudaSuccess)
         {
-            head_kernel<<<(rows + 7) / 8, 256, 0, s>>>(m->h2, m->W3(), m->B3(), rows, m->z, m->p);
+            head_kernel<<<(rows + 7) / 8, 256, 0, s>>>(m->h2, m->W3(), m->B3(), rows, m->p);
             e = cudaGetLastError();
         }
         if (e != cudaSuccess)
@@ -443,45 +380,43 @@ namespace vg
         return VG_OK;
     }
 
-    // backward for a batch already run forward: gradients into m->grad; loss added to m->loss
-    static int mlp_backward(vg_mlp *m, const uint8_t *valid, int n, int rows, cudaStream_t s)
+    // One step on `rows` rows (a multiple of 128, the first n of them configurations q[n][dim]):
+    // gradients to m->grad (lr 0) or an Adam update; the loss is added to m->loss.  x: row-major
+    // features wanted (null: not).
+    static int mlp_step(vg_mlp *m, const float *q, const uint8_t *valid, int n, int rows, float lr, __nv_bfloat16 *x,
+                        cudaStream_t s)
     {
-        float *gr = m->grad;
-        head_backward_kernel<<<(rows + 7) / 8, 256, 0, s>>>(m->h2, m->W3(), m->p, m->z, valid, n, rows, m->dz, m->dh2, m->loss);
-        colsum_kernel<__nv_bfloat16><<<kHidden / 32, dim3(32, 32), 0, s>>>(m->h2, m->dz, rows, kHidden, m->G(gr, m->W3()));  // dw3
-        colsum_kernel<float><<<1, dim3(32, 32), 0, s>>>(m->dz, nullptr, rows, 1, m->G(gr, m->B3()));                     // db3
-        colsum_kernel<__nv_bfloat16><<<kHidden / 32, dim3(32, 32), 0, s>>>(m->dh2, nullptr, rows, kHidden, m->G(gr, m->B2()));  // db2
-        // dW2[j][i] = sum_r dH2[r][j] H1[r][i]
-        const dim3 tb(32, 8);
-        transpose_kernel<<<dim3(kHidden / 32, rows / 32), tb, 0, s>>>(m->dh2, m->t0, rows, kHidden);
-        transpose_kernel<<<dim3(kHidden / 32, rows / 32), tb, 0, s>>>(m->h1, m->t1, rows, kHidden);
-        GemmParams gw2{m->t0, m->t1, m->G(gr, m->W2()), nullptr, nullptr, kHidden, kHidden, rows, m->err};
-        gw2.wait_limit = m->wait_limit;
-        cudaError_t e = gemm_bf16(gw2, kEpiStoreF32, s);
-        // dH1 = (dH2 W2) * (H1 > 0): B operand is W2^T as [i][j]
-        GemmParams gh1{m->dh2, m->w2tb, m->f32, nullptr, nullptr, rows, kHidden, kHidden, m->err};
-        gh1.wait_limit = m->wait_limit;
+        RowsParams rp{q, valid, n, m->dim, m->kin, m->core.w1, m->core.w2, m->core.w2t, m->B1(), m->B2(), m->W3(), m->B3(), m->step_buf, x,
+                      m->loss, m->err, m->wait_limit};
+        WeightsParams wp{m->step_buf, rows, m->kin, m->w, m->grad, m->m1, m->m2, lr > 0.0f, lr, 0.9f, 0.999f, 1e-8f, 1.0f, 1.0f,
+                         m->core, m->err, m->wait_limit};
+        if (wp.adam)
+        {
+            ++m->step;
+            wp.c1 = 1.0f - std::pow(wp.b1, static_cast<float>(m->step));
+            wp.c2 = 1.0f - std::pow(wp.b2, static_cast<float>(m->step));
+        }
+        // each kernel starts up under the one before (programmatic dependent launch): at 1,024 rows
+        // the two take 21 us and the gaps between plain launches were 15
+        cudaLaunchAttribute overlap{};
+        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        overlap.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t c{};
+        c.attrs = &overlap;
+        c.numAttrs = 1;
+        c.stream = s;
+        c.gridDim = dim3(rows / 128);
+        c.blockDim = dim3(kTrainThreads);
+        c.dynamicSmemBytes = rows_smem_bytes();
+        cudaError_t e = cudaLaunchKernelEx(&c, mlp_rows_kernel, rp);
+        c.gridDim = dim3(weights_grid());
+        c.blockDim = dim3(kWeightsThreads);
+        c.dynamicSmemBytes = weights_smem_bytes();
         if (e == cudaSuccess)
-            e = gemm_bf16(gh1, kEpiStoreF32, s);
+            e = cudaLaunchKernelEx(&c, mlp_weights_kernel, wp);
         if (e != cudaSuccess)
-            return set_error(VG_ERR_CUDA, std::string("MLP backward: ") + cudaGetErrorString(e));
-        relu_mask_kernel<<<(rows * kHidden + 255) / 256, 256, 0, s>>>(m->f32, m->h1, rows * kHidden, m->dh1);
-        colsum_kernel<__nv_bfloat16><<<kHidden / 32, dim3(32, 32), 0, s>>>(m->dh1, nullptr, rows, kHidden, m->G(gr, m->B1()));  // db1
-        // dW1[i][c] = sum_r dH1[r][i] X[r][c]
-        transpose_kernel<<<dim3(kHidden / 32, rows / 32), tb, 0, s>>>(m->dh1, m->t0, rows, kHidden);
-        transpose_kernel<<<dim3((m->kin + 31) / 32, rows / 32), tb, 0, s>>>(m->x, m->t1, rows, m->kin);
-        GemmParams gw1{m->t0, m->t1, m->G(gr, m->W1()), nullptr, nullptr, kHidden, m->kin, rows, m->err};
-        gw1.wait_limit = m->wait_limit;
-        e = gemm_bf16(gw1, kEpiStoreF32, s);
-        if (e != cudaSuccess)
-            return set_error(VG_ERR_CUDA, std::string("MLP backward: ") + cudaGetErrorString(e));
+            return set_error(VG_ERR_CUDA, std::string("MLP training step: ") + cudaGetErrorString(e));
         return VG_OK;
-    }
-
-    static void refresh_w2t(vg_mlp *m, cudaStream_t s)
-    {
-        // W2^T as bf16 [i][j] for the dH1 GEMM
-        transpose_kernel<<<dim3(kHidden / 32, kHidden / 32), dim3(32, 8), 0, s>>>(m->w2b, m->w2tb, kHidden, kHidden);
     }
 
     static int mlp_check_err(vg_mlp *m)
@@ -520,7 +455,7 @@ vg_mlp *vg_mlp_create(int dim, uint64_t seed)
     if (e == cudaSuccess) e = cudaMalloc(&m->m2, n * 4);
     if (e == cudaSuccess) e = cudaMalloc(&m->w1b, m->n_w1() * 2);
     if (e == cudaSuccess) e = cudaMalloc(&m->w2b, 256 * 256 * 2);
-    if (e == cudaSuccess) e = cudaMalloc(&m->w2tb, 256 * 256 * 2);
+    if (e == cudaSuccess) e = cudaMalloc(&m->core.w2, 2 * 256 * 256 * 2 + m->n_w1() * 2);
     if (e == cudaSuccess) e = cudaMalloc(&m->loss, 4);
     if (e == cudaSuccess) e = cudaMalloc(&m->err, 4);
     if (e != cudaSuccess)
@@ -555,8 +490,9 @@ vg_mlp *vg_mlp_create(int dim, uint64_t seed)
     cudaMemset(m->m1, 0, n * 4);
     cudaMemset(m->m2, 0, n * 4);
     cudaMemset(m->err, 0, 4);
-    sync_bf16(m, 0);
-    refresh_w2t(m, 0);
+    m->core.w2t = m->core.w2 + 256 * 256 * 2;
+    m->core.w1 = m->core.w2t + 256 * 256 * 2;
+    pack_weights(m, 0);
     cudaDeviceSynchronize();
     return m;
 }
@@ -565,8 +501,8 @@ void vg_mlp_destroy(vg_mlp *m)
 {
     if (!m)
         return;
-    void *ptrs[] = {m->w, m->grad, m->m1, m->m2, m->w1b, m->w2b, m->w2tb, m->x, m->h1, m->h2, m->dh2, m->dh1, m->t0, m->t1,
-                    m->f32, m->z, m->p, m->dz, m->loss, m->err, m->scores};
+    void *ptrs[] = {m->w, m->grad, m->m1, m->m2, m->w1b, m->w2b, m->core.w2, m->x, m->h1, m->h2, m->p, m->step_mem, m->loss,
+                    m->err, m->scores};
     for (void *p : ptrs)
         if (p)
             cudaFree(p);
@@ -588,8 +524,7 @@ int vg_mlp_set_params(vg_mlp *m, const float *in)
         return set_error(VG_ERR_ARG, "vg_mlp_set_params: bad argument");
     if (cudaMemcpy(m->w, in, m->count() * 4, cudaMemcpyHostToDevice) != cudaSuccess)
         return set_error(VG_ERR_CUDA, "vg_mlp_set_params: copy failed");
-    sync_bf16(m, 0);
-    refresh_w2t(m, 0);
+    pack_weights(m, 0);
     return cudaDeviceSynchronize() == cudaSuccess ? VG_OK : set_error(VG_ERR_CUDA, "vg_mlp_set_params");
 }
 
@@ -625,10 +560,10 @@ int vg_mlp_gradients(vg_mlp *m, const float *q_dev, const uint8_t *valid_dev, si
     const int rows = static_cast<int>((n + 127) / 128 * 128);
     if (int rc = mlp_reserve(m, rows))
         return rc;
-    cudaMemset(m->loss, 0, 4);
-    if (int rc = mlp_forward(m, q_dev, static_cast<int>(n), rows, 0))
+    if (int rc = mlp_reserve_step(m, rows))
         return rc;
-    if (int rc = mlp_backward(m, valid_dev, static_cast<int>(n), rows, 0))
+    cudaMemset(m->loss, 0, 4);
+    if (int rc = mlp_step(m, q_dev, valid_dev, static_cast<int>(n), rows, 0.0f, m->x, 0))
         return rc;
     if (cudaDeviceSynchronize() != cudaSuccess)
         return set_error(VG_ERR_CUDA, "vg_mlp_gradients: kernel failure");
@@ -655,7 +590,7 @@ int vg_mlp_train_device(vg_mlp *m, const float *q_dev, const uint8_t *valid_dev,
     if (!m || !q_dev || !valid_dev || n < 128 || epochs < 1 || batch < 128 || batch % 128 || !(lr > 0))
         return set_error(VG_ERR_ARG, "vg_mlp_train_device: bad argument (batch must be a multiple of 128)");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (int rc = mlp_reserve(m, batch))
+    if (int rc = mlp_reserve_step(m, batch))
         return rc;
     const size_t steps = n / batch;
     for (int ep = 0; ep < epochs; ++ep)
@@ -664,11 +599,8 @@ int vg_mlp_train_device(vg_mlp *m, const float *q_dev, const uint8_t *valid_dev,
         for (size_t st = 0; st < steps; ++st)
         {
             const size_t off = st * batch;
-            if (int rc = mlp_forward(m, q_dev + off * m->dim, batch, batch, s))
+            if (int rc = mlp_step(m, q_dev + off * m->dim, valid_dev + off, batch, batch, lr, nullptr, s))
                 return rc;
-            if (int rc = mlp_backward(m, valid_dev + off, batch, batch, s))
-                return rc;
-            ++m->step;
             if (ep == 0 && st == 0)
             {
                 // the first step shows whether the tensor-core kernels work on this device
@@ -677,14 +609,9 @@ int vg_mlp_train_device(vg_mlp *m, const float *q_dev, const uint8_t *valid_dev,
                 if (int rc = mlp_check_err(m))
                     return rc;
             }
-            const float b1 = 0.9f, b2 = 0.999f;
-            const float c1 = 1.0f - std::pow(b1, static_cast<float>(m->step));
-            const float c2 = 1.0f - std::pow(b2, static_cast<float>(m->step));
-            const int cnt = static_cast<int>(m->count());
-            adam_kernel<<<(cnt + 255) / 256, 256, 0, s>>>(m->w, m->grad, m->m1, m->m2, cnt, lr, b1, b2, 1e-8f, c1, c2, nullptr);
-            sync_bf16(m, s);
-            refresh_w2t(m, s);
         }
+        if (ep + 1 == epochs)
+            pack_weights(m, s);  // the row-major copies; the steps keep the others
         if (losses)
         {
             float l = 0;
@@ -798,15 +725,16 @@ namespace vg
             tc::mbar_init(&bar2, 1);
         }
         // weights into core-matrix layout, 16-byte units
+        // (8 lanes take the 8 rows of a core matrix: 128 consecutive bytes of shared memory)
         for (int u = tid; u < kHidden * (KIN / 8); u += kInferThreads)
         {
-            const int r = u / (KIN / 8), g = u % (KIN / 8);
+            const int r = (u & 7) + 8 * ((u >> 3) / (KIN / 8)), g = (u >> 3) % (KIN / 8);
             *reinterpret_cast<uint4 *>(sw1 + tc::tile_offset(r, 8 * g, KIN)) =
                 *reinterpret_cast<const uint4 *>(p.w1 + static_cast<size_t>(r) * KIN + 8 * g);
         }
         for (int u = tid; u < kHidden * (kHidden / 8); u += kInferThreads)
         {
-            const int r = u / (kHidden / 8), g = u % (kHidden / 8);
+            const int r = (u & 7) + 8 * (u >> 8), g = u >> 3 & 31;
             *reinterpret_cast<uint4 *>(sw2 + tc::tile_offset(r, 8 * g, kHidden)) =
                 *reinterpret_cast<const uint4 *>(p.w2 + static_cast<size_t>(r) * kHidden + 8 * g);
         }

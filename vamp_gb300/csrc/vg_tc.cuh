@@ -125,6 +125,62 @@ namespace vg::tc
         return false;
     }
 
+    // Programmatic dependent launch: waits until the kernel before in the stream has completed and
+    // its writes are visible; lets the kernel after start up to its own wait.
+    __device__ __forceinline__ void wait_previous_kernel()
+    {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+
+    __device__ __forceinline__ void start_next_kernel()
+    {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+
+    // 16 bytes from global to shared memory, asynchronously (both 16-byte aligned)
+    __device__ __forceinline__ void copy16_async(void *dst, const void *src)
+    {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    }
+
+    __device__ __forceinline__ void copies_commit()
+    {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+
+    // Waits until at most N of this thread's committed groups of copies are in flight.
+    template <int N>
+    __device__ __forceinline__ void copies_wait()
+    {
+        asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+    }
+
+    // Expects `bytes` of bulk copies on the barrier's current phase (and arrives).
+    __device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes)
+    {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+    }
+
+    // `bytes` (a multiple of 16) of contiguous global memory into shared memory by the copy engine;
+    // both addresses 16-byte aligned; completes on the barrier.
+    __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+    {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                     "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                     : "memory");
+    }
+
+    // Four 8 x 8 matrices of 16-bit elements, transposed: lanes 8 i .. 8 i + 7 give the addresses of
+    // matrix i's rows (16 bytes each); lane t gets elements (2 (t % 4), t / 4) and (2 (t % 4) + 1,
+    // t / 4) of each.
+    __device__ __forceinline__ void ldmatrix_x4_trans(const void *row, uint32_t *r)
+    {
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(smem_u32(row))
+                     : "memory");
+    }
+
     // 32 consecutive FP32 accumulator columns of this thread's TMEM lane (warp w of the CTA reads
     // lanes 32 (w % 4) .. 32 (w % 4) + 31).
     __device__ __forceinline__ void tmem_load32(uint32_t taddr, float *v)
