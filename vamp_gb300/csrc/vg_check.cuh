@@ -389,20 +389,18 @@ namespace vg
             return t_zcuboid(o, x, y, z, rsq);
     }
 
-    // One kind's sorted primitive list against NS query spheres.
+    // One kind's sorted primitive list against a query sphere.
     //
     // The reference walks the list per sphere and stops at the first object whose min_distance
     // minus max_extent has a clear sign bit in every lane of the block.  Since min_distance is
     // sorted and rounding is monotone, that stop is the first object with min_distance >= M, M
     // being the largest max_extent over the block's lanes; the objects before it are tested and a
-    // collision is any lane's test with its sign bit set.  Here each object record is read once
-    // for the NS spheres; sphere s tests it while min_distance < Mw[s] (the warp's largest M for
-    // that sphere, a uniform branch) and counts the result only while min_distance < M[s] (its
-    // own segment's bound).  Sign bits are OR-ed into bits[]; the segment vote happens once.
-    template <int KIND, int NS>
-    __device__ __forceinline__ void kind_pass(
-        const EnvView &e, float Mall, const float *Mw, const float *M, const float *x, const float *y,
-        const float *z, const float *r, const float *rsq, unsigned *bits)
+    // collision is any lane's test with its sign bit set.  Here the warp walks while min_distance <
+    // Mw (its largest M, a uniform branch) and a lane counts a result only while min_distance < M
+    // (its own segment's bound).  Sign bits are OR-ed into bits; the segment vote happens once.
+    template <int KIND>
+    __device__ __forceinline__ void kind_pass(const EnvView &e, float Mw, float M, float x, float y, float z, float r, float rsq,
+                                              unsigned &bits)
     {
         const float4 *rec = e.rec[KIND];
         const int n = e.n[KIND];
@@ -411,19 +409,12 @@ namespace vg
         {
             const float4 *o = rec + i * rec_f4(KIND);
             const float md = reinterpret_cast<const float *>(o)[min_d_offset(KIND)];
-            if (!(md < Mall))
+            if (!(md < Mw))
             {
                 break;
             }
-#pragma unroll
-            for (int s = 0; s < NS; ++s)
-            {
-                if (md < Mw[s])
-                {
-                    const float t = prim_test<KIND>(o, x[s], y[s], z[s], r[s], rsq[s]);
-                    bits[s] |= md < M[s] ? __float_as_uint(t) : 0u;
-                }
-            }
+            const float t = prim_test<KIND>(o, x, y, z, r, rsq);
+            bits |= md < M ? __float_as_uint(t) : 0u;
         }
     }
 
@@ -596,73 +587,49 @@ namespace vg
         return __ballot_sync(kFull, hit);
     }
 
-    // sphere_environment_in_collision (validity.hh:47-150) for NS spheres at once, sphere s over
-    // the segments in mask[s].  hit[s] receives the lanes of the segments whose block collides for
-    // sphere s.  Warp-uniform; all 32 lanes must call.
-    // kExt: also the heightfields (kernels built for environments with heightfields or an
-    // attachment; the default kernels leave them out)
-    template <int W, int NS, bool kExt = false>
-    __device__ __forceinline__ void env_multi(const EnvView &e, const float4 *sph, const unsigned *mask, unsigned *hit)
+    // sphere_environment_in_collision (validity.hh:47-150) for each lane's sphere over the segments
+    // in `mask`: the lanes of the segments whose block collides.  may: the lanes of `mask` whose
+    // sphere may touch something; the pointclouds are asked for no others.  Warp-uniform; all 32
+    // lanes must call.  kExt: also the heightfields (kernels built for environments with heightfields or
+    // an attachment; the default kernels leave them out).
+    template <int W, bool kExt = false>
+    __device__ __forceinline__ unsigned env_query(const EnvView &e, float x, float y, float z, float r, unsigned mask, unsigned may)
     {
         const int lane = threadIdx.x & 31;
-        float x[NS], y[NS], z[NS], r[NS], rsq[NS], M[NS], Mw[NS];
-        unsigned bits[NS];
-        float Mall = -__int_as_float(0x7f800000);
-#pragma unroll
-        for (int s = 0; s < NS; ++s)
-        {
-            const float4 c = sph[s];
-            const bool on = (mask[s] >> lane) & 1u;
-            x[s] = c.x;
-            y[s] = c.y;
-            z[s] = c.z;
-            r[s] = c.w;
-            rsq[s] = __fmul_rn(c.w, c.w);
-            const float v = __fmaf_rn(c.x, c.x, __fmaf_rn(c.z, c.z, __fmul_rn(c.y, c.y)));
-            const float m = seg_max<W>(max_extent(e, v, c.w));
-            M[s] = on ? m : -__int_as_float(0x7f800000);
-            // max_extent is >= 0 (or +inf): as unsigned integers its bit patterns order like the
-            // floats, so one warp reduction gives the warp-wide bound (inactive lanes count as 0)
-            Mw[s] = __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(m) : 0u));
-            Mall = fmaxf(Mall, Mw[s]);
-            bits[s] = 0u;
-        }
-        kind_pass<0, NS>(e, Mall, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<1, NS>(e, Mall, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<2, NS>(e, Mall, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<3, NS>(e, Mall, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<4, NS>(e, Mall, Mw, M, x, y, z, r, rsq, bits);
+        const bool on = (mask >> lane) & 1u;
+        const float rsq = __fmul_rn(r, r);
+        const float v = __fmaf_rn(x, x, __fmaf_rn(z, z, __fmul_rn(y, y)));
+        const float m = seg_max<W>(max_extent(e, v, r));
+        const float M = on ? m : -__int_as_float(0x7f800000);
+        // max_extent is >= 0 (or +inf): as unsigned integers its bit patterns order like the
+        // floats, so one warp reduction gives the warp-wide bound (inactive lanes count as 0)
+        const float Mw = __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(m) : 0u));
+        unsigned bits = 0u;
+        kind_pass<0>(e, Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<1>(e, Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<2>(e, Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<3>(e, Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<4>(e, Mw, M, x, y, z, r, rsq, bits);
         if constexpr (kExt)
         {
 #pragma unroll 1
             for (int h = 0; h < e.n_hf; ++h)
             {
-#pragma unroll
-                for (int s = 0; s < NS; ++s)
-                {
-                    bits[s] |= __float_as_uint(t_heightfield(e.hf[h], x[s], y[s], z[s], r[s]));
-                }
+                bits |= __float_as_uint(t_heightfield(e.hf[h], x, y, z, r));
             }
         }
-#pragma unroll
-        for (int s = 0; s < NS; ++s)
-        {
-            hit[s] = seg_any<W>(__ballot_sync(kFull, bits[s] >> 31)) & mask[s];
-        }
+        unsigned hit = seg_any<W>(__ballot_sync(kFull, bits >> 31)) & mask;
         // pointclouds, for the blocks the primitives did not already put in collision
 #pragma unroll 1
         for (int c = 0; c < e.n_clouds; ++c)
         {
-#pragma unroll
-            for (int s = 0; s < NS; ++s)
+            const unsigned ask = may & ~hit;
+            if (ask)
             {
-                const bool ask = ((mask[s] & ~hit[s]) >> lane) & 1u;
-                if (mask[s] & ~hit[s])
-                {
-                    hit[s] |= seg_any<W>(capt_warp(e.clouds[c], x[s], y[s], z[s], r[s], ask)) & mask[s];
-                }
+                hit |= seg_any<W>(capt_warp(e.clouds[c], x, y, z, r, (ask >> lane) & 1u)) & mask;
             }
         }
+        return hit;
     }
 
     // A frame as 12 floats: R row-major, then t.
@@ -686,16 +653,6 @@ namespace vg
             c[r] = acc;
         }
         return make_float4(c[0], c[1], c[2], o.w);
-    }
-
-    // Single-sphere query, inlined into the caller.
-    template <int W, bool kExt = false>
-    __device__ __forceinline__ unsigned env_query_inline(const EnvView &e, float x, float y, float z, float r, unsigned mask)
-    {
-        const float4 s = make_float4(x, y, z, r);
-        unsigned hit;
-        env_multi<W, 1, kExt>(e, &s, &mask, &hit);
-        return hit;
     }
 
     // sphere_sphere_self_collision (validity.hh:23-44) for the segments in `mask`.
@@ -742,9 +699,9 @@ namespace vg
         // this thread's column of the robot's shared-memory stage: element i at stage[i * kStageStride]
         float *stage = nullptr;
 
-        __device__ __forceinline__ unsigned env_hit(float x, float y, float z, float r, unsigned mask)
+        __device__ __forceinline__ unsigned env_hit(const float4 s, unsigned mask, unsigned may)
         {
-            return env_query_inline<W, kExt>(env, x, y, z, r, mask);
+            return env_query<W, kExt>(env, s.x, s.y, s.z, s.w, mask, may);
         }
 
         // the field's value at a point (0, which rules nothing out, without a field)
@@ -759,9 +716,10 @@ namespace vg
             return seg_any<W>(__ballot_sync(kFull, may) & mask);
         }
 
-        __device__ __forceinline__ unsigned near(const float4 s, unsigned mask)
+        // the lanes of `mask` whose sphere may touch something
+        __device__ __forceinline__ unsigned may_touch(const float4 s, unsigned mask)
         {
-            return vote_near(clearance(s.x, s.y, s.z) < field_reach(s.w), mask);
+            return __ballot_sync(kFull, clearance(s.x, s.y, s.z) < field_reach(s.w)) & mask;
         }
 
         __device__ __forceinline__ unsigned self_hit(

@@ -879,7 +879,8 @@ namespace vg
                     const float dz = __fsub_rn(__ldg(spheres + 4 * k + 2), z), rs = __fadd_rn(__ldg(spheres + 4 * k + 3), radius);
                     valid &= !(__fsub_rn(__fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy))), __fmul_rn(rs, rs)) < 0.0f);
                 }
-                const unsigned hit = env_query_inline<1>(ev, x, y, z, radius, __ballot_sync(kFull, valid));
+                const unsigned ask = __ballot_sync(kFull, valid);
+                const unsigned hit = env_query<1>(ev, x, y, z, radius, ask, ask);
                 if (in)
                     flags[i] = valid && !((hit >> lane) & 1u) ? 1u : 0u;
             }

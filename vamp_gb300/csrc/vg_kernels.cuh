@@ -116,10 +116,10 @@ namespace vg
         for (int k = 0; k < ev.n_att && need; ++k)
         {
             const float4 c = posed(k);
-            const unsigned may = ctx.near(c, need);
+            const unsigned may = ctx.may_touch(c, need);
             if (!may)
                 continue;
-            const unsigned hit = ctx.env_hit(c.x, c.y, c.z, c.w, may);
+            const unsigned hit = ctx.env_hit(c, seg_any<W>(may), may);
             ctx.alive &= ~hit;
             need &= ~hit;
         }

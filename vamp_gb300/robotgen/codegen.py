@@ -867,8 +867,8 @@ while (todo)
         for (int slot = e.x;; slot = next++)
         {{
             const float4 c = vg::frame_point(f, {pre}SlotOff[slot]);
-            const unsigned may = ctx.near(c, need);
-            const unsigned hit = may ? ctx.env_hit(c.x, c.y, c.z, c.w, may) : 0u;
+            const unsigned may = ctx.may_touch(c, need);
+            const unsigned hit = may ? ctx.env_hit(c, vg::seg_any<Ctx::kW>(may), may) : 0u;
             if (coarse)
             {{
                 need = hit;
