@@ -204,3 +204,27 @@ def test_a_stream_under_capture_runs_without_building_the_field():
     want = vg.panda.validate_batch(q, env)
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("n", [6143, 6144, 6145, 7168, 20001])
+def test_motions_handed_out_long_ones_first_are_those_handed_out_as_given(n):
+    """Edge counts about the threshold and the rank kernel's tiles: verdicts and block counts land on
+    their own edges (the segment-per-edge schedule takes edges as given)."""
+    import torch
+
+    import vamp_gb300 as vg
+    from vamp_gb300 import scenes
+
+    rb = vg.ur5
+    a, b = scenes.edges(rb.s_m, rb.s_a, n, 31)
+    rng = np.random.default_rng(2)
+    b = a + (b - a) * rng.random((n, 1), dtype=np.float32) ** 4  # many one-block edges
+    b[::97] = a[::97] + 300.0  # more blocks than the kernel tells apart
+    a, b = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    result = []
+    for schedule in (1, 0):
+        env = _base()
+        env.set_schedule(schedule)
+        blocks = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+        result.append((rb.validate_motion_batch(a, b, env, blocks=blocks), blocks))
+    assert torch.equal(result[0][0], result[1][0]) and torch.equal(result[0][1], result[1][1])

@@ -582,6 +582,40 @@ namespace vg
         }
     }
 
+    bool ranked(const MotionLaunch &m)
+    {
+        // fewer edges than kRankEdges are all handed out at once or nearly so
+        return !m.env->extended() && (m.scores || m.schedule == 1 || m.schedule == 2) && m.n >= kRankEdges;
+    }
+
+    unsigned *rank_scratch(vg_env *env, const MotionLaunch &m, cudaStream_t s)
+    {
+        if (!ranked(m))
+        {
+            return nullptr;
+        }
+        if (m.n > env->rank_cap)
+        {
+            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
+            {
+                cudaGetLastError();
+                return nullptr;  // no allocation under capture: the edges go as given
+            }
+            if (env->d_rank)
+                cudaFree(env->d_rank);
+            env->d_rank = nullptr;
+            env->rank_cap = 0;
+            if (cudaMalloc(&env->d_rank, m.n * sizeof(unsigned)) != cudaSuccess)
+            {
+                cudaGetLastError();
+                return nullptr;
+            }
+            env->rank_cap = m.n;
+        }
+        return env->d_rank;
+    }
+
     int launch_motions(const MotionLaunch &m, cudaStream_t s)
     {
         const RobotOps *r = m.r;
@@ -605,7 +639,7 @@ namespace vg
             return rc;
         if (m.blocks_per_sm > 0 && m.blocks_per_sm < occ)
             occ = m.blocks_per_sm;
-        VG_CUDA(cudaMemsetAsync(m.counter, 0, sizeof(unsigned), s), "reset work counter");
+        VG_CUDA(cudaMemsetAsync(m.counter, 0, 3 * sizeof(unsigned), s), "reset work counter");
         // edges handled at once by one block of threads: a warp each (same-edge schedule) or a
         // segment each
         const int per_block = grouped ? kBlock / 32 : kBlock / env->lanes;
@@ -613,6 +647,11 @@ namespace vg
         const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));
         EdgesParams p{m.a, m.b, static_cast<int>(m.n), m.resolution, m.out, m.blocks, m.counter, env_device(env), m.scores, m.probes,
                       m.dist, m.order};
+        if (grouped && !packed && m.rank && ranked(m))
+        {
+            p.rank = m.rank;
+            VG_CUDA(r->edge_rank[which](p, s), "edge rank kernel launch");
+        }
         if (learned)
         {
             // each edge's group order first (one warp per edge), on the same stream
@@ -633,6 +672,7 @@ namespace vg
     }
 
     // ------------------------------------------------------------ allocation-free variant
+    // (edges go as given: the hand-out order would need scratch)
     //
     // Scratch for vg_validate_motions_device_noalloc: the edge kernel's work counter lives in
     // this fixed array instead of memory the library allocates.  Every GPU that loads the
@@ -744,6 +784,8 @@ void vg_env_destroy(vg_env *env)
         cudaFree(env->d_stage);
     if (env->d_order)
         cudaFree(env->d_order);
+    if (env->d_rank)
+        cudaFree(env->d_rank);
     if (env->d_field)
         cudaFree(env->d_field);
     for (const CloudPoints &p : env->d_points)
@@ -1148,6 +1190,7 @@ int vg_validate_motions_device(
     want_field(env, kEdgeStates * static_cast<double>(n), static_cast<cudaStream_t>(stream));
     MotionLaunch m{r, env, a, b, n, resolution, nullptr, 0, out, blocks, env->d_counter};
     tuned_for(env, r, &m.schedule, &m.blocks_per_sm);
+    m.rank = rank_scratch(env, m, static_cast<cudaStream_t>(stream));
     return launch_motions(m, static_cast<cudaStream_t>(stream));
 }
 
@@ -1180,6 +1223,7 @@ int vg_validate_vectors_device(
     MotionLaunch m{r, env, start, vector, n, resolution, nullptr, 0, out, blocks, env->d_counter};
     m.dist = distance;
     tuned_for(env, r, &m.schedule, &m.blocks_per_sm);
+    m.rank = rank_scratch(env, m, static_cast<cudaStream_t>(stream));
     return launch_motions(m, static_cast<cudaStream_t>(stream));
 }
 
@@ -1225,6 +1269,7 @@ int vg_validate_motions_scored_device(
     m.order = env->d_order;
     int schedule = 1;
     tuned_for(env, r, &schedule, &m.blocks_per_sm);
+    m.rank = rank_scratch(env, m, static_cast<cudaStream_t>(stream));
     return launch_motions(m, static_cast<cudaStream_t>(stream));
 }
 

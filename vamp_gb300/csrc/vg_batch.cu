@@ -34,6 +34,7 @@ struct vg_batch
     unsigned *counters = nullptr;  // one work counter per part (64 bytes apart)
     size_t counters_cap = 0;
     std::vector<float *> scores;   // per part with an MLP: [n][probes]
+    std::vector<unsigned *> ranks; // per part whose edges are handed out in an order of their own
     std::vector<uint8_t *> orders; // per part with an MLP: its edges' group orders, 16 bytes each
     cudaStream_t capture = nullptr;  // the graph is captured here (the caller's stream may be the legacy default stream, which cannot be captured)
     std::vector<cudaStream_t> side;
@@ -87,9 +88,15 @@ namespace
             bt->scores.push_back(nullptr);
         while (bt->orders.size() < bt->parts.size())
             bt->orders.push_back(nullptr);
+        while (bt->ranks.size() < bt->parts.size())
+            bt->ranks.push_back(nullptr);
         for (size_t i = 0; i < bt->parts.size(); ++i)
         {
             const auto &p = bt->parts[i];
+            if (p.n >= kRankEdges && !bt->ranks[i])
+            {
+                VG_CUDA(cudaMalloc(&bt->ranks[i], p.n * sizeof(unsigned)), "cudaMalloc(batch edge orders)");
+            }
             if (p.mlp && !bt->scores[i])
             {
                 VG_CUDA(cudaMalloc(&bt->scores[i], p.n * p.probes * sizeof(float)), "cudaMalloc(batch scores)");
@@ -135,6 +142,7 @@ namespace
             MotionLaunch m{p.r, p.env, p.a, p.b, p.n, p.resolution, p.mlp ? bt->scores[i] : nullptr, p.probes,
                            p.out, p.blocks, bt->counters + 16 * i};
             m.order = p.mlp ? bt->orders[i] : nullptr;
+            m.rank = bt->ranks[i];
             tuned_for(p.env, p.r, &m.schedule, &m.blocks_per_sm);
             if (int rc = launch_motions(m, st))
                 return rc;
@@ -160,6 +168,9 @@ void vg_batch_destroy(vg_batch *b)
     if (b->counters)
         cudaFree(b->counters);
     for (uint8_t *p : b->orders)
+        if (p)
+            cudaFree(p);
+    for (unsigned *p : b->ranks)
         if (p)
             cudaFree(p);
     for (float *p : b->scores)
@@ -261,6 +272,7 @@ int vg_autotune_motions(const char *robot, vg_env *env, const float *a, const fl
         for (int bps = occ; bps >= 1 && rc == VG_OK; --bps)
         {
             MotionLaunch m{r, env, a, b, n, resolution, nullptr, 0, out, nullptr, env->d_counter, sched, bps};
+            m.rank = rank_scratch(env, m, s);
             float t = 1e30f;
             for (int rep = 0; rep < 3 && rc == VG_OK; ++rep)
             {

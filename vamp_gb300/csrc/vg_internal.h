@@ -45,6 +45,8 @@ namespace vg
         // next edge
         cudaError_t (*edges_packed[2])(const EdgesParams &, int grid, int block, int smem, cudaStream_t);
         const void *edges_packed_fn[2];
+        // the order in which the same-edge schedules hand edges out (EdgesParams::rank)
+        cudaError_t (*edge_rank[2])(const EdgesParams &, cudaStream_t);
         // each edge's group order from its scores (before the learned-order check)
         cudaError_t (*edge_order[2])(const EdgesParams &, int grid, int block, int smem, cudaStream_t);
         // same-edge schedule in a learned block order (EdgesParams::order)
@@ -155,6 +157,9 @@ struct vg_env
     // learned-order group orders (vg_validate_motions_scored_device), 16 bytes per edge
     uint8_t *d_order = nullptr;
     size_t order_cap = 0;
+    // hand-out order of the same-edge schedules (rank_scratch), 4 bytes per edge
+    unsigned *d_rank = nullptr;
+    size_t rank_cap = 0;
     // library-owned scratch: work counter, staging for host-pointer calls
     unsigned *d_counter = nullptr;
     void *d_stage = nullptr;
@@ -189,6 +194,7 @@ namespace vg
         int blocks_per_sm = 0;  // 0: as many as fit
         const float *dist = nullptr;  // validate_vector form: b holds vectors, dist their lengths
         uint8_t *order = nullptr;     // with scores: scratch of n x 16 bytes for the group orders
+        unsigned *rank = nullptr;     // scratch of n x 4 bytes for the hand-out order (null: edges as given)
     };
 
     int commit(vg_env *e);
@@ -196,6 +202,8 @@ namespace vg
     // States checked in an environment since its last change from which its clearance field is
     // built (about 0.1 ms, allocations and the synchronisation included).
     constexpr double kFieldStates = 131072.0;
+    // Edges from which they are handed out in edge_rank_kernel's order.
+    constexpr size_t kRankEdges = 6144;
     // states an edge is taken to hold where its length is not known on the host
     constexpr double kEdgeStates = 64.0;
     // Counts `states` about to be checked on stream s in a committed environment and builds its
@@ -205,4 +213,8 @@ namespace vg
     int prepare_kernel(const void *fn, int smem, int block, int *blocks_per_sm);
     void tuned_for(const vg_env *env, const RobotOps *r, int *schedule, int *blocks_per_sm);
     int launch_motions(const MotionLaunch &m, cudaStream_t s);
+    // whether launch_motions hands the edges out in edge_rank_kernel's order
+    bool ranked(const MotionLaunch &m);
+    // the environment's scratch for that order (null where the edges go as given, or without memory)
+    unsigned *rank_scratch(vg_env *env, const MotionLaunch &m, cudaStream_t s);
 }  // namespace vg

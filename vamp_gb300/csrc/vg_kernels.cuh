@@ -257,7 +257,8 @@ namespace vg
         int resolution;
         uint8_t *out;        // 1 = valid
         int32_t *blocks;     // optional: blocks checked per edge
-        unsigned *head;      // work counter, zero before launch
+        unsigned *head;      // work counters, zero before launch: [0] the edges handed out; [1], [2]
+                             // edge_rank_kernel's ends of the long and the short edges
         EnvDevice env;
         // learned order (same-edge schedule only): per-edge collision scores of `probes` states
         // at fractions (p + 0.5) / probes along the edge; null = the reference's block order
@@ -269,6 +270,9 @@ namespace vg
         // learned order: per edge kOrderMax / (32 / W) group indices in checking order, written
         // by edge_order_kernel from the scores
         uint8_t *order = nullptr;
+        // same-edge schedules: the order in which edges are handed out, from edge_rank_kernel (null:
+        // as given)
+        unsigned *rank = nullptr;
     };
 
     constexpr int kOrderMax = 64;  // blocks of an edge the learned order ranks; later ones follow in order
@@ -408,6 +412,102 @@ namespace vg
                 p.order[e * kGroups + lane] = order[lane];
             }
             __syncwarp();
+        }
+    }
+
+    // Blocks of edge e, exactly as the edge kernels count them.
+    template <int D, int W>
+    __device__ __forceinline__ int block_count(const EdgesParams &p, long long e)
+    {
+        float len;
+        if (p.dist)
+        {
+            len = p.dist[e];
+        }
+        else
+        {
+            float v[D];
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+            {
+                v[d] = __fsub_rn(p.b[e * D + d], p.a[e * D + d]);
+            }
+            len = edge_length<D>(v);
+        }
+        const float nf = ceilf(__fmul_rn(__fdiv_rn(len, static_cast<float>(W)), static_cast<float>(p.resolution)));
+        return static_cast<int>(nf > 1.0f ? nf : 1.0f);
+    }
+
+    // An order for handing edges out in which long ones come early: the launch's last edges, which
+    // leave most warps idle until the longest of them is done, are then short.  Each block of
+    // threads sorts its kRankTile edges by block count (longest first, counts of kRankBins and more
+    // alike), takes the longer half's places from the front of the order and the shorter half's
+    // from the back.  One pass over the end points; verdicts and block counts do not depend on the
+    // order.
+    constexpr int kRankTile = 1024;
+    constexpr int kRankBins = 256;
+
+    template <int D, int W>
+    __global__ void __launch_bounds__(kRankBins) edge_rank_kernel(EdgesParams p)
+    {
+        constexpr int kEach = kRankTile / kRankBins;
+        __shared__ unsigned bins[kRankBins];
+        __shared__ unsigned warp_sum[kRankBins / 32], front, back;
+        const int t = threadIdx.x, lane = t & 31;
+        const long long base = static_cast<long long>(blockIdx.x) * kRankTile;
+        const unsigned count = static_cast<unsigned>(min(static_cast<long long>(kRankTile), p.n - base));
+        bins[t] = 0u;
+        __syncthreads();
+        int bin[kEach];
+        unsigned place[kEach];
+#pragma unroll
+        for (int k = 0; k < kEach; ++k)
+        {
+            const long long e = base + t + kRankBins * k;
+            bin[k] = -1;
+            if (e < p.n)
+            {
+                bin[k] = kRankBins - min(block_count<D, W>(p, e), kRankBins);  // longest first
+                place[k] = atomicAdd(&bins[bin[k]], 1u);
+            }
+        }
+        __syncthreads();
+        // exclusive sums of the bins
+        const unsigned mine = bins[t];
+        unsigned sum = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const unsigned v = __shfl_up_sync(kFull, sum, o);
+            sum += lane >= o ? v : 0u;
+        }
+        if (lane == 31)
+        {
+            warp_sum[t >> 5] = sum;
+        }
+        const unsigned half = count / 2;
+        if (t == 0)
+        {
+            front = atomicAdd(p.head + 1, half);
+            back = atomicAdd(p.head + 2, count - half);
+        }
+        __syncthreads();
+        unsigned before = 0u;
+        for (int w = 0; w < t >> 5; ++w)
+        {
+            before += warp_sum[w];
+        }
+        bins[t] = before + sum - mine;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kEach; ++k)
+        {
+            if (bin[k] >= 0)
+            {
+                const unsigned r = bins[bin[k]] + place[k];
+                const unsigned at = r < half ? front + r : static_cast<unsigned>(p.n) - 1u - (back + (count - 1u - r));
+                p.rank[at] = static_cast<unsigned>(base + t + kRankBins * k);
+            }
         }
     }
 
@@ -552,7 +652,7 @@ namespace vg
             {
                 break;
             }
-            const int e = static_cast<int>(got);
+            const int e = static_cast<int>(p.rank ? p.rank[got] : got);
             float q[D], bs[D], v[D];
 #pragma unroll
             for (int d = 0; d < D; ++d)

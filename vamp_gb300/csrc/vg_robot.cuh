@@ -52,6 +52,14 @@ namespace vg
         return cudaGetLastError();
     }
 
+    template <typename R, int W>
+    cudaError_t launch_edge_rank(const EdgesParams &p, cudaStream_t s)
+    {
+        edge_rank_kernel<R::kDim, W><<<static_cast<unsigned>((static_cast<long long>(p.n) + kRankTile - 1) / kRankTile), kRankBins, 0,
+                                       s>>>(p);
+        return cudaGetLastError();
+    }
+
     template <typename R, int W, int kMinBlocks>
     cudaError_t launch_edges_packed(const EdgesParams &p, int grid, int block, int smem, cudaStream_t s)
     {
@@ -129,6 +137,8 @@ namespace vg
         o.edges_learned[1] = &launch_edges_grouped<R, 4, true>;
         o.edges_learned_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, true>);
         o.edges_learned_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, true>);
+        o.edge_rank[0] = &launch_edge_rank<R, 8>;
+        o.edge_rank[1] = &launch_edge_rank<R, 4>;
         o.edge_order[0] = &launch_edge_order<R, 8>;
         o.edge_order[1] = &launch_edge_order<R, 4>;
         // extended checks (heightfields, fkcc_attach): the segment-per-edge and states kernels
