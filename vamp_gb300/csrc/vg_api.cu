@@ -786,8 +786,7 @@ void vg_env_destroy(vg_env *env)
         cudaFree(env->d_order);
     if (env->d_rank)
         cudaFree(env->d_rank);
-    if (env->d_field)
-        cudaFree(env->d_field);
+    release_field(env);
     for (const CloudPoints &p : env->d_points)
     {
         if (p.d)

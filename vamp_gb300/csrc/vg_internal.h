@@ -209,6 +209,8 @@ namespace vg
     // Counts `states` about to be checked on stream s in a committed environment and builds its
     // clearance field when due.  Failure to build leaves the environment without one.
     void want_field(vg_env *e, double states, cudaStream_t s);
+    // Gives the field's buffer back (waits for the device).
+    void release_field(vg_env *e);
     int sm_count();
     int prepare_kernel(const void *fn, int smem, int block, int *blocks_per_sm);
     void tuned_for(const vg_env *env, const RobotOps *r, int *schedule, int *blocks_per_sm);
