@@ -265,6 +265,44 @@ namespace vg
         }
     }
 
+    // A sphere, in the attachment's own coordinates, whose pose contains the pose of every sphere of
+    // the attachment, 0.1 mm to spare (its relative transform may scale: distances grow by at most
+    // the Frobenius norm of its 3 x 3 part).  Not finite (contains everything) where they are not.
+    static float4 attachment_bound(const vg_env *e)
+    {
+        double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0}, norm2 = 0.0, size = 1.0;
+        for (int r = 0; r < 3; ++r)
+        {
+            for (int c = 0; c < 3; ++c)
+                norm2 += static_cast<double>(e->att[4 * r + c]) * e->att[4 * r + c];
+            size += std::fabs(static_cast<double>(e->att[4 * r + 3]));
+        }
+        const float *s = e->att.data() + 12;
+        for (int k = 0; k < e->n_att; ++k)
+        {
+            for (int c = 0; c < 3; ++c)
+            {
+                lo[c] = k ? std::min(lo[c], static_cast<double>(s[4 * k + c])) : s[4 * k + c];
+                hi[c] = k ? std::max(hi[c], static_cast<double>(s[4 * k + c])) : s[4 * k + c];
+            }
+        }
+        const float m[3] = {static_cast<float>(0.5 * (lo[0] + hi[0])), static_cast<float>(0.5 * (lo[1] + hi[1])),
+                            static_cast<float>(0.5 * (lo[2] + hi[2]))};
+        double radius = 0.0;
+        bool finite = std::isfinite(norm2) && std::isfinite(size);
+        for (int k = 0; k < e->n_att; ++k)
+        {
+            const double dx = s[4 * k] - static_cast<double>(m[0]), dy = s[4 * k + 1] - static_cast<double>(m[1]),
+                         dz = s[4 * k + 2] - static_cast<double>(m[2]);
+            const double d = std::sqrt(norm2 * (dx * dx + dy * dy + dz * dz)) + std::fabs(static_cast<double>(s[4 * k + 3]));
+            finite = finite && std::isfinite(d);
+            radius = std::max(radius, d);
+            size = std::max(size, d + std::sqrt(norm2) * (std::fabs(m[0]) + std::fabs(m[1]) + std::fabs(m[2])));
+        }
+        const double r = radius + 1e-4 + 1e-5 * size;
+        return make_float4(m[0], m[1], m[2], finite ? static_cast<float>(r) : INFINITY);
+    }
+
     // Uploads the environment image if it changed; records the current device.
     int commit(vg_env *e)
     {
@@ -302,12 +340,13 @@ namespace vg
             img.resize(at + sizeof(HeightView) / sizeof(float4));
             std::memcpy(&img[at], &v, sizeof(HeightView));
         }
-        // the attachment: 3 transform rows, then its spheres
+        // the attachment: 3 transform rows, then its spheres and the sphere that contains them
         e->att_off = static_cast<int>(img.size());
         if (e->n_att >= 0)
         {
             for (int k = 0; k < 3 + e->n_att; ++k)
                 img.push_back(make_float4(e->att[4 * k], e->att[4 * k + 1], e->att[4 * k + 2], e->att[4 * k + 3]));
+            img.push_back(attachment_bound(e));
         }
         if (img.size() > e->image_cap)
         {
@@ -585,7 +624,7 @@ namespace vg
     bool ranked(const MotionLaunch &m)
     {
         // fewer edges than kRankEdges are all handed out at once or nearly so
-        return !m.env->extended() && (m.scores || m.schedule == 1 || m.schedule == 2) && m.n >= kRankEdges;
+        return (m.env->extended() || m.scores || m.schedule == 1 || m.schedule == 2) && m.n >= kRankEdges;
     }
 
     unsigned *rank_scratch(vg_env *env, const MotionLaunch &m, cudaStream_t s)
@@ -622,14 +661,13 @@ namespace vg
         const vg_env *env = m.env;
         const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4)) + r->stage_floats * kBlock * 4;
         const int which = env->lanes == 8 ? 0 : 1;
-        // with heightfields or an attachment every schedule runs the extended checks in the
-        // segment-per-edge kernel (the block order does not change verdicts, so a learned order
-        // is not needed there)
+        // with heightfields or an attachment every schedule runs the extended checks in the same-edge
+        // kernel (the block order does not change verdicts, so a learned order is not needed there)
         const bool ext = env->extended();
         const bool learned = !ext && m.scores != nullptr;
-        const bool grouped = !ext && (learned || m.schedule >= 1);
-        const bool wide = grouped && !learned && m.schedule == 2;
-        const bool packed = grouped && !learned && m.schedule == 3;
+        const bool grouped = ext || learned || m.schedule >= 1;
+        const bool wide = !ext && !learned && m.schedule == 2;
+        const bool packed = !ext && !learned && m.schedule == 3;
         const void *fn = ext ? r->edges_ext_fn[which]
                              : learned ? r->edges_learned_fn[which]
                              : packed  ? r->edges_packed_fn[which]

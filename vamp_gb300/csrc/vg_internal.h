@@ -53,7 +53,7 @@ namespace vg
         cudaError_t (*edges_learned[2])(const EdgesParams &, int grid, int block, int smem, cudaStream_t);
         const void *edges_learned_fn[2];
         // extended forms (heightfields in the environment, or an attachment: fkcc_attach): states,
-        // and edges a segment each
+        // and edges in the same-edge schedule
         cudaError_t (*states_ext)(const StatesParams &, int grid, int block, int smem, cudaStream_t);
         const void *states_ext_fn;
         cudaError_t (*edges_ext[2])(const EdgesParams &, int grid, int block, int smem, cudaStream_t);

@@ -80,18 +80,22 @@ namespace vg
     }
 
     // The attachment part of Robot::fkcc_attach (robots/panda.hh:15308-15445) for the segments
-    // in `alive`: the attachment's spheres posed at the end effector (Attachment::pose,
+    // in ctx.alive: the attachment's spheres posed at the end effector (Attachment::pose,
     // collision/attachments.hh:43-55: p_tf * tf, then each centre) against the environment
     // (attachment_environment_collision, validity.hh:251-268), then, per robot link the
     // reference lists, its coarse sphere gating its fine spheres against the posed spheres
-    // (attachment_sphere_collision, validity.hh:270-293).  Returns the segments still valid.
+    // (attachment_sphere_collision, validity.hh:270-293).  Clears the colliding segments.
     // Every product is a chain of fused multiply-adds, first term first.
-    template <typename Robot, int W, bool kExt>
-    __device__ __noinline__ unsigned attach_check(const EnvView &ev, const float *q, unsigned alive)
+    //
+    // Frames come from the stage (recomputing the kinematics and every slot of the robot, through
+    // local memory, took most of this part), and the posed spheres' containing sphere stands for
+    // them until something comes near it.
+    template <typename Robot, int W, typename Ctx>
+    __device__ __forceinline__ void attach_check(Ctx &ctx, const float *st)
     {
-        CheckCtx<W, kExt> ctx{ev, alive, false, nullptr};
+        const EnvView &ev = ctx.env;
         float T[12], NR[9], Nt[3];
-        Robot::ee_pose(q, T);
+        Robot::ee_of(Robot::frame_at(st, Robot::kEeFrame), T);
         const float4 *A = ev.att;
         const float a[3][4] = {{A[0].x, A[0].y, A[0].z, A[0].w}, {A[1].x, A[1].y, A[1].z, A[1].w},
                                {A[2].x, A[2].y, A[2].z, A[2].w}};
@@ -111,49 +115,59 @@ namespace vg
                 c[r] = __fmaf_rn(NR[3 * r + 2], s.z, __fmaf_rn(NR[3 * r + 1], s.y, __fmaf_rn(NR[3 * r], s.x, Nt[r])));
             return make_float4(c[0], c[1], c[2], s.w);
         };
-        unsigned need = ctx.alive;
-#pragma unroll 1
-        for (int k = 0; k < ev.n_att && need; ++k)
+        const float4 whole = posed(ev.n_att);  // contains every posed sphere (attachment_bound)
+        if (ctx.may_touch(whole, ctx.alive))
         {
-            const float4 c = posed(k);
-            const unsigned may = ctx.may_touch(c, need);
-            if (!may)
-                continue;
-            const unsigned hit = ctx.env_hit(c, seg_any<W>(may), may);
-            ctx.alive &= ~hit;
-            need &= ~hit;
+#pragma unroll 1
+            for (int k = 0; k < ev.n_att; ++k)
+            {
+                const float4 c = posed(k);
+                const unsigned may = ctx.may_touch(c, ctx.alive);
+                if (may)
+                {
+                    const unsigned hit = ctx.env_hit(c, seg_any<W>(may), may);
+                    if (hit && !ctx.kill(hit))
+                    {
+                        return;
+                    }
+                }
+            }
         }
-        if (!need)
-            return ctx.alive;
-        float S[Robot::kSlots * 4];
-        Robot::spheres(q, S);
-        // any posed sphere against robot slot `slot`, for the segments in m
-        auto robot_hit = [&](int slot, unsigned m) {
+        // any posed sphere against robot sphere s, for the segments in m
+        auto robot_hit = [&](const float4 s, unsigned m) {
             unsigned hit = 0;
 #pragma unroll 1
             for (int k = 0; k < ev.n_att && (m & ~hit); ++k)
             {
                 const float4 c = posed(k);
-                hit |= ctx.self_hit(S[4 * slot], S[4 * slot + 1], S[4 * slot + 2], S[4 * slot + 3], c.x, c.y, c.z, c.w,
-                                    m & ~hit);
+                hit |= ctx.self_hit(s.x, s.y, s.z, s.w, c.x, c.y, c.z, c.w, m & ~hit);
             }
             return hit;
         };
 #pragma unroll 1
-        for (int L = 0; L < Robot::kAttachLinks && need; ++L)
+        for (int L = 0; L < Robot::kAttachLinks; ++L)
         {
             const int4 li = Robot::attach_link(L);
-            unsigned gate = robot_hit(li.x, need);
-#pragma unroll 1
-            for (int f = li.y; f < li.z && gate; ++f)
+            const Frame f = Robot::frame_at(st, li.w);
+            const float4 coarse = frame_point(f, Robot::slot_offset(li.x));
+            unsigned gate = ctx.self_hit(coarse.x, coarse.y, coarse.z, coarse.w, whole.x, whole.y, whole.z, whole.w, ctx.alive);
+            if (!gate)
             {
-                const unsigned hit = robot_hit(Robot::attach_fine(f), gate);
-                ctx.alive &= ~hit;
-                need &= ~hit;
+                continue;
+            }
+            gate = robot_hit(coarse, gate);
+#pragma unroll 1
+            for (int i = li.y; i < li.z && gate; ++i)
+            {
+                const unsigned hit = robot_hit(frame_point(f, Robot::slot_offset(Robot::attach_fine(i))), gate);
                 gate &= ~hit;
+                if (hit && !ctx.kill(hit))
+                {
+                    return;
+                }
+                gate &= ctx.alive;
             }
         }
-        return ctx.alive;
     }
 
     // kExt: the extended checks, for environments with heightfields or an attachment: every
@@ -168,7 +182,7 @@ namespace vg
         if constexpr (kExt)
         {
             if (ctx.alive && ev.n_att >= 0)
-                ctx.alive = attach_check<Robot, W, kExt>(ev, q, ctx.alive);
+                attach_check<Robot, W>(ctx, stage);
         }
         return ctx.alive;
     }
@@ -511,7 +525,7 @@ namespace vg
         }
     }
 
-    template <typename Robot, int W, bool kExt = false>
+    template <typename Robot, int W>
     __global__ void __launch_bounds__(128, VG_MIN_BLOCKS) edges_kernel(EdgesParams p)
     {
         extern __shared__ float4 smem[];
@@ -582,7 +596,7 @@ namespace vg
             {
                 break;
             }
-            const unsigned alive = run_fkcc<Robot, W, kExt>(ev, q, active, stage);
+            const unsigned alive = run_fkcc<Robot, W>(ev, q, active, stage);
             bool finish = false;
             if (e >= 0)
             {
@@ -624,7 +638,8 @@ namespace vg
     // (block i = block 0 minus v / (W n), i times).  The edge is invalid if any checked block is,
     // and the reference would have stopped at the first invalid block, so the block count
     // reported is that block's index + 1.
-    template <typename Robot, int W, bool kLearned, int kMinBlocks = Robot::kEdgeBlocks>
+    // kExt: the extended checks (heightfields, fkcc_attach).
+    template <typename Robot, int W, bool kLearned, int kMinBlocks = Robot::kEdgeBlocks, bool kExt = false>
     __global__ void __launch_bounds__(128, kMinBlocks) edges_grouped_kernel(EdgesParams p)
     {
         extern __shared__ float4 smem[];
@@ -716,7 +731,7 @@ namespace vg
                         }
                     }
                     const unsigned mask = __ballot_sync(kFull, active);
-                    const unsigned alive = run_fkcc<Robot, W, false, true>(ev, q, mask, stage);
+                    const unsigned alive = run_fkcc<Robot, W, kExt, true>(ev, q, mask, stage);
                     const unsigned dead = mask & ~alive;
                     // one bit per active segment (its first lane)
                     const unsigned leaders = mask & kSegLeaders;
@@ -745,7 +760,7 @@ namespace vg
                 {
                     const bool active = i0 + seg < n;
                     const unsigned mask = __ballot_sync(kFull, active);
-                    const unsigned alive = run_fkcc<Robot, W, false, true>(ev, q, mask, stage);
+                    const unsigned alive = run_fkcc<Robot, W, kExt, true>(ev, q, mask, stage);
                     const unsigned dead = mask & ~alive;
                     if (dead)
                     {

@@ -20,10 +20,10 @@ namespace vg
         return cudaGetLastError();
     }
 
-    template <typename R, int W, bool kExt = false>
+    template <typename R, int W>
     cudaError_t launch_edges(const EdgesParams &p, int grid, int block, int smem, cudaStream_t s)
     {
-        edges_kernel<R, W, kExt><<<grid, block, smem, s>>>(p);
+        edges_kernel<R, W><<<grid, block, smem, s>>>(p);
         return cudaGetLastError();
     }
 
@@ -38,10 +38,10 @@ namespace vg
         return cudaGetLastError();
     }
 
-    template <typename R, int W, bool kLearned, int kMinBlocks = R::kEdgeBlocks>
+    template <typename R, int W, bool kLearned, int kMinBlocks = R::kEdgeBlocks, bool kExt = false>
     cudaError_t launch_edges_grouped(const EdgesParams &p, int grid, int block, int smem, cudaStream_t s)
     {
-        edges_grouped_kernel<R, W, kLearned, kMinBlocks><<<grid, block, smem, s>>>(p);
+        edges_grouped_kernel<R, W, kLearned, kMinBlocks, kExt><<<grid, block, smem, s>>>(p);
         return cudaGetLastError();
     }
 
@@ -141,13 +141,13 @@ namespace vg
         o.edge_rank[1] = &launch_edge_rank<R, 4>;
         o.edge_order[0] = &launch_edge_order<R, 8>;
         o.edge_order[1] = &launch_edge_order<R, 4>;
-        // extended checks (heightfields, fkcc_attach): the segment-per-edge and states kernels
+        // extended checks (heightfields, fkcc_attach): the states and same-edge kernels
         o.states_ext = &launch_states<R, true>;
         o.states_ext_fn = reinterpret_cast<const void *>(&states_kernel<R, true>);
-        o.edges_ext[0] = &launch_edges<R, 8, true>;
-        o.edges_ext[1] = &launch_edges<R, 4, true>;
-        o.edges_ext_fn[0] = reinterpret_cast<const void *>(&edges_kernel<R, 8, true>);
-        o.edges_ext_fn[1] = reinterpret_cast<const void *>(&edges_kernel<R, 4, true>);
+        o.edges_ext[0] = &launch_edges_grouped<R, 8, false, R::kEdgeBlocks, true>;
+        o.edges_ext[1] = &launch_edges_grouped<R, 4, false, R::kEdgeBlocks, true>;
+        o.edges_ext_fn[0] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 8, false, R::kEdgeBlocks, true>);
+        o.edges_ext_fn[1] = reinterpret_cast<const void *>(&edges_grouped_kernel<R, 4, false, R::kEdgeBlocks, true>);
         o.ee_pose = &launch_ee_pose<R>;
         o.stage_floats = R::kStage;
         o.spheres = &launch_spheres<R>;

@@ -720,8 +720,9 @@ def gen_cuda(model: dict) -> str:
     w("    // the widened joint limits; global memory)")
     w(f"    __device__ const int2 {pre}AllPair[{max(1, len(all_pairs))}] = {{{', '.join('{%d, %d}' % p for p in all_pairs) or '{0, 0}'}}};")
     arows, afine = attach_tables(model, coarse_slot)
-    w("    // links checked against an attachment (fkcc_attach): coarse slot, fine range; fine slots")
-    w(f"    __device__ const int4 {pre}AttachLink[{max(1, len(arows))}] = {{{', '.join('{%d, %d, %d, 0}' % r for r in arows) or '{0, 0, 0, 0}'}}};")
+    w("    // links checked against an attachment (fkcc_attach): coarse slot, fine range, staged frame; fine")
+    w("    // slots")
+    table("__device__ const", "int4", "AttachLink", [r + (lay["frames"][kin.sphere_in_frame(*slots[r[0]][:2])[0]],) for r in arows], i4)
     w(f"    __device__ const int {pre}AttachFine[{max(1, len(afine))}] = {{{', '.join(map(str, afine)) or '0'}}};")
     w("")
 
@@ -773,7 +774,22 @@ def gen_cuda(model: dict) -> str:
     for l in body:
         w("        " + l)
     w("    }")
-    w("    // links checked against an attachment, in the reference's order: coarse slot, fine range")
+    # the same transform from the staged frame of the end effector's link
+    ee_fid = kin.link_frame[model["end_effector"]][0]
+    em = Emitter("cuda", SNAP32)
+    R0, t0 = fr[ee_fid]
+    entry = lambda v, i: v if isinstance(v, float) else f"f.m[{i}]"  # noqa: E731
+    staged = ([[entry(R0[r][c], 3 * r + c) for c in range(3)] for r in range(3)], [entry(t0[r], 9 + r) for r in range(3)])
+    vals = emit_ee_pose(em, {ee_fid: staged}, kin, model["end_effector"])
+    w(f"    // The same from the staged frame kEeFrame.")
+    w(f"    static constexpr int kEeFrame = {lay['frames'][ee_fid]};")
+    w("    static __device__ __forceinline__ void ee_of(const vg::Frame &f, float *T)")
+    w("    {")
+    for l in em.lines + [" ".join(f"T[{i}] = {em.ref(v)};" for i, v in enumerate(vals))]:
+        w("        " + l)
+    w("    }")
+    w(f"    static __device__ __forceinline__ float4 slot_offset(int i) {{ return {pre}SlotOff[i]; }}")
+    w("    // links checked against an attachment, in the reference's order: coarse slot, fine range, frame")
     w(f"    static constexpr int kAttachLinks = {len(arows)};")
     w(f"    static __device__ __forceinline__ int4 attach_link(int i) {{ return k{S}AttachLink[i]; }}")
     w(f"    static __device__ __forceinline__ int attach_fine(int i) {{ return k{S}AttachFine[i]; }}")
