@@ -6,6 +6,7 @@
 #include "../../include/vamp_gb300.h"
 #include "vg_internal.h"
 #include "vg_capt_gpu.h"
+#include "vg_pool.h"
 #include "x86_rsqrt_table.h"
 
 #include <cmath>
@@ -166,13 +167,14 @@ namespace vg
 
     static_assert(sizeof(CaptView) % sizeof(float4) == 0, "CaptView must pack into float4s");
 
-    // A device copy of a pointcloud's points for the clearance field.  Without memory for it the
+    // A device copy of a host-built pointcloud's points for the clearance field.  Without memory for it the
     // field reads the tree's blocks instead (CloudPoints::n = 0).
-    static CloudPoints keep_points(const float *xyz, size_t n, cudaMemcpyKind kind, cudaStream_t s)
+    static CloudPoints keep_points(const float *xyz, size_t n)
     {
         CloudPoints p;
         const size_t bytes = 3 * n * sizeof(float);
-        if (n && cudaMalloc(&p.d, bytes) == cudaSuccess && cudaMemcpyAsync(p.d, xyz, bytes, kind, s) == cudaSuccess)
+        if (n && pool_take(reinterpret_cast<void **>(&p.d), bytes, 0) == cudaSuccess &&
+            cudaMemcpy(p.d, xyz, bytes, cudaMemcpyHostToDevice) == cudaSuccess)
         {
             p.n = n;
         }
@@ -184,8 +186,8 @@ namespace vg
     }
 
     // Uploads each pointcloud's tree once: kCloudBuffers device buffers per cloud (tests, aabbs,
-    // starts, the reference-layout blocks, the ring-ordered blocks the queries scan, and the
-    // query tables).  A host-built cloud's reference-layout blocks are freed once ordered (the
+    // starts, the reference-layout blocks, and the ring-ordered blocks the queries scan with the
+    // query tables behind them).  A host-built cloud's reference-layout blocks are freed once ordered (the
     // host copy answers layout queries).
     static int upload_clouds(vg_env *e)
     {
@@ -198,7 +200,7 @@ namespace vg
             void *dst[4] = {nullptr, nullptr, nullptr, nullptr};
             for (int k = 0; k < 4; ++k)
             {
-                cudaError_t err = cudaMalloc(&dst[k], bytes[k]);
+                cudaError_t err = pool_take(&dst[k], bytes[k], 0);
                 if (err == cudaSuccess && src[k] && (k != 3 || !c.aff.empty()))
                 {
                     err = cudaMemcpy(dst[k], src[k], k == 3 ? c.aff.size() * sizeof(float) : bytes[k], cudaMemcpyHostToDevice);
@@ -206,23 +208,20 @@ namespace vg
                 if (err != cudaSuccess)
                 {
                     for (int j = 0; j <= k; ++j)
-                    {
-                        if (dst[j])
-                            cudaFree(dst[j]);
-                    }
+                        pool_give(dst[j], 0);
                     return cuda_fail(err, "upload pointcloud");
                 }
             }
             CaptQuery q;
             const int rc = capt_query_layout(static_cast<const float *>(dst[0]), c.nlog2, static_cast<const float *>(dst[1]),
                                              static_cast<const uint32_t *>(dst[2]), static_cast<const float *>(dst[3]), c.blocks(),
-                                             c.r_max, c.r_point, q);
-            cudaFree(dst[3]);
+                                             c.r_max, c.r_point, c.tests.data(), 0, q);
+            pool_give(dst[3], 0);
             dst[3] = nullptr;
             if (rc != VG_OK)
             {
                 for (int j = 0; j < 3; ++j)
-                    cudaFree(dst[j]);
+                    pool_give(dst[j], 0);
                 return rc;
             }
             for (int k = 0; k < 4; ++k)
@@ -230,9 +229,8 @@ namespace vg
                 e->d_clouds.push_back(dst[k]);
             }
             e->d_clouds.push_back(q.aff_q);
-            e->d_clouds.push_back(q.tables);
             e->capt_q.push_back(q);
-            e->d_points.push_back(keep_points(c.points.data(), c.points.size() / 3, cudaMemcpyHostToDevice, 0));
+            e->d_points.push_back(keep_points(c.points.data(), c.points.size() / 3));
         }
         return VG_OK;
     }
@@ -352,17 +350,19 @@ namespace vg
         {
             if (e->d_image)
             {
-                cudaFree(e->d_image);
+                cudaDeviceSynchronize();  // checks on any stream may be reading it
+                pool_give(e->d_image, 0);
                 e->d_image = nullptr;
+                e->d_counter = nullptr;
+                e->image_cap = 0;
             }
-            VG_CUDA(cudaMalloc(&e->d_image, img.size() * sizeof(float4)), "cudaMalloc(environment)");
-            e->image_cap = img.size();
+            // room to grow, and the work counter behind
+            const size_t cap = img.size() + img.size() / 2;
+            VG_CUDA(pool_take(reinterpret_cast<void **>(&e->d_image), cap * sizeof(float4) + 64, 0), "allocate environment");
+            e->image_cap = cap;
+            e->d_counter = reinterpret_cast<unsigned *>(e->d_image + cap);
         }
         VG_CUDA(cudaMemcpy(e->d_image, img.data(), img.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload environment");
-        if (!e->d_counter)
-        {
-            VG_CUDA(cudaMalloc(&e->d_counter, 64), "cudaMalloc(counter)");
-        }
         e->image_f4 = img.size();
         e->field_ready.store(false);
         e->field_states = 0.0;
@@ -814,10 +814,14 @@ void vg_env_destroy(vg_env *env)
     {
         return;
     }
-    if (env->d_image)
-        cudaFree(env->d_image);
-    if (env->d_counter)
-        cudaFree(env->d_counter);
+    // checks on any stream of its device may still be using what is given back
+    int dev = -1;
+    const bool away = env->device >= 0 && cudaGetDevice(&dev) == cudaSuccess && dev != env->device;
+    if (away)
+        cudaSetDevice(env->device);
+    if (env->d_image || !env->d_clouds.empty())
+        cudaDeviceSynchronize();
+    pool_give(env->d_image, 0);
     if (env->d_stage)
         cudaFree(env->d_stage);
     if (env->d_order)
@@ -827,15 +831,22 @@ void vg_env_destroy(vg_env *env)
     release_field(env);
     for (const CloudPoints &p : env->d_points)
     {
-        if (p.d)
-            cudaFree(p.d);
+        if (p.owned)
+            pool_give(p.d, 0);
     }
     if (env->h_pin)
         cudaFreeHost(env->h_pin);
-    for (void *p : env->d_clouds)
-        cudaFree(p);
+    for (size_t i = 0; i < env->d_clouds.size(); ++i)
+    {
+        // a device-built tree's first buffer holds its boxes, starts and points too
+        const size_t part = i % kCloudBuffers;
+        if ((part != 1 && part != 2) || !env->clouds[i / kCloudBuffers].on_device)
+            pool_give(env->d_clouds[i], 0);
+    }
     for (void *p : env->d_hf)
         cudaFree(p);
+    if (away)
+        cudaSetDevice(dev);
     delete env;
 }
 
@@ -972,12 +983,17 @@ int vg_env_add_pointcloud_device(vg_env *env, const float *xyz, size_t n, float 
     if (int rc = capt_build_device(xyz, n, r_min, r_max, r_point, static_cast<cudaStream_t>(stream), d))
         return rc;
     CaptQuery q;
-    if (int rc = capt_query_layout(d.tests, d.nlog2, d.aabbs, d.starts, d.aff, d.blocks, r_max, r_point, q))
+    if (int rc = capt_query_layout(d.tests, d.nlog2, d.aabbs, d.starts, d.aff, d.blocks, r_max, r_point, d.top_tests,
+                                   static_cast<cudaStream_t>(stream), q))
     {
         d.release();
         return rc;
     }
-    env->d_points.push_back(keep_points(xyz, n, cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream)));
+    CloudPoints pts;
+    pts.d = d.points;
+    pts.n = n;
+    pts.owned = false;
+    env->d_points.push_back(pts);
     CaptHost c;
     c.nlog2 = d.nlog2;
     std::memcpy(c.top, d.top, sizeof(c.top));
@@ -992,7 +1008,6 @@ int vg_env_add_pointcloud_device(vg_env *env, const float *xyz, size_t n, float 
     env->d_clouds.push_back(d.starts);
     env->d_clouds.push_back(d.aff);  // reference layout, kept for vg_env_pointcloud_layout
     env->d_clouds.push_back(q.aff_q);
-    env->d_clouds.push_back(q.tables);
     env->capt_q.push_back(q);
     env->device = dev;
     env->dirty = true;

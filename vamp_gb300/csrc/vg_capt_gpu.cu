@@ -4,16 +4,25 @@
 // The host builder splits recursively; this one goes level by level.  At level d every node
 // holds N >> d consecutive entries of the point order: a bitonic network sorts each node's
 // entries by (coordinate on axis d mod 3, current position), which is exactly the host's stable
-// sort.  Each node's split value, the two scans of its sorted halves (capt.hh:226-233) and its
-// children's cells follow from the sorted keys.  Its affordance list (the points of other nodes
-// within r_max of its cell) is filtered into its children's lists in order, one thread block per
-// node (ordered compaction), and the scanned ranges are appended, as the host builder does.  At
-// the leaves, each leaf's representative and its afforded points that pass the cell test become
-// its 8-point blocks, its box and its block range.
+// sort.  Each node's split value and the two scans of its sorted halves (capt.hh:226-233) follow
+// from the sorted keys.  Its affordance list (the points of other nodes within r_max of its cell)
+// is filtered into its children's lists in order, one thread block per node (ordered compaction),
+// and the scanned ranges are appended, as the host builder does.  At the leaves, each leaf's
+// representative and its afforded points that pass the cell test become its 8-point blocks, its
+// box and its block range.
+//
+// What bounds a build of a few thousand points is launches and waits, not work: a launch per step
+// and level, and a host wait per level for the size of its lists, made 5,271 points 1.54 ms.  So
+// the levels whose nodes fit a tile sort in one launch (a block takes a subtree down to its
+// leaves, keeping each level's order), a node's lists take their room from a counter instead of a
+// scan, within room guessed before (the build starts again with more when that runs out), and the
+// host waits once, for the size of the blocks.
 #include "vg_capt_gpu.h"
 
 #include "../../include/vamp_gb300.h"
 #include "vg_internal.h"
+#include "vg_pool.h"
+#include "vg_sort.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -26,6 +35,7 @@ namespace vg
     {
         constexpr float kInf = __builtin_huge_valf();
         constexpr int kListBlock = 128;  // threads per node in the list passes
+        constexpr long long kOrdersMax = 1ll << 24;  // entries up to which the subtrees' orders are kept
 
         __global__ void init_points(const float *xyz, long long n, long long N, float *px, float *py, float *pz,
                                     uint32_t *ord)
@@ -74,52 +84,58 @@ namespace vg
         }
 
         constexpr int kSortTile = 2048;  // entries per shared-memory tile of the sort
+        constexpr int kSmallTile = 512;
+
+        // An entry under sort: its key, its position before the level's sort (breaks ties), its point.
+        struct Entry
+        {
+            float key;
+            uint32_t pos, ord;
+        };
+
+        __device__ __forceinline__ Entry shuffle_xor(Entry v, int lanes)
+        {
+            return {__shfl_xor_sync(0xffffffffu, v.key, lanes), __shfl_xor_sync(0xffffffffu, v.pos, lanes),
+                    __shfl_xor_sync(0xffffffffu, v.ord, lanes)};
+        }
+
+        struct After
+        {
+            __device__ __forceinline__ bool operator()(const Entry &a, const Entry &b) const
+            {
+                return a.key > b.key || (a.key == b.key && a.pos > b.pos);
+            }
+        };
 
         // All compare-exchange stages of sizes k in [k0, k1] and strides below the tile, on tiles
         // of T = min(S, 2048) entries (S: the sorted segment size, a power of two).
-        __global__ void bitonic_tile(float *key, uint32_t *pos, uint32_t *ord, long long S, long long k0, long long k1)
+        __global__ void __launch_bounds__(kSortTile / 2) bitonic_tile(float *key, uint32_t *pos, uint32_t *ord, long long S,
+                                                                      long long k0, long long k1)
         {
-            __shared__ float sk[kSortTile];
-            __shared__ uint32_t sp[kSortTile], so[kSortTile];
-            const long long T = S < kSortTile ? S : kSortTile;
+            __shared__ Entry sm[kSortTile];
+            const int T = static_cast<int>(S < kSortTile ? S : kSortTile), t = threadIdx.x;
             const long long base = static_cast<long long>(blockIdx.x) * T;
-            for (long long t = threadIdx.x; t < T; t += blockDim.x)
+            Entry v[2] = {};
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
             {
-                sk[t] = key[base + t];
-                sp[t] = pos[base + t];
-                so[t] = ord[base + t];
+                const long long i = base + 2 * t + e;
+                if (2 * t + e < T)
+                    v[e] = {key[i], pos[i], ord[i]};
             }
-            __syncthreads();
-            for (long long k = k0; k <= k1; k <<= 1)
+            const unsigned b = static_cast<unsigned>(base), all = static_cast<unsigned>(S);
+            sort_steps(v, sm, T, static_cast<unsigned>(k0), static_cast<unsigned>(k1), After{},
+                       [&](unsigned i, unsigned k) { return k == all || ((b + i) & k) == 0; });
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
             {
-                for (long long j = (k >> 1) < (T >> 1) ? (k >> 1) : (T >> 1); j > 0; j >>= 1)
+                const long long i = base + 2 * t + e;
+                if (2 * t + e < T)
                 {
-                    for (long long t = threadIdx.x; t < (T >> 1); t += blockDim.x)
-                    {
-                        const long long i = 2 * t - (t & (j - 1)), q = i + j;
-                        const bool up = k == S || ((base + i) & k) == 0;
-                        const float ki = sk[i], kq = sk[q];
-                        const bool greater = ki > kq || (ki == kq && sp[i] > sp[q]);
-                        if (greater == up)
-                        {
-                            sk[i] = kq;
-                            sk[q] = ki;
-                            const uint32_t a = sp[i];
-                            sp[i] = sp[q];
-                            sp[q] = a;
-                            const uint32_t o = so[i];
-                            so[i] = so[q];
-                            so[q] = o;
-                        }
-                    }
-                    __syncthreads();
+                    key[i] = v[e].key;
+                    pos[i] = v[e].pos;
+                    ord[i] = v[e].ord;
                 }
-            }
-            for (long long t = threadIdx.x; t < T; t += blockDim.x)
-            {
-                key[base + t] = sk[t];
-                pos[base + t] = sp[t];
-                ord[base + t] = so[t];
             }
         }
 
@@ -143,17 +159,12 @@ namespace vg
             return lo;
         }
 
-        // per node of level d: split value, scan ends, children's cells
-        __global__ void split_nodes(const float *key, long long N, int d, float r_max, const float *cell, float *tests,
-                                    NodeInfo *info, float *child_cell)
+        // A node's split value (returned) and scan ends from its S sorted keys at key[begin ..]; the ends
+        // are shifted by `base`, the tile's place in the whole order.
+        __device__ float split_node(const float *key, long long begin, long long S, long long base, float r_max, NodeInfo &ni)
         {
-            const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (t >= (1ll << d))
-                return;
-            const long long S = N >> d, half = S >> 1, begin = t * S;
+            const long long half = S >> 1;
             const float test = __fmul_rn(__fadd_rn(key[begin + half - 1], key[begin + half]), 0.5f);
-            tests[(1ll << d) - 1 + t] = test;
-            NodeInfo ni;
             ni.up = __fadd_rn(test, r_max);
             ni.down = __fsub_rn(test, r_max);
             // lower half, from its smallest key: while key >= down and finite
@@ -167,16 +178,78 @@ namespace vg
                 const long long f = upper_bound(key, begin + half, begin + S, __int_as_float(0x7f7fffff));
                 ni.l = ni.l < f ? ni.l : f;
             }
-            info[t] = ni;
-            const int ax = d % 3;
-            float *lo = child_cell + 12 * t, *hi = lo + 6;
-            for (int k = 0; k < 6; ++k)
+            ni.h += base;
+            ni.l += base;
+            return test;
+        }
+
+        // split_node for every node of level d (heap order)
+        __global__ void split_nodes(const float *key, long long N, int d, float r_max, float *tests, NodeInfo *info)
+        {
+            const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+            if (t < (1ll << d))
             {
-                lo[k] = cell[6 * t + k];
-                hi[k] = cell[6 * t + k];
+                const long long S = N >> d, at = (1ll << d) - 1 + t;
+                tests[at] = split_node(key, t * S, S, 0, r_max, info[at]);
             }
-            lo[3 + ax] = test;  // lower child: upper bound on the axis
-            hi[ax] = test;      // upper child: lower bound on the axis
+        }
+
+        // Levels d0 .. d1 - 1 of subtrees whose nodes at level d0 hold at most T entries: a block of T / 2
+        // threads per tile of T entries sorts every level, splits its nodes and leaves each level's
+        // order in orders[(d - d0) N ..], the last one in ord.  The network of each level is
+        // bitonic_tile's.
+        __global__ void __launch_bounds__(kSortTile / 2) sort_subtrees(const float *px, const float *py, const float *pz, long long N,
+                                                                       int d0, int d1, int T, float r_max, uint32_t *ord,
+                                                                       uint32_t *orders, float *tests, NodeInfo *info)
+        {
+            __shared__ Entry sm[kSortTile];
+            __shared__ float sk[kSortTile];
+            const long long base = static_cast<long long>(blockIdx.x) * T;
+            const int t = threadIdx.x;
+            Entry v[2] = {};
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+            {
+                if (2 * t + e < T)
+                    v[e].ord = ord[base + 2 * t + e];
+            }
+            for (int d = d0; d < d1; ++d)
+            {
+                const long long S = N >> d;
+                const float *axis = d % 3 == 0 ? px : d % 3 == 1 ? py : pz;
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                {
+                    v[e].pos = static_cast<uint32_t>(base + 2 * t + e);
+                    if (2 * t + e < T)
+                        v[e].key = axis[v[e].ord];
+                }
+                const unsigned b = static_cast<unsigned>(base), all = static_cast<unsigned>(S);
+                sort_steps(v, sm, all, 2u, all, After{}, [&](unsigned i, unsigned k) { return k == all || ((b + i) & k) == 0; });
+                uint32_t *order = orders + static_cast<long long>(d - d0) * N + base;
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                {
+                    if (2 * t + e < T)
+                    {
+                        sk[2 * t + e] = v[e].key;
+                        order[2 * t + e] = v[e].ord;
+                    }
+                }
+                __syncthreads();
+                for (int n = t; n < T / S; n += blockDim.x)
+                {
+                    const long long at = (1ll << d) - 1 + base / S + n;
+                    tests[at] = split_node(sk, static_cast<long long>(n) * S, S, base, r_max, info[at]);
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+            {
+                if (2 * t + e < T)
+                    ord[base + 2 * t + e] = v[e].ord;
+            }
         }
 
         // block-wide exclusive scan of one flag per thread; returns the thread's offset, *total
@@ -221,43 +294,27 @@ namespace vg
             return all;
         }
 
-        // children's list sizes of each node (one block per node)
-        __global__ void count_children(const unsigned long long *off, const uint32_t *items, const float *axis, long long N,
-                                       int d, const NodeInfo *info, unsigned long long *sizes)
+        // The children's lists of each node of level d (one block per node): the node's list filtered in
+        // order, then the scanned range.  A node's two lists take their room in `out` from the level's
+        // counter, in any order; range[n] is node n's list.  Past the room `cap` nothing is written (the
+        // counter still says what the level needs) and *full is set.
+        __global__ void child_lists(const ulonglong2 *range, const uint32_t *items, const float *axis, long long N, int d,
+                                    const NodeInfo *info, const uint32_t *ord, unsigned long long cap, unsigned long long *used,
+                                    int *full, ulonglong2 *child_range, uint32_t *out)
         {
+            __shared__ unsigned long long room;
             const long long t = blockIdx.x;
-            const NodeInfo ni = info[t];
-            unsigned long long n_lo = 0, n_hi = 0;
-            for (unsigned long long i = off[t] + threadIdx.x; i < off[t + 1]; i += blockDim.x)
-            {
-                const float v = axis[items[i]];
-                n_lo += v <= ni.up;
-                n_hi += v >= ni.down;
-            }
-            n_lo = block_sum(n_lo);
-            n_hi = block_sum(n_hi);
-            if (threadIdx.x == 0)
-            {
-                const long long S = N >> d, begin = t * S;
-                sizes[2 * t] = n_lo + static_cast<unsigned long long>(ni.l - (begin + S / 2));
-                sizes[2 * t + 1] = n_hi + static_cast<unsigned long long>(ni.h - begin);
-            }
-        }
-
-        // children's lists: the node's list filtered in order, then the scanned range
-        __global__ void write_children(const unsigned long long *off, const uint32_t *items, const float *axis, long long N,
-                                       int d, const NodeInfo *info, const uint32_t *ord, const unsigned long long *child_off,
-                                       uint32_t *child_items)
-        {
-            const long long t = blockIdx.x;
-            const NodeInfo ni = info[t];
-            unsigned long long w_lo = child_off[2 * t], w_hi = child_off[2 * t + 1];
-            const unsigned long long a0 = off[t], a1 = off[t + 1];
-            for (unsigned long long c = a0; c < a1; c += blockDim.x)
-            {
-                const unsigned long long i = c + threadIdx.x;
-                uint32_t it = 0;
-                bool lo = false, hi = false;
+            const NodeInfo ni = info[(1ll << d) - 1 + t];
+            const unsigned long long a0 = range[t].x, a1 = range[t].y;
+            const long long S = N >> d, begin = t * S, half = S / 2;
+            const unsigned long long s_lo = static_cast<unsigned long long>(ni.l - (begin + half)),
+                                     s_hi = static_cast<unsigned long long>(ni.h - begin);
+            // lists of one pass are read once
+            const bool once = a1 - a0 <= kListBlock;
+            uint32_t it = 0;
+            bool lo = false, hi = false;
+            auto load = [&](unsigned long long i) {
+                lo = hi = false;
                 if (i < a1)
                 {
                     it = items[i];
@@ -265,21 +322,99 @@ namespace vg
                     lo = v <= ni.up;
                     hi = v >= ni.down;
                 }
-                unsigned tot_lo, tot_hi;
-                const unsigned p_lo = block_scan(lo ? 1u : 0u, &tot_lo);
-                const unsigned p_hi = block_scan(hi ? 1u : 0u, &tot_hi);
-                if (lo)
-                    child_items[w_lo + p_lo] = it;
-                if (hi)
-                    child_items[w_hi + p_hi] = it;
-                w_lo += tot_lo;
-                w_hi += tot_hi;
+            };
+            unsigned long long n_lo = 0, n_hi = 0;
+            unsigned p_lo = 0, p_hi = 0, tot_lo = 0, tot_hi = 0;
+            if (once)
+            {
+                load(a0 + threadIdx.x);
+                p_lo = block_scan(lo ? 1u : 0u, &tot_lo);
+                p_hi = block_scan(hi ? 1u : 0u, &tot_hi);
+                n_lo = tot_lo;
+                n_hi = tot_hi;
             }
-            const long long S = N >> d, begin = t * S, half = S / 2;
+            else
+            {
+                for (unsigned long long i = a0 + threadIdx.x; i < a1; i += blockDim.x)
+                {
+                    load(i);
+                    n_lo += lo;
+                    n_hi += hi;
+                }
+                n_lo = block_sum(n_lo);
+                n_hi = block_sum(n_hi);
+            }
+            const unsigned long long need = n_lo + s_lo + n_hi + s_hi;
+            if (threadIdx.x == 0)
+                room = need ? atomicAdd(used + d, need) : 0ull;
+            __syncthreads();
+            unsigned long long w_lo = room, w_hi = room + n_lo + s_lo;
+            const bool fits = room + need <= cap;
+            if (threadIdx.x == 0)
+            {
+                child_range[2 * t] = fits ? make_ulonglong2(w_lo, w_hi) : make_ulonglong2(0, 0);
+                child_range[2 * t + 1] = fits ? make_ulonglong2(w_hi, room + need) : make_ulonglong2(0, 0);
+                if (!fits)
+                    *full = 1;
+            }
+            if (!fits)
+                return;
+            if (once)
+            {
+                if (lo)
+                    out[w_lo + p_lo] = it;
+                if (hi)
+                    out[w_hi + p_hi] = it;
+            }
+            else
+            {
+                for (unsigned long long c = a0; c < a1; c += blockDim.x)
+                {
+                    load(c + threadIdx.x);
+                    p_lo = block_scan(lo ? 1u : 0u, &tot_lo);
+                    p_hi = block_scan(hi ? 1u : 0u, &tot_hi);
+                    if (lo)
+                        out[w_lo + p_lo] = it;
+                    if (hi)
+                        out[w_hi + p_hi] = it;
+                    w_lo += tot_lo;
+                    w_hi += tot_hi;
+                }
+                n_lo = n_hi = 0;
+            }
             for (long long i = begin + half + threadIdx.x; i < ni.l; i += blockDim.x)
-                child_items[w_lo + (i - begin - half)] = ord[i];
+                out[w_lo + n_lo + (i - begin - half)] = ord[i];
             for (long long i = begin + threadIdx.x; i < ni.h; i += blockDim.x)
-                child_items[w_hi + (i - begin)] = ord[i];
+                out[w_hi + n_hi + (i - begin)] = ord[i];
+        }
+
+        // each leaf's cell: the split planes along its path (right child: coordinate >= test)
+        __global__ void leaf_cells(const float *tests, int nlog2, float *cell)
+        {
+            const long long leaf = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+            if (leaf >= 1ll << nlog2)
+                return;
+            float lo[3] = {-kInf, -kInf, -kInf}, hi[3] = {kInf, kInf, kInf};
+            long long idx = 0;
+            for (int d = 0; d < nlog2; ++d)
+            {
+                const bool right = (leaf >> (nlog2 - 1 - d)) & 1;
+                const float t = tests[idx];
+                for (int k = 0; k < 3; ++k)
+                {
+                    if (k == d % 3)
+                    {
+                        lo[k] = right ? t : lo[k];
+                        hi[k] = right ? hi[k] : t;
+                    }
+                }
+                idx = 2 * idx + 1 + right;
+            }
+            for (int k = 0; k < 3; ++k)
+            {
+                cell[6 * leaf + k] = lo[k];
+                cell[6 * leaf + 3 + k] = hi[k];
+            }
         }
 
         __device__ float cell_distsq(const float *c, float x, float y, float z)
@@ -309,7 +444,7 @@ namespace vg
 
         struct LeafParams
         {
-            const unsigned long long *off;
+            const ulonglong2 *range;
             const uint32_t *items;
             const float *px, *py, *pz;
             const uint32_t *ord;
@@ -318,7 +453,7 @@ namespace vg
         };
 
         // number of 8-point blocks of each leaf (one block of threads per leaf)
-        __global__ void count_leaves(const LeafParams p, unsigned long long *blocks)
+        __global__ void count_leaves(const LeafParams p, uint32_t *blocks)
         {
             const long long t = blockIdx.x;
             const uint32_t rep = p.ord[t];
@@ -328,7 +463,8 @@ namespace vg
             const bool finite = rx < kInf && rx > -kInf;
             if (finite && !cell_inside_ball(c, rx, ry, rz, p.min_l2))
             {
-                for (unsigned long long i = p.off[t] + threadIdx.x; i < p.off[t + 1]; i += blockDim.x)
+                const ulonglong2 list = p.range[t];
+                for (unsigned long long i = list.x + threadIdx.x; i < list.y; i += blockDim.x)
                 {
                     const uint32_t it = p.items[i];
                     acc += cell_distsq(c, p.px[it], p.py[it], p.pz[it]) <= p.max_l2;
@@ -336,7 +472,7 @@ namespace vg
             }
             acc = block_sum(acc);
             if (threadIdx.x == 0)
-                blocks[t] = finite ? (acc + 1 + 7) / 8 : 0;
+                blocks[t] = static_cast<uint32_t>(finite ? (acc + 1 + 7) / 8 : 0);
         }
 
         __device__ float block_min(float v)
@@ -356,7 +492,7 @@ namespace vg
 
         // each leaf's blocks (its representative, then its accepted points in list order, padded
         // with +inf) and its box
-        __global__ void write_leaves(const LeafParams p, const unsigned long long *starts, float *aff, float *aabbs)
+        __global__ void write_leaves(const LeafParams p, const uint32_t *starts, float *aff, float *aabbs)
         {
             const long long t = blockIdx.x;
             const uint32_t rep = p.ord[t];
@@ -380,12 +516,13 @@ namespace vg
                 unsigned long long w = 1;
                 if (!cell_inside_ball(c, rx, ry, rz, p.min_l2))
                 {
-                    for (unsigned long long s = p.off[t]; s < p.off[t + 1]; s += blockDim.x)
+                    const ulonglong2 list = p.range[t];
+                    for (unsigned long long s = list.x; s < list.y; s += blockDim.x)
                     {
                         const unsigned long long i = s + threadIdx.x;
                         bool ok = false;
                         float x = 0, y = 0, z = 0;
-                        if (i < p.off[t + 1])
+                        if (i < list.y)
                         {
                             const uint32_t it = p.items[i];
                             x = p.px[it];
@@ -426,14 +563,80 @@ namespace vg
             }
         }
 
-        // box of every finite representative (one block)
-        __global__ void top_box(const uint32_t *ord, const float *px, const float *py, const float *pz, long long N,
-                                float *top)
+        // what the host needs of a finished tree
+        struct Summary
         {
-            float mn[3] = {kInf, kInf, kInf}, mx[3] = {-kInf, -kInf, -kInf};
-            for (long long t = threadIdx.x; t < N; t += blockDim.x)
+            unsigned long long blocks;
+            float top[6];        // box of every finite representative
+            float top_tests[3];  // the first split values
+            int full;
+        };
+
+        // The leaves' first blocks (exclusive sums of their counts, starts[N] the total) by block 0, the
+        // box of the finite representatives by block 1.
+        __global__ void __launch_bounds__(1024) finish_tree(const uint32_t *blocks, long long N, uint32_t *starts, const uint32_t *ord,
+                                                            const float *px, const float *py, const float *pz,
+                                                            const float *tests, const int *full, Summary *sum)
+        {
+            const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+            if (blockIdx.x == 0)
             {
-                const uint32_t r = ord[t];
+                __shared__ unsigned long long wsum[32];
+                // 1024 consecutive counts a round, the sums of the rounds before carried
+                __shared__ unsigned long long carry;
+                if (t == 0)
+                    carry = 0;
+                for (long long c = 0; c < N; c += 1024 * 8)
+                {
+                    // eight consecutive counts a thread
+                    uint32_t v[8];
+                    unsigned long long mine = 0;
+                    const long long i0 = c + 8 * t;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                    {
+                        v[k] = i0 + k < N ? blocks[i0 + k] : 0u;
+                        mine += v[k];
+                    }
+                    unsigned long long x = mine;
+                    for (int o = 1; o < 32; o <<= 1)
+                    {
+                        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+                        if (lane >= o)
+                            x += y;
+                    }
+                    if (lane == 31)
+                        wsum[warp] = x;
+                    __syncthreads();
+                    unsigned long long at = carry + x - mine;
+                    for (int w = 0; w < warp; ++w)
+                        at += wsum[w];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                    {
+                        if (i0 + k < N)
+                            starts[i0 + k] = static_cast<uint32_t>(at);
+                        at += v[k];
+                    }
+                    __syncthreads();
+                    if (t == 1023)
+                        carry = at;
+                    __syncthreads();
+                }
+                if (t == 0)
+                {
+                    starts[N] = static_cast<uint32_t>(carry);
+                    sum->blocks = carry;
+                    sum->full = *full;
+                    for (int k = 0; k < 3; ++k)
+                        sum->top_tests[k] = k < N - 1 ? tests[k] : 0.0f;
+                }
+                return;
+            }
+            float mn[3] = {kInf, kInf, kInf}, mx[3] = {-kInf, -kInf, -kInf};
+            for (long long i = t; i < N; i += 1024)
+            {
+                const uint32_t r = ord[i];
                 const float v[3] = {px[r], py[r], pz[r]};
                 if (v[0] < kInf && v[0] > -kInf)
                 {
@@ -444,75 +647,28 @@ namespace vg
                     }
                 }
             }
+            __shared__ float part[6][32];
             for (int k = 0; k < 3; ++k)
             {
-                const float a = block_min(mn[k]), b = -block_min(-mx[k]);
-                if (threadIdx.x == 0)
+                for (int o = 16; o > 0; o >>= 1)
                 {
-                    top[k] = a;
-                    top[3 + k] = b;
+                    mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
+                    mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+                }
+                if (lane == 0)
+                {
+                    part[k][warp] = mn[k];
+                    part[3 + k][warp] = mx[k];
                 }
             }
-        }
-
-        // exclusive scan of n values (one block), out[n] = total
-        __global__ void scan_small(const unsigned long long *in, long long n, unsigned long long *out)
-        {
-            __shared__ unsigned long long carry;
-            if (threadIdx.x == 0)
-                carry = 0;
             __syncthreads();
-            for (long long c = 0; c < n; c += blockDim.x)
+            if (t < 6)
             {
-                const long long i = c + threadIdx.x;
-                const unsigned long long v = i < n ? in[i] : 0;
-                // inclusive scan within the block (warp shuffles, then warp totals)
-                __shared__ unsigned long long wsum[32];
-                unsigned long long x = v;
-                const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-                for (int o = 1; o < 32; o <<= 1)
-                {
-                    const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o)
-                        x += y;
-                }
-                if (lane == 31)
-                    wsum[warp] = x;
-                __syncthreads();
-                unsigned long long base = 0;
-                for (int w = 0; w < warp; ++w)
-                    base += wsum[w];
-                if (i < n)
-                    out[i] = carry + base + x - v;
-                __syncthreads();
-                if (threadIdx.x == blockDim.x - 1)
-                    carry += base + x;
-                __syncthreads();
+                float v = part[t][0];
+                for (int w = 1; w < 32; ++w)
+                    v = t < 3 ? fminf(v, part[t][w]) : fmaxf(v, part[t][w]);
+                sum->top[t] = v;
             }
-            if (threadIdx.x == 0)
-                out[n] = carry;
-        }
-
-        __global__ void narrow_starts(const unsigned long long *in, long long n, uint32_t *out)
-        {
-            const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (i < n)
-                out[i] = static_cast<uint32_t>(in[i]);
-        }
-
-        template <typename T>
-        cudaError_t grow(T **p, size_t *cap, size_t need)
-        {
-            if (need <= *cap)
-                return cudaSuccess;
-            if (*p)
-                cudaFree(*p);
-            *p = nullptr;
-            *cap = 0;
-            const cudaError_t e = cudaMalloc(p, std::max<size_t>(need, 1) * sizeof(T));
-            if (e == cudaSuccess)
-                *cap = need;
-            return e;
         }
 
         unsigned grid_of(long long n, int block)
@@ -535,154 +691,197 @@ namespace vg
         out.r_min = r_min;
         out.r_max = r_max;
         out.r_point = r_point;
-        float *px = nullptr, *py = nullptr, *pz = nullptr, *key = nullptr, *cell = nullptr, *child_cell = nullptr;
-        uint32_t *ord = nullptr, *pos = nullptr, *items = nullptr, *child_items = nullptr;
-        unsigned long long *off = nullptr, *child_off = nullptr, *sizes = nullptr;
-        NodeInfo *info = nullptr;
-        size_t items_cap = 0, child_cap = 0;
+        // the first level whose nodes fit a tile: its subtrees sort in one launch, where their levels'
+        // orders (4 bytes an entry and level) are no burden
+        int d0 = 0;
+        while ((N >> d0) > kSortTile)
+            ++d0;
+        int d1 = d0;  // the first level of nodes of kSmallTile entries (d0 in smaller trees)
+        while ((N >> d1) > kSmallTile)
+            ++d1;
+        const bool subtrees = N <= kOrdersMax;
+        const int T = static_cast<int>(std::min<long long>(N, kSortTile));
+        // Room for a level's lists: 104 entries a leaf in the Panda's tree of 50,000 points.  A tree for
+        // larger spheres needs more, and starts again.
+        unsigned long long cap = static_cast<unsigned long long>(
+            std::min<long long>(std::max<long long>(160 * N, 1 << 18), std::max<long long>(1ll << 28, 2 * N)));
+        unsigned long long least = 0;  // what the last level that ran out needs
         cudaError_t e = cudaSuccess;
-        // the fixed-size scratch in one allocation (carved in 256-byte aligned pieces)
-        char *scratch = nullptr;
+        // results: split values, boxes, starts and the points, in one allocation
         {
-            size_t used = 0;
+            const size_t tests = (static_cast<size_t>(N) * sizeof(float) + 255) & ~size_t(255);
+            const size_t boxes = (6 * static_cast<size_t>(N) * sizeof(float) + 255) & ~size_t(255);
+            const size_t starts = ((static_cast<size_t>(N) + 1) * sizeof(uint32_t) + 255) & ~size_t(255);
+            char *base = nullptr;
+            e = pool_take(reinterpret_cast<void **>(&base), tests + boxes + starts + 3 * n * sizeof(float), s);
+            if (e == cudaSuccess)
+            {
+                out.tests = reinterpret_cast<float *>(base);
+                out.aabbs = reinterpret_cast<float *>(base + tests);
+                out.starts = reinterpret_cast<uint32_t *>(base + tests + boxes);
+                out.points = reinterpret_cast<float *>(base + tests + boxes + starts);
+                e = cudaMemcpyAsync(out.points, xyz, 3 * n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+            }
+        }
+        Summary sum{};
+        while (e == cudaSuccess)
+        {
+            float *px, *py, *pz, *key, *cell;
+            uint32_t *ord, *pos, *orders, *items, *child_items, *blocks;
+            ulonglong2 *range, *child_range;
+            unsigned long long *used;
+            NodeInfo *info;
+            Summary *d_sum;
+            int *full;
+            char *scratch = nullptr;
+            size_t bytes = 0;
             auto carve = [&](auto **p, size_t count) {
-                const size_t at = used;
-                used += (std::max<size_t>(count, 1) * sizeof(**p) + 255) & ~size_t(255);
+                const size_t at = bytes;
+                bytes += (std::max<size_t>(count, 1) * sizeof(**p) + 255) & ~size_t(255);
                 *p = scratch ? reinterpret_cast<std::remove_reference_t<decltype(*p)>>(scratch + at) : nullptr;
             };
             auto carve_all = [&]() {
-                used = 0;
+                bytes = 0;
+                carve(&used, 32);
+                carve(&full, 1);
+                carve(&d_sum, 1);
                 carve(&px, N);
                 carve(&py, N);
                 carve(&pz, N);
                 carve(&key, N);
                 carve(&ord, N);
                 carve(&pos, N);
+                carve(&orders, subtrees ? N * (nlog2 - d0) : 1);
                 carve(&cell, 6 * N);
-                carve(&child_cell, 6 * N);
-                carve(&off, N + 1);
-                carve(&child_off, N + 1);
-                carve(&sizes, N);
-                carve(&info, N / 2 > 0 ? N / 2 : 1);
+                carve(&range, N);
+                carve(&child_range, N);
+                carve(&info, N);
+                carve(&blocks, N);
+                carve(&items, cap);
+                carve(&child_items, cap);
             };
             carve_all();
-            e = cudaMalloc(&scratch, used);
-            if (e == cudaSuccess)
-                carve_all();
-        }
-        auto alloc = [&](auto **p, size_t count) {
-            if (e == cudaSuccess)
-                e = cudaMalloc(p, std::max<size_t>(count, 1) * sizeof(**p));
-        };
-        alloc(&out.tests, N - 1);
-        alloc(&out.aabbs, 6 * N);
-        alloc(&out.starts_dev, N + 1);
-        alloc(&out.top_dev, 6);
-        const float *axis[3] = {px, py, pz};
-        if (e == cudaSuccess)
-        {
-            init_points<<<grid_of(N, 256), 256, 0, s>>>(xyz, static_cast<long long>(n), N, px, py, pz, ord);
-            const float root[6] = {-kInf, -kInf, -kInf, kInf, kInf, kInf};
-            e = cudaMemcpyAsync(cell, root, sizeof(root), cudaMemcpyHostToDevice, s);
-        }
-        if (e == cudaSuccess)
-            e = cudaMemsetAsync(off, 0, 2 * sizeof(unsigned long long), s);  // root: empty list
-        for (int d = 0; d < nlog2 && e == cudaSuccess; ++d)
-        {
-            const long long nodes = 1ll << d, S = N >> d;
-            load_keys<<<grid_of(N, 256), 256, 0, s>>>(ord, axis[d % 3], N, key, pos);
-            // strides below the tile in shared memory, the longer ones one launch each
-            const long long T = std::min<long long>(S, kSortTile);
-            const unsigned tiles = static_cast<unsigned>(N / T), threads = static_cast<unsigned>(std::max<long long>(T / 2, 1));
-            bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, 2, T);
-            for (long long k = 2 * T; k <= S; k <<= 1)
+            e = pool_take(reinterpret_cast<void **>(&scratch), bytes, s);
+            if (e == cudaErrorMemoryAllocation && least && cap > least)
             {
-                for (long long j = k >> 1; j >= T; j >>= 1)
-                    bitonic_stage<<<grid_of(N, 256), 256, 0, s>>>(key, pos, ord, N, k, j, S);
-                bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, k, k);
+                // not four times as much, then
+                cudaGetLastError();
+                cap = least;
+                e = cudaSuccess;
+                continue;
             }
-            split_nodes<<<grid_of(nodes, 128), 128, 0, s>>>(key, N, d, r_max, cell, out.tests, info, child_cell);
-            count_children<<<static_cast<unsigned>(nodes), kListBlock, 0, s>>>(off, items, axis[d % 3], N, d, info, sizes);
-            scan_small<<<1, 1024, 0, s>>>(sizes, 2 * nodes, child_off);
-            unsigned long long total = 0;
-            e = cudaMemcpyAsync(&total, child_off + 2 * nodes, sizeof(total), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess)
-                e = cudaStreamSynchronize(s);
-            if (e == cudaSuccess)
-                e = grow(&child_items, &child_cap, total);
             if (e != cudaSuccess)
                 break;
-            write_children<<<static_cast<unsigned>(nodes), kListBlock, 0, s>>>(off, items, axis[d % 3], N, d, info, ord,
-                                                                                child_off, child_items);
-            e = cudaGetLastError();
-            std::swap(off, child_off);
-            std::swap(items, child_items);
-            std::swap(items_cap, child_cap);
-            std::swap(cell, child_cell);
-        }
-        // leaves
-        LeafParams lp{off, items, px, py, pz, ord, cell, 0.0f, 0.0f};
-        {
-            const float l1 = r_max + r_point, l0 = r_min + r_point;
-            lp.max_l2 = l1 * l1;
-            lp.min_l2 = l0 * l0;
-        }
-        if (e == cudaSuccess)
-        {
-            count_leaves<<<static_cast<unsigned>(N), kListBlock, 0, s>>>(lp, sizes);
-            scan_small<<<1, 1024, 0, s>>>(sizes, N, out.starts_dev);
-            unsigned long long total = 0;
-            e = cudaMemcpyAsync(&total, out.starts_dev + N, sizeof(total), cudaMemcpyDeviceToHost, s);
+            carve_all();
+            const float *axis[3] = {px, py, pz};
+            // counters, *full and the root's empty list are zeros
+            e = cudaMemsetAsync(used, 0, reinterpret_cast<char *>(d_sum) - reinterpret_cast<char *>(used), s);
             if (e == cudaSuccess)
-                e = cudaStreamSynchronize(s);
-            out.blocks = total;
-            if (e == cudaSuccess)
-                e = cudaMalloc(&out.aff, std::max<size_t>(24 * total, 4) * sizeof(float));
+                e = cudaMemsetAsync(range, 0, sizeof(ulonglong2), s);
+            init_points<<<grid_of(N, 256), 256, 0, s>>>(xyz, static_cast<long long>(n), N, px, py, pz, ord);
+            for (int d = 0; d < nlog2 && e == cudaSuccess; ++d)
+            {
+                const long long nodes = 1ll << d, S = N >> d;
+                const uint32_t *order = ord;
+                if (subtrees && d >= d0)
+                {
+                    if (d == d0 || d == d1)
+                    {
+                        // full tiles down to nodes of kSmallTile entries, which then sort on more SMs
+                        // (2,048 entries on one: 94 us for all eleven levels)
+                        const int tile = d == d1 ? static_cast<int>(S) : T;
+                        sort_subtrees<<<static_cast<unsigned>(N / tile), std::max(tile / 2, 32), 0, s>>>(
+                            px, py, pz, N, d, d < d1 ? d1 : nlog2, tile, r_max, ord, orders + static_cast<long long>(d - d0) * N,
+                            out.tests, info);
+                    }
+                    order = orders + static_cast<long long>(d - d0) * N;
+                }
+                else
+                {
+                    load_keys<<<grid_of(N, 256), 256, 0, s>>>(ord, axis[d % 3], N, key, pos);
+                    // strides below the tile in shared memory, the longer ones one launch each
+                    const long long st = std::min<long long>(S, kSortTile);
+                    const unsigned tiles = static_cast<unsigned>(N / st),
+                                   threads = static_cast<unsigned>(std::max<long long>(st / 2, 32));
+                    bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, 2, st);
+                    for (long long k = 2 * st; k <= S; k <<= 1)
+                    {
+                        for (long long j = k >> 1; j >= st; j >>= 1)
+                            bitonic_stage<<<grid_of(N, 256), 256, 0, s>>>(key, pos, ord, N, k, j, S);
+                        bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, k, k);
+                    }
+                    split_nodes<<<grid_of(nodes, 128), 128, 0, s>>>(key, N, d, r_max, out.tests, info);
+                }
+                child_lists<<<static_cast<unsigned>(nodes), kListBlock, 0, s>>>(range, items, axis[d % 3], N, d, info, order, cap,
+                                                                               used, full, child_range, child_items);
+                e = cudaGetLastError();
+                std::swap(range, child_range);
+                std::swap(items, child_items);
+            }
+            LeafParams lp{range, items, px, py, pz, ord, cell, 0.0f, 0.0f};
+            {
+                const float l1 = r_max + r_point, l0 = r_min + r_point;
+                lp.max_l2 = l1 * l1;
+                lp.min_l2 = l0 * l0;
+            }
+            unsigned long long h_used[32] = {};
             if (e == cudaSuccess)
             {
-                write_leaves<<<static_cast<unsigned>(N), kListBlock, 0, s>>>(lp, out.starts_dev, out.aff, out.aabbs);
-                top_box<<<1, kListBlock, 0, s>>>(ord, px, py, pz, N, out.top_dev);
+                leaf_cells<<<grid_of(N, 256), 256, 0, s>>>(out.tests, nlog2, cell);
+                count_leaves<<<static_cast<unsigned>(N), kListBlock, 0, s>>>(lp, blocks);
+                finish_tree<<<2, 1024, 0, s>>>(blocks, N, out.starts, ord, px, py, pz, out.tests, full, d_sum);
                 e = cudaGetLastError();
             }
             if (e == cudaSuccess)
-                e = cudaMalloc(&out.starts, (N + 1) * sizeof(uint32_t));
+                e = cudaMemcpyAsync(&sum, d_sum, sizeof(sum), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess)
-            {
-                narrow_starts<<<grid_of(N + 1, 256), 256, 0, s>>>(out.starts_dev, N + 1, out.starts);
-                e = cudaMemcpyAsync(out.top, out.top_dev, sizeof(out.top), cudaMemcpyDeviceToHost, s);
-            }
+                e = cudaMemcpyAsync(h_used, used, sizeof(h_used), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess)
                 e = cudaStreamSynchronize(s);
-            if (out.starts_dev)
-                cudaFree(out.starts_dev);
-            if (out.top_dev)
-                cudaFree(out.top_dev);
-            out.starts_dev = nullptr;
-            out.top_dev = nullptr;
+            if (e == cudaSuccess && !sum.full)
+            {
+                e = pool_take(reinterpret_cast<void **>(&out.aff), std::max<size_t>(24 * sum.blocks, 4) * sizeof(float), s);
+                if (e == cudaSuccess)
+                {
+                    write_leaves<<<static_cast<unsigned>(N), kListBlock, 0, s>>>(lp, out.starts, out.aff, out.aabbs);
+                    e = cudaGetLastError();
+                }
+            }
+            pool_give(scratch, s);
+            if (e != cudaSuccess || !sum.full)
+                break;
+            // a level ran out of room: as much as the first such level needs, and four times more for
+            // the levels below
+            for (int d = 0; d < nlog2; ++d)
+            {
+                if (h_used[d] > cap)
+                {
+                    least = h_used[d];
+                    cap = 4 * least;
+                    break;
+                }
+            }
         }
-        for (void *p : {static_cast<void *>(scratch), static_cast<void *>(items), static_cast<void *>(child_items)})
+        if (e == cudaSuccess)
         {
-            if (p)
-                cudaFree(p);
+            out.blocks = sum.blocks;
+            for (int k = 0; k < 6; ++k)
+                out.top[k] = sum.top[k];
+            for (int k = 0; k < 3; ++k)
+                out.top_tests[k] = sum.top_tests[k];
+            return VG_OK;
         }
-        if (e != cudaSuccess)
-        {
-            out.release();
-            return set_error(VG_ERR_CUDA, std::string("CAPT build on the GPU: ") + cudaGetErrorString(e));
-        }
-        return VG_OK;
+        cudaStreamSynchronize(s);
+        out.release();
+        return set_error(VG_ERR_CUDA, std::string("CAPT build on the GPU: ") + cudaGetErrorString(e));
     }
 
     void DeviceCapt::release()
     {
-        for (void *p : {static_cast<void *>(tests), static_cast<void *>(aabbs), static_cast<void *>(starts_dev),
-                        static_cast<void *>(aff), static_cast<void *>(top_dev), static_cast<void *>(starts)})
-        {
-            if (p)
-                cudaFree(p);
-        }
-        tests = aabbs = aff = top_dev = nullptr;
-        starts_dev = nullptr;
+        // tests is the start of one allocation with aabbs, starts and points
+        pool_give(tests, 0);
+        pool_give(aff, 0);
+        tests = aabbs = aff = points = nullptr;
         starts = nullptr;
     }
 }  // namespace vg

@@ -24,6 +24,7 @@
 
 #include "../../include/vamp_gb300.h"
 #include "vg_internal.h"
+#include "vg_pool.h"
 
 #include <cmath>
 #include <string>
@@ -173,7 +174,7 @@ namespace vg
     }  // namespace
 
     int capt_query_layout(const float *tests, int nlog2, const float *aabbs, const uint32_t *starts, const float *aff,
-                          size_t blocks, float r_max, float r_point, CaptQuery &q)
+                          size_t blocks, float r_max, float r_point, const float *top_tests, cudaStream_t s, CaptQuery &q)
     {
         q = CaptQuery{};
         q.rem = nlog2 % 3;
@@ -186,39 +187,39 @@ namespace vg
         const size_t node_bytes = static_cast<size_t>(n_nodes) * 2 * sizeof(float4);
         const size_t leaf_bytes = static_cast<size_t>(leaves) * 2 * sizeof(float4);
         const size_t end_bytes = static_cast<size_t>(leaves) * kCaptRings * sizeof(uint32_t);
-        cudaError_t e = cudaMalloc(&q.aff_q, std::max<size_t>(blocks, 1) * 24 * sizeof(float));
-        if (e == cudaSuccess)
-            e = cudaMalloc(&q.tables, node_bytes + leaf_bytes + end_bytes);
+        const size_t aff_bytes = (std::max<size_t>(blocks, 1) * 24 * sizeof(float) + 255) & ~size_t(255);
+        char *base = nullptr;
+        cudaError_t e = pool_take(reinterpret_cast<void **>(&base), aff_bytes + node_bytes + leaf_bytes + end_bytes, s);
         if (e == cudaSuccess)
         {
-            char *base = static_cast<char *>(q.tables);
+            q.aff_q = reinterpret_cast<float *>(base);
+            base += aff_bytes;
             q.nodes = reinterpret_cast<float4 *>(base);
             q.leaves = reinterpret_cast<float4 *>(base + node_bytes);
             q.ends = reinterpret_cast<uint32_t *>(base + node_bytes + leaf_bytes);
             const int top = static_cast<int>(std::min<long long>(3, leaves - 1));
-            if (top > 0)
+            for (int k = 0; top_tests && k < top; ++k)
+                q.top_tests[k] = top_tests[k];
+            if (!top_tests && top > 0)
                 e = cudaMemcpy(q.top_tests, tests, top * sizeof(float), cudaMemcpyDeviceToHost);
         }
         if (e == cudaSuccess && n_nodes > 0)
         {
             const int grid = static_cast<int>(std::min<long long>((n_nodes + 255) / 256, 4096));
-            nodes_kernel<<<grid, 256>>>(tests, q.rem, n_nodes, q.nodes);
+            nodes_kernel<<<grid, 256, 0, s>>>(tests, q.rem, n_nodes, q.nodes);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess)
         {
-            leaf_kernel<<<static_cast<unsigned>(leaves), kRingThreads>>>(tests, nlog2, aabbs, starts, aff, step, q.aff_q,
+            leaf_kernel<<<static_cast<unsigned>(leaves), kRingThreads, 0, s>>>(tests, nlog2, aabbs, starts, aff, step, q.aff_q,
                                                                          q.leaves, q.ends);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess)
-            e = cudaDeviceSynchronize();
+            e = cudaStreamSynchronize(s);
         if (e != cudaSuccess)
         {
-            if (q.aff_q)
-                cudaFree(q.aff_q);
-            if (q.tables)
-                cudaFree(q.tables);
+            pool_give(q.aff_q, s);
             q = CaptQuery{};
             return set_error(VG_ERR_CUDA, std::string("CAPT query tables: ") + cudaGetErrorString(e));
         }

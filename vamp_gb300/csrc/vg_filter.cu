@@ -6,7 +6,7 @@
 //   1. codes: one 64-bit key per entry, (Morton code << 32) | position, so that sorting the keys
 //      is the stable sort by code; the coordinate range of the next pass is reduced on the side;
 //   2. a sort of the keys: a stable radix sort on the code for long lists, a bitonic network
-//      (shared-memory tiles of 2048 for the short strides) for short ones;
+//      (tiles of 8192 in registers for the short strides) for short ones;
 //   3. next[j]: the first entry after j that is farther than min_dist from entry j, found by a
 //      forward scan that skips 32-, 1024- and 32768-entry tiles whose bounding box lies inside
 //      the min_dist ball (tested in double with a margin, so a skipped entry is never "far");
@@ -22,6 +22,8 @@
 // single entry placed after the passing points.
 #include "../../include/vamp_gb300.h"
 #include "vg_internal.h"
+#include "vg_pool.h"
+#include "vg_sort.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -32,7 +34,9 @@ namespace vg
     namespace
     {
         constexpr int kTile = 1024;      // entries per scan tile and per chain chunk
-        constexpr int kSortTile = 2048;  // entries per shared-memory bitonic tile
+        constexpr int kSortTile = 8192;  // keys per bitonic tile
+        constexpr int kSortPer = 8;      // of them per thread
+        constexpr int kSortMin = 256;    // keys of the smallest sort (a warp's tile)
         constexpr int kCodeBlock = 256;
         constexpr long long kRadixMin = 16384;  // lists longer than this are radix-sorted
 
@@ -111,17 +115,24 @@ namespace vg
             int cull;
         };
 
-        __global__ void cull_kernel(const float *xyz, long long n, CullParams c, uint32_t *flags)
+        // flags of the points that pass, and how many do in each tile
+        __global__ void __launch_bounds__(kTile) cull_kernel(const float *xyz, long long n, CullParams c, uint32_t *flags,
+                                                             uint32_t *sums)
         {
-            const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (i >= n)
-                return;
-            const float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
-            bool pass = true;
-            if (c.cull)
-                pass = sqdist(x, y, z, c.ox, c.oy, c.oz) < c.sq_range && c.lo[0] <= x && x <= c.hi[0] && c.lo[1] <= y &&
-                       y <= c.hi[1] && c.lo[2] <= z && z <= c.hi[2];
-            flags[i] = pass ? 1u : 0u;
+            const long long i = static_cast<long long>(blockIdx.x) * kTile + threadIdx.x;
+            bool pass = false;
+            if (i < n)
+            {
+                const float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+                pass = true;
+                if (c.cull)
+                    pass = sqdist(x, y, z, c.ox, c.oy, c.oz) < c.sq_range && c.lo[0] <= x && x <= c.hi[0] && c.lo[1] <= y &&
+                           y <= c.hi[1] && c.lo[2] <= z && z <= c.hi[2];
+                flags[i] = pass ? 1u : 0u;
+            }
+            const int total = __syncthreads_count(pass);
+            if (threadIdx.x == 0)
+                sums[blockIdx.x] = static_cast<uint32_t>(total);
         }
 
         __global__ void tile_sums(const uint32_t *flags, long long n, uint32_t *sums)
@@ -156,16 +167,33 @@ namespace vg
                 out[n] = carry;
         }
 
-        // out[offset of j] = src ? src[j] : j, for every flagged j, in order
-        __global__ void compact(const uint32_t *flags, long long n, const uint32_t *offs, const uint32_t *src,
-                                uint32_t *out)
+        // out[offset of j] = src ? src[j] : j, for every flagged j, in order.  A tile's offset is the sum of
+        // the tiles before it: of up to kDirectTiles sums each block adds them up itself, of more `sums`
+        // holds the offsets already (scan_tiles).  The last block writes the total to *count.
+        constexpr long long kDirectTiles = 2048;
+
+        __global__ void __launch_bounds__(kTile) compact(const uint32_t *flags, long long n, const uint32_t *sums, long long tiles,
+                                                         const uint32_t *src, uint32_t *out, uint32_t *count)
         {
             const long long i = static_cast<long long>(blockIdx.x) * kTile + threadIdx.x;
             const uint32_t f = i < n ? flags[i] : 0u;
-            uint32_t total;
+            uint32_t total, offset;
             const uint32_t at = block_scan(f, &total);
+            if (tiles <= kDirectTiles)
+            {
+                uint32_t mine = 0u;
+                for (long long k = threadIdx.x; k < blockIdx.x; k += kTile)
+                    mine += sums[k];
+                block_scan(mine, &offset);
+            }
+            else
+            {
+                offset = sums[blockIdx.x];
+            }
             if (f)
-                out[offs[blockIdx.x] + at] = src ? src[i] : static_cast<uint32_t>(i);
+                out[offset + at] = src ? src[i] : static_cast<uint32_t>(i);
+            if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+                *count = offset + total;
         }
 
         // --- one pass ---------------------------------------------------------------------
@@ -269,32 +297,33 @@ namespace vg
             }
         }
 
-        // all merge steps of stride < T for sizes k in [k0, k1], on tiles of T = min(M, 2048) keys
-        __global__ void bitonic_tile(unsigned long long *keys, long long M, long long k0, long long k1)
+        // all merge steps of stride < T for sizes k in [k0, k1], on tiles of T = min(M, 8192) keys, eight
+        // a thread (M >= 256)
+        __global__ void __launch_bounds__(kSortTile / kSortPer) bitonic_tile(unsigned long long *keys, long long M, long long k0,
+                                                                             long long k1)
         {
-            __shared__ unsigned long long s[kSortTile];
-            const long long T = M < kSortTile ? M : kSortTile;
+            extern __shared__ unsigned long long tile_smem[];
+            const int T = static_cast<int>(M < kSortTile ? M : kSortTile), t = threadIdx.x;
             const long long base = static_cast<long long>(blockIdx.x) * T;
-            for (long long t = threadIdx.x; t < T; t += blockDim.x)
-                s[t] = keys[base + t];
-            __syncthreads();
-            for (long long k = k0; k <= k1; k <<= 1)
+            unsigned long long v[kSortPer];
+            ulonglong2 *at = reinterpret_cast<ulonglong2 *>(keys + base + kSortPer * t);
+#pragma unroll
+            for (int e = 0; e < kSortPer; e += 2)
             {
-                for (long long j = (k >> 1) < (T >> 1) ? (k >> 1) : (T >> 1); j > 0; j >>= 1)
-                {
-                    for (long long t = threadIdx.x; t < (T >> 1); t += blockDim.x)
-                    {
-                        const long long i = 2 * t - (t & (j - 1));  // lower element of the t-th pair
-                        cmp_swap(s[i], s[i + j], ((base + i) & k) == 0);
-                    }
-                    __syncthreads();
-                }
+                const ulonglong2 p = at[e / 2];
+                v[e] = p.x;
+                v[e + 1] = p.y;
             }
-            for (long long t = threadIdx.x; t < T; t += blockDim.x)
-                keys[base + t] = s[t];
+            const unsigned b = static_cast<unsigned>(base);
+            sort_steps(v, tile_smem, T, static_cast<unsigned>(k0), static_cast<unsigned>(k1),
+                       [](unsigned long long x, unsigned long long y) { return x > y; },
+                       [&](unsigned i, unsigned k) { return ((b + i) & k) == 0; });
+#pragma unroll
+            for (int e = 0; e < kSortPer; e += 2)
+                at[e / 2] = make_ulonglong2(v[e], v[e + 1]);
         }
 
-        // one merge step of stride j >= 2048
+        // one merge step of stride j >= 8192
         __global__ void bitonic_step(unsigned long long *keys, long long M, long long k, long long j)
         {
             const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -363,59 +392,58 @@ namespace vg
             }
         }
 
-        // the sorted entries' point indices and coordinates
-        __global__ void gather_sorted(const unsigned long long *keys, const uint32_t *list, long long m, const float *xyz,
-                                      uint32_t *sidx, float4 *sp)
-        {
-            const long long j = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (j >= m)
-                return;
-            const uint32_t idx = list[static_cast<uint32_t>(keys[j])];
-            sidx[j] = idx;
-            const float *p = xyz + 3 * static_cast<size_t>(idx);
-            sp[j] = make_float4(p[0], p[1], p[2], 0.0f);
-        }
-
         struct Box
         {
             float lo[3], hi[3];
         };
 
-        // bounding box of every 32 consecutive entries (one warp per tile; NaN coordinates are
-        // left out, which is safe: a NaN entry is never farther than min_dist)
-        __global__ void boxes_of_points(const float4 *sp, long long m, long long tiles, Box *out)
+        // The box of a warp's 32 boxes, in every lane.
+        __device__ __forceinline__ void join_boxes(Box &b)
         {
-            const long long w = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-            const int lane = threadIdx.x & 31;
-            if (w >= tiles)
-                return;
-            const long long j = 32 * w + lane;
-            const float inf = __int_as_float(0x7f800000);
-            float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
-            if (j < m)
-            {
-                const float4 p = sp[j];
-                lo[0] = hi[0] = p.x;
-                lo[1] = hi[1] = p.y;
-                lo[2] = hi[2] = p.z;
-            }
             for (int k = 0; k < 3; ++k)
             {
                 for (int o = 16; o > 0; o >>= 1)
                 {
-                    lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
-                    hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+                    b.lo[k] = fminf(b.lo[k], __shfl_xor_sync(0xffffffffu, b.lo[k], o));
+                    b.hi[k] = fmaxf(b.hi[k], __shfl_xor_sync(0xffffffffu, b.hi[k], o));
                 }
             }
+        }
+
+        // The sorted entries' point indices and coordinates, and the bounding boxes of every 32 and
+        // every 1024 (= kTile) of them.  NaN coordinates are left out of the boxes, which is safe: a NaN
+        // entry is never farther than min_dist.
+        __global__ void __launch_bounds__(kTile) gather_sorted(const unsigned long long *keys, const uint32_t *list, long long m,
+                                                               const float *xyz, uint32_t *sidx, float4 *sp, Box *b32, Box *b1k)
+        {
+            const long long j = static_cast<long long>(blockIdx.x) * kTile + threadIdx.x;
+            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            const float inf = __int_as_float(0x7f800000);
+            Box b = {{inf, inf, inf}, {-inf, -inf, -inf}};
+            if (j < m)
+            {
+                const uint32_t idx = list[static_cast<uint32_t>(keys[j])];
+                sidx[j] = idx;
+                const float *p = xyz + 3 * static_cast<size_t>(idx);
+                sp[j] = make_float4(p[0], p[1], p[2], 0.0f);
+                for (int k = 0; k < 3; ++k)
+                    b.lo[k] = b.hi[k] = p[k];
+            }
+            join_boxes(b);
+            __shared__ Box part[kTile / 32];
             if (lane == 0)
             {
-                Box b;
-                for (int k = 0; k < 3; ++k)
-                {
-                    b.lo[k] = lo[k];
-                    b.hi[k] = hi[k];
-                }
-                out[w] = b;
+                part[warp] = b;
+                if (j < m)
+                    b32[j >> 5] = b;
+            }
+            __syncthreads();
+            if (warp == 0)
+            {
+                b = part[lane];
+                join_boxes(b);
+                if (lane == 0)
+                    b1k[blockIdx.x] = b;
             }
         }
 
@@ -598,10 +626,37 @@ namespace vg
             }
         }
 
+        // The chain's entry point into each of up to kFewChunks chunks, walked directly (0xFFFFFFFF for
+        // the chunks it skips).
+        constexpr long long kFewChunks = 32;
+
+        __global__ void walk_chunks(const uint32_t *exit_of, long long m, int chunks, uint32_t *entry, uint32_t *err)
+        {
+            if (threadIdx.x < chunks)
+                entry[threadIdx.x] = 0xFFFFFFFFu;
+            __syncwarp();
+            if (threadIdx.x > 0)
+                return;
+            long long x = 0;
+            for (int h = 0; h < chunks && x < m; ++h)
+            {
+                entry[x / kTile] = static_cast<uint32_t>(x);
+                const long long y = exit_of[x];
+                if (y < (x / kTile + 1) * kTile && y < m)
+                {
+                    *err = 1u;  // not reached: every exit leaves its chunk
+                    return;
+                }
+                x = y;
+            }
+        }
+
         // kept flags of each chunk: its chain members from the entry point.  Each thread lifts
         // from the entry with the doubling tables J_k = next^(2^k) (restricted to the chunk):
         // the last chain element at or before its own index is itself exactly when it is kept.
-        __global__ void mark_kept(const uint32_t *next, long long m, const uint32_t *entry, uint32_t *kept, uint32_t *err)
+        // sums: the flags set in each chunk
+        __global__ void mark_kept(const uint32_t *next, long long m, const uint32_t *entry, uint32_t *kept, uint32_t *sums,
+                                  uint32_t *err)
         {
             __shared__ uint32_t J[10][kTile];
             const long long c0 = static_cast<long long>(blockIdx.x) * kTile;
@@ -612,6 +667,8 @@ namespace vg
             {
                 if (c0 + t < c1)
                     kept[c0 + t] = 0u;
+                if (t == 0)
+                    sums[blockIdx.x] = 0u;
                 return;  // uniform: the chain skips this chunk
             }
             J[0][t] = c0 + t < c1 ? next[c0 + t] : static_cast<uint32_t>(c1);
@@ -622,9 +679,9 @@ namespace vg
                 J[k][t] = v < c1 && v > c0 ? J[k - 1][v - c0] : v;
                 __syncthreads();
             }
+            uint32_t mine = 0u;
             if (c0 + t < c1)
             {
-                uint32_t mine = 0u;
                 const uint32_t me = static_cast<uint32_t>(c0 + t);
                 if (e0 < c0 || e0 >= c1)
                 {
@@ -643,6 +700,9 @@ namespace vg
                 }
                 kept[c0 + t] = mine;
             }
+            const int total = __syncthreads_count(mine != 0u);
+            if (t == 0)
+                sums[blockIdx.x] = static_cast<uint32_t>(total);
         }
 
         __global__ void gather_points(const float *xyz, const uint32_t *list, long long m, float *out)
@@ -661,11 +721,11 @@ namespace vg
             return static_cast<unsigned>((n + per - 1) / per);
         }
 
-        // device buffers of one filter call
         // device buffers of one filter call, carved out of one allocation: a first round of get()
         // calls measures, allocate() reserves the total, a second round hands out the pointers
         struct FilterBuffers
         {
+            cudaStream_t stream;
             char *base = nullptr;
             size_t used = 0;
             bool measuring = true;
@@ -682,15 +742,14 @@ namespace vg
 
             void allocate()
             {
-                err = cudaMalloc(&base, used);
+                err = pool_take(reinterpret_cast<void **>(&base), used, stream);
                 used = 0;
                 measuring = false;
             }
 
             ~FilterBuffers()
             {
-                if (base)
-                    cudaFree(base);
+                pool_give(base, stream);
             }
         };
 
@@ -699,13 +758,13 @@ namespace vg
                              cudaStream_t s)
         {
             const long long N = static_cast<long long>(n);
-            long long M = 1;
+            long long M = kSortMin;
             while (M < N + 1)
                 M <<= 1;
             const long long tiles = blocks_of(N + 1, kTile);
-            FilterBuffers fb;
+            FilterBuffers fb{s};
             uint32_t *flags, *list, *list2, *sums, *offs, *sidx, *next, *exit_of, *entry, *exit_super, *entry_super;
-            uint32_t *rcount, *rstart, *rsums, *roffs, *err;
+            uint32_t *rcount, *rstart, *rsums, *roffs, *counts;
             unsigned long long *keys, *keys2;
             float4 *sp;
             Box *b32, *b1k, *b32k;
@@ -717,7 +776,7 @@ namespace vg
                 flags = fb.get<uint32_t>(N + 1);
                 list = fb.get<uint32_t>(N + 1);
                 list2 = fb.get<uint32_t>(N + 1);
-                sums = fb.get<uint32_t>(tiles);
+                sums = fb.get<uint32_t>(tiles + 1);
                 offs = fb.get<uint32_t>(tiles + 1);
                 sidx = fb.get<uint32_t>(N + 1);
                 next = fb.get<uint32_t>(N + 1);
@@ -738,7 +797,7 @@ namespace vg
                 part_lo = fb.get<float>(code_blocks);
                 part_hi = fb.get<float>(code_blocks);
                 range = fb.get<Range>(1);
-                err = fb.get<uint32_t>(1);
+                counts = fb.get<uint32_t>(2);  // entries kept, error code
             };
             carve();
             fb.allocate();
@@ -746,13 +805,17 @@ namespace vg
                 return cuda_fail(fb.err, "vg_filter_pointcloud: cudaMalloc");
             carve();
 
+            VG_CUDA(cudaFuncSetAttribute(bitonic_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kSortTile * sizeof(unsigned long long)),
+                    "vg_filter_pointcloud: sort kernel");
             const float sq = min_dist * min_dist, sq_range = max_range * max_range;
             // collision/filter.hh:194-197: both ends are minima over the axes
             Range r0;
             r0.lo = std::min({origin[0] - max_range, origin[1] - max_range, origin[2] - max_range});
             r0.hi = std::min({origin[0] + max_range, origin[1] + max_range, origin[2] + max_range});
             VG_CUDA(cudaMemcpyAsync(range, &r0, sizeof(r0), cudaMemcpyHostToDevice, s), "vg_filter_pointcloud: copy");
-            VG_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), s), "vg_filter_pointcloud: memset");
+            VG_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), s), "vg_filter_pointcloud: memset");
+            uint32_t *const err = counts + 1;
 
             // the work list: the passing points in order, then one copy of point 0 if any failed
             CullParams cp{origin[0], origin[1], origin[2], sq_range, {}, {}, cull};
@@ -762,12 +825,19 @@ namespace vg
                 cp.hi[k] = workcell_max[k];
             }
             const long long in_tiles = blocks_of(N, kTile);
-            cull_kernel<<<blocks_of(N, 256), 256, 0, s>>>(xyz, N, cp, flags);
-            tile_sums<<<static_cast<unsigned>(in_tiles), kTile, 0, s>>>(flags, N, sums);
-            scan_tiles<<<1, kTile, 0, s>>>(sums, in_tiles, offs);
-            compact<<<static_cast<unsigned>(in_tiles), kTile, 0, s>>>(flags, N, offs, nullptr, list);
+            // tile sums beyond what a compaction adds up itself become offsets, in place
+            auto offsets = [&](long long t) {
+                if (t > kDirectTiles)
+                {
+                    scan_tiles<<<1, kTile, 0, s>>>(sums, t, offs);
+                    std::swap(sums, offs);
+                }
+            };
+            cull_kernel<<<static_cast<unsigned>(in_tiles), kTile, 0, s>>>(xyz, N, cp, flags, sums);
+            offsets(in_tiles);
+            compact<<<static_cast<unsigned>(in_tiles), kTile, 0, s>>>(flags, N, sums, in_tiles, nullptr, list, counts);
             uint32_t h = 0;
-            VG_CUDA(cudaMemcpyAsync(&h, offs + in_tiles, sizeof(h), cudaMemcpyDeviceToHost, s), "vg_filter_pointcloud: copy");
+            VG_CUDA(cudaMemcpyAsync(&h, counts, sizeof(h), cudaMemcpyDeviceToHost, s), "vg_filter_pointcloud: copy");
             VG_CUDA(cudaStreamSynchronize(s), "vg_filter_pointcloud");
             long long m = h;
             if (static_cast<long long>(h) < N)
@@ -783,7 +853,7 @@ namespace vg
             const double limit = static_cast<double>(sq) / (1.0 + 1e-5) - 1e-38;
             for (int pass = 0; pass < 6; ++pass)
             {
-                long long Mp = 1;
+                long long Mp = kSortMin;
                 while (Mp < m)
                     Mp <<= 1;
                 const long long cb = blocks_of(Mp, kCodeBlock);
@@ -806,43 +876,46 @@ namespace vg
                     }
                     // four passes: the result is back in keys
                 }
-                else if (Mp > 1)
+                else
                 {
                     const long long T = std::min<long long>(Mp, kSortTile);
-                    const unsigned tb = static_cast<unsigned>(Mp / T), tt = static_cast<unsigned>(T / 2);
-                    bitonic_tile<<<tb, tt, 0, s>>>(keys, Mp, 2, T);
+                    const unsigned tb = static_cast<unsigned>(Mp / T), tt = static_cast<unsigned>(T / kSortPer);
+                    const size_t tile_bytes = static_cast<size_t>(T) * sizeof(unsigned long long);
+                    bitonic_tile<<<tb, tt, tile_bytes, s>>>(keys, Mp, 2, T);
                     for (long long k = 2 * T; k <= Mp; k <<= 1)
                     {
                         for (long long j = k >> 1; j >= T; j >>= 1)
                             bitonic_step<<<blocks_of(Mp / 2, 256), 256, 0, s>>>(keys, Mp, k, j);
-                        bitonic_tile<<<tb, tt, 0, s>>>(keys, Mp, k, k);
+                        bitonic_tile<<<tb, tt, tile_bytes, s>>>(keys, Mp, k, k);
                     }
                 }
-                gather_sorted<<<blocks_of(m, 256), 256, 0, s>>>(keys, list, m, xyz, sidx, sp);
-                const long long t32 = blocks_of(m, 32), t1k = blocks_of(t32, 32), t32k = blocks_of(t1k, 32);
-                boxes_of_points<<<blocks_of(32 * t32, 256), 256, 0, s>>>(sp, m, t32, b32);
-                boxes_of_boxes<<<blocks_of(32 * t1k, 256), 256, 0, s>>>(b32, t32, t1k, b1k);
-                boxes_of_boxes<<<blocks_of(32 * t32k, 256), 256, 0, s>>>(b1k, t1k, t32k, b32k);
+                gather_sorted<<<blocks_of(m, kTile), kTile, 0, s>>>(keys, list, m, xyz, sidx, sp, b32, b1k);
+                const long long t1k = blocks_of(m, kTile), t32k = blocks_of(t1k, 32);
+                if (m >= 65536)  // no scan looks at one below
+                    boxes_of_boxes<<<blocks_of(32 * t32k, 256), 256, 0, s>>>(b1k, t1k, t32k, b32k);
                 next_kernel<<<blocks_of(m, 128), 128, 0, s>>>(NextParams{sp, m, sq, limit, b32, b1k, b32k, next});
                 const long long chunks = blocks_of(m, kTile);
                 chunk_exit<<<static_cast<unsigned>(chunks), kTile, 0, s>>>(next, m, exit_of);
-                const long long supers = blocks_of(chunks, kSuper);
-                VG_CUDA(cudaMemsetAsync(entry, 0xFF, chunks * sizeof(uint32_t), s), "vg_filter_pointcloud: memset");
-                VG_CUDA(cudaMemsetAsync(entry_super, 0xFF, supers * sizeof(uint32_t), s), "vg_filter_pointcloud: memset");
-                super_exit<<<blocks_of(m, 256), 256, 0, s>>>(exit_of, m, exit_super, err);
-                chain_walk<<<1, 1, 0, s>>>(exit_super, m, entry_super, err);
-                chunk_entries<<<blocks_of(supers, 128), 128, 0, s>>>(exit_of, m, entry_super, supers, entry);
-                mark_kept<<<static_cast<unsigned>(chunks), kTile, 0, s>>>(next, m, entry, flags, err);
-                tile_sums<<<static_cast<unsigned>(chunks), kTile, 0, s>>>(flags, m, sums);
-                scan_tiles<<<1, kTile, 0, s>>>(sums, chunks, offs);
-                compact<<<static_cast<unsigned>(chunks), kTile, 0, s>>>(flags, m, offs, sidx, list2);
+                if (chunks <= kFewChunks)
+                {
+                    walk_chunks<<<1, 32, 0, s>>>(exit_of, m, static_cast<int>(chunks), entry, err);
+                }
+                else
+                {
+                    const long long supers = blocks_of(chunks, kSuper);
+                    VG_CUDA(cudaMemsetAsync(entry, 0xFF, chunks * sizeof(uint32_t), s), "vg_filter_pointcloud: memset");
+                    VG_CUDA(cudaMemsetAsync(entry_super, 0xFF, supers * sizeof(uint32_t), s), "vg_filter_pointcloud: memset");
+                    super_exit<<<blocks_of(m, 256), 256, 0, s>>>(exit_of, m, exit_super, err);
+                    chain_walk<<<1, 1, 0, s>>>(exit_super, m, entry_super, err);
+                    chunk_entries<<<blocks_of(supers, 128), 128, 0, s>>>(exit_of, m, entry_super, supers, entry);
+                }
+                mark_kept<<<static_cast<unsigned>(chunks), kTile, 0, s>>>(next, m, entry, flags, sums, err);
+                offsets(chunks);
+                compact<<<static_cast<unsigned>(chunks), kTile, 0, s>>>(flags, m, sums, chunks, sidx, list2, counts);
                 std::swap(list, list2);
                 VG_CUDA(cudaGetLastError(), "vg_filter_pointcloud: launch");
                 uint32_t kept[2] = {0, 0};
-                VG_CUDA(cudaMemcpyAsync(&kept[0], offs + chunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
-                        "vg_filter_pointcloud: copy");
-                VG_CUDA(cudaMemcpyAsync(&kept[1], err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
-                        "vg_filter_pointcloud: copy");
+                VG_CUDA(cudaMemcpyAsync(kept, counts, sizeof(kept), cudaMemcpyDeviceToHost, s), "vg_filter_pointcloud: copy");
                 VG_CUDA(cudaStreamSynchronize(s), "vg_filter_pointcloud");
                 if (kept[1] || kept[0] == 0 || kept[0] > m)
                     return set_error(VG_ERR_STATE, "vg_filter_pointcloud: inconsistent chain (code " +
@@ -930,9 +1003,9 @@ int vg_filter_self_from_pointcloud_device(const char *robot, vg_env *env, const 
         return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const long long N = static_cast<long long>(n), tiles = blocks_of(N, kTile);
-    FilterBuffers fb;
+    FilterBuffers fb{s};
     float *dq, *sph;
-    uint32_t *flags, *sums, *offs, *idx;
+    uint32_t *flags, *sums, *offs, *idx, *count;
     auto carve = [&]() {
         dq = fb.get<float>(r->dim);
         sph = fb.get<float>(4 * r->slots);
@@ -940,6 +1013,7 @@ int vg_filter_self_from_pointcloud_device(const char *robot, vg_env *env, const 
         sums = fb.get<uint32_t>(tiles);
         offs = fb.get<uint32_t>(tiles + 1);
         idx = fb.get<uint32_t>(N);
+        count = fb.get<uint32_t>(1);
     };
     carve();
     fb.allocate();
@@ -955,11 +1029,15 @@ int vg_filter_self_from_pointcloud_device(const char *robot, vg_env *env, const 
     const int grid = static_cast<int>(std::min<long long>(blocks_of(N, 256), static_cast<long long>(sm_count()) * occ));
     filter_self_kernel<<<grid, 256, smem, s>>>(xyz, N, point_radius, sph, r->fine, env_device(env), flags);
     tile_sums<<<static_cast<unsigned>(tiles), kTile, 0, s>>>(flags, N, sums);
-    scan_tiles<<<1, kTile, 0, s>>>(sums, tiles, offs);
-    compact<<<static_cast<unsigned>(tiles), kTile, 0, s>>>(flags, N, offs, nullptr, idx);
+    if (tiles > kDirectTiles)
+    {
+        scan_tiles<<<1, kTile, 0, s>>>(sums, tiles, offs);
+        std::swap(sums, offs);
+    }
+    compact<<<static_cast<unsigned>(tiles), kTile, 0, s>>>(flags, N, sums, tiles, nullptr, idx, count);
     VG_CUDA(cudaGetLastError(), "vg_filter_self_from_pointcloud: launch");
     uint32_t m = 0;
-    VG_CUDA(cudaMemcpyAsync(&m, offs + tiles, sizeof(m), cudaMemcpyDeviceToHost, s), "vg_filter_self_from_pointcloud: copy");
+    VG_CUDA(cudaMemcpyAsync(&m, count, sizeof(m), cudaMemcpyDeviceToHost, s), "vg_filter_self_from_pointcloud: copy");
     VG_CUDA(cudaStreamSynchronize(s), "vg_filter_self_from_pointcloud");
     if (m > 0)
     {

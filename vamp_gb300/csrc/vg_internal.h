@@ -86,8 +86,8 @@ namespace vg
     } while (0)
 
     // device buffers per pointcloud: tests, aabbs, starts, reference-layout blocks (device-built
-    // clouds only), ring-ordered blocks, query tables
-    constexpr size_t kCloudBuffers = 6;
+    // clouds only), ring-ordered blocks with the query tables
+    constexpr size_t kCloudBuffers = 5;
 
     // threads per block of every checking kernel (the robots' stage stride)
     constexpr int kBlock = 128;
@@ -108,6 +108,7 @@ namespace vg
     {
         float *d = nullptr;
         size_t n = 0;
+        bool owned = true;  // false: part of a device-built tree's first buffer
     };
 }  // namespace vg
 

@@ -1,0 +1,61 @@
+// Device memory that comes and goes with calls and environments (the pointcloud filter's and tree
+// builds' scratch, trees, environment images): a private
+// stream-ordered pool per device, which keeps up to kPoolKeep bytes between calls (an allocation of
+// tens of megabytes from the driver takes longer than the work in it) and returns the rest to the
+// driver.  Safe with several threads and streams: allocations and releases are ordered on their
+// streams, and the pool orders reuse across streams.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+#include <mutex>
+
+namespace vg
+{
+    constexpr uint64_t kPoolKeep = uint64_t{256} << 20;
+
+    // `bytes` of device memory for work on stream s.
+    inline cudaError_t pool_take(void **p, size_t bytes, cudaStream_t s)
+    {
+        constexpr int kDevices = 64;
+        static std::mutex mu;
+        static cudaMemPool_t pools[kDevices] = {};
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess)
+            return e;
+        if (dev >= kDevices)
+            return cudaMalloc(p, bytes);
+        cudaMemPool_t pool = nullptr;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!pools[dev])
+            {
+                cudaMemPoolProps props{};
+                props.allocType = cudaMemAllocationTypePinned;
+                props.location.type = cudaMemLocationTypeDevice;
+                props.location.id = dev;
+                e = cudaMemPoolCreate(&pools[dev], &props);
+                uint64_t keep = kPoolKeep;
+                if (e == cudaSuccess)
+                    e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+                if (e != cudaSuccess)
+                    return e;
+            }
+            pool = pools[dev];
+        }
+        return cudaMallocFromPoolAsync(p, bytes, pool, s);
+    }
+
+    // Releases memory from pool_take once the work already on s is done.
+    inline void pool_give(void *p, cudaStream_t s)
+    {
+        if (p && cudaFreeAsync(p, s) != cudaSuccess)
+        {
+            cudaGetLastError();
+            cudaFree(p);
+        }
+    }
+}  // namespace vg
