@@ -504,16 +504,16 @@ namespace vg
     // Blocks of a host batch above which the batch goes to the edge kernels.
     constexpr size_t kSmallBlocks = 4096;
 
-    // A small host batch of edges checked block by block.  Every block of every edge is built on
-    // the host with the edge kernels' arithmetic (the length summed in the x86 order and rounded
-    // once, n = max(ceil(length / W * resolution), 1), block 0 at fractions (k + 1) / W of the
-    // edge, block i = block 0 minus i steps of v / (W n), planning/validate.hh:24-56), the blocks
-    // go to the caller-given-blocks kernel in one launch, and an edge is valid when all of its
-    // blocks are: the verdicts of the edge kernels, which stop at the first colliding block.  All
-    // blocks of an edge run at once, where the edge kernels give one warp the whole edge, which
-    // is what the latency of a single edge (a planner's extension step) needs.  dist == nullptr:
-    // b holds goals (validate_motion), otherwise motion vectors and dist the lengths
+    // A small host batch of edges checked block by block: the host counts each edge's blocks with the
+    // edge kernels' arithmetic (the length summed in the x86 order and rounded once, n =
+    // max(ceil(length / W * resolution), 1), planning/validate.hh:24-56) and one launch of
+    // edge_blocks_kernel checks them all at once; an edge is valid when all of its blocks are, which is
+    // the verdict of the edge kernels, which stop at the first colliding block.  dist == nullptr: b
+    // holds goals (validate_motion), otherwise motion vectors and dist the lengths
     // (validate_vector).  *handled = 0 when the batch has more than kSmallBlocks blocks.
+    //
+    // Blocks built on the host, copied up and their verdicts copied down took 32 us for one motion
+    // and 97 for 256 (a third of it the host's subtractions).
     static int small_motions(const RobotOps *r, vg_env *env, const float *a, const float *b, const float *dist, size_t n,
                              int resolution, uint8_t *out, int *handled)
     {
@@ -552,57 +552,40 @@ namespace vg
             if (total > kSmallBlocks)
                 return VG_OK;
         }
-        const size_t qb = total * W * D * sizeof(float);
-        const size_t qa = (qb + 255) & ~size_t(255);
-        if (int rc = ensure_pinned(env, qa + total))
+        const size_t ab = (n * D * sizeof(float) + 255) & ~size_t(255);
+        const size_t items_at = 2 * ab, out_at = items_at + total * sizeof(int2);
+        if (int rc = ensure_pinned(env, out_at + n))
             return rc;
-        if (int rc = ensure_stage(env, qa + total))
-            return rc;
-        float *hq = static_cast<float *>(env->h_pin);
-        uint8_t *hv = static_cast<uint8_t *>(env->h_pin) + qa;
-        float q[8][32], bs[32];
-        size_t blk = 0;
+        char *pin = static_cast<char *>(env->h_pin);
+        std::memcpy(pin, a, n * D * sizeof(float));
+        std::memcpy(pin + ab, b, n * D * sizeof(float));
+        int2 *items = reinterpret_cast<int2 *>(pin + items_at);
         for (size_t e = 0; e < n; ++e)
         {
-            for (int d = 0; d < D; ++d)
-                v[d] = dist ? b[e * D + d] : b[e * D + d] - a[e * D + d];
-            const float denom = static_cast<float>(W * nb[e]);
-            for (int d = 0; d < D; ++d)
-                bs[d] = v[d] / denom;
-            for (int k = 0; k < W; ++k)
-            {
-                const float pct = static_cast<float>(k + 1) / static_cast<float>(W);
-                for (int d = 0; d < D; ++d)
-                    q[k][d] = std::fma(v[d], pct, a[e * D + d]);
-            }
-            for (int i = 0; i < nb[e]; ++i, ++blk)
-            {
-                for (int k = 0; k < W; ++k)
-                {
-                    for (int d = 0; d < D; ++d)
-                    {
-                        hq[(blk * W + k) * D + d] = q[k][d];
-                        q[k][d] = q[k][d] - bs[d];
-                    }
-                }
-            }
-        }
-        float *dq = static_cast<float *>(env->d_stage);
-        uint8_t *dv = static_cast<uint8_t *>(env->d_stage) + qa;
-        VG_CUDA(cudaMemcpyAsync(dq, hq, qb, cudaMemcpyHostToDevice, 0), "copy configuration blocks");
-        if (int rc = vg_fkcc_blocks_device(r->name, env, dq, total, dv, nullptr))
-            return rc;
-        VG_CUDA(cudaMemcpyAsync(hv, dv, total, cudaMemcpyDeviceToHost, 0), "copy block verdicts");
-        VG_CUDA(cudaStreamSynchronize(0), "synchronize");
-        blk = 0;
-        for (size_t e = 0; e < n; ++e)
-        {
-            uint8_t ok = 1;
             for (int i = 0; i < nb[e]; ++i)
-                ok &= hv[blk + i];
-            out[e] = ok;
-            blk += static_cast<size_t>(nb[e]);
+                *items++ = make_int2(static_cast<int>(e), i | nb[e] << 16);
         }
+        uint8_t *verdicts = reinterpret_cast<uint8_t *>(pin + out_at);
+        std::memset(verdicts, 1, n);
+        const int ext = env->extended() ? 1 : 0, which = W == 8 ? 0 : 1;
+        const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4)) + r->stage_floats * kBlock * 4;
+        int occ = 0;
+        if (int rc = prepare_kernel(r->edge_blocks_fn[ext][which], smem, kBlock, &occ))
+            return rc;
+        want_field(env, static_cast<double>(total) * W, 0);
+        // Blocks of one warp run the union of their tests, so few blocks are spread over more warps, up
+        // to 16 an SM, about what is resident: 256 planner steps of Panda 57.5 us with 4 blocks a warp, 49.
+        int spread = 1;
+        while (spread < 32 / W && total > static_cast<size_t>(sm_count()) * 16 * spread)
+            spread *= 2;
+        const long long per_block = (kBlock / 32) * spread;
+        const int grid = static_cast<int>(std::min<long long>((static_cast<long long>(total) + per_block - 1) / per_block,
+                                                              static_cast<long long>(sm_count()) * occ));
+        EdgeBlocksParams p{reinterpret_cast<const float *>(pin), reinterpret_cast<const float *>(pin + ab), dist ? 1 : 0,
+                           reinterpret_cast<const int2 *>(pin + items_at), static_cast<int>(total), spread, verdicts, env_device(env)};
+        VG_CUDA(r->edge_blocks[ext][which](p, grid, kBlock, smem, 0), "edge blocks kernel launch");
+        VG_CUDA(cudaStreamSynchronize(0), "synchronize");
+        std::memcpy(out, verdicts, n);
         *handled = 1;
         return VG_OK;
     }

@@ -32,6 +32,9 @@ namespace vg
         const void *blocks_fn[2];
         cudaError_t (*blocks_ext[2])(const StatesParams &, int grid, int block, int smem, cudaStream_t);
         const void *blocks_ext_fn[2];
+        // every block of a small batch of edges: [extended][0 = 8-lane blocks, 1 = 4-lane]
+        cudaError_t (*edge_blocks[2][2])(const EdgeBlocksParams &, int grid, int block, int smem, cudaStream_t);
+        const void *edge_blocks_fn[2][2];
         // edges: index 0 = 8-lane blocks, 1 = 4-lane blocks
         cudaError_t (*edges[2])(const EdgesParams &, int grid, int block, int smem, cudaStream_t);
         const void *edges_fn[2];
@@ -165,7 +168,8 @@ struct vg_env
     unsigned *d_counter = nullptr;
     void *d_stage = nullptr;
     size_t stage_cap = 0;
-    // pinned host staging of small host-pointer edge batches (their blocks, then their verdicts)
+    // pinned host memory of small host-pointer edge batches, which their kernel reads and writes:
+    // starts, goals, blocks, verdicts
     void *h_pin = nullptr;
     size_t pin_cap = 0;
     // per-robot picks of vg_autotune_motions (cleared by vg_env_set_schedule)

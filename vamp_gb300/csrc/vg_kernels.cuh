@@ -261,6 +261,86 @@ namespace vg
         }
     }
 
+    // ---------------------------------------------------------------------- blocks of edges
+
+    // Every block of a small batch of edges, one W-lane segment each, all at once: what one motion's
+    // latency needs, where the edge kernels give a warp the whole edge.  Inputs and verdicts lie in
+    // pinned host memory: a batch is a few kilobytes, and two copies would take longer than reading
+    // them across.
+    struct EdgeBlocksParams
+    {
+        const float *a, *b;  // as EdgesParams
+        int vectors;         // 1: b holds the motion vectors
+        const int2 *items;   // per block: its edge, and its index + (the edge's blocks << 16)
+        int n;               // blocks
+        int spread;          // blocks a warp checks at once, at most 32 / W
+        uint8_t *out;        // per edge, 1 before the launch; 0 = some block collides
+        EnvDevice env;
+    };
+
+    template <typename Robot, int W, bool kExt = false>
+    __global__ void __launch_bounds__(128, VG_MIN_BLOCKS) edge_blocks_kernel(EdgeBlocksParams p)
+    {
+        extern __shared__ float4 smem[];
+        constexpr int D = Robot::kDim;
+        const int lane = threadIdx.x & 31, sl = lane % W, seg = lane / W;
+        const float pct = __fdiv_rn(static_cast<float>(sl + 1), static_cast<float>(W));
+        const int stride = gridDim.x * (blockDim.x >> 5) * p.spread;
+        int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * p.spread;
+        // the first items' round trip to the host runs under the staging of the environment
+        int2 it = make_int2(0, 1 << 16);
+        float av[D], v[D];
+        auto load = [&](bool in) {
+            if (in)
+            {
+                it = p.items[base + seg];
+#pragma unroll
+                for (int d = 0; d < D; ++d)
+                {
+                    av[d] = p.a[static_cast<long long>(it.x) * D + d];
+                    v[d] = p.b[static_cast<long long>(it.x) * D + d];
+                }
+            }
+        };
+        load(seg < p.spread && base + seg < p.n);
+        const EnvView ev = stage_env(p.env, smem);
+        float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
+        for (bool first = true; base < p.n; base += stride, first = false)
+        {
+            const bool in = seg < p.spread && base + seg < p.n;
+            if (!first)
+            {
+                load(in);
+            }
+            // block i of the edge: block 0 minus i repeated steps, as the edge kernels reach it
+            const int i = it.y & 0xffff;
+            const float denom = static_cast<float>(W * (it.y >> 16));
+            float q[D], bs[D];
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+            {
+                const float vd = in ? (p.vectors ? v[d] : __fsub_rn(v[d], av[d])) : 0.0f;
+                q[d] = __fmaf_rn(vd, pct, in ? av[d] : 0.0f);
+                bs[d] = __fdiv_rn(vd, denom);
+            }
+            const int steps = static_cast<int>(__reduce_max_sync(kFull, static_cast<unsigned>(in ? i : 0)));
+#pragma unroll 1
+            for (int k = 0; k < steps; ++k)
+            {
+#pragma unroll
+                for (int d = 0; d < D; ++d)
+                {
+                    q[d] = k < i ? __fsub_rn(q[d], bs[d]) : q[d];
+                }
+            }
+            const unsigned alive = run_fkcc<Robot, W, kExt>(ev, q, __ballot_sync(kFull, in), stage);
+            if (in && sl == 0 && !((alive >> lane) & 1u))
+            {
+                p.out[it.x] = 0;
+            }
+        }
+    }
+
     // ------------------------------------------------------------------------------- edges
 
     struct EdgesParams

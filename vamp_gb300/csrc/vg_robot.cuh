@@ -20,6 +20,13 @@ namespace vg
         return cudaGetLastError();
     }
 
+    template <typename R, int W, bool kExt>
+    cudaError_t launch_edge_blocks(const EdgeBlocksParams &p, int grid, int block, int smem, cudaStream_t s)
+    {
+        edge_blocks_kernel<R, W, kExt><<<grid, block, smem, s>>>(p);
+        return cudaGetLastError();
+    }
+
     template <typename R, int W>
     cudaError_t launch_edges(const EdgesParams &p, int grid, int block, int smem, cudaStream_t s)
     {
@@ -115,6 +122,14 @@ namespace vg
         o.blocks_ext[1] = &launch_blocks<R, 4, true>;
         o.blocks_ext_fn[0] = reinterpret_cast<const void *>(&blocks_kernel<R, 8, true>);
         o.blocks_ext_fn[1] = reinterpret_cast<const void *>(&blocks_kernel<R, 4, true>);
+        o.edge_blocks[0][0] = &launch_edge_blocks<R, 8, false>;
+        o.edge_blocks[0][1] = &launch_edge_blocks<R, 4, false>;
+        o.edge_blocks[1][0] = &launch_edge_blocks<R, 8, true>;
+        o.edge_blocks[1][1] = &launch_edge_blocks<R, 4, true>;
+        o.edge_blocks_fn[0][0] = reinterpret_cast<const void *>(&edge_blocks_kernel<R, 8, false>);
+        o.edge_blocks_fn[0][1] = reinterpret_cast<const void *>(&edge_blocks_kernel<R, 4, false>);
+        o.edge_blocks_fn[1][0] = reinterpret_cast<const void *>(&edge_blocks_kernel<R, 8, true>);
+        o.edge_blocks_fn[1][1] = reinterpret_cast<const void *>(&edge_blocks_kernel<R, 4, true>);
         o.edges[0] = &launch_edges<R, 8>;
         o.edges[1] = &launch_edges<R, 4>;
         o.edges_fn[0] = reinterpret_cast<const void *>(&edges_kernel<R, 8>);
