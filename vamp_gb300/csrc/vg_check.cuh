@@ -678,6 +678,12 @@ namespace vg
         return sql2(a.x, a.y, a.z, b.x, b.y, b.z) < __fmul_rn(rr, rr);
     }
 
+    // whether the joints (qa, qb) lie in a danger box (lo0, hi0, lo1, hi1)
+    __device__ __forceinline__ bool in_box(const float4 box, float qa, float qb)
+    {
+        return (qa >= box.x) & (qa <= box.y) & (qb >= box.z) & (qb <= box.w);
+    }
+
     // Threads per block of every checking kernel, and the stride of the per-thread columns of
     // the robots' shared-memory stage.
     constexpr int kStageStride = 128;

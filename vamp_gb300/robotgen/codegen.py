@@ -420,17 +420,14 @@ def f32_up(v: float) -> float:
 BIG = 3.0e38  # an unbounded box side (joint values are finite)
 
 
-def danger_boxes(model: dict, cull) -> tuple:
-    """Per self check ((joint indices, index of its first pair box or -1), union box) and the
-    boxes of the analysed checks' live pairs, as FP32 bounds rounded outwards; unanalysed checks
-    get an unbounded union box and no pair boxes."""
-    checks, pairs = [], []
+def danger_boxes(model: dict, cull) -> list:
+    """Per self check its two joint indices, whether it was analysed, and the union of its live
+    pairs' boxes as FP32 bounds rounded outwards (unbounded if not analysed)."""
+    checks = []
     for ci, e in enumerate(model["self_checks"]):
         bx = None if cull is None or "boxes" not in cull else cull["boxes"][ci]
-        sel = range(len(e["fine"])) if cull is None or cull["live"][ci] is None else cull["live"][ci]
-        n_live = len(list(sel))
         if not bx:
-            checks.append(((0, 0, -1), (-BIG, BIG, -BIG, BIG)))
+            checks.append(((0, 0, False), (-BIG, BIG, -BIG, BIG)))
             continue
         j = bx[0]["joints"]
         two = len(j) == 2
@@ -440,9 +437,8 @@ def danger_boxes(model: dict, cull) -> tuple:
             lo1, hi1 = (b["lo"][1], b["hi"][1]) if two else (-BIG, BIG)
             per.append((f32_down(b["lo"][0]), f32_up(b["hi"][0]), f32_down(lo1) if two else -BIG, f32_up(hi1) if two else BIG))
         union = (min(p[0] for p in per), max(p[1] for p in per), min(p[2] for p in per), max(p[3] for p in per))
-        checks.append(((jj[0], jj[1], len(pairs)), union))
-        pairs += per
-    return checks, pairs
+        checks.append(((jj[0], jj[1], True), union))
+    return checks
 
 
 # Resident 128-thread blocks per SM that the same-edge kernels are built for: five for the robots
@@ -540,8 +536,8 @@ def stage_layout(model: dict, kin, cull) -> dict:
             row_c.append(0.0)
         fslots.append(row_s)
         fconsts.append(row_c)
-    checks, _ = danger_boxes(model, cull)
-    joints = sorted({j for (j0, j1, b0), _ in checks if b0 >= 0 for j in (j0, j1)})
+    checks = danger_boxes(model, cull)
+    joints = sorted({j for (j0, j1, found), _ in checks if found for j in (j0, j1)})
     return {"frames": frames, "slots": fslots, "consts": fconsts, "values": list(values),
             "joints": joints, "joint_pos": {j: i for i, j in enumerate(joints)},
             "q0": len(values), "total": len(values) + len(joints)}
@@ -616,7 +612,7 @@ def gen_cuda(model: dict) -> str:
     members, pairs = groups["members"], groups["pairs"]
     n_groups = len(members)
     assert n_groups <= 32, "one bit of a word per link group"
-    boxes_of, live_boxes = danger_boxes(model, cull)
+    boxes_of = danger_boxes(model, cull)
     all_pairs = [tuple(p_) for e in model["self_checks"] for p_ in e["fine"]]
     lines = []
     w = lines.append
@@ -656,10 +652,11 @@ def gen_cuda(model: dict) -> str:
         offs.append((em0.const(float(v[0])), em0.const(float(v[1])), em0.const(float(v[2])), r))
     w("    // slot -> its centre's offset in its frame, and its radius")
     table("__constant__", "float4", "SlotOff", offs, f4)
-    w("    // per staged frame and entry: its stage slot, or -1 and the constant value")
+    w("    // per staged frame and entry: its stage slot, or -1 and the constant value (global memory: see")
+    w("    // self_checks)")
     nfr = len(lay["slots"])
-    w(f"    __constant__ int {pre}FrameSlot[{nfr}][12] = {{{', '.join('{' + ', '.join(map(str, r)) + '}' for r in lay['slots'])}}};")
-    w(f"    __constant__ float {pre}FrameConst[{nfr}][12] = {{{', '.join('{' + ', '.join(lit32(v) for v in r) + '}' for r in lay['consts'])}}};")
+    w(f"    __device__ const int {pre}FrameSlot[{nfr}][12] = {{{', '.join('{' + ', '.join(map(str, r)) + '}' for r in lay['slots'])}}};")
+    w(f"    __device__ const float {pre}FrameConst[{nfr}][12] = {{{', '.join('{' + ', '.join(lit32(v) for v in r) + '}' for r in lay['consts'])}}};")
     env_rows, group_rows = [], []
     for g, fid in enumerate(groups["frames"]):
         first = len(env_rows)
@@ -671,7 +668,7 @@ def gen_cuda(model: dict) -> str:
     w("    // fine slots")
     table("__constant__", "int4", "Group", group_rows, i4)
     table("__constant__", "int4", "Env", env_rows, i4)
-    pair_rows, check_a, check_b, check_box, contain, row_rows, row_b, row_box = [], [], [], [], [], [], [], []
+    pair_rows, check_a, check_b, check_box, contain, row_rows, row_b = [], [], [], [], [], [], []
     full0 = [0]
     for e in model["self_checks"]:
         full0.append(full0[-1] + len(e["fine"]))
@@ -680,20 +677,19 @@ def gen_cuda(model: dict) -> str:
         for c in cs:
             e = model["self_checks"][c]
             sel = range(len(e["fine"])) if cull is None or cull["live"][c] is None else cull["live"][c]
-            (j0, j1, box0), union = boxes_of[c]
+            (j0, j1, found), union = boxes_of[c]
             r0 = len(row_rows)
             last = None
-            for n_, i in enumerate(sel):
+            for i in sel:
                 x, y = e["fine"][i]
                 if x != last:
                     row_rows.append([x, len(row_b), len(row_b), 0])
                     last = x
                 row_b.append(y)
                 row_rows[-1][2] = len(row_b)
-                row_box.append(box0 + n_ if box0 >= 0 else -1)
             check_a.append((coarse_slot[e["links"][0]], coarse_slot[e["links"][1]], r0, len(row_rows)))
             jp = lay["joint_pos"]
-            check_b.append((full0[c], full0[c + 1], jp[j0] if box0 >= 0 else -1, jp[j1] if box0 >= 0 else -1))
+            check_b.append((full0[c], full0[c + 1], jp[j0] if found else -1, jp[j1] if found else -1))
             check_box.append(union)
             contain.append(f32_up(containing_radius(model, kin, model["env_checks"][groups["env_ix"][e["links"][1]]]) + CONTAIN_MARGIN))
         fa, fb = groups["frames"][ga], groups["frames"][gb]
@@ -710,12 +706,12 @@ def gen_cuda(model: dict) -> str:
     w(f"    // centre that contains B's fine spheres with {CONTAIN_MARGIN} m to spare")
     table("__constant__", "float4", "CheckBox", check_box, f4)
     w(f"    __constant__ float {pre}ContainR[{len(contain)}] = {{{', '.join(lit32(v) for v in contain)}}};")
-    w("    // rows: a fine slot of A, its live pairs' range; per live pair the fine slot of B, and the box")
-    table("__constant__", "int4", "Row", row_rows, i4)
+    w("    // rows: a fine sphere of A (offset and radius), its live pairs' range; per live pair the fine")
+    w("    // slot of B, and its sphere (global memory: see self_checks)")
+    table("__constant__", "float4", "RowA", [offs[r[0]] for r in row_rows], f4)
+    table("__constant__", "int2", "Row", row_rows, lambda r: "{%d, %d}" % (tuple(r[1:3]) if r else (0, 0)))
+    table("__device__ const", "float4", "RowSphere", [offs[y] for y in row_b], f4)
     w(f"    __constant__ int {pre}RowB[{max(1, len(row_b))}] = {{{', '.join(map(str, row_b)) or '0'}}};")
-    if live_boxes:
-        boxed = [live_boxes[i] if i >= 0 else (-BIG, BIG, -BIG, BIG) for i in row_box]
-        table("__constant__", "float4", "RowBox", boxed, f4)
     w("    // every fine self pair, in the reference's order (debug reports, and configurations outside")
     w("    // the widened joint limits; global memory)")
     w(f"    __device__ const int2 {pre}AllPair[{max(1, len(all_pairs))}] = {{{', '.join('{%d, %d}' % p for p in all_pairs) or '{0, 0}'}}};")
@@ -841,7 +837,7 @@ def gen_cuda(model: dict) -> str:
             # contains it
             body.append(f"over{wd} = vg::shift_in(over{wd}, vg::self_bits({', '.join(A)}, {', '.join(B)}, "
                         f"__fadd_rn({lit32(ra)}, {lit32(rb)})));")
-            if all(boxes_of[c][0][2] >= 0 for c in pairs[(ga, gb)]):
+            if all(boxes_of[c][0][2] for c in pairs[(ga, gb)]):
                 gate.append((len(part) - 1 - j, [boxes_of[c] for c in pairs[(ga, gb)]]))
         body.append(f"unsigned boxed{wd} = ~0u;")
         if gate:
@@ -912,32 +908,22 @@ if (!self_checks(ctx, st, over{wd}, boxed{wd}, on, {32 * wd + len(part) - 1}))
 {{
     return;
 }}""".split("\n")
-    box_gate = box_row = ""
-    if live_boxes:
+    box_gate = ""
+    if any(found for (_, _, found), _ in boxes_of):
         box_gate = f"""
                 const int4 cb4 = {pre}CheckB[k];
                 float qa = 0.0f, qb = 0.0f;
                 if (cb4.z >= 0)
                 {{
-                    // only while some lane's joints lie in the check's danger box
-                    const float4 bx = {pre}CheckBox[k];
+                    // only the lanes whose joints lie in the check's danger box
                     qa = st[({lay['q0']} + cb4.z) * vg::kStageStride];
                     qb = st[({lay['q0']} + cb4.w) * vg::kStageStride];
-                    const bool in = (qa >= bx.x) & (qa <= bx.y) & (qb >= bx.z) & (qb <= bx.w);
-                    if (!(__ballot_sync(vg::kFull, in) & need))
+                    mine &= __ballot_sync(vg::kFull, vg::in_box({pre}CheckBox[k], qa, qb));
+                    if (!mine)
                     {{
                         continue;
                     }}
                 }}"""
-        box_row = f"""
-                        if (cb4.z >= 0)
-                        {{
-                            const float4 bx = {pre}RowBox[i];
-                            if (!__any_sync(vg::kFull, (qa >= bx.x) & (qa <= bx.y) & (qb >= bx.z) & (qb <= bx.w)))
-                            {{
-                                continue;
-                            }}
-                        }}"""
     w(f"""    // Staged frame f: its non-constant entries from this thread's stage, the rest constants.
     static __device__ __forceinline__ vg::Frame frame_at(const float *st, int f)
     {{
@@ -956,6 +942,15 @@ if (!self_checks(ctx, st, over{wd}, boxed{wd}, on, {32 * wd + len(part) - 1}))
     // Each pair's checks run the reference's coarse test; where it overlaps, each fine sphere of A
     // against B's containing sphere (every fine sphere of B lies inside it with CONTAIN_MARGIN to
     // spare), and only rows that may touch it against B's spheres.  False once no segment is left.
+    //
+    // What bounds it is the latency of its tables, which are many times what the constant cache
+    // holds.  The frames' entries lie in global memory, where the L1 cache holds them.  Single
+    // configurations, whose warps walk nearly every check, read the pairs' spheres there too, two
+    // rows and two pairs a step, and only for lanes inside the check's danger box and not yet found
+    // colliding: 1,048,576 of Panda 598 -> 352 us (570 with constant tables, 390 with every table in
+    // global memory; Fetch 2,172 -> 1,186, 1,643 and 1,337; a danger box per pair cost more than it
+    // saved).  Segments, whose lanes are neighbours, walk few rows: one at a time from the constant
+    // tables, 65,536 Panda motions 639 us and 646 from global memory, 648 in the other form.
     template <typename Ctx>
     static __device__ __forceinline__ bool self_checks(Ctx &ctx, const float *st, unsigned over, unsigned boxed, unsigned on, int last)
     {{
@@ -1001,23 +996,64 @@ if (!self_checks(ctx, st, over{wd}, boxed{wd}, on, {32 * wd + len(part) - 1}))
                         return false;
                     }}
                     continue;
-                }}{box_gate}
+                }}
+                unsigned mine = need;  // the lanes still in question{box_gate}
                 cb.w = {pre}ContainR[k];
-                const bool mine = (need >> lane) & 1u;
-#pragma unroll 1
-                for (int r = ck.z; r < ck.w; ++r)
+                if constexpr (Ctx::kW > 1)  // one row at a time
                 {{
-                    const int4 row = {pre}Row[r];
-                    const float4 sa = vg::frame_point(a, {pre}SlotOff[row.x]);
-                    if (!__any_sync(vg::kFull, mine && vg::spheres_meet(sa, cb)))
-                    {{
-                        continue;
-                    }}
 #pragma unroll 1
-                    for (int i = row.y; i < row.z; ++i)
-                    {{{box_row}
-                        const float4 sb = vg::frame_point(b, {pre}SlotOff[{pre}RowB[i]]);
-                        acc |= vg::self_bits(sa.x, sa.y, sa.z, sb.x, sb.y, sb.z, __fadd_rn(sa.w, sb.w));
+                    for (int r = ck.z; r < ck.w; ++r)
+                    {{
+                        const int2 row = {pre}Row[r];
+                        const float4 sa = vg::frame_point(a, {pre}RowA[r]);
+                        if (!(__ballot_sync(vg::kFull, vg::spheres_meet(sa, cb)) & mine))
+                        {{
+                            continue;
+                        }}
+#pragma unroll 1
+                        for (int i = row.x; i < row.y; ++i)
+                        {{
+                            const float4 sb = vg::frame_point(b, {pre}SlotOff[{pre}RowB[i]]);
+                            acc |= vg::self_bits(sa.x, sa.y, sa.z, sb.x, sb.y, sb.z, __fadd_rn(sa.w, sb.w));
+                        }}
+                    }}
+                    const unsigned hit = ctx.vote(acc, need);
+                    if (hit && !ctx.kill(hit))
+                    {{
+                        return false;
+                    }}
+                    continue;
+                }}
+                constexpr int kRows = 2;
+#pragma unroll 1
+                for (int r = ck.z; r < ck.w && mine; r += kRows)
+                {{
+                    unsigned meet = 0u;
+#pragma unroll
+                    for (int j = 0; j < kRows; ++j)
+                    {{
+                        const bool hit = vg::spheres_meet(vg::frame_point(a, {pre}RowA[min(r + j, ck.w - 1)]), cb);
+                        meet |= hit && r + j < ck.w ? 1u << j : 0u;
+                    }}
+                    unsigned rows = __reduce_or_sync(vg::kFull, (mine >> lane) & 1u ? meet : 0u);
+#pragma unroll 1
+                    for (; rows; rows &= rows - 1u)
+                    {{
+                        const int j = __ffs(static_cast<int>(rows)) - 1;
+                        const unsigned m = __ballot_sync(vg::kFull, (meet >> j) & 1u) & mine;
+                        if (!m)
+                        {{
+                            continue;
+                        }}
+                        const int2 row = {pre}Row[r + j];
+                        const float4 sa = vg::frame_point(a, {pre}RowA[r + j]);
+#pragma unroll 2
+                        for (int i = row.x; i < row.y; ++i)
+                        {{
+                            const float4 sb = vg::frame_point(b, {pre}RowSphere[i]);
+                            acc |= vg::self_bits(sa.x, sa.y, sa.z, sb.x, sb.y, sb.z, __fadd_rn(sa.w, sb.w));
+                        }}
+                        mine &= ~__ballot_sync(vg::kFull, acc >> 31);
                     }}
                 }}
                 const unsigned hit = ctx.vote(acc, need);
