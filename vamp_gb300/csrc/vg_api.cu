@@ -501,6 +501,21 @@ namespace vg
         return VG_OK;
     }
 
+    // Configurations (or blocks) a warp checks at once, a power of two up to `most`.  Those of a warp
+    // run the union of their tests, so a small batch is spread over as many warps as are resident
+    // at once (occ thread blocks per SM) before a warp takes more; a second round of warps costs
+    // more than a fuller one saves (4,096 Baxter configurations with a cloud: 12 warps an SM resident,
+    // 186 us at 8, 239 at 16).  Measured against full warps: 4,096 Panda configurations 64 -> 56 us, with a
+    // 50,000-point cloud 138 -> 97, 1,024 Baxter with one 460 -> 114, 32 of them 387 -> 107; 65,536
+    // and more fill the warps.  256 planner steps of Panda 57.5 -> 49 us.
+    static int warp_share(size_t total, int occ, int most)
+    {
+        int share = 1;
+        while (share < most && total > static_cast<size_t>(sm_count()) * static_cast<size_t>(occ) * (kBlock / 32) * share)
+            share *= 2;
+        return share;
+    }
+
     // Blocks of a host batch above which the batch goes to the edge kernels.
     constexpr size_t kSmallBlocks = 4096;
 
@@ -573,11 +588,7 @@ namespace vg
         if (int rc = prepare_kernel(r->edge_blocks_fn[ext][which], smem, kBlock, &occ))
             return rc;
         want_field(env, static_cast<double>(total) * W, 0);
-        // Blocks of one warp run the union of their tests, so few blocks are spread over more warps, up
-        // to 16 an SM, about what is resident: 256 planner steps of Panda 57.5 us with 4 blocks a warp, 49.
-        int spread = 1;
-        while (spread < 32 / W && total > static_cast<size_t>(sm_count()) * 16 * spread)
-            spread *= 2;
+        const int spread = warp_share(total, occ, 32 / W);
         const long long per_block = (kBlock / 32) * spread;
         const int grid = static_cast<int>(std::min<long long>((static_cast<long long>(total) + per_block - 1) / per_block,
                                                               static_cast<long long>(sm_count()) * occ));
@@ -1092,9 +1103,11 @@ int vg_validate_states_device(const char *robot, vg_env *env, const float *q, si
     if (int rc = prepare_kernel(ext ? r->states_ext_fn : r->states_fn, smem, kBlock, &occ))
         return rc;
     want_field(env, static_cast<double>(n), static_cast<cudaStream_t>(stream));
-    const long long want = (static_cast<long long>(n) + kBlock - 1) / kBlock;
+    const int spread = warp_share(n, occ, 32);
+    const long long per_block = (kBlock / 32) * spread;
+    const long long want = (static_cast<long long>(n) + per_block - 1) / per_block;
     const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));
-    StatesParams p{q, static_cast<long long>(n), out, env_device(env)};
+    StatesParams p{q, static_cast<long long>(n), out, env_device(env), spread};
     VG_CUDA((ext ? r->states_ext : r->states)(p, grid, kBlock, smem, static_cast<cudaStream_t>(stream)),
             "states kernel launch");
     return VG_OK;
@@ -1397,10 +1410,11 @@ int vg_fkcc_blocks_device(const char *robot, vg_env *env, const float *q, size_t
     if (int rc = prepare_kernel(ext ? r->blocks_ext_fn[which] : r->blocks_fn[which], smem, kBlock, &occ))
         return rc;
     want_field(env, static_cast<double>(n_blocks) * env->lanes, static_cast<cudaStream_t>(stream));
-    const long long per_block = (kBlock / 32) * (32 / env->lanes);  // configuration blocks per thread block
+    const int spread = warp_share(n_blocks, occ, 32 / env->lanes);
+    const long long per_block = (kBlock / 32) * spread;  // configuration blocks per thread block
     const long long want = (static_cast<long long>(n_blocks) + per_block - 1) / per_block;
     const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));
-    StatesParams p{q, static_cast<long long>(n_blocks), out, env_device(env)};
+    StatesParams p{q, static_cast<long long>(n_blocks), out, env_device(env), spread};
     VG_CUDA((ext ? r->blocks_ext[which] : r->blocks[which])(p, grid, kBlock, smem, static_cast<cudaStream_t>(stream)),
             "blocks kernel launch");
     return VG_OK;

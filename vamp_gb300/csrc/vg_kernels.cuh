@@ -195,6 +195,7 @@ namespace vg
         long long n;
         uint8_t *out;    // 1 = valid
         EnvDevice env;
+        int spread;      // configurations (blocks) a warp checks at once, at most 32 (32 / W)
     };
 
     template <typename Robot, bool kExt = false>
@@ -205,13 +206,14 @@ namespace vg
         // this thread's column of the robot's shared-memory stage (blocks of kStageStride threads)
         float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
         constexpr int D = Robot::kDim;
-        const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+        const int lane = threadIdx.x & 31;
+        const long long stride = static_cast<long long>(gridDim.x) * (blockDim.x >> 5) * p.spread;
         // every lane of a warp iterates the same number of times (warp-uniform loop)
-        const long long base0 = static_cast<long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31);
+        const long long base0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * p.spread;
         for (long long base = base0; base < p.n; base += stride)
         {
-            const long long idx = base + (threadIdx.x & 31);
-            const bool in = idx < p.n;
+            const long long idx = base + lane;
+            const bool in = lane < p.spread && idx < p.n;
             float q[D];
 #pragma unroll
             for (int d = 0; d < D; ++d)
@@ -221,7 +223,7 @@ namespace vg
             const unsigned alive = run_fkcc<Robot, 1, kExt>(ev, q, __ballot_sync(kFull, in), stage);
             if (in)
             {
-                p.out[idx] = static_cast<uint8_t>((alive >> (threadIdx.x & 31)) & 1u);
+                p.out[idx] = static_cast<uint8_t>((alive >> lane) & 1u);
             }
         }
     }
@@ -239,14 +241,13 @@ namespace vg
         const EnvView ev = stage_env(p.env, smem);
         float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
         constexpr int D = Robot::kDim;
-        constexpr int S = 32 / W;  // blocks per warp
         const int lane = threadIdx.x & 31;
-        const long long stride = static_cast<long long>(gridDim.x) * (blockDim.x >> 5) * S;
-        for (long long base = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * S; base < p.n;
-             base += stride)
+        const long long stride = static_cast<long long>(gridDim.x) * (blockDim.x >> 5) * p.spread;
+        for (long long base = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * p.spread;
+             base < p.n; base += stride)
         {
             const long long blk = base + lane / W;
-            const bool in = blk < p.n;
+            const bool in = lane / W < p.spread && blk < p.n;
             float q[D];
 #pragma unroll
             for (int d = 0; d < D; ++d)
