@@ -1203,14 +1203,14 @@ int vg_eefk(const char *robot, const float *q, size_t n, float *out)
         return VG_OK;
     float *d = nullptr;
     const size_t in_bytes = n * r->dim * sizeof(float), out_bytes = n * 16 * sizeof(float);
-    VG_CUDA(cudaMalloc(&d, in_bytes + out_bytes), "vg_eefk: cudaMalloc");
+    VG_CUDA(pool_take(reinterpret_cast<void **>(&d), in_bytes + out_bytes, 0), "vg_eefk: allocate");
     cudaError_t e = cudaMemcpy(d, q, in_bytes, cudaMemcpyHostToDevice);
     float *d_out = d + n * r->dim;
     if (e == cudaSuccess)
         e = r->ee_pose(d, static_cast<long long>(n), d_out, nullptr);
     if (e == cudaSuccess)
         e = cudaMemcpy(out, d_out, out_bytes, cudaMemcpyDeviceToHost);
-    cudaFree(d);
+    pool_give(d, 0);
     VG_CUDA(e, "vg_eefk");
     return VG_OK;
 }
@@ -1519,20 +1519,20 @@ int vg_sphere_fk(const char *robot, const float *q, size_t n, float *out)
         return VG_OK;
     float *dq = nullptr, *dout = nullptr;
     const size_t qb = n * r->dim * sizeof(float), ob = n * r->slots * 4 * sizeof(float);
-    VG_CUDA(cudaMalloc(&dq, qb), "cudaMalloc");
-    cudaError_t e = cudaMalloc(&dout, ob);
+    VG_CUDA(pool_take(reinterpret_cast<void **>(&dq), qb, 0), "vg_sphere_fk: allocate");
+    cudaError_t e = pool_take(reinterpret_cast<void **>(&dout), ob, 0);
     if (e != cudaSuccess)
     {
-        cudaFree(dq);
-        return cuda_fail(e, "cudaMalloc");
+        pool_give(dq, 0);
+        return cuda_fail(e, "vg_sphere_fk: allocate");
     }
     e = cudaMemcpy(dq, q, qb, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = r->spheres(dq, static_cast<long long>(n), dout, 0);
     if (e == cudaSuccess)
         e = cudaMemcpy(out, dout, ob, cudaMemcpyDeviceToHost);
-    cudaFree(dq);
-    cudaFree(dout);
+    pool_give(dq, 0);
+    pool_give(dout, 0);
     if (e != cudaSuccess)
         return cuda_fail(e, "vg_sphere_fk");
     return VG_OK;

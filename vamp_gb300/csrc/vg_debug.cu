@@ -3,6 +3,7 @@
 // (bindings/robot_helper.hh:249-253).
 #include "../../include/vamp_gb300.h"
 #include "vg_internal.h"
+#include "vg_pool.h"
 
 #include <algorithm>
 #include <string>
@@ -143,9 +144,9 @@ int vg_debug_device(const char *robot, vg_env *env, const float *q, size_t n, ui
     const long long chunk = std::min<long long>(static_cast<long long>(n), kDebugChunk);
     int *d_ids = nullptr;
     float *d_sph = nullptr;
-    cudaError_t e = cudaMalloc(&d_ids, ids.size() * sizeof(int));
+    cudaError_t e = pool_take(reinterpret_cast<void **>(&d_ids), ids.size() * sizeof(int), s);
     if (e == cudaSuccess)
-        e = cudaMalloc(&d_sph, static_cast<size_t>(chunk) * r->slots * 4 * sizeof(float));
+        e = pool_take(reinterpret_cast<void **>(&d_sph), static_cast<size_t>(chunk) * r->slots * 4 * sizeof(float), s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_ids, ids.data(), ids.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     const int words = debug_words(env);
@@ -171,8 +172,8 @@ int vg_debug_device(const char *robot, vg_env *env, const float *q, size_t n, ui
     }
     // the scratch is released once the launches that read it have run
     const cudaError_t se = cudaStreamSynchronize(s);
-    cudaFree(d_sph);
-    cudaFree(d_ids);
+    pool_give(d_sph, s);
+    pool_give(d_ids, s);
     if (e != cudaSuccess || se != cudaSuccess)
         return set_error(VG_ERR_CUDA, std::string("vg_debug_device: ") + cudaGetErrorString(e != cudaSuccess ? e : se));
     return VG_OK;
@@ -188,7 +189,7 @@ int vg_debug(const char *robot, vg_env *env, const float *q, size_t n, uint32_t 
     const int words = debug_words(env);
     const size_t qb = n * r->dim * sizeof(float), bb = n * r->fine * words * sizeof(uint32_t), pb = n * r->self_pairs;
     void *d = nullptr;
-    if (cudaMalloc(&d, qb + bb + pb) != cudaSuccess)
+    if (pool_take(&d, qb + bb + pb, 0) != cudaSuccess)
         return set_error(VG_ERR_NOMEM, "vg_debug: device buffers");
     char *base = static_cast<char *>(d);
     int rc = VG_OK;
@@ -200,7 +201,7 @@ int vg_debug(const char *robot, vg_env *env, const float *q, size_t n, uint32_t 
     if (rc == VG_OK && (cudaMemcpy(env_bits, base + qb, bb, cudaMemcpyDeviceToHost) != cudaSuccess ||
                         cudaMemcpy(pairs, base + qb + bb, pb, cudaMemcpyDeviceToHost) != cudaSuccess))
         rc = set_error(VG_ERR_CUDA, "vg_debug: copy out");
-    cudaFree(d);
+    pool_give(d, 0);
     return rc;
 }
 

@@ -1058,7 +1058,7 @@ int vg_filter_self_from_pointcloud(const char *robot, vg_env *env, const float *
     if (n == 0)
         return VG_OK;
     float *d_in = nullptr;
-    VG_CUDA(cudaMalloc(&d_in, 2 * n * 3 * sizeof(float)), "vg_filter_self_from_pointcloud: cudaMalloc");
+    VG_CUDA(pool_take(reinterpret_cast<void **>(&d_in), 2 * n * 3 * sizeof(float), 0), "vg_filter_self_from_pointcloud: allocate");
     float *d_out = d_in + 3 * n;
     int rc = VG_OK;
     cudaError_t e = cudaMemcpy(d_in, xyz, n * 3 * sizeof(float), cudaMemcpyHostToDevice);
@@ -1066,7 +1066,7 @@ int vg_filter_self_from_pointcloud(const char *robot, vg_env *env, const float *
         rc = vg_filter_self_from_pointcloud_device(robot, env, d_in, n, point_radius, q, d_out, n_out, nullptr);
     if (e == cudaSuccess && rc == VG_OK && *n_out)
         e = cudaMemcpy(out, d_out, *n_out * 3 * sizeof(float), cudaMemcpyDeviceToHost);
-    cudaFree(d_in);
+    pool_give(d_in, 0);
     if (e != cudaSuccess)
         return cuda_fail(e, "vg_filter_self_from_pointcloud: copy");
     return rc;
@@ -1083,7 +1083,7 @@ int vg_filter_pointcloud(const float *xyz, size_t n, float min_dist, float max_r
     if (n > 0)
     {
         float *d_in = nullptr;
-        VG_CUDA(cudaMalloc(&d_in, 2 * n * 3 * sizeof(float)), "vg_filter_pointcloud: cudaMalloc");
+        VG_CUDA(pool_take(reinterpret_cast<void **>(&d_in), 2 * n * 3 * sizeof(float), 0), "vg_filter_pointcloud: allocate");
         float *d_out = d_in + 3 * n;
         int rc = VG_OK;
         cudaError_t e = cudaMemcpy(d_in, xyz, n * 3 * sizeof(float), cudaMemcpyHostToDevice);
@@ -1092,7 +1092,7 @@ int vg_filter_pointcloud(const float *xyz, size_t n, float min_dist, float max_r
                                   nullptr);
         if (e == cudaSuccess && rc == VG_OK && *n_out)
             e = cudaMemcpy(out, d_out, *n_out * 3 * sizeof(float), cudaMemcpyDeviceToHost);
-        cudaFree(d_in);
+        pool_give(d_in, 0);
         if (e != cudaSuccess)
             return cuda_fail(e, "vg_filter_pointcloud: copy");
         if (rc != VG_OK)

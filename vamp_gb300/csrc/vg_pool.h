@@ -1,5 +1,5 @@
-// Device memory that comes and goes with calls and environments (the pointcloud filter's and tree
-// builds' scratch, trees, environment images): a private
+// Device memory that comes and goes with calls and environments (the pointcloud filter's, tree
+// builds' and debug reports' scratch, host calls' buffers, trees, environment images): a private
 // stream-ordered pool per device, which keeps up to kPoolKeep bytes between calls (an allocation of
 // tens of megabytes from the driver takes longer than the work in it) and returns the rest to the
 // driver.  Safe with several threads and streams: allocations and releases are ordered on their
