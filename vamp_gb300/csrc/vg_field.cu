@@ -126,7 +126,7 @@ namespace vg
             {
                 const int l = t + 256 * i;
                 const int ix = 8 * bx + (l & 7), iy = 8 * by + (l >> 3 & 7), iz = 8 * bz + (l >> 6);
-                cell[i] = (iz << (2 * kFieldBits)) + (iy << kFieldBits) + ix;
+                cell[i] = field_at(ix, iy, iz);
                 p[i] = cell_centre(ix, iy, iz);
                 best[i] = kCap;
             }
@@ -280,7 +280,7 @@ namespace vg
             auto value = [&](int b, uint8_t have) {
                 return static_cast<uint8_t>(min(static_cast<unsigned>(have), step_of(sqrtf(static_cast<float>(b)) * kCell - less)));
             };
-            uchar4 *cell = reinterpret_cast<uchar4 *>(out) + z * kPlane + at;
+            uchar4 *cell = reinterpret_cast<uchar4 *>(out + field_at(4 * threadIdx.x, blockIdx.x * kLines + threadIdx.y, z));
             const uchar4 have = *cell;
             *cell = make_uchar4(value(best[0], have.x), value(best[1], have.y), value(best[2], have.z), value(best[3], have.w));
         }
@@ -356,7 +356,7 @@ namespace vg
             }
             for (int iz = 0; iz < kFieldCells; ++iz)
             {
-                uint8_t *cell = out + (iz << (2 * kFieldBits)) + (iy << kFieldBits) + ix;
+                uint8_t *cell = out + field_at(ix, iy, iz);
                 const float z = (static_cast<float>(iz) - kFieldZ) * kCell;
                 float clear = 0.0f;
 #pragma unroll
