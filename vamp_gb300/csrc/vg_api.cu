@@ -265,7 +265,8 @@ namespace vg
 
     // A sphere, in the attachment's own coordinates, whose pose contains the pose of every sphere of
     // the attachment, 0.1 mm to spare (its relative transform may scale: distances grow by at most
-    // the Frobenius norm of its 3 x 3 part).  Not finite (contains everything) where they are not.
+    // the Frobenius norm of its 3 x 3 part).  Where they are not finite its centre or radius is not
+    // either, which rules nothing out (attach_check).
     static float4 attachment_bound(const vg_env *e)
     {
         double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0}, norm2 = 0.0, size = 1.0;

@@ -150,7 +150,11 @@ namespace vg
             const int4 li = Robot::attach_link(L);
             const Frame f = Robot::frame_at(st, li.w);
             const float4 coarse = frame_point(f, Robot::slot_offset(li.x));
-            unsigned gate = ctx.self_hit(coarse.x, coarse.y, coarse.z, coarse.w, whole.x, whole.y, whole.z, whole.w, ctx.alive);
+            // not (apart): where the containing sphere is not finite, or the squares overflow, the value
+            // is NaN or -inf, which rules nothing out
+            const float rs = __fadd_rn(coarse.w, whole.w);
+            const float apart = __fmaf_rn(-rs, rs, sql2(coarse.x, coarse.y, coarse.z, whole.x, whole.y, whole.z));
+            unsigned gate = ctx.vote(apart > 0.0f ? 0u : 0x80000000u, ctx.alive);
             if (!gate)
             {
                 continue;
