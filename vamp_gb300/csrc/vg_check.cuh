@@ -711,6 +711,9 @@ namespace vg
         // every active lane's configuration lies inside the joint limits widened by the culling
         // slack: fine self pairs proven unable to collide there may be skipped
         bool in_limits = false;
+        // some active lane's configuration is so far out that its frames may not be rigid: a sphere
+        // that contains others by their distances in a frame may not contain them
+        bool far = false;
         // this thread's column of the robot's shared-memory stage: element i at stage[i * kStageStride]
         float *stage = nullptr;
 

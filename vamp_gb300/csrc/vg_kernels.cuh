@@ -115,7 +115,8 @@ namespace vg
                 c[r] = __fmaf_rn(NR[3 * r + 2], s.z, __fmaf_rn(NR[3 * r + 1], s.y, __fmaf_rn(NR[3 * r], s.x, Nt[r])));
             return make_float4(c[0], c[1], c[2], s.w);
         };
-        const float4 whole = posed(ev.n_att);  // contains every posed sphere (attachment_bound)
+        float4 whole = posed(ev.n_att);  // contains every posed sphere (attachment_bound)
+        whole.w = ctx.far ? __int_as_float(0x7f800000) : whole.w;
         if (ctx.may_touch(whole, ctx.alive))
         {
 #pragma unroll 1
@@ -181,7 +182,8 @@ namespace vg
     template <typename Robot, int W, bool kExt = false, bool kOrdered = false>
     __device__ __forceinline__ unsigned run_fkcc(const EnvView &ev, const float *q, unsigned alive, float *stage)
     {
-        CheckCtx<W, kExt, kOrdered> ctx{ev, alive, false, stage};
+        CheckCtx<W, kExt, kOrdered> ctx{ev, alive};
+        ctx.stage = stage;
         Robot::fkcc(q, ctx);
         if constexpr (kExt)
         {

@@ -447,6 +447,11 @@ def danger_boxes(model: dict, cull) -> list:
 # Baxter's stage leaves room for three (built for 4, with spills: 1,270 us; for 3: 1,224).
 EDGE_BLOCKS = {"panda": 5, "ur5": 5, "fetch": 5, "baxter": 3}
 CONTAIN_MARGIN = 1e-4  # metres between a link's fine spheres and its containing sphere
+# A joint value beyond this (radians or metres) may leave frames that do not keep distances: the sine
+# and the cosine each round the angle, so they stand for angles that differ by up to half a unit of
+# its last place.  At 64 that is 4e-6 a joint, under 0.02 mm over seven joints and a group's half
+# metre, a fifth of CONTAIN_MARGIN; at 10^6 it is 0.03, and containing spheres contain no more.
+FAR_JOINT = 64.0
 
 
 def containing_radius(model: dict, kin, env_check: dict) -> float:
@@ -822,7 +827,7 @@ def gen_cuda(model: dict) -> str:
             xyz = emit_point(em, fr[fid], c, f"g{g}_")
         body += em.lines
         group_sphere.append((xyz, float(r)))
-        body.append(f"const unsigned v{g} = ctx.clearance({', '.join(xyz)});")
+        body.append(f"unsigned v{g} = ctx.clearance({', '.join(xyz)});")
     em.lines = []
     body.append("// per lane: the pairs of groups that overlap, and those whose joints lie in a danger box")
     plist = list(pairs)
@@ -848,6 +853,17 @@ def gen_cuda(model: dict) -> str:
                     b[0][0], lit32(b[1][0]), b[0][0], lit32(b[1][1]), b[0][1], lit32(b[1][2]), b[0][1], lit32(b[1][3])) for b in bs)
                 body.append(f"    boxed{wd} &= {cond} ? ~0u : ~{1 << bit}u;")
             body.append("}")
+    body.append("if (!ctx.in_limits)")
+    body.append("{")
+    near = " & ".join(f"(fabsf(q[{d}]) <= {lit32(FAR_JOINT)})" for d in range(dim))
+    body.append(f"    ctx.far = __any_sync(vg::kFull, !({near}) && ((ctx.alive >> (threadIdx.x & 31)) & 1u));")
+    body.append("    if (ctx.far)  // what stands for a group contains nothing for sure: every check is run")
+    body.append("    {")
+    body.append("        %s = 0u;" % " = ".join(f"v{g}" for g in range(n_groups)))
+    for wd in range(n_words):
+        body.append(f"        over{wd} = {hex((1 << len(plist[32 * wd:32 * wd + 32])) - 1)}u;")
+    body.append("    }")
+    body.append("}")
     body.append("// per lane: the groups that may touch something")
     body.append("unsigned near = 0u;")
     for g in range(n_groups):
