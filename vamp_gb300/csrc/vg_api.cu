@@ -347,11 +347,13 @@ namespace vg
                 img.push_back(make_float4(e->att[4 * k], e->att[4 * k + 1], e->att[4 * k + 2], e->att[4 * k + 3]));
             img.push_back(attachment_bound(e));
         }
+        // checks already queued, on any stream, still have the image before to read
+        if (e->d_image)
+            VG_CUDA(cudaDeviceSynchronize(), "wait for the checks before");
         if (img.size() > e->image_cap)
         {
             if (e->d_image)
             {
-                cudaDeviceSynchronize();  // checks on any stream may be reading it
                 pool_give(e->d_image, 0);
                 e->d_image = nullptr;
                 e->d_counter = nullptr;
@@ -364,6 +366,9 @@ namespace vg
             e->d_counter = reinterpret_cast<unsigned *>(e->d_image + cap);
         }
         VG_CUDA(cudaMemcpy(e->d_image, img.data(), img.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload environment");
+        // a copy from pageable memory may return before it has landed, and the default stream does not
+        // order it before checks on streams that do not synchronise with it
+        VG_CUDA(cudaStreamSynchronize(0), "upload environment");
         e->image_f4 = img.size();
         e->field_ready.store(false);
         e->field_states = 0.0;
