@@ -633,14 +633,16 @@ namespace vg
         {
             return nullptr;
         }
+        // A caller's graph would hold the buffer past the next larger batch, which frees it, and the
+        // graph cannot allocate its own: captured launches hand the edges out as given.
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
+        {
+            cudaGetLastError();
+            return nullptr;
+        }
         if (m.n > env->rank_cap)
         {
-            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
-            {
-                cudaGetLastError();
-                return nullptr;  // no allocation under capture: the edges go as given
-            }
             if (env->d_rank)
                 cudaFree(env->d_rank);
             env->d_rank = nullptr;
