@@ -130,10 +130,9 @@ namespace vg
     }
 
     // Packs the sorted host rows into the device image (layouts in vg_check.cuh).
-    static void pack_image(const vg_env *e, std::vector<float4> &img, int off[5], int n[5])
+    // Appends the primitive records, and enters their offsets and counts in the image's head.
+    static void pack_records(const vg_env *e, std::vector<float4> &img, int off[5], int n[5])
     {
-        img.assign(kRsqrtF4, make_float4(0, 0, 0, 0));
-        std::memcpy(img.data(), kX86RsqrtTable, sizeof(uint32_t) * 2048);
         for (int k = 0; k < 5; ++k)
         {
             const int w = kFields[k] + 1;
@@ -163,6 +162,9 @@ namespace vg
                 }
             }
         }
+        int *head = reinterpret_cast<int *>(img.data() + kRsqrtF4);
+        std::copy(off, off + 5, head);
+        std::copy(n, n + 5, head + 5);
     }
 
     static_assert(sizeof(CaptView) % sizeof(float4) == 0, "CaptView must pack into float4s");
@@ -326,8 +328,8 @@ namespace vg
             e->d_hf.push_back(p);
             VG_CUDA(cudaMemcpy(p, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice), "upload heightfield");
         }
-        std::vector<float4> img;
-        pack_image(e, img, e->off, e->n);
+        std::vector<float4> img(kHeadF4, make_float4(0, 0, 0, 0));
+        std::memcpy(img.data(), kX86RsqrtTable, sizeof(uint32_t) * 2048);
         pack_clouds(e, img, &e->cloud_off);
         static_assert(sizeof(HeightView) % sizeof(float4) == 0, "HeightView must pack into float4s");
         e->hf_off = static_cast<int>(img.size());
@@ -347,6 +349,7 @@ namespace vg
                 img.push_back(make_float4(e->att[4 * k], e->att[4 * k + 1], e->att[4 * k + 2], e->att[4 * k + 3]));
             img.push_back(attachment_bound(e));
         }
+        pack_records(e, img, e->off, e->n);
         // checks already queued, on any stream, still have the image before to read
         if (e->d_image)
             VG_CUDA(cudaDeviceSynchronize(), "wait for the checks before");
@@ -382,10 +385,10 @@ namespace vg
     {
         EnvDevice d{};
         d.buf = e->d_image;
-        d.n_f4 = static_cast<int>(e->image_f4);
+        d.staged = static_cast<int>(e->image_f4) - kHeadF4;
         for (int k = 0; k < 5; ++k)
         {
-            d.n[k] = e->n[k];
+            d.n[k] = d.near[k] = e->n[k];
             d.off[k] = e->off[k];
         }
         d.sqrt_mode = e->sqrt_mode;
@@ -420,6 +423,49 @@ namespace vg
             counts[dev].store(c, std::memory_order_relaxed);
         }
         return c;
+    }
+
+    static int shared_limit()
+    {
+        // per device, as sm_count
+        constexpr int kDevices = 64;
+        static std::atomic<int> limits[kDevices] = {};
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 0 && dev < kDevices && (v = limits[dev].load(std::memory_order_relaxed)) > 0)
+        {
+            return v;
+        }
+        cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (dev >= 0 && dev < kDevices)
+        {
+            limits[dev].store(v, std::memory_order_relaxed);
+        }
+        return v;
+    }
+
+    int stage_split(EnvDevice &d, int beside, int *smem)
+    {
+        const int limit = shared_limit(), image = d.staged * static_cast<int>(sizeof(float4));
+        *smem = image + beside;
+        if (*smem <= limit)
+        {
+            return VG_OK;
+        }
+        if (image > limit)
+        {
+            return set_error(VG_ERR_LIMIT, "the environment needs " + std::to_string(image) +
+                                               " bytes, more than the GPU's " + std::to_string(limit) +
+                                               " of shared memory per block (too many primitives)");
+        }
+        d.staged = (limit - beside) / static_cast<int>(sizeof(float4));
+        d.cut = kHeadF4 + d.staged;
+        for (int k = 0; k < 5; ++k)
+        {
+            d.near[k] = records_before(d.cut, d.off[k], d.n[k], rec_f4(k));
+        }
+        *smem = d.staged * static_cast<int>(sizeof(float4)) + beside;
+        return VG_OK;
     }
 
     int prepare_kernel(const void *fn, int smem, int block, int *blocks_per_sm)
@@ -589,17 +635,20 @@ namespace vg
         uint8_t *verdicts = reinterpret_cast<uint8_t *>(pin + out_at);
         std::memset(verdicts, 1, n);
         const int ext = env->extended() ? 1 : 0, which = W == 8 ? 0 : 1;
-        const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4)) + r->stage_floats * kBlock * 4;
+        want_field(env, static_cast<double>(total) * W, 0);
+        EnvDevice dev = env_device(env);
+        int smem = 0;
+        if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
+            return rc;
         int occ = 0;
         if (int rc = prepare_kernel(r->edge_blocks_fn[ext][which], smem, kBlock, &occ))
             return rc;
-        want_field(env, static_cast<double>(total) * W, 0);
         const int spread = warp_share(total, occ, 32 / W);
         const long long per_block = (kBlock / 32) * spread;
         const int grid = static_cast<int>(std::min<long long>((static_cast<long long>(total) + per_block - 1) / per_block,
                                                               static_cast<long long>(sm_count()) * occ));
         EdgeBlocksParams p{reinterpret_cast<const float *>(pin), reinterpret_cast<const float *>(pin + ab), dist ? 1 : 0,
-                           reinterpret_cast<const int2 *>(pin + items_at), static_cast<int>(total), spread, verdicts, env_device(env)};
+                           reinterpret_cast<const int2 *>(pin + items_at), static_cast<int>(total), spread, verdicts, dev};
         VG_CUDA(r->edge_blocks[ext][which](p, grid, kBlock, smem, 0), "edge blocks kernel launch");
         VG_CUDA(cudaStreamSynchronize(0), "synchronize");
         std::memcpy(out, verdicts, n);
@@ -661,7 +710,10 @@ namespace vg
     {
         const RobotOps *r = m.r;
         const vg_env *env = m.env;
-        const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4)) + r->stage_floats * kBlock * 4;
+        EnvDevice dev = env_device(env);
+        int smem = 0;
+        if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
+            return rc;
         const int which = env->lanes == 8 ? 0 : 1;
         // with heightfields or an attachment every schedule runs the extended checks in the same-edge
         // kernel (the block order does not change verdicts, so a learned order is not needed there)
@@ -685,7 +737,7 @@ namespace vg
         const int per_block = grouped ? kBlock / 32 : kBlock / env->lanes;
         const long long want = (static_cast<long long>(m.n) + per_block - 1) / per_block;
         const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));
-        EdgesParams p{m.a, m.b, static_cast<int>(m.n), m.resolution, m.out, m.blocks, m.counter, env_device(env), m.scores, m.probes,
+        EdgesParams p{m.a, m.b, static_cast<int>(m.n), m.resolution, m.out, m.blocks, m.counter, dev, m.scores, m.probes,
                       m.dist, m.order};
         if (grouped && !packed && m.rank && ranked(m))
         {
@@ -1105,17 +1157,20 @@ int vg_validate_states_device(const char *robot, vg_env *env, const float *q, si
         return VG_OK;
     if (int rc = commit(env))
         return rc;
-    const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4)) + r->stage_floats * kBlock * 4;
+    want_field(env, static_cast<double>(n), static_cast<cudaStream_t>(stream));
+    EnvDevice dev = env_device(env);
+    int smem = 0;
+    if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
+        return rc;
     const bool ext = env->extended();
     int occ = 0;
     if (int rc = prepare_kernel(ext ? r->states_ext_fn : r->states_fn, smem, kBlock, &occ))
         return rc;
-    want_field(env, static_cast<double>(n), static_cast<cudaStream_t>(stream));
     const int spread = warp_share(n, occ, 32);
     const long long per_block = (kBlock / 32) * spread;
     const long long want = (static_cast<long long>(n) + per_block - 1) / per_block;
     const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));
-    StatesParams p{q, static_cast<long long>(n), out, env_device(env), spread};
+    StatesParams p{q, static_cast<long long>(n), out, dev, spread};
     VG_CUDA((ext ? r->states_ext : r->states)(p, grid, kBlock, smem, static_cast<cudaStream_t>(stream)),
             "states kernel launch");
     return VG_OK;
@@ -1413,16 +1468,19 @@ int vg_fkcc_blocks_device(const char *robot, vg_env *env, const float *q, size_t
         return rc;
     const int which = env->lanes == 8 ? 0 : 1;
     const bool ext = env->extended();
-    const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4)) + r->stage_floats * kBlock * 4;
+    want_field(env, static_cast<double>(n_blocks) * env->lanes, static_cast<cudaStream_t>(stream));
+    EnvDevice dev = env_device(env);
+    int smem = 0;
+    if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
+        return rc;
     int occ = 0;
     if (int rc = prepare_kernel(ext ? r->blocks_ext_fn[which] : r->blocks_fn[which], smem, kBlock, &occ))
         return rc;
-    want_field(env, static_cast<double>(n_blocks) * env->lanes, static_cast<cudaStream_t>(stream));
     const int spread = warp_share(n_blocks, occ, 32 / env->lanes);
     const long long per_block = (kBlock / 32) * spread;  // configuration blocks per thread block
     const long long want = (static_cast<long long>(n_blocks) + per_block - 1) / per_block;
     const int grid = static_cast<int>(std::min<long long>(want, static_cast<long long>(sm_count()) * occ));
-    StatesParams p{q, static_cast<long long>(n_blocks), out, env_device(env), spread};
+    StatesParams p{q, static_cast<long long>(n_blocks), out, dev, spread};
     VG_CUDA((ext ? r->blocks_ext[which] : r->blocks[which])(p, grid, kBlock, smem, static_cast<cudaStream_t>(stream)),
             "blocks kernel launch");
     return VG_OK;

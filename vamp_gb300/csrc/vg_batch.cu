@@ -252,6 +252,10 @@ int vg_autotune_motions(const char *robot, vg_env *env, const float *a, const fl
         return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     want_field(env, kEdgeStates * static_cast<double>(n), s);
+    EnvDevice dev = env_device(env);
+    int smem = 0;
+    if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
+        return rc;
     uint8_t *out = nullptr;
     VG_CUDA(cudaMalloc(&out, n), "cudaMalloc(autotune)");
     cudaEvent_t e0, e1;
@@ -260,7 +264,6 @@ int vg_autotune_motions(const char *robot, vg_env *env, const float *a, const fl
     int best_s = 1, best_b = 0, rc = VG_OK;
     float best = 1e30f;
     const int which = env->lanes == 8 ? 0 : 1;
-    const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4)) + r->stage_floats * kBlock * 4;
     for (int sched = 0; sched < 4 && rc == VG_OK; ++sched)
     {
         int occ = 0;

@@ -217,7 +217,20 @@ namespace vg
         const HeightView *hf;
         int n_hf;
         const uint8_t *field;  // clearance field (below); null: not built
+        const float4 *image;   // the whole image in global memory
+        int cut;               // where its staged part ends (0: all of it is staged)
     };
+
+    // The image's head: the RSQRTPS table, then five record offsets and five counts.
+    constexpr int kRsqrtF4 = 2048 / 4;
+    constexpr int kHeadF4 = kRsqrtF4 + 3;
+
+    // Records of a kind, `off` float4s into an image and `n` of them, that lie whole before `cut`.
+    __host__ __device__ constexpr int records_before(int cut, int off, int n, int size)
+    {
+        const int room = cut > off ? (cut - off) / size : 0;
+        return room < n ? room : n;
+    }
 
     // ------------------------------------------------------------------- clearance field
     //
@@ -408,11 +421,9 @@ namespace vg
     // Mw (its largest M, a uniform branch) and a lane counts a result only while min_distance < M
     // (its own segment's bound).  Sign bits are OR-ed into bits; the segment vote happens once.
     template <int KIND>
-    __device__ __forceinline__ void kind_pass(const EnvView &e, float Mw, float M, float x, float y, float z, float r, float rsq,
+    __device__ __forceinline__ void kind_pass(const float4 *rec, int n, float Mw, float M, float x, float y, float z, float r, float rsq,
                                               unsigned &bits)
     {
-        const float4 *rec = e.rec[KIND];
-        const int n = e.n[KIND];
 #pragma unroll 1
         for (int i = 0; i < n; ++i)
         {
@@ -425,6 +436,33 @@ namespace vg
             const float t = prim_test<KIND>(o, x, y, z, r, rsq);
             bits |= md < M ? __float_as_uint(t) : 0u;
         }
+    }
+
+    // kind_pass over a kind's records past `cut`, read from the image in global memory
+    template <int KIND>
+    __device__ __forceinline__ void far_kind(const float4 *image, int cut, float Mw, float M, float x, float y, float z, float r,
+                                             float rsq, unsigned &bits)
+    {
+        const int *head = reinterpret_cast<const int *>(image + kRsqrtF4);
+        const int off = __ldg(head + KIND), n = __ldg(head + 5 + KIND);
+        const int near = records_before(cut, off, n, rec_f4(KIND));
+        kind_pass<KIND>(image + off + near * rec_f4(KIND), n - near, Mw, M, x, y, z, r, rsq, bits);
+    }
+
+    // The sign bits of the records that did not fit the shared memory beside the robot's stage (26 to 58 KB a
+    // block): environments of up to 227 KB are accepted for every robot.  Out of the kernels' way, a
+    // call behind one uniform branch, because few environments are that large.
+    static __device__ __noinline__ unsigned far_records(const float4 *image, int cut, float Mw, float M, float x, float y, float z,
+                                                        float r)
+    {
+        const float rsq = __fmul_rn(r, r);
+        unsigned bits = 0u;
+        far_kind<0>(image, cut, Mw, M, x, y, z, r, rsq, bits);
+        far_kind<1>(image, cut, Mw, M, x, y, z, r, rsq, bits);
+        far_kind<2>(image, cut, Mw, M, x, y, z, r, rsq, bits);
+        far_kind<3>(image, cut, Mw, M, x, y, z, r, rsq, bits);
+        far_kind<4>(image, cut, Mw, M, x, y, z, r, rsq, bits);
+        return bits;
     }
 
 #ifndef VG_CAPT_SHARED_WEIGHT
@@ -614,11 +652,15 @@ namespace vg
         // floats, so one warp reduction gives the warp-wide bound (inactive lanes count as 0)
         const float Mw = __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(m) : 0u));
         unsigned bits = 0u;
-        kind_pass<0>(e, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<1>(e, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<2>(e, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<3>(e, Mw, M, x, y, z, r, rsq, bits);
-        kind_pass<4>(e, Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<0>(e.rec[0], e.n[0], Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<1>(e.rec[1], e.n[1], Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<2>(e.rec[2], e.n[2], Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<3>(e.rec[3], e.n[3], Mw, M, x, y, z, r, rsq, bits);
+        kind_pass<4>(e.rec[4], e.n[4], Mw, M, x, y, z, r, rsq, bits);
+        if (e.cut)
+        {
+            bits |= far_records(e.image, e.cut, Mw, M, x, y, z, r);
+        }
         if constexpr (kExt)
         {
 #pragma unroll 1

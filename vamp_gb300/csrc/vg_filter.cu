@@ -1022,12 +1022,15 @@ int vg_filter_self_from_pointcloud_device(const char *robot, vg_env *env, const 
     carve();
     VG_CUDA(cudaMemcpyAsync(dq, q, r->dim * sizeof(float), cudaMemcpyHostToDevice, s), "vg_filter_self_from_pointcloud: copy");
     VG_CUDA(r->spheres(dq, 1, sph, s), "vg_filter_self_from_pointcloud: sphere_fk");
-    const int smem = static_cast<int>(staged_f4(static_cast<int>(env->image_f4)) * sizeof(float4));
+    EnvDevice dev = env_device(env);
+    int smem = 0;
+    if (int rc = stage_split(dev, 0, &smem))
+        return rc;
     int occ = 0;
     if (int rc = prepare_kernel(reinterpret_cast<const void *>(&filter_self_kernel), smem, 256, &occ))
         return rc;
     const int grid = static_cast<int>(std::min<long long>(blocks_of(N, 256), static_cast<long long>(sm_count()) * occ));
-    filter_self_kernel<<<grid, 256, smem, s>>>(xyz, N, point_radius, sph, r->fine, env_device(env), flags);
+    filter_self_kernel<<<grid, 256, smem, s>>>(xyz, N, point_radius, sph, r->fine, dev, flags);
     tile_sums<<<static_cast<unsigned>(tiles), kTile, 0, s>>>(flags, N, sums);
     if (tiles > kDirectTiles)
     {

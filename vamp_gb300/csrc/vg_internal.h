@@ -217,6 +217,10 @@ namespace vg
     // Gives the field's buffer back (waits for the device).
     void release_field(vg_env *e);
     int sm_count();
+    // Splits an environment between shared and global memory for kernels that need `beside` bytes of shared
+    // memory for themselves: *smem is what a block needs in all.  VG_ERR_LIMIT where the image alone
+    // is more than a block can have.
+    int stage_split(EnvDevice &d, int beside, int *smem);
     int prepare_kernel(const void *fn, int smem, int block, int *blocks_per_sm);
     void tuned_for(const vg_env *env, const RobotOps *r, int *schedule, int *blocks_per_sm);
     int launch_motions(const MotionLaunch &m, cudaStream_t s);

@@ -25,16 +25,19 @@
 #endif
 namespace vg
 {
-    // Device image of an environment: the x86 RSQRTPS table followed by the primitive records
-    // of each kind (layouts in vg_check.cuh), all float4 aligned.
+    // Device image of an environment: the x86 RSQRTPS table, the records' offsets and counts per kind
+    // (EnvDevice::off and n), the descriptors of clouds and heightfields, the attachment, then
+    // the primitive records of each kind (layouts in vg_check.cuh), all float4 aligned.
     struct EnvDevice
     {
         const float4 *buf;  // whole image
-        int n_f4;           // image size in float4
+        int staged;         // float4s after the head that a thread block stages into shared memory
+        int cut;            // where they end in the image (0: with the image)
         int n[5];           // objects per kind
+        int near[5];        // those of them that are staged, the first ones
         int off[5];         // record offset of each kind, in float4 from the image start
         int sqrt_mode;
-        int n_clouds;       // CaptView descriptors at the end of the image
+        int n_clouds;       // CaptView descriptors
         int cloud_off;      // their offset, in float4
         int n_att;          // attachment spheres (-1: no attachment)
         int att_off;        // attachment block: 3 transform rows, then the spheres, in float4
@@ -43,38 +46,33 @@ namespace vg
         const uint8_t *field;  // clearance field (null: not built)
     };
 
-    constexpr int kRsqrtF4 = 2048 / 4;
-
-    // Float4s of the image each block stages into shared memory: all but the RSQRTPS table,
-    // which stays in global memory (read through the L1 cache), so that shared memory goes to
-    // more resident warps.
-    __host__ __device__ constexpr int staged_f4(int n_f4)
-    {
-        return n_f4 - kRsqrtF4;
-    }
-
+    // Each block stages the image into shared memory, all but its head (the RSQRTPS table, which is read
+    // through the L1 cache, so that shared memory goes to more resident warps, and the counts).
+    // Of an environment that does not fit beside the robot's own stage the last records stay in
+    // global memory, too (far_records, vg_check.cuh).
     __device__ __forceinline__ EnvView stage_env(const EnvDevice &d, float4 *smem)
     {
-        const int n = staged_f4(d.n_f4);
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
+        for (int i = threadIdx.x; i < d.staged; i += blockDim.x)
         {
-            smem[i] = d.buf[kRsqrtF4 + i];
+            smem[i] = d.buf[kHeadF4 + i];
         }
         __syncthreads();
         EnvView v;
         v.rsqrt_tab = reinterpret_cast<const uint32_t *>(d.buf);
         v.sqrt_mode = d.sqrt_mode;
-        v.clouds = reinterpret_cast<const CaptView *>(smem + d.cloud_off - kRsqrtF4);
+        v.clouds = reinterpret_cast<const CaptView *>(smem + d.cloud_off - kHeadF4);
         v.n_clouds = d.n_clouds;
-        v.att = smem + d.att_off - kRsqrtF4;
+        v.att = smem + d.att_off - kHeadF4;
         v.n_att = d.n_att;
-        v.hf = reinterpret_cast<const HeightView *>(smem + d.hf_off - kRsqrtF4);
+        v.hf = reinterpret_cast<const HeightView *>(smem + d.hf_off - kHeadF4);
         v.n_hf = d.n_hf;
         v.field = d.field;
+        v.image = d.buf;
+        v.cut = d.cut;
         for (int k = 0; k < 5; ++k)
         {
-            v.rec[k] = smem + d.off[k] - kRsqrtF4;
-            v.n[k] = d.n[k];
+            v.rec[k] = smem + d.off[k] - kHeadF4;
+            v.n[k] = d.near[k];
         }
         return v;
     }
@@ -210,7 +208,7 @@ namespace vg
         extern __shared__ float4 smem[];
         const EnvView ev = stage_env(p.env, smem);
         // this thread's column of the robot's shared-memory stage (blocks of kStageStride threads)
-        float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
+        float *const stage = reinterpret_cast<float *>(smem + p.env.staged) + threadIdx.x;
         constexpr int D = Robot::kDim;
         const int lane = threadIdx.x & 31;
         const long long stride = static_cast<long long>(gridDim.x) * (blockDim.x >> 5) * p.spread;
@@ -245,7 +243,7 @@ namespace vg
     {
         extern __shared__ float4 smem[];
         const EnvView ev = stage_env(p.env, smem);
-        float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
+        float *const stage = reinterpret_cast<float *>(smem + p.env.staged) + threadIdx.x;
         constexpr int D = Robot::kDim;
         const int lane = threadIdx.x & 31;
         const long long stride = static_cast<long long>(gridDim.x) * (blockDim.x >> 5) * p.spread;
@@ -311,7 +309,7 @@ namespace vg
         };
         load(seg < p.spread && base + seg < p.n);
         const EnvView ev = stage_env(p.env, smem);
-        float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
+        float *const stage = reinterpret_cast<float *>(smem + p.env.staged) + threadIdx.x;
         for (bool first = true; base < p.n; base += stride, first = false)
         {
             const bool in = seg < p.spread && base + seg < p.n;
@@ -618,7 +616,7 @@ namespace vg
         extern __shared__ float4 smem[];
         const EnvView ev = stage_env(p.env, smem);
         // this thread's column of the robot's shared-memory stage (blocks of kStageStride threads)
-        float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
+        float *const stage = reinterpret_cast<float *>(smem + p.env.staged) + threadIdx.x;
         constexpr int D = Robot::kDim;
         const int lane = threadIdx.x & 31;
         const int sl = lane % W;                  // lane within the segment
@@ -732,7 +730,7 @@ namespace vg
         extern __shared__ float4 smem[];
         const EnvView ev = stage_env(p.env, smem);
         // this thread's column of the robot's shared-memory stage (blocks of kStageStride threads)
-        float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
+        float *const stage = reinterpret_cast<float *>(smem + p.env.staged) + threadIdx.x;
         constexpr int D = Robot::kDim;
         constexpr int S = 32 / W;                 // segments (blocks) per warp
         const int lane = threadIdx.x & 31;
@@ -893,7 +891,7 @@ namespace vg
         static_assert(W == 8 || W == 4, "packed schedule: 4 or 8 segments per warp");
         extern __shared__ float4 smem[];
         const EnvView ev = stage_env(p.env, smem);
-        float *const stage = reinterpret_cast<float *>(smem + staged_f4(p.env.n_f4)) + threadIdx.x;
+        float *const stage = reinterpret_cast<float *>(smem + p.env.staged) + threadIdx.x;
         constexpr int D = Robot::kDim;
         constexpr int S = 32 / W;  // segments (blocks) per warp
         const int lane = threadIdx.x & 31;
