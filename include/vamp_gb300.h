@@ -162,6 +162,11 @@ int vg_env_set_mode(vg_env *env, int lanes, int sqrt_mode);
  * (vg_autotune_motions) takes precedence until this is called again.
  * No reference counterpart: the reference validates one edge at a time on one core. */
 int vg_env_set_schedule(vg_env *env, int schedule);
+/* 1 if the environment's clearance field stands (0: not, -1: null environment): a grid of lower bounds
+ * of the distance to anything in it, which the checks build on the GPU once enough configurations
+ * have been checked since the environment's last change, and skip exact tests by.  Verdicts and
+ * block counts do not depend on it.  No reference counterpart. */
+int vg_env_field_ready(const vg_env *env);
 /* Number of objects of a kind (0 spheres, 1 capsules, 2 z-capsules, 3 cuboids, 4 z-cuboids)
  * and the fields of one, in checking order, followed by its min_distance. */
 int vg_env_count(const vg_env *env, int kind, size_t *count);

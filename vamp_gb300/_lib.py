@@ -64,6 +64,7 @@ def _load() -> ctypes.CDLL:
         "vg_env_add_heightfield_fields": ([_p, _p, _sz, _sz, _p], _i),
         "vg_fkcc_blocks_device": ([_s, _p, _p, _sz, _p, _p], _i),
         "vg_fkcc_blocks": ([_s, _p, _p, _sz, _p], _i),
+        "vg_env_field_ready": ([_p], _i),
         "vg_env_count": ([_p, _i, _p], _i),
         "vg_env_get": ([_p, _i, _sz, _p], _i),
         "vg_validate_states_device": ([_s, _p, _p, _sz, _p, _p], _i),
@@ -146,6 +147,7 @@ EXPORTED = (
     "vg_env_add_heightfield_fields",
     "vg_fkcc_blocks_device",
     "vg_fkcc_blocks",
+    "vg_env_field_ready",
     "vg_env_count",
     "vg_env_get",
     "vg_validate_states_device",

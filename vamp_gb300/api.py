@@ -67,6 +67,11 @@ class Environment:
         check(lib.vg_env_set_mode(self._h, lanes, sqrt_mode))
         self.lanes, self.sqrt_mode = lanes, sqrt_mode
 
+    def field_ready(self) -> bool:
+        """Whether the environment's clearance field stands (vg_env_field_ready): checks build it once
+        enough configurations have been checked since the last change.  Results do not depend on it."""
+        return lib.vg_env_field_ready(self._h) == 1
+
     def set_schedule(self, schedule: int) -> None:
         """GPU edge schedule: 1 a warp per edge, 0 a lane-block per edge, 2 a warp per edge with
         the register-rich build, 3 as 2 with the segments an edge leaves free starting on the

@@ -1129,6 +1129,11 @@ int vg_env_set_schedule(vg_env *env, int schedule)
     return VG_OK;
 }
 
+int vg_env_field_ready(const vg_env *env)
+{
+    return env ? !env->dirty && env->field_ready.load(std::memory_order_acquire) : -1;
+}
+
 int vg_env_count(const vg_env *env, int kind, size_t *count)
 {
     if (!env || kind < 0 || kind > 4 || !count)
