@@ -174,7 +174,8 @@ int vg_env_get(const vg_env *env, int kind, size_t index, float *out);
 
 /* ----------------------------------------------------------------------- checks (device)
  * Inputs and outputs in device memory; asynchronous on `stream` (a cudaStream_t, or NULL for
- * the default stream).  Configurations are row-major [n][dim] float32. */
+ * the default stream), but for the first check after a change of the environment, which waits for
+ * the device to upload it.  Configurations are row-major [n][dim] float32. */
 
 /* Per-configuration validity: out[i] = 1 if configuration i is collision free.
  * Replaces Robot::fkcc on a broadcast block, i.e. the Python binding's validate()

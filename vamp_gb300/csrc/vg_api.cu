@@ -381,7 +381,7 @@ namespace vg
         return VG_OK;
     }
 
-    EnvDevice env_device(const vg_env *e)
+    EnvDevice env_device(const vg_env *e, const uint8_t *field)
     {
         EnvDevice d{};
         d.buf = e->d_image;
@@ -398,7 +398,7 @@ namespace vg
         d.att_off = e->att_off;
         d.n_hf = static_cast<int>(e->hf.size());
         d.hf_off = e->hf_off;
-        d.field = e->field_ready.load(std::memory_order_acquire) ? e->d_field : nullptr;
+        d.field = field;
         return d;
     }
 
@@ -636,7 +636,7 @@ namespace vg
         std::memset(verdicts, 1, n);
         const int ext = env->extended() ? 1 : 0, which = W == 8 ? 0 : 1;
         want_field(env, static_cast<double>(total) * W, 0);
-        EnvDevice dev = env_device(env);
+        EnvDevice dev = env_device(env, usable_field(env, 0));
         int smem = 0;
         if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
             return rc;
@@ -710,7 +710,8 @@ namespace vg
     {
         const RobotOps *r = m.r;
         const vg_env *env = m.env;
-        EnvDevice dev = env_device(env);
+        const bool ordered = m.replayed && env->field_ready.load(std::memory_order_acquire);
+        EnvDevice dev = env_device(env, ordered ? env->d_field : usable_field(env, s));
         int smem = 0;
         if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
             return rc;
@@ -1163,7 +1164,7 @@ int vg_validate_states_device(const char *robot, vg_env *env, const float *q, si
     if (int rc = commit(env))
         return rc;
     want_field(env, static_cast<double>(n), static_cast<cudaStream_t>(stream));
-    EnvDevice dev = env_device(env);
+    EnvDevice dev = env_device(env, usable_field(env, static_cast<cudaStream_t>(stream)));
     int smem = 0;
     if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
         return rc;
@@ -1474,7 +1475,7 @@ int vg_fkcc_blocks_device(const char *robot, vg_env *env, const float *q, size_t
     const int which = env->lanes == 8 ? 0 : 1;
     const bool ext = env->extended();
     want_field(env, static_cast<double>(n_blocks) * env->lanes, static_cast<cudaStream_t>(stream));
-    EnvDevice dev = env_device(env);
+    EnvDevice dev = env_device(env, usable_field(env, static_cast<cudaStream_t>(stream)));
     int smem = 0;
     if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
         return rc;

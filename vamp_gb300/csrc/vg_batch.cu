@@ -143,6 +143,7 @@ namespace
                            p.out, p.blocks, bt->counters + 16 * i};
             m.order = p.mlp ? bt->orders[i] : nullptr;
             m.rank = bt->ranks[i];
+            m.replayed = true;
             tuned_for(p.env, p.r, &m.schedule, &m.blocks_per_sm);
             if (int rc = launch_motions(m, st))
                 return rc;
@@ -233,6 +234,8 @@ int vg_batch_launch(vg_batch *b, void *stream)
             b->versions.push_back(p.env->version);
         b->stale = false;
     }
+    for (const auto &p : b->parts)
+        usable_field(p.env, s);  // orders this launch behind a field still being built
     VG_CUDA(cudaGraphLaunch(b->exec, s), "cudaGraphLaunch");
     return VG_OK;
 }
@@ -252,7 +255,7 @@ int vg_autotune_motions(const char *robot, vg_env *env, const float *a, const fl
         return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     want_field(env, kEdgeStates * static_cast<double>(n), s);
-    EnvDevice dev = env_device(env);
+    EnvDevice dev = env_device(env, nullptr);
     int smem = 0;
     if (int rc = stage_split(dev, r->stage_floats * kBlock * 4, &smem))
         return rc;

@@ -152,7 +152,7 @@ int vg_debug_device(const char *robot, vg_env *env, const float *q, size_t n, ui
     const int words = debug_words(env);
     p.slots = r->slots;
     p.fine = r->fine;
-    p.env = env_device(env);
+    p.env = env_device(env, nullptr);
     p.ids = d_ids;
     p.words = words;
     for (long long c0 = 0; e == cudaSuccess && c0 < static_cast<long long>(n); c0 += chunk)

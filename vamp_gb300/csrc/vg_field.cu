@@ -17,11 +17,10 @@
 // their 8 x 8 x 8 block).
 #include "../../include/vamp_gb300.h"
 #include "vg_internal.h"
+#include "vg_pool.h"
 
 #include <algorithm>
 #include <mutex>
-#include <utility>
-#include <vector>
 
 namespace vg
 {
@@ -377,7 +376,7 @@ namespace vg
         cudaError_t launch_build(vg_env *e, cudaStream_t s)
         {
             unsigned char *scratch = e->d_field + kCells;
-            field_primitives<<<kCells / 512, 256, 0, s>>>(env_device(e), e->d_field);
+            field_primitives<<<kCells / 512, 256, 0, s>>>(env_device(e, nullptr), e->d_field);
             cudaError_t err = cudaGetLastError();
             if (!e->clouds.empty() && err == cudaSuccess)
             {
@@ -423,50 +422,44 @@ namespace vg
         }
     }  // namespace
 
-    // Field buffers (a field and its scratch, 8.8 MB) of destroyed environments, for later ones: an
-    // allocation of that size takes longer than the build.  At most kKept, each for its device.
     namespace
     {
-        constexpr size_t kKept = 4;
-        std::mutex kept_mu;
-        std::vector<std::pair<int, uint8_t *>> kept;
-
-        cudaError_t take_buffer(int device, uint8_t **buffer)
+        // This thread's calls do not count as unsafe for another thread's capture (in the default, global
+        // mode, an allocation or an event's query anywhere would end it).
+        struct OutsideCaptures
         {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+
+            OutsideCaptures()
             {
-                std::lock_guard<std::mutex> lock(kept_mu);
-                for (size_t i = 0; i < kept.size(); ++i)
-                {
-                    if (kept[i].first == device)
-                    {
-                        *buffer = kept[i].second;
-                        kept.erase(kept.begin() + static_cast<long>(i));
-                        return cudaSuccess;
-                    }
-                }
+                cudaThreadExchangeStreamCaptureMode(&mode);
             }
-            return cudaMalloc(buffer, kCells + kScratch);
+
+            ~OutsideCaptures()
+            {
+                cudaThreadExchangeStreamCaptureMode(&mode);
+            }
+        };
+
+        bool captured(cudaStream_t s)
+        {
+            cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(s, &status) != cudaSuccess)
+            {
+                cudaGetLastError();
+                return true;
+            }
+            return status != cudaStreamCaptureStatusNone;
         }
     }  // namespace
 
     void release_field(vg_env *e)
     {
-        if (!e->d_field)
-            return;
-        // kept only when idle: the next environment fills it on a stream of its own
-        int dev = -1;
-        const bool idle = cudaGetDevice(&dev) == cudaSuccess && dev == e->device && cudaDeviceSynchronize() == cudaSuccess;
-        {
-            std::lock_guard<std::mutex> lock(kept_mu);
-            if (idle && kept.size() < kKept)
-            {
-                kept.emplace_back(e->device, e->d_field);
-                e->d_field = nullptr;
-            }
-        }
-        if (e->d_field)
-            cudaFree(e->d_field);
+        pool_give(e->d_field, 0);
         e->d_field = nullptr;
+        if (e->field_built)
+            cudaEventDestroy(e->field_built);
+        e->field_built = nullptr;
     }
 
     void want_field(vg_env *e, double states, cudaStream_t s)
@@ -481,22 +474,22 @@ namespace vg
         {
             return;
         }
-        // a stream under capture takes no allocation and no synchronisation: its launches run
-        // without the field
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
+        // the build belongs to no graph: launches under capture run without the field
+        if (captured(s))
         {
-            cudaGetLastError();
             return;
         }
+        const OutsideCaptures outside;
         cudaError_t err = cudaSuccess;
-        if (!e->d_field)
-            err = take_buffer(e->device, &e->d_field);
+        if (!e->field_built)
+            err = cudaEventCreateWithFlags(&e->field_built, cudaEventDisableTiming);
+        if (err == cudaSuccess && !e->d_field)
+            err = pool_take(reinterpret_cast<void **>(&e->d_field), kCells + kScratch, s);
         if (err == cudaSuccess)
             err = launch_build(e, s);
-        // complete before any other stream or thread can see it
+        // the call waits for nothing: checks on other streams queue behind this (usable_field)
         if (err == cudaSuccess)
-            err = cudaStreamSynchronize(s);
+            err = cudaEventRecord(e->field_built, s);
         if (err != cudaSuccess)
         {
             // without a field the checks are as they were; not tried again before the next change
@@ -504,7 +497,34 @@ namespace vg
             e->field_states = -1e300;
             return;
         }
+        e->field_done.store(false, std::memory_order_relaxed);
         ++e->version;  // graphs captured without the field are captured again
         e->field_ready.store(true, std::memory_order_release);
+    }
+
+    const uint8_t *usable_field(const vg_env *e, cudaStream_t s)
+    {
+        if (!e->field_ready.load(std::memory_order_acquire))
+        {
+            return nullptr;
+        }
+        if (e->field_done.load(std::memory_order_acquire))
+        {
+            return e->d_field;
+        }
+        const OutsideCaptures outside;
+        if (cudaEventQuery(e->field_built) == cudaSuccess)
+        {
+            e->field_done.store(true, std::memory_order_release);
+            return e->d_field;
+        }
+        cudaGetLastError();  // not ready
+        // a graph cannot wait for the build
+        if (captured(s) || cudaStreamWaitEvent(s, e->field_built, 0) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return e->d_field;
     }
 }  // namespace vg

@@ -1022,7 +1022,7 @@ int vg_filter_self_from_pointcloud_device(const char *robot, vg_env *env, const 
     carve();
     VG_CUDA(cudaMemcpyAsync(dq, q, r->dim * sizeof(float), cudaMemcpyHostToDevice, s), "vg_filter_self_from_pointcloud: copy");
     VG_CUDA(r->spheres(dq, 1, sph, s), "vg_filter_self_from_pointcloud: sphere_fk");
-    EnvDevice dev = env_device(env);
+    EnvDevice dev = env_device(env, nullptr);
     int smem = 0;
     if (int rc = stage_split(dev, 0, &smem))
         return rc;

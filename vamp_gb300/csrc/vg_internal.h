@@ -155,7 +155,9 @@ struct vg_env
     // clearance field (vg_field.cu): built by want_field once the states checked since the last
     // upload make it worth while, dropped by the next upload
     uint8_t *d_field = nullptr;
-    std::atomic<bool> field_ready{false};
+    std::atomic<bool> field_ready{false};         // queued for building, field_built recorded behind
+    mutable std::atomic<bool> field_done{false};  // known to be complete
+    cudaEvent_t field_built = nullptr;
     double field_states = 0.0;
     std::mutex field_mu;
     // learned-order group orders (vg_validate_motions_scored_device), 16 bytes per edge
@@ -200,10 +202,12 @@ namespace vg
         const float *dist = nullptr;  // validate_vector form: b holds vectors, dist their lengths
         uint8_t *order = nullptr;     // with scores: scratch of n x 16 bytes for the group orders
         unsigned *rank = nullptr;     // scratch of n x 4 bytes for the hand-out order (null: edges as given)
+        bool replayed = false;        // recorded in a graph that each launch orders behind the field's build
     };
 
     int commit(vg_env *e);
-    EnvDevice env_device(const vg_env *e);
+    // `field`: from usable_field, or null
+    EnvDevice env_device(const vg_env *e, const uint8_t *field);
     // States checked in an environment since its last change from which its clearance field is
     // built (about 0.1 ms, allocations and the synchronisation included).
     constexpr double kFieldStates = 131072.0;
@@ -211,10 +215,14 @@ namespace vg
     constexpr size_t kRankEdges = 6144;
     // states an edge is taken to hold where its length is not known on the host
     constexpr double kEdgeStates = 64.0;
-    // Counts `states` about to be checked on stream s in a committed environment and builds its
-    // clearance field when due.  Failure to build leaves the environment without one.
+    // Counts `states` about to be checked on stream s in a committed environment and queues the
+    // build of its clearance field there when due.  Waits for nothing.  Failure to build leaves the
+    // environment without one.
     void want_field(vg_env *e, double states, cudaStream_t s);
-    // Gives the field's buffer back (waits for the device).
+    // The environment's field for checks queued on stream s from here on (null: none, or not to be
+    // had by a stream under capture yet).
+    const uint8_t *usable_field(const vg_env *e, cudaStream_t s);
+    // Gives the field's buffer back, its checks being done.
     void release_field(vg_env *e);
     int sm_count();
     // Splits an environment between shared and global memory for kernels that need `beside` bytes of shared
