@@ -59,8 +59,9 @@ namespace
 
     int record(vg_batch *bt, cudaStream_t s);
 
-    // every allocation and upload a launch needs, done outside any capture
-    int prepare(vg_batch *bt, cudaStream_t s)
+    // The environments uploaded, and every launch's edges counted towards their clearance fields: one
+    // that falls due changes its environment's version, so the graph is captured again.
+    int commit_parts(vg_batch *bt, cudaStream_t s)
     {
         int dev = 0;
         VG_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
@@ -74,6 +75,12 @@ namespace
         }
         for (auto &p : bt->parts)
             want_field(p.env, kEdgeStates * static_cast<double>(p.n), s);
+        return VG_OK;
+    }
+
+    // every allocation a launch needs, done outside any capture
+    int prepare(vg_batch *bt)
+    {
         const size_t need = bt->parts.size() * 16;
         if (need > bt->counters_cap)
         {
@@ -206,14 +213,16 @@ int vg_batch_launch(vg_batch *b, void *stream)
     if (!b || b->parts.empty())
         return set_error(VG_ERR_ARG, "vg_batch_launch: empty batch");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (int rc = commit_parts(b, s))
+        return rc;
     bool changed = b->versions.size() != b->parts.size();
     for (size_t i = 0; i < b->parts.size() && !changed; ++i)
-        changed = b->parts[i].env->dirty || b->parts[i].env->version != b->versions[i];
+        changed = b->parts[i].env->version != b->versions[i];
     if (changed)
-        drop_graph(b);  // an environment changed since the capture: upload it and capture again
+        drop_graph(b);  // an environment changed since the capture: capture again
     if (b->stale)
     {
-        if (int rc = prepare(b, s))
+        if (int rc = prepare(b))
             return rc;
         // the capture records the launches without running them
         VG_CUDA(cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
