@@ -452,6 +452,12 @@ CONTAIN_MARGIN = 1e-4  # metres between a link's fine spheres and its containing
 # its last place.  At 64 that is 4e-6 a joint, under 0.02 mm over seven joints and a group's half
 # metre, a fifth of CONTAIN_MARGIN; at 10^6 it is 0.03, and containing spheres contain no more.
 FAR_JOINT = 64.0
+# Where such lanes are dealt with: between the lookups and their words, a branch that also keeps the
+# compiler from drawing the lookups forward (16,384 Panda motions 295 -> 287 us, UR5 338 -> 336, Baxter
+# equal), or, for the Fetch, whose states kernel then needs 114 registers and loses its fifth resident
+# block (262,144 configurations 321 -> 352 us, 32,768 blocks 277 -> 321), after the words (324 and 279).
+# Its motions take 421 or 425 us, 405 without the test.
+FAR_LATE = {"fetch"}
 
 
 def containing_radius(model: dict, kin, env_check: dict) -> float:
@@ -808,6 +814,10 @@ def gen_cuda(model: dict) -> str:
     fr = frames_block(em)
     body = list(em.lines)
     body += limits_code(model, cull)
+    near = " & ".join(f"(fabsf(q[{d}]) <= {lit32(FAR_JOINT)})" for d in range(dim))
+    far_test = f"ctx.far = __any_sync(vg::kFull, !({near}) && ((ctx.alive >> (threadIdx.x & 31)) & 1u));"
+    if name in FAR_LATE:
+        body += ["if (__builtin_expect(!ctx.in_limits, 0))", "{", f"    {far_test}", "}"]
     body.append("float *const st = ctx.stage;")
     vals_ = [f"(-{v[1:]})" if v.startswith("-") else v for v in lay["values"]]
     for i in range(0, len(vals_), 6):
@@ -832,10 +842,10 @@ def gen_cuda(model: dict) -> str:
     body.append("// per lane: the pairs of groups that overlap, and those whose joints lie in a danger box")
     plist = list(pairs)
     n_words = -(-len(plist) // 32)
+    gate = []
     for wd in range(n_words):
         part = plist[32 * wd:32 * wd + 32]
         body.append(f"unsigned over{wd} = 0u;")
-        gate = []
         for j, (ga, gb) in enumerate(part):
             (A, ra), (B, rb) = group_sphere[ga], group_sphere[gb]
             # the reference's own coarse test where both groups are single links, else one that
@@ -843,31 +853,29 @@ def gen_cuda(model: dict) -> str:
             body.append(f"over{wd} = vg::shift_in(over{wd}, vg::self_bits({', '.join(A)}, {', '.join(B)}, "
                         f"__fadd_rn({lit32(ra)}, {lit32(rb)})));")
             if all(boxes_of[c][0][2] for c in pairs[(ga, gb)]):
-                gate.append((len(part) - 1 - j, [boxes_of[c] for c in pairs[(ga, gb)]]))
+                gate.append((wd, len(part) - 1 - j, [boxes_of[c] for c in pairs[(ga, gb)]]))
         body.append(f"unsigned boxed{wd} = ~0u;")
-        if gate:
-            body.append("if (ctx.in_limits)")
-            body.append("{")
-            for bit, bs in gate:
-                cond = " | ".join("((q[%d] >= %s) & (q[%d] <= %s) & (q[%d] >= %s) & (q[%d] <= %s))" % (
-                    b[0][0], lit32(b[1][0]), b[0][0], lit32(b[1][1]), b[0][1], lit32(b[1][2]), b[0][1], lit32(b[1][3])) for b in bs)
-                body.append(f"    boxed{wd} &= {cond} ? ~0u : ~{1 << bit}u;")
-            body.append("}")
-    body.append("if (!ctx.in_limits)")
+    body.append("if (ctx.in_limits)")
     body.append("{")
-    near = " & ".join(f"(fabsf(q[{d}]) <= {lit32(FAR_JOINT)})" for d in range(dim))
-    body.append(f"    ctx.far = __any_sync(vg::kFull, !({near}) && ((ctx.alive >> (threadIdx.x & 31)) & 1u));")
-    body.append("    if (ctx.far)  // what stands for a group contains nothing for sure: every check is run")
-    body.append("    {")
-    body.append("        %s = 0u;" % " = ".join(f"v{g}" for g in range(n_groups)))
-    for wd in range(n_words):
-        body.append(f"        over{wd} = {hex((1 << len(plist[32 * wd:32 * wd + 32])) - 1)}u;")
-    body.append("    }")
+    for wd, bit, bs in gate:
+        cond = " | ".join("((q[%d] >= %s) & (q[%d] <= %s) & (q[%d] >= %s) & (q[%d] <= %s))" % (
+            b[0][0], lit32(b[1][0]), b[0][0], lit32(b[1][1]), b[0][1], lit32(b[1][2]), b[0][1], lit32(b[1][3])) for b in bs)
+        body.append(f"    boxed{wd} &= {cond} ? ~0u : ~{1 << bit}u;")
     body.append("}")
+    # far lanes: what stands for a group contains nothing for sure, so every check is run
+    far_over = [f"over{wd} = {hex((1 << len(plist[32 * wd:32 * wd + 32])) - 1)}u;" for wd in range(n_words)]
+    if name not in FAR_LATE:
+        body += ["else", "{", f"    {far_test}", "    if (ctx.far)  // no sphere that stands for others is relied on", "    {"]
+        body += [f"        {line}" for line in far_over]
+        body += ["        %s = 0u;" % " = ".join(f"v{g}" for g in range(n_groups)), "    }", "}"]
     body.append("// per lane: the groups that may touch something")
     body.append("unsigned near = 0u;")
     for g in range(n_groups):
         body.append(f"near = vg::shift_in(near, v{g} - vg::field_reach({lit32(group_sphere[g][1])}));")
+    if name in FAR_LATE:
+        body += ["if (__builtin_expect(ctx.far, 0))  // no sphere that stands for others is relied on", "{"]
+        body += [f"    {line}" for line in far_over]
+        body += [f"    near = {hex((1 << n_groups) - 1)}u;", "}"]
     body.append("const unsigned on = (ctx.alive >> (threadIdx.x & 31)) & 1u ? ~0u : 0u;")
     body += f"""// environment checks of those groups
 unsigned todo = __reduce_or_sync(vg::kFull, near & on);
