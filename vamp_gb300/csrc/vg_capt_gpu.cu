@@ -18,6 +18,7 @@
 // scan, within room guessed before (the build starts again with more when that runs out), and the
 // host waits once, for the size of the blocks.
 #include "vg_capt_gpu.h"
+#include "vg_capt_room.h"
 
 #include "../../include/vamp_gb300.h"
 #include "vg_internal.h"
@@ -699,13 +700,9 @@ namespace vg
         int d1 = d0;  // the first level of nodes of kSmallTile entries (d0 in smaller trees)
         while ((N >> d1) > kSmallTile)
             ++d1;
-        const bool subtrees = N <= kOrdersMax;
+        bool subtrees = N <= kOrdersMax;
         const int T = static_cast<int>(std::min<long long>(N, kSortTile));
-        // Room for a level's lists: 104 entries a leaf in the Panda's tree of 50,000 points.  A tree for
-        // larger spheres needs more, and starts again.
-        unsigned long long cap = static_cast<unsigned long long>(
-            std::min<long long>(std::max<long long>(160 * N, 1 << 18), std::max<long long>(1ll << 28, 2 * N)));
-        unsigned long long least = 0;  // what the last level that ran out needs
+        ListRoom room(N);
         cudaError_t e = cudaSuccess;
         // results: split values, boxes, starts and the points, in one allocation
         {
@@ -740,6 +737,7 @@ namespace vg
                 bytes += (std::max<size_t>(count, 1) * sizeof(**p) + 255) & ~size_t(255);
                 *p = scratch ? reinterpret_cast<std::remove_reference_t<decltype(*p)>>(scratch + at) : nullptr;
             };
+            const unsigned long long cap = room.entries();
             auto carve_all = [&]() {
                 bytes = 0;
                 carve(&used, 32);
@@ -762,11 +760,11 @@ namespace vg
             };
             carve_all();
             e = pool_take(reinterpret_cast<void **>(&scratch), bytes, s);
-            if (e == cudaErrorMemoryAllocation && least && cap > least)
+            if (e == cudaErrorMemoryAllocation && (room.shrink() || subtrees))
             {
-                // not four times as much, then
+                // with less, then; at the least without the subtrees' orders
                 cudaGetLastError();
-                cap = least;
+                subtrees = subtrees && room.entries() < cap;
                 e = cudaSuccess;
                 continue;
             }
@@ -850,14 +848,11 @@ namespace vg
             pool_give(scratch, s);
             if (e != cudaSuccess || !sum.full)
                 break;
-            // a level ran out of room: as much as the first such level needs, and four times more for
-            // the levels below
             for (int d = 0; d < nlog2; ++d)
             {
                 if (h_used[d] > cap)
                 {
-                    least = h_used[d];
-                    cap = 4 * least;
+                    room.grow(h_used[d]);  // the first level that ran out
                     break;
                 }
             }
