@@ -362,9 +362,10 @@ namespace vg
                 e->d_counter = nullptr;
                 e->image_cap = 0;
             }
-            // room to grow, and the work counter behind
+            // room to grow, and the work counters behind
             const size_t cap = img.size() + img.size() / 2;
-            VG_CUDA(pool_take(reinterpret_cast<void **>(&e->d_image), cap * sizeof(float4) + 64, 0), "allocate environment");
+            const size_t bytes = cap * sizeof(float4) + kEdgeCounters * sizeof(unsigned);
+            VG_CUDA(pool_take(reinterpret_cast<void **>(&e->d_image), bytes, 0), "allocate environment");
             e->image_cap = cap;
             e->d_counter = reinterpret_cast<unsigned *>(e->d_image + cap);
         }
@@ -732,7 +733,7 @@ namespace vg
             return rc;
         if (m.blocks_per_sm > 0 && m.blocks_per_sm < occ)
             occ = m.blocks_per_sm;
-        VG_CUDA(cudaMemsetAsync(m.counter, 0, 3 * sizeof(unsigned), s), "reset work counter");
+        VG_CUDA(cudaMemsetAsync(m.counter, 0, kEdgeCounters * sizeof(unsigned), s), "reset work counters");
         // edges handled at once by one block of threads: a warp each (same-edge schedule) or a
         // segment each
         const int per_block = grouped ? kBlock / 32 : kBlock / env->lanes;
@@ -767,14 +768,14 @@ namespace vg
     // ------------------------------------------------------------ allocation-free variant
     // (edges go as given: the hand-out order would need scratch)
     //
-    // Scratch for vg_validate_motions_device_noalloc: the edge kernel's work counter lives in
+    // Scratch for vg_validate_motions_device_noalloc: the edge kernel's work counters live in
     // this fixed array instead of memory the library allocates.  Every GPU that loads the
-    // library holds these bytes until the process exits.  All calls share it: the counter is
+    // library holds these bytes until the process exits.  All calls share it: the counters are
     // cleared on the caller's stream before each launch, and calls whose kernels overlap on the
     // GPU race on it.
     constexpr size_t kNoAllocScratchBytes = 256;
     static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
-    static_assert(sizeof(unsigned) <= kNoAllocScratchBytes, "the work counter must fit the scratch array");
+    static_assert(kEdgeCounters * sizeof(unsigned) <= kNoAllocScratchBytes, "the work counters must fit the scratch array");
 
     // Device address of the scratch array on each device, looked up once per device with that
     // device current (host code cannot use the array's name as a device pointer).

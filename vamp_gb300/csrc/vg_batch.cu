@@ -81,6 +81,7 @@ namespace
     // every allocation a launch needs, done outside any capture
     int prepare(vg_batch *bt)
     {
+        static_assert(kEdgeCounters <= 16, "a part's counters");
         const size_t need = bt->parts.size() * 16;
         if (need > bt->counters_cap)
         {

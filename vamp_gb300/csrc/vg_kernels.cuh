@@ -348,6 +348,8 @@ namespace vg
 
     // ------------------------------------------------------------------------------- edges
 
+    constexpr int kEdgeCounters = 3;  // of EdgesParams::head
+
     struct EdgesParams
     {
         const float *a;  // [n][dim] start configurations
@@ -356,7 +358,7 @@ namespace vg
         int resolution;
         uint8_t *out;        // 1 = valid
         int32_t *blocks;     // optional: blocks checked per edge
-        unsigned *head;      // work counters, zero before launch: [0] the edges handed out; [1], [2]
+        unsigned *head;      // kEdgeCounters, zero before launch: [0] the edges handed out; [1], [2]
                              // edge_rank_kernel's ends of the long and the short edges
         EnvDevice env;
         // learned order (same-edge schedule only): per-edge collision scores of `probes` states

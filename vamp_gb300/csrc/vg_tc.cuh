@@ -137,24 +137,6 @@ namespace vg::tc
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
 
-    // 16 bytes from global to shared memory, asynchronously (both 16-byte aligned)
-    __device__ __forceinline__ void copy16_async(void *dst, const void *src)
-    {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-    }
-
-    __device__ __forceinline__ void copies_commit()
-    {
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-
-    // Waits until at most N of this thread's committed groups of copies are in flight.
-    template <int N>
-    __device__ __forceinline__ void copies_wait()
-    {
-        asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-    }
-
     // Expects `bytes` of bulk copies on the barrier's current phase (and arrives).
     __device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes)
     {
