@@ -368,19 +368,6 @@ def fk_flops(model: dict) -> dict:
     return {"frames": em.flops + SINCOS_FLOPS * n_rev, "centre": CENTRE_FLOPS, "slots": len(slots)}
 
 
-def frame_values(kin: Kin, frames) -> list:
-    """Every frame (root first, then movable frames in order) as 12 values: R row-major, t."""
-    out = []
-    for fid in ["root"] + [f["id"] for f in kin.frames]:
-        R, t = frames[fid]
-        out.append([R[r][c] for r in range(3) for c in range(3)] + list(t))
-    return out
-
-
-def frame_index(kin: Kin) -> dict:
-    return {fid: i for i, fid in enumerate(["root"] + [f["id"] for f in kin.frames])}
-
-
 def struct_name(name: str) -> str:
     return name[0].upper() + name[1:]
 
@@ -594,20 +581,10 @@ def link_groups(model: dict, kin) -> dict:
     for c, e in enumerate(model["self_checks"]):
         a, b = of[env_ix[e["links"][0]]], of[env_ix[e["links"][1]]]
         assert a != b, "links of one rigid group are not checked against each other"
+        A, B = (list(dict.fromkeys(p[k] for p in e["fine"])) for k in (0, 1))
+        assert [[x, y] for x in A for y in B] == e["fine"], "fine self pairs are a cross product"
         pairs.setdefault((a, b), []).append(c)
     return {"frames": order, "members": [groups[f] for f in order], "pairs": pairs, "env_ix": env_ix}
-
-
-def _pairs_ab(e):
-    A, B = [], []
-    for sa, sb in e["fine"]:
-        if sa not in A:
-            A.append(sa)
-        if sb not in B:
-            B.append(sb)
-    # the reference's fine pairs for a link pair are the cross product of the two links' spheres
-    assert [[x, y] for x in A for y in B] == e["fine"], "fine self pairs are not a cross product"
-    return A, B
 
 
 def gen_cuda(model: dict) -> str:
