@@ -15,8 +15,8 @@
 // and level, and a host wait per level for the size of its lists, made 5,271 points 1.54 ms.  So
 // the levels whose nodes fit a tile sort in one launch (a block takes a subtree down to its
 // leaves, keeping each level's order), a node's lists take their room from a counter instead of a
-// scan, within room guessed before (the build starts again with more when that runs out), and the
-// host waits once, for the size of the blocks.
+// scan, within room guessed before (a level that runs out is done again in a larger buffer), and
+// the host waits once, for the size of the blocks, and once for each level that ran out.
 #include "vg_capt_gpu.h"
 #include "vg_capt_room.h"
 
@@ -50,10 +50,12 @@ namespace vg
             ord[i] = static_cast<uint32_t>(i);
         }
 
-        __global__ void load_keys(const uint32_t *ord, const float *axis, long long N, float *key, uint32_t *pos)
+        // `full` (here and below): not zero once a level's lists ran out of room (its number + 1).  What is
+        // queued for the levels below then does nothing, so that the build can go on from that level.
+        __global__ void load_keys(const uint32_t *ord, const float *axis, long long N, const int *full, float *key, uint32_t *pos)
         {
             const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (i >= N)
+            if (i >= N || *full)
                 return;
             key[i] = axis[ord[i]];
             pos[i] = static_cast<uint32_t>(i);
@@ -62,11 +64,11 @@ namespace vg
         // One compare-exchange stage of a bitonic network that sorts every aligned segment of S
         // entries ascending by (key, pos).
         __global__ void bitonic_stage(float *key, uint32_t *pos, uint32_t *ord, long long N, long long k, long long j,
-                                      long long S)
+                                      long long S, const int *full)
         {
             const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
             const long long p = i ^ j;
-            if (i >= N || p <= i)
+            if (i >= N || p <= i || *full)
                 return;
             const bool up = k == S || (i & k) == 0;
             const float ki = key[i], kp = key[p];
@@ -111,9 +113,11 @@ namespace vg
         // All compare-exchange stages of sizes k in [k0, k1] and strides below the tile, on tiles
         // of T = min(S, 2048) entries (S: the sorted segment size, a power of two).
         __global__ void __launch_bounds__(kSortTile / 2) bitonic_tile(float *key, uint32_t *pos, uint32_t *ord, long long S,
-                                                                      long long k0, long long k1)
+                                                                      long long k0, long long k1, const int *full)
         {
             __shared__ Entry sm[kSortTile];
+            if (*full)
+                return;
             const int T = static_cast<int>(S < kSortTile ? S : kSortTile), t = threadIdx.x;
             const long long base = static_cast<long long>(blockIdx.x) * T;
             Entry v[2] = {};
@@ -185,10 +189,10 @@ namespace vg
         }
 
         // split_node for every node of level d (heap order)
-        __global__ void split_nodes(const float *key, long long N, int d, float r_max, float *tests, NodeInfo *info)
+        __global__ void split_nodes(const float *key, long long N, int d, float r_max, const int *full, float *tests, NodeInfo *info)
         {
             const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (t < (1ll << d))
+            if (t < (1ll << d) && !*full)
             {
                 const long long S = N >> d, at = (1ll << d) - 1 + t;
                 tests[at] = split_node(key, t * S, S, 0, r_max, info[at]);
@@ -200,11 +204,13 @@ namespace vg
         // order in orders[(d - d0) N ..], the last one in ord.  The network of each level is
         // bitonic_tile's.
         __global__ void __launch_bounds__(kSortTile / 2) sort_subtrees(const float *px, const float *py, const float *pz, long long N,
-                                                                       int d0, int d1, int T, float r_max, uint32_t *ord,
-                                                                       uint32_t *orders, float *tests, NodeInfo *info)
+                                                                       int d0, int d1, int T, float r_max, const int *full,
+                                                                       uint32_t *ord, uint32_t *orders, float *tests, NodeInfo *info)
         {
             __shared__ Entry sm[kSortTile];
             __shared__ float sk[kSortTile];
+            if (*full)
+                return;
             const long long base = static_cast<long long>(blockIdx.x) * T;
             const int t = threadIdx.x;
             Entry v[2] = {};
@@ -298,12 +304,15 @@ namespace vg
         // The children's lists of each node of level d (one block per node): the node's list filtered in
         // order, then the scanned range.  A node's two lists take their room in `out` from the level's
         // counter, in any order; range[n] is node n's list.  Past the room `cap` nothing is written (the
-        // counter still says what the level needs) and *full is set.
+        // counter still says what the level needs) and *full is set to d + 1.
         __global__ void child_lists(const ulonglong2 *range, const uint32_t *items, const float *axis, long long N, int d,
                                     const NodeInfo *info, const uint32_t *ord, unsigned long long cap, unsigned long long *used,
                                     int *full, ulonglong2 *child_range, uint32_t *out)
         {
             __shared__ unsigned long long room;
+            const int ran_out = *static_cast<volatile int *>(full);
+            if (__syncthreads_or(ran_out != 0 && ran_out != d + 1))
+                return;  // a level above
             const long long t = blockIdx.x;
             const NodeInfo ni = info[(1ll << d) - 1 + t];
             const unsigned long long a0 = range[t].x, a1 = range[t].y;
@@ -356,7 +365,7 @@ namespace vg
                 child_range[2 * t] = fits ? make_ulonglong2(w_lo, w_hi) : make_ulonglong2(0, 0);
                 child_range[2 * t + 1] = fits ? make_ulonglong2(w_hi, room + need) : make_ulonglong2(0, 0);
                 if (!fits)
-                    *full = 1;
+                    *full = d + 1;
             }
             if (!fits)
                 return;
@@ -390,10 +399,10 @@ namespace vg
         }
 
         // each leaf's cell: the split planes along its path (right child: coordinate >= test)
-        __global__ void leaf_cells(const float *tests, int nlog2, float *cell)
+        __global__ void leaf_cells(const float *tests, int nlog2, const int *full, float *cell)
         {
             const long long leaf = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (leaf >= 1ll << nlog2)
+            if (leaf >= 1ll << nlog2 || *full)
                 return;
             float lo[3] = {-kInf, -kInf, -kInf}, hi[3] = {kInf, kInf, kInf};
             long long idx = 0;
@@ -454,8 +463,10 @@ namespace vg
         };
 
         // number of 8-point blocks of each leaf (one block of threads per leaf)
-        __global__ void count_leaves(const LeafParams p, uint32_t *blocks)
+        __global__ void count_leaves(const LeafParams p, const int *full, uint32_t *blocks)
         {
+            if (*full)
+                return;
             const long long t = blockIdx.x;
             const uint32_t rep = p.ord[t];
             const float rx = p.px[rep], ry = p.py[rep], rz = p.pz[rep];
@@ -570,7 +581,7 @@ namespace vg
             unsigned long long blocks;
             float top[6];        // box of every finite representative
             float top_tests[3];  // the first split values
-            int full;
+            int full;            // a level that ran out of room + 1 (0: none; only then is the rest filled in)
         };
 
         // The leaves' first blocks (exclusive sums of their counts, starts[N] the total) by block 0, the
@@ -580,6 +591,12 @@ namespace vg
                                                             const float *tests, const int *full, Summary *sum)
         {
             const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+            if (*full)
+            {
+                if (blockIdx.x == 0 && t == 0)
+                    sum->full = *full;
+                return;
+            }
             if (blockIdx.x == 0)
             {
                 __shared__ unsigned long long wsum[32];
@@ -628,7 +645,7 @@ namespace vg
                 {
                     starts[N] = static_cast<uint32_t>(carry);
                     sum->blocks = carry;
-                    sum->full = *full;
+                    sum->full = 0;
                     for (int k = 0; k < 3; ++k)
                         sum->top_tests[k] = k < N - 1 ? tests[k] : 0.0f;
                 }
@@ -720,24 +737,24 @@ namespace vg
                 e = cudaMemcpyAsync(out.points, xyz, 3 * n * sizeof(float), cudaMemcpyDeviceToDevice, s);
             }
         }
-        Summary sum{};
+        // scratch of fixed size, and the lists' two buffers: level d's lists lie in the one, its
+        // children's go to the other
+        float *px = nullptr, *py = nullptr, *pz = nullptr, *key = nullptr, *cell = nullptr;
+        uint32_t *ord = nullptr, *pos = nullptr, *orders = nullptr, *blocks = nullptr, *items[2] = {nullptr, nullptr};
+        ulonglong2 *range[2] = {nullptr, nullptr};
+        unsigned long long *used = nullptr, cap[2] = {0, 0};
+        NodeInfo *info = nullptr;
+        Summary *d_sum = nullptr;
+        int *full = nullptr;
+        char *scratch = nullptr;
         while (e == cudaSuccess)
         {
-            float *px, *py, *pz, *key, *cell;
-            uint32_t *ord, *pos, *orders, *items, *child_items, *blocks;
-            ulonglong2 *range, *child_range;
-            unsigned long long *used;
-            NodeInfo *info;
-            Summary *d_sum;
-            int *full;
-            char *scratch = nullptr;
             size_t bytes = 0;
             auto carve = [&](auto **p, size_t count) {
                 const size_t at = bytes;
                 bytes += (std::max<size_t>(count, 1) * sizeof(**p) + 255) & ~size_t(255);
                 *p = scratch ? reinterpret_cast<std::remove_reference_t<decltype(*p)>>(scratch + at) : nullptr;
             };
-            const unsigned long long cap = room.entries();
             auto carve_all = [&]() {
                 bytes = 0;
                 carve(&used, 32);
@@ -751,72 +768,86 @@ namespace vg
                 carve(&pos, N);
                 carve(&orders, subtrees ? N * (nlog2 - d0) : 1);
                 carve(&cell, 6 * N);
-                carve(&range, N);
-                carve(&child_range, N);
+                carve(&range[0], N);
+                carve(&range[1], N);
                 carve(&info, N);
                 carve(&blocks, N);
-                carve(&items, cap);
-                carve(&child_items, cap);
             };
             carve_all();
             e = pool_take(reinterpret_cast<void **>(&scratch), bytes, s);
+            for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+            {
+                cap[k] = room.entries();
+                e = pool_take(reinterpret_cast<void **>(&items[k]), cap[k] * sizeof(uint32_t), s);
+            }
+            if (e == cudaSuccess)
+            {
+                carve_all();
+                break;
+            }
+            for (void *p : {static_cast<void *>(scratch), static_cast<void *>(items[0]), static_cast<void *>(items[1])})
+                pool_give(p, s);
+            scratch = nullptr;
+            items[0] = items[1] = nullptr;
+            const unsigned long long tried = room.entries();
             if (e == cudaErrorMemoryAllocation && (room.shrink() || subtrees))
             {
                 // with less, then; at the least without the subtrees' orders
                 cudaGetLastError();
-                subtrees = subtrees && room.entries() < cap;
+                subtrees = subtrees && room.entries() < tried;
                 e = cudaSuccess;
-                continue;
             }
-            if (e != cudaSuccess)
-                break;
-            carve_all();
-            const float *axis[3] = {px, py, pz};
-            // counters, *full and the root's empty list are zeros
+        }
+        const float *axis[3] = {px, py, pz};
+        // counters, *full and the root's empty list are zeros
+        if (e == cudaSuccess)
             e = cudaMemsetAsync(used, 0, reinterpret_cast<char *>(d_sum) - reinterpret_cast<char *>(used), s);
-            if (e == cudaSuccess)
-                e = cudaMemsetAsync(range, 0, sizeof(ulonglong2), s);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(range[0], 0, sizeof(ulonglong2), s);
+        if (e == cudaSuccess)
             init_points<<<grid_of(N, 256), 256, 0, s>>>(xyz, static_cast<long long>(n), N, px, py, pz, ord);
-            for (int d = 0; d < nlog2 && e == cudaSuccess; ++d)
+        Summary sum{};
+        // Every level is queued without a look at its lists.  If one ran out of room the levels below did
+        // nothing: it gets a buffer of what the counter says and the build goes on from there.
+        int from = 0;
+        while (e == cudaSuccess)
+        {
+            for (int d = from; d < nlog2 && e == cudaSuccess; ++d)
             {
                 const long long nodes = 1ll << d, S = N >> d;
-                const uint32_t *order = ord;
-                if (subtrees && d >= d0)
+                const bool tree = subtrees && d >= d0, sorted = d == from && sum.full;
+                const uint32_t *order = tree ? orders + static_cast<long long>(d - d0) * N : ord;
+                if (tree && !sorted && (d == d0 || d == d1))
                 {
-                    if (d == d0 || d == d1)
-                    {
-                        // full tiles down to nodes of kSmallTile entries, which then sort on more SMs
-                        // (2,048 entries on one: 94 us for all eleven levels)
-                        const int tile = d == d1 ? static_cast<int>(S) : T;
-                        sort_subtrees<<<static_cast<unsigned>(N / tile), std::max(tile / 2, 32), 0, s>>>(
-                            px, py, pz, N, d, d < d1 ? d1 : nlog2, tile, r_max, ord, orders + static_cast<long long>(d - d0) * N,
-                            out.tests, info);
-                    }
-                    order = orders + static_cast<long long>(d - d0) * N;
+                    // full tiles down to nodes of kSmallTile entries, which then sort on more SMs
+                    // (2,048 entries on one: 94 us for all eleven levels)
+                    const int tile = d == d1 ? static_cast<int>(S) : T;
+                    sort_subtrees<<<static_cast<unsigned>(N / tile), std::max(tile / 2, 32), 0, s>>>(
+                        px, py, pz, N, d, d < d1 ? d1 : nlog2, tile, r_max, full, ord, orders + static_cast<long long>(d - d0) * N,
+                        out.tests, info);
                 }
-                else
+                else if (!tree && !sorted)
                 {
-                    load_keys<<<grid_of(N, 256), 256, 0, s>>>(ord, axis[d % 3], N, key, pos);
+                    load_keys<<<grid_of(N, 256), 256, 0, s>>>(ord, axis[d % 3], N, full, key, pos);
                     // strides below the tile in shared memory, the longer ones one launch each
                     const long long st = std::min<long long>(S, kSortTile);
                     const unsigned tiles = static_cast<unsigned>(N / st),
                                    threads = static_cast<unsigned>(std::max<long long>(st / 2, 32));
-                    bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, 2, st);
+                    bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, 2, st, full);
                     for (long long k = 2 * st; k <= S; k <<= 1)
                     {
                         for (long long j = k >> 1; j >= st; j >>= 1)
-                            bitonic_stage<<<grid_of(N, 256), 256, 0, s>>>(key, pos, ord, N, k, j, S);
-                        bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, k, k);
+                            bitonic_stage<<<grid_of(N, 256), 256, 0, s>>>(key, pos, ord, N, k, j, S, full);
+                        bitonic_tile<<<tiles, threads, 0, s>>>(key, pos, ord, S, k, k, full);
                     }
-                    split_nodes<<<grid_of(nodes, 128), 128, 0, s>>>(key, N, d, r_max, out.tests, info);
+                    split_nodes<<<grid_of(nodes, 128), 128, 0, s>>>(key, N, d, r_max, full, out.tests, info);
                 }
-                child_lists<<<static_cast<unsigned>(nodes), kListBlock, 0, s>>>(range, items, axis[d % 3], N, d, info, order, cap,
-                                                                               used, full, child_range, child_items);
+                const int p = d & 1, c = 1 - p;
+                child_lists<<<static_cast<unsigned>(nodes), kListBlock, 0, s>>>(range[p], items[p], axis[d % 3], N, d, info, order, cap[c],
+                                                                               used, full, range[c], items[c]);
                 e = cudaGetLastError();
-                std::swap(range, child_range);
-                std::swap(items, child_items);
             }
-            LeafParams lp{range, items, px, py, pz, ord, cell, 0.0f, 0.0f};
+            LeafParams lp{range[nlog2 & 1], items[nlog2 & 1], px, py, pz, ord, cell, 0.0f, 0.0f};
             {
                 const float l1 = r_max + r_point, l0 = r_min + r_point;
                 lp.max_l2 = l1 * l1;
@@ -825,8 +856,8 @@ namespace vg
             unsigned long long h_used[32] = {};
             if (e == cudaSuccess)
             {
-                leaf_cells<<<grid_of(N, 256), 256, 0, s>>>(out.tests, nlog2, cell);
-                count_leaves<<<static_cast<unsigned>(N), kListBlock, 0, s>>>(lp, blocks);
+                leaf_cells<<<grid_of(N, 256), 256, 0, s>>>(out.tests, nlog2, full, cell);
+                count_leaves<<<static_cast<unsigned>(N), kListBlock, 0, s>>>(lp, full, blocks);
                 finish_tree<<<2, 1024, 0, s>>>(blocks, N, out.starts, ord, px, py, pz, out.tests, full, d_sum);
                 e = cudaGetLastError();
             }
@@ -836,7 +867,9 @@ namespace vg
                 e = cudaMemcpyAsync(h_used, used, sizeof(h_used), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess)
                 e = cudaStreamSynchronize(s);
-            if (e == cudaSuccess && !sum.full)
+            if (e != cudaSuccess)
+                break;
+            if (!sum.full)
             {
                 e = pool_take(reinterpret_cast<void **>(&out.aff), std::max<size_t>(24 * sum.blocks, 4) * sizeof(float), s);
                 if (e == cudaSuccess)
@@ -844,19 +877,22 @@ namespace vg
                     write_leaves<<<static_cast<unsigned>(N), kListBlock, 0, s>>>(lp, out.starts, out.aff, out.aabbs);
                     e = cudaGetLastError();
                 }
-            }
-            pool_give(scratch, s);
-            if (e != cudaSuccess || !sum.full)
                 break;
-            for (int d = 0; d < nlog2; ++d)
-            {
-                if (h_used[d] > cap)
-                {
-                    room.grow(h_used[d]);  // the first level that ran out
-                    break;
-                }
             }
+            // what the buffer holds, the lists of the level above, has been read
+            from = sum.full - 1;
+            const int c = 1 - (from & 1);
+            pool_give(items[c], s);
+            items[c] = nullptr;
+            cap[c] = h_used[from];
+            e = pool_take(reinterpret_cast<void **>(&items[c]), cap[c] * sizeof(uint32_t), s);
+            if (e == cudaSuccess)
+                e = cudaMemsetAsync(used + from, 0, sizeof(*used), s);
+            if (e == cudaSuccess)
+                e = cudaMemsetAsync(full, 0, sizeof(*full), s);
         }
+        for (void *p : {static_cast<void *>(scratch), static_cast<void *>(items[0]), static_cast<void *>(items[1])})
+            pool_give(p, s);
         if (e == cudaSuccess)
         {
             out.blocks = sum.blocks;

@@ -1,6 +1,7 @@
-// Room for the affordance lists of a tree built level by level on the GPU (vg_capt_gpu.cu): entries of
-// each of its two list buffers.  Guessed before the build, which starts again with more where a
-// level runs out, and tries with less where the memory cannot be had.
+// Room for the affordance lists of a tree built level by level on the GPU (vg_capt_gpu.cu), in entries
+// of each of its two list buffers: a guess before the build.  A level that runs out gets a buffer of what
+// it needs and is done again (twice that, for the levels below, took as long: the waits it saves are
+// short against the mapping of the memory).
 #pragma once
 
 #include <algorithm>
@@ -10,7 +11,7 @@ namespace vg
     class ListRoom
     {
     public:
-        // 160 entries a leaf: a tree for the Panda's spheres needs 104 (50,000 points), one for larger
+        // 160 entries a leaf: a tree for the Panda's spheres needs 89 (50,000 points), one for larger
         // spheres more.  `leaves` is a power of two.
         explicit ListRoom(long long leaves)
           : floor_(2ull * static_cast<unsigned long long>(leaves)),
@@ -23,26 +24,18 @@ namespace vg
             return entries_;
         }
 
-        // The memory for this room cannot be had.  False where no smaller room can do.
+        // The memory for the guess cannot be had.  False where it has come down to two entries a leaf.
         bool shrink()
         {
-            if (needed_ ? entries_ <= needed_ : entries_ <= floor_)
+            if (entries_ <= floor_)
             {
                 return false;
             }
-            entries_ = needed_ ? needed_ : std::max(entries_ / 4, floor_);
+            entries_ = std::max(entries_ / 4, floor_);
             return true;
-        }
-
-        // A level ran out of room and needs `entries`: four times that for the levels below.
-        void grow(unsigned long long entries)
-        {
-            needed_ = entries;
-            entries_ = 4 * entries;
         }
 
     private:
         unsigned long long floor_, entries_;
-        unsigned long long needed_ = 0;  // by the last level that ran out
     };
 }  // namespace vg
