@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 def test_the_build_goes_on_where_the_room_ran_out(n, r_max):
     rng = np.random.default_rng(n)
     pts = rng.uniform(-0.5, 0.5, (n, 3)).astype(np.float32)
-    _same(pts, 0.01, r_max)
+    _same(pts, 0.01, r_max)  # the larger trees take blocks beyond what the pool keeps
     if n <= 4097:
         pts[::3] = np.round(pts[::3] * 8) / 8  # ties and repeats
         _same(pts, 0.0, r_max)
