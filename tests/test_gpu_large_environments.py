@@ -104,3 +104,31 @@ def test_the_limit_is_the_same_for_every_robot(robot):
         env = vg.Environment.from_scene({"cuboids": cuboids[:n]})
         s = torch.cuda.current_stream().cuda_stream
         assert lib.vg_validate_states_device(rb.name.encode(), env.handle, q.data_ptr(), 64, out.data_ptr(), s) == code
+
+
+@pytest.mark.parametrize("robot", ["panda", "ur5", "fetch", "baxter"])
+def test_sizes_about_the_ones_that_split_the_records(port, robot):
+    """All records staged, three eighths left behind for a second resident block, all staged again,
+    and left behind because even one block cannot hold them: verdicts are the oracle's each time."""
+    import torch
+
+    import vamp_gb300 as vg
+    from vamp_gb300 import scenes
+
+    rb, prb = getattr(vg, robot), port.robot(robot)
+    stage = {"panda": 65, "ur5": 52, "fetch": 59, "baxter": 114}[robot] * 128 * 4
+    pair = (LIMIT + 1024) // 2 - 1024 - stage
+    q = scenes.configurations(rb.s_m, rb.s_a, 400, 23)
+    a, b = scenes.edges(rb.s_m, rb.s_a, 60, 29)
+    b = (a + 0.15 * (b - a)).astype(np.float32)
+    cuboids = _cuboids(np.random.default_rng(37), LIMIT // 64)
+    for room in (pair, pair * 8 // 5, LIMIT - stage):
+        for n in (room // 64 - 1, room // 64, room // 64 + 1):
+            scene = {"cuboids": cuboids[:n]}
+            env, penv = vg.Environment.from_scene(scene), port.env(scene)
+            got = rb.validate_batch(torch.from_numpy(q).cuda(), env).cpu().numpy()
+            assert np.array_equal(got, penv.validate_states(prb, q, threads=THREADS)), n
+            want, count = penv.validate_motions(prb, a, b, rb.resolution(), 8, threads=THREADS)
+            blocks = torch.empty(len(a), dtype=torch.int32, device="cuda")
+            ok = rb.validate_motion_batch(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), env, blocks=blocks)
+            assert np.array_equal(ok.cpu().numpy(), want) and np.array_equal(blocks.cpu().numpy(), count), n
