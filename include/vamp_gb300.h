@@ -210,7 +210,7 @@ int vg_validate_motions_device(
  * memory while they run (a real-time planner that reserves all memory up front so no call can
  * block on the allocator or run out of memory mid-plan; a framework that owns device memory
  * through its own pool).  No counterpart in the reference, which runs on the CPU.  Same verdicts
- * and block counts; allocates nothing.  Its only scratch, the edge kernel's work counter, is a
+ * and block counts; allocates nothing.  Its only scratch, the edge kernel's work counters, is a
  * fixed 256-byte device array inside the library that every GPU loading the library keeps until
  * exit.  Requirements: env already uploaded to the current device by an earlier ordinary check
  * call and unchanged since (VG_ERR_STATE otherwise); n <= 2^31 - 1 (VG_ERR_LIMIT).  The first
@@ -219,7 +219,7 @@ int vg_validate_motions_device(
  * allocate: let the earlier ordinary call be a vg_validate_motions_device with the same robot,
  * environment settings and schedule (so the same kernel is already loaded), or run with
  * CUDA_MODULE_LOADING=EAGER.
- * All calls share the array (the counter is cleared on `stream` before each launch): calls whose
+ * All calls share the array (the counters are cleared on `stream` before each launch): calls whose
  * kernels overlap on the GPU race, so issue them on one stream or wait between them. */
 int vg_validate_motions_device_noalloc(
     const char *robot,
@@ -248,9 +248,10 @@ int vg_fkcc_blocks(const char *robot, vg_env *env, const float *q, size_t n_bloc
  * Same as the device forms with host buffers: copies in, checks, copies out, and waits.
  * Pinned buffers (vg_host_alloc) make the copies fastest.  Staging memory is owned by env.
  * vg_validate_motions and vg_validate_vectors check a batch of at most 4,096 blocks in all (a
- * planner's single edge, say) block by block: the blocks are built on the host with the edge
- * kernels' arithmetic and checked at once by the blocks kernel, an edge being valid when all its
- * blocks are; larger batches go to the edge kernels.  The verdicts are the same either way. */
+ * planner's single edge, say) block by block: the host counts the blocks with the edge kernels'
+ * arithmetic, one kernel reads the edges in pinned host memory and checks all their blocks at
+ * once, an edge being valid when all its blocks are; larger batches go to the edge kernels.  The
+ * verdicts are the same either way. */
 int vg_validate_states(const char *robot, vg_env *env, const float *q, size_t n, uint8_t *out);
 int vg_validate_motions(
     const char *robot, vg_env *env, const float *a, const float *b, size_t n, int resolution, uint8_t *out);

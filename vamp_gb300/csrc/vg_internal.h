@@ -209,7 +209,7 @@ namespace vg
     // `field`: from usable_field, or null
     EnvDevice env_device(const vg_env *e, const uint8_t *field);
     // States checked in an environment since its last change from which its clearance field is
-    // built (about 0.1 ms, allocations and the synchronisation included).
+    // built (0.06 ms among 60 primitives, 0.13 with a cloud of 20,000 points, 0.24 with a terrain).
     constexpr double kFieldStates = 131072.0;
     // Edges from which they are handed out in edge_rank_kernel's order.
     constexpr size_t kRankEdges = 6144;
