@@ -447,17 +447,18 @@ namespace vg
 
     int stage_split(EnvDevice &d, int beside, int *smem)
     {
-        const int limit = shared_limit(), image = d.staged * static_cast<int>(sizeof(float4));
-        *smem = image + beside;
+        const int limit = shared_limit();
+        const long long image = static_cast<long long>(d.staged) * static_cast<long long>(sizeof(float4));
         // Two resident blocks rather than one where that leaves no more than three eighths of the records
         // behind (131,072 configurations among 900 and 1,290 cuboids: Baxter 7.8 -> 4.9 and 11.8 -> 8.8
         // ms, among 1,800 the Panda 9.7 -> 6.1, UR5 15.4 -> 10.6; with half of them behind, Baxter among
         // 1,800, 18.2 and 18.1, its motions 8.3 -> 10.5, UR5's among 2,500 18.6 -> 28.7).
         constexpr int kReserved = 1024;  // of an SM's shared memory per resident block
         const int pair = (limit + kReserved) / 2 - kReserved;
-        const int room = beside > 0 && *smem > pair && 8ll * (pair - beside) >= 5ll * image ? pair : limit;
-        if (*smem <= room)
+        const int room = beside > 0 && image + beside > pair && 8ll * (pair - beside) >= 5 * image ? pair : limit;
+        if (image + beside <= room)
         {
+            *smem = static_cast<int>(image) + beside;
             return VG_OK;
         }
         if (image > limit)
